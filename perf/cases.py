@@ -1,0 +1,612 @@
+"""What the speed of this framework is measured on: one pass of each case is one request, as a user's program makes it.
+
+A request resets the session, prefills its prompts and decodes: every step is given its tokens (a server that runs its own
+stop rules or sampler feeds them back like this) and returns its picks, the last one its logits too. The training-side case
+is one call of the expert's forward over a batch of rows. Models are random stand-ins of this repository's shapes, written in
+the formats of its loaders and loaded once per process, as a server does; sessions are kept per size for the same reason. The
+prompts, the fed tokens and the training rows come from the seed.
+
+Weights are scaled as trained ones are: every block adds a fraction of the residual stream, and the rows of the head are those
+of the embedding, so that picks stand clear of rounding."""
+import json
+import math
+import os
+import shutil
+import struct
+import sys
+import tempfile
+
+import numpy as np
+import torch
+
+sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "tensor-ffn_b200"))
+
+# Shapes of synth.SHAPES and of the layer-list stacks in bench.py. The larger Qwen2 shapes keep their widths, heads and
+# vocabulary but fewer layers, so that a file of weights is written in seconds.
+QWEN = {
+    "q0.5b": dict(hidden_size=896, num_hidden_layers=24, num_attention_heads=14, num_key_value_heads=2, intermediate_size=4864,
+                  vocab_size=151936, tie_word_embeddings=True),
+    "q1.5b": dict(hidden_size=1536, num_hidden_layers=12, num_attention_heads=12, num_key_value_heads=2, intermediate_size=8960,
+                  vocab_size=151936, tie_word_embeddings=True),
+    "q3b": dict(hidden_size=2048, num_hidden_layers=8, num_attention_heads=16, num_key_value_heads=2, intermediate_size=11008,
+                vocab_size=151936, tie_word_embeddings=True),
+    "q7b": dict(hidden_size=3584, num_hidden_layers=4, num_attention_heads=28, num_key_value_heads=4, intermediate_size=18944,
+                vocab_size=152064, tie_word_embeddings=False),
+}
+STACKS = {
+    "w896": dict(width=896, heads=14, dim=64, d_kv=14, experts=16, ff=1792, chunk=1024, rank=64),
+    "z896": dict(width=896, heads=14, dim=64, d_kv=14, rot=32, kv_rank=256, q_rank=384, blocks=14, ff=4864),
+    "z2048": dict(width=2048, heads=16, dim=128, d_kv=8, rot=64, kv_rank=512, q_rank=768, blocks=16, ff=4096),
+}
+DEPTH, STACK_VOCAB, CONV, TOP, IDENTITY, EPS = 8, 32768, 4, 4, 2, 1e-5
+KV_HEADS = 2
+RESIDUAL_MULT, LOGIT_SCALE = 0.5, 0.7
+EXPERT_SCALE = 0.1
+ROPE_THETA = {"qwen": 1e6, "stack": 1e4}
+
+
+def listed():
+    def request(name, model, seqs, prompt, steps, expert=False, ragged=False, dtype="bfloat16"):
+        return {"name": name, "model": model, "expert": expert, "dtype": dtype, "seqs": seqs, "prompt": prompt, "ragged": ragged, "steps": steps}
+    return [
+        # one user, one answer: the repository's batch-1 setting
+        request("reply", "q0.5b", 1, 128, 128, expert=True),
+        # a short question answered in a word: latency and launches
+        request("short", "q0.5b", 1, 9, 8),
+        # the benchmark's workload: a full batch of equal prompts
+        request("batch64", "q0.5b", 64, 512, 128, expert=True),
+        # what a server's batch looks like: 13 prompts of unequal, odd lengths, base model
+        request("ragged13", "q0.5b", 13, 701, 33, ragged=True),
+        # documents read on the 128-wide heads, mostly prefill
+        request("documents", "q1.5b", 8, 2048, 48, expert=True),
+        # one long context
+        request("long", "q3b", 1, 4001, 32, expert=True),
+        # the widest layers in a batch
+        request("wide32", "q7b", 32, 768, 32, expert=True),
+        # the trainer's forward of the expert over a batch of rows
+        {"name": "train_rows", "model": "q0.5b", "rows": 2048},
+        # the layer-list families: experts and delta rule in a batch; latent attention and recurrences in a ragged batch and on
+        # one long prompt; the fp32 sessions that numbers are checked with
+        request("experts64", "w896", 64, 512, 64),
+        request("latent16", "z896", 16, 397, 48, ragged=True),
+        request("latent_long", "z2048", 1, 3000, 64),
+        request("latent_fp32", "z896", 3, 150, 8, dtype="float32"),
+    ]
+
+
+# per model: most prompt tokens of a request in all, longest prompt, most sequences
+DRAWN = {"q0.5b": (64 * 512, 2048, 64), "q1.5b": (8 * 2048, 2048, 32), "q3b": (4096, 4096, 16), "q7b": (32 * 768, 1024, 32),
+         "w896": (64 * 512, 2048, 64), "z896": (32 * 512, 2048, 64), "z2048": (8 * 1024, 3000, 32)}
+
+
+def draw(rng):
+    def size(lo, hi):
+        return min(hi, int(round(math.exp(rng.uniform(math.log(lo), math.log(hi + 1))))))
+    if rng.random() < 0.1:
+        return {"model": "q0.5b", "rows": size(16, 2048)}
+    model = rng.choice(sorted(DRAWN) + ["q0.5b"] * 3)
+    total, longest, most = DRAWN[model]
+    f32 = model in STACKS and rng.random() < 0.2
+    if f32:
+        total, longest, most = 512, 256, 4
+    seqs = 1 if rng.random() < 0.3 else size(2, most)
+    return {"model": model, "expert": model in QWEN and rng.random() < 0.6, "dtype": "float32" if f32 else "bfloat16", "seqs": seqs,
+            "prompt": size(8, min(longest, total // seqs)), "ragged": seqs > 1 and rng.random() < 0.5, "steps": size(4, 12 if f32 else 64)}
+
+
+def lengths(case):
+    if not case["ragged"]:
+        return [case["prompt"]] * case["seqs"]
+    return [1 + int((case["prompt"] - 1) * (((i + 1) * 0.6180339887) % 1.0)) for i in range(case["seqs"])]
+
+
+# ------------------------------------------------------------------------------------------- configurations and weights
+def config(model):
+    if model in QWEN:
+        return dict(QWEN[model], max_position_embeddings=32768, rms_norm_eps=1e-6, rope_theta=ROPE_THETA["qwen"], eos_token_id=151645,
+                    bos_token_id=151643, model_type="qwen2", torch_dtype="bfloat16")
+    s = STACKS[model]
+    h, d, H = s["heads"], s["dim"], s["width"]
+    layers = []
+    rot = lambda dims: {"base": ROPE_THETA["stack"], "dims": dims}  # noqa: E731
+    rec = {"heads": h, "kv_heads": s["d_kv"], "dim": d, "vdim": d, "conv": CONV}
+    if "experts" in s:
+        mlp = {"kind": "moe", "expert": {"ff": s["ff"]}, "router": {"experts": s["experts"], "identity": IDENTITY, "top": TOP}}
+        att = {"heads": h, "kv_heads": KV_HEADS, "dim": d, "vdim": d, "scale": d ** -0.5, "rot": rot(d), "mask": {"size": s["chunk"]}}
+        layers = [{"type": "channel_delta" if i % 2 else "attention", "mixer": rec if i % 2 else att, "mlp": mlp} for i in range(DEPTH)]
+        return {"architecture": "Rafilix", "width": H, "vocab": STACK_VOCAB, "norm": {"eps": EPS}, "layers": layers}
+    lat = {"heads": h, "dim": d, "rot_dim": s["rot"], "vdim": d, "kv_rank": s["kv_rank"], "q_rank": s["q_rank"], "scale": (d + s["rot"]) ** -0.5,
+           "rot": rot(s["rot"])}
+    for i in range(0, DEPTH, 4):
+        layers += [("latent_attention", lat), ("rglru", {"width": H, "blocks": s["blocks"], "conv": CONV}), ("delta", rec),
+                   ("latent_attention", dict(lat, kv_from=i))]
+    return {"architecture": "Razesun", "width": H, "vocab": STACK_VOCAB, "norm": {"eps": EPS}, "residual_mult": RESIDUAL_MULT,
+            "logit_scale": LOGIT_SCALE, "layers": [{"type": t, "mixer": m, "mlp": {"kind": "dense", "ff": s["ff"]}} for t, m in layers]}
+
+
+EMBED_STD = 0.05  # of the Qwen2 stand-ins; what a block adds to the stream is scaled by it
+
+
+def specs(model):
+    """(name, shape, mean, standard deviation) of every tensor, in the order of the file"""
+    cfg = config(model)
+    out = []
+    lin = lambda name, n, k, gain=1.0: out.append((name, (n, k), 0.0, gain * k ** -0.5))  # noqa: E731
+    vec = lambda name, n, mean, std: out.append((name, n if isinstance(n, tuple) else (n,), mean, std))  # noqa: E731
+    if model in QWEN:
+        H, I, V = cfg["hidden_size"], cfg["intermediate_size"], cfg["vocab_size"]
+        nh, nkv = cfg["num_attention_heads"], cfg["num_key_value_heads"]
+        hd = H // nh
+        out.append(("model.embed_tokens.weight", (V, H), 0.0, EMBED_STD))
+        for i in range(cfg["num_hidden_layers"]):
+            p = "model.layers.%d." % i
+            for t, n, gain in (("q", nh * hd, 1.3), ("k", nkv * hd, 1.3), ("v", nkv * hd, 1.0)):
+                lin(p + "self_attn.%s_proj.weight" % t, n, H, gain)
+                vec(p + "self_attn.%s_proj.bias" % t, n, 0.0, 0.1)
+            lin(p + "self_attn.o_proj.weight", H, nh * hd, 0.5 * EMBED_STD)
+            vec(p + "input_layernorm.weight", H, 1.0, 0.1)
+            vec(p + "post_attention_layernorm.weight", H, 1.0, 0.1)
+            lin(p + "mlp.gate_proj.weight", I, H)
+            lin(p + "mlp.up_proj.weight", I, H)
+            lin(p + "mlp.down_proj.weight", H, I, 0.5 * EMBED_STD)
+        vec("model.norm.weight", H, 1.0, 0.1)
+        if not cfg["tie_word_embeddings"]:
+            out.append(("lm_head.weight", (V, H), 0.0, EMBED_STD))
+        return out
+    H = cfg["width"]
+    sublayer = 0.1  # weight of the norm behind a Rafilix sublayer
+    out.append(("embed", (cfg["vocab"], H), 0.0, 0.5))
+    razesun = cfg["architecture"] == "Razesun"
+    if razesun:
+        vec("embed.norm", H, 1.0, 0.1)
+    for i, layer in enumerate(cfg["layers"]):
+        m, n = layer["mixer"], "l%d." % i
+        p, f = n + "mix.", n + "mlp."
+        vec(n + "norm1", H, 1.0, 0.1)
+        if not razesun:
+            vec(n + "norm1b", H, sublayer, 0.1 * sublayer)
+        if layer["type"] == "attention":
+            h, g, d, v = m["heads"], m["kv_heads"], m["dim"], m["vdim"]
+            lin(p + "q", h * d, H), lin(p + "k", g * d, H), lin(p + "v", g * v, H)
+            vec(p + "q.norm", d, 1.0, 0.1), vec(p + "k.norm", d, 1.0, 0.1)
+            width = h * v
+        elif layer["type"] in ("channel_delta", "delta"):
+            h, g, d, v = m["heads"], m["kv_heads"], m["dim"], m["vdim"]
+            lin(p + "q", g * d, H), lin(p + "k", g * d, H), lin(p + "v", h * v, H)
+            for t, c in (("q", g * d), ("k", g * d), ("v", h * v)):
+                vec(p + t + ".conv", (c, m["conv"]), 0.0, 0.6)
+            lin(p + "b", h, H)
+            vec(p + "A_log", h, -1.0, 0.8)
+            vec(p + "norm", v, 1.0, 0.1)
+            if layer["type"] == "delta":
+                lin(p + "a", h, H), vec(p + "dt_bias", h, -1.5, 1.0), lin(p + "g", h * v, H)
+            else:
+                r = STACKS[model]["rank"]
+                lin(p + "a1", r, H), lin(p + "a2", h * d, r), vec(p + "dt_bias", h * d, -1.5, 1.0), lin(p + "g1", r, H), lin(p + "g2", h * v, r)
+            width = h * v
+        elif layer["type"] == "latent_attention":
+            h, d, rd, v, r, q = (m[k] for k in ("heads", "dim", "rot_dim", "vdim", "kv_rank", "q_rank"))
+            lin(p + "dq", q, H), vec(p + "dq.norm", q, 1.0, 0.1), lin(p + "uq", h * (d + rd), q)
+            if "kv_from" not in m:
+                lin(p + "dkv", r + rd, H), vec(p + "dkv.norm", r, 1.0, 0.1)
+            lin(p + "uk", h * d, r), lin(p + "uv", h * v, r), lin(p + "g", h, H)
+            width = h * v
+        else:
+            w, b = m["width"], m["blocks"]
+            for t in ("y", "x"):
+                lin(p + t, w, H), vec(p + t + ".b", w, 0.0, 0.3)
+            vec(p + "conv", (w, m["conv"]), 0.0, 0.6), vec(p + "conv.b", w, 0.0, 0.3)
+            for t in ("ra", "ri"):
+                out.append((p + t, (b, w // b, w // b), 0.0, (w // b) ** -0.5)), vec(p + t + ".b", (b, w // b), 0.0, 0.5)
+            vec(p + "lam", w, -2.5, 1.5)
+            width = w
+        lin(p + "o", H, width, 0.4 if razesun else 1.0)
+        if razesun:
+            ff = layer["mlp"]["ff"]
+            vec(n + "norm2", H, 1.0, 0.1), lin(f + "gate", ff, H), lin(f + "up", ff, H), lin(f + "down", H, ff, 0.4)
+            continue
+        ff, r = layer["mlp"]["expert"]["ff"], layer["mlp"]["router"]
+        vec(n + "norm2", H, 1.0, 0.1), vec(n + "norm2b", H, sublayer, 0.1 * sublayer)
+        for e in range(r["experts"]):
+            lin("%se%d.up" % (f, e), ff, H), lin("%se%d.down" % (f, e), H, ff)
+        lin(f + "router", r["experts"] + r["identity"], H, 2.0)
+        vec(f + "correction", r["experts"] + r["identity"], 0.0, 0.05)
+    vec("final.norm", H, 1.0, 0.1)
+    if razesun:
+        lin("head", cfg["vocab"], H)
+    return out
+
+
+def tensor(seed, shape, mean, std, dtype=torch.bfloat16):
+    g = torch.Generator("cuda").manual_seed(seed)
+    return torch.randn(shape, generator=g, device="cuda").mul_(std).add_(mean).to(dtype)
+
+
+def weight(model, i, spec):
+    """tensor i of a model; an untied head has the embedding's rows"""
+    name, shape, mean, std = spec
+    return tensor(1000 + (0 if name in ("lm_head.weight", "head") else i), shape, mean, std)
+
+
+def weights(model):
+    return {s[0]: (lambda i=i, s=s: weight(model, i, s)) for i, s in enumerate(specs(model))}
+
+
+def expert_matrix(model, layer, which):
+    """gate, up [I, H] or down [H, I] of the trained delta, whole fp32 as the trainer writes it"""
+    cfg = config(model)
+    H, I = cfg["hidden_size"], cfg["intermediate_size"]
+    shape = (H, I) if which == 2 else (I, H)
+    return tensor(900000 + 3 * layer + which, shape, 0.0, (EMBED_STD if which == 2 else 1.0) * shape[1] ** -0.5, torch.float32)
+
+
+_kept = {}
+
+
+def loaded(model, with_expert=False):
+    """the model and its expert delta, loaded once per process"""
+    import tffn
+    if model not in _kept:
+        base = "/dev/shm" if os.path.isdir("/dev/shm") and shutil.disk_usage("/dev/shm").free > 16 << 30 else None
+        with tempfile.TemporaryDirectory(dir=base) as folder:
+            with open(os.path.join(folder, "config.json"), "w") as f:
+                json.dump(config(model), f)
+            head, at = {}, 0
+            for name, shape, _, _ in specs(model):
+                n = 2 * math.prod(shape)
+                head[name] = {"dtype": "BF16", "shape": list(shape), "data_offsets": [at, at + n]}
+                at += n
+            text = json.dumps(head).encode()
+            text += b" " * (-len(text) % 8)
+            with open(os.path.join(folder, "model.safetensors"), "wb") as f:
+                f.write(struct.pack("<Q", len(text)) + text)
+                for i, s in enumerate(specs(model)):
+                    weight(model, i, s).view(torch.int16).cpu().numpy().tofile(f)
+            _kept[model] = tffn.load_model(folder)
+    if with_expert and (model, "expert") not in _kept:
+        cfg = config(model)
+        base = "/dev/shm" if os.path.isdir("/dev/shm") and shutil.disk_usage("/dev/shm").free > 16 << 30 else None
+        with tempfile.NamedTemporaryFile(dir=base, suffix=".bin") as f:
+            f.write(struct.pack("<5I", 0x45585054, 1, cfg["num_hidden_layers"], cfg["hidden_size"], cfg["intermediate_size"]))
+            for layer in range(cfg["num_hidden_layers"]):
+                for which in range(3):
+                    f.write(expert_matrix(model, layer, which).cpu().numpy().data)
+            f.flush()
+            _kept[model, "expert"] = tffn.checkpoint_load(f.name, _kept[model], EXPERT_SCALE)
+    return _kept[model], _kept[model, "expert"] if with_expert else None
+
+
+def session(case):
+    import tffn
+    longest = (case["prompt"] + case["steps"] + 63) // 64 * 64
+    key = (case["model"], case["expert"], case["dtype"], case["seqs"], longest)
+    if key not in _kept:
+        model, expert = loaded(case["model"], case["expert"])
+        _kept[key] = tffn.Session(model, expert, max_batch=case["seqs"], max_seq=longest, compute=case["dtype"])
+        _kept[key].set_launch_mode(2)
+    return _kept[key]
+
+
+def request_tokens(case, seed):
+    rng = np.random.default_rng([seed, 11])
+    vocab = 151643 if case["model"] in QWEN else STACK_VOCAB
+    return [rng.integers(0, vocab, n, dtype=np.int32) for n in lengths(case)], rng.integers(0, vocab, (case["steps"], case["seqs"]), dtype=np.int32)
+
+
+def training_rows(case, seed):
+    cfg = config(case["model"])
+    return tensor(seed, (cfg["num_hidden_layers"], case["rows"], cfg["hidden_size"]), 0.0, 1.0)
+
+
+def prepare(case, seed):
+    if "rows" in case:
+        x = training_rows(case, seed)
+        return {"expert": loaded(case["model"], True)[1], "x": x, "out": torch.empty(x.shape, dtype=torch.float32, device="cuda"), "rows": case["rows"]}
+    prompts, fed = request_tokens(case, seed)
+    return {"session": session(case), "prompts": prompts, "fed": fed}
+
+
+def run(state):
+    if "x" in state:
+        state["expert"].expert_forward(state["x"].data_ptr(), state["out"].data_ptr(), state["rows"])
+        return {"delta": state["out"]}
+    s, fed = state["session"], state["fed"]
+    s.qwen_reset()
+    picks = [s.prefill(state["prompts"])[0]]
+    for tokens in fed[:-1]:
+        picks.append(s.decode_step(tokens)[0])
+    last, logits = s.decode_step(fed[-1], want_logits=True)
+    return {"picks": np.stack(picks + [last]), "logits": logits}
+
+
+# ------------------------------------------------------------------------------------------- what a pass cannot do without
+def work(case):
+    """Prefill: every weight once, its products over all prompt tokens, the cache written once. Each step: every weight it
+    uses once, each sequence's cache or state once, one token's products. Causal attention counts the half that is seen."""
+    cfg = config(case["model"])
+    if "rows" in case:
+        n, L = 3 * cfg["hidden_size"] * cfg["intermediate_size"], cfg["num_hidden_layers"]
+        return {"bytes": L * (2 * n + 6 * case["rows"] * cfg["hidden_size"]), "flops": 2 * L * case["rows"] * n}
+    lens, steps, n = lengths(case), case["steps"], case["seqs"]
+    elem = 4 if case["dtype"] == "float32" else 2
+    tokens, b, f = sum(lens), 0.0, 0.0
+    pairs = sum(t * (t + 1) / 2 for t in lens)  # (query, key) pairs of the prompts
+    seen = sum(t * steps + steps * (steps + 1) / 2 for t in lens)  # of the steps
+
+    def matrix(params, used_by=1.0):  # by all prompt tokens and all steps
+        nonlocal b, f
+        b += 2 * params * (1 + steps)
+        f += 2 * params * used_by * (tokens + n * steps)
+
+    def cache(width, per_pair, window=None):  # elements of a cached row; products of one (query, key) pair
+        nonlocal b, f
+        p, s = pairs, seen
+        if window:
+            p = sum((t // window) * window * (window + 1) / 2 + (t % window) * (t % window + 1) / 2 for t in lens)
+            s = sum(sum((t + k) % window + 1 for k in range(steps)) for t in lens)
+        b += elem * width * (tokens + n * steps + s)
+        f += 2 * per_pair * (p + s)
+
+    if case["model"] in QWEN:
+        H, I = cfg["hidden_size"], cfg["intermediate_size"]
+        nh, nkv = cfg["num_attention_heads"], cfg["num_key_value_heads"]
+        hd = H // nh
+        for _ in range(cfg["num_hidden_layers"]):
+            matrix((nh + 2 * nkv) * hd * H + H * nh * hd + 3 * H * I * (2 if case["expert"] else 1))
+            cache(2 * nkv * hd, 2 * nh * hd)
+        vocab = cfg["vocab_size"]
+    else:
+        H, vocab = cfg["width"], cfg["vocab"]
+        for layer in cfg["layers"]:
+            m = layer["mixer"]
+            if layer["type"] == "attention":
+                h, g, d, v = m["heads"], m["kv_heads"], m["dim"], m["vdim"]
+                matrix((h * d + g * (d + v) + h * v) * H)
+                cache(g * (d + v), h * (d + v), m["mask"]["size"])
+            elif layer["type"] == "latent_attention":
+                h, d, rd, v, r, q = (m[k] for k in ("heads", "dim", "rot_dim", "vdim", "kv_rank", "q_rank"))
+                matrix((q + h + h * v + (0 if "kv_from" in m else r + rd)) * H + h * (d + rd) * q + h * (d + v) * r)
+                cache(r + rd, h * (d + rd + v))
+            elif layer["type"] == "rglru":
+                w = m["width"]
+                matrix(3 * w * H + 2 * w * w // m["blocks"])
+                b += 8 * w * n * (1 + steps)
+            else:
+                h, g, d, v = m["heads"], m["kv_heads"], m["dim"], m["vdim"]
+                r = STACKS[case["model"]].get("rank")
+                matrix((2 * g * d + 2 * h * v + h) * H + (2 * r * H + r * h * (d + v) if r else (h + h * v) * H))
+                b += 8 * h * d * v * n * (1 + steps)
+                f += 8 * h * d * v * (tokens + n * steps)
+            if "expert" in layer["mlp"]:
+                r, ff = layer["mlp"]["router"], layer["mlp"]["expert"]["ff"]
+                outs = r["experts"] + r["identity"]
+                matrix(outs * H)
+                b += 4 * H * ff * r["experts"] * sum(1 - (1 - r["top"] / outs) ** t for t in [tokens] + [n] * steps)
+                f += 4 * H * ff * r["top"] * r["experts"] / outs * (tokens + n * steps)
+            else:
+                matrix(3 * H * layer["mlp"]["ff"])
+    b += 2 * vocab * H * (1 + steps) + 4 * n * vocab
+    f += 2 * vocab * H * n * (1 + steps)
+    return {"bytes": b, "flops": f}
+
+
+def tolerance(case):
+    # against 64 bits, in norm: 0.2 to 1.8 % on the bf16 requests (the Qwen2 stream is rounded to bf16 twice per layer; a router
+    # near a tie may choose another expert), 0.3 % on the training rows, 8e-7 in the fp32 sessions
+    if case.get("dtype") == "float32":
+        return {"rel": 1e-5, "max": 1e-3, "differ": 0.01}
+    return {"rel": 0.012, "max": 0.3} if "rows" in case else {"rel": 0.03, "max": 0.5, "differ": 0.01}
+
+
+# ------------------------------------------------------------------------------------------- the same in plain 64-bit torch
+D = torch.float64
+
+
+def rms(x, w, eps):
+    return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps) * w.to(D)
+
+
+def linear(x, w):
+    return x @ w.to(D).T
+
+
+def angles(T, dims, base):
+    f = base ** (-torch.arange(0, dims, 2, device="cuda", dtype=D) / dims)
+    a = torch.arange(T, device="cuda", dtype=D)[:, None] * f
+    return a.cos()[:, None], a.sin()[:, None]
+
+
+def halves(x, cs, sn):
+    """rotate x [T, heads, dims]: dimension i and i + dims/2 are a pair"""
+    u, v = x.chunk(2, -1)
+    return torch.cat([u * cs - v * sn, v * cs + u * sn], -1)
+
+
+def neighbours(x, cs, sn):
+    u, v = x[..., 0::2], x[..., 1::2]
+    return torch.stack([u * cs - v * sn, v * cs + u * sn], -1).flatten(-2)
+
+
+def attend(q, k, v, scale, window=None):
+    """q [T, heads, d], k and v [T, kv heads, d] of one sequence, in blocks of queries"""
+    T, h, g = q.shape[0], q.shape[1], k.shape[1]
+    out = []
+    pos = torch.arange(T, device="cuda")
+    for a in range(0, T, 512):
+        i = pos[a:a + 512]
+        s = torch.einsum("tgrd,sgd->grts", q[a:a + 512].unflatten(1, (g, h // g)), k[: a + 512]) * scale
+        j = pos[: a + 512]
+        hidden = j[None] > i[:, None]
+        if window:
+            hidden |= j[None] < (i // window * window)[:, None]
+        s = s.masked_fill(hidden, -math.inf).softmax(-1)
+        out.append(torch.einsum("grts,sgd->tgrd", s, v[: a + 512]).flatten(1, 2))
+    return torch.cat(out)
+
+
+def by_sequence(f, *xs):
+    return torch.stack([f(*(x[i] for x in xs)) for i in range(xs[0].shape[0])])
+
+
+def conv(x, taps, bias=None):
+    """x [n, T, channels]: causal, the last column weighs the current token"""
+    T, taps = x.shape[1], taps.to(D)
+    y = sum(torch.nn.functional.pad(x, (0, 0, taps.shape[1] - 1 - j, 0))[:, :T] * taps[:, j] for j in range(taps.shape[1]))
+    return y if bias is None else y + bias.to(D)
+
+
+def unit(x):
+    return x * torch.rsqrt((x * x).sum(-1, keepdim=True) + 1e-6)
+
+
+def delta_rule(h, w, p, m, per_channel):
+    n, T = h.shape[:2]
+    H, G, d, v = m["heads"], m["kv_heads"], m["dim"], m["vdim"]
+    silu = torch.nn.functional.silu
+    q, k, x = (silu(conv(linear(h, w[p + t]()), w[p + t + ".conv"]())) for t in "qkv")
+    q = (unit(q.unflatten(-1, (G, d))) * d ** -0.5).repeat_interleave(H // G, 2)
+    k = unit(k.unflatten(-1, (G, d))).repeat_interleave(H // G, 2)
+    x = x.unflatten(-1, (H, v))
+    beta = linear(h, w[p + "b"]()).sigmoid()
+    rate = w[p + "A_log"]().to(D).exp()
+    bias = w[p + "dt_bias"]().to(D)
+    if per_channel:
+        z = linear(linear(h, w[p + "a1"]()), w[p + "a2"]()) + bias
+        g = torch.exp(-rate[:, None] * torch.nn.functional.softplus(z).unflatten(-1, (H, d)))[..., None]
+        gate = linear(linear(h, w[p + "g1"]()), w[p + "g2"]()).sigmoid()
+    else:
+        g = torch.exp(-rate * torch.nn.functional.softplus(linear(h, w[p + "a"]()) + bias))[..., None, None]
+        gate = silu(linear(h, w[p + "g"]()))
+    S, o = torch.zeros(n, H, d, v, device="cuda", dtype=D), torch.empty(n, T, H, v, device="cuda", dtype=D)
+    for t in range(T):
+        S = S * g[:, t]
+        u = beta[:, t, :, None] * (x[:, t] - torch.einsum("nhdv,nhd->nhv", S, k[:, t]))
+        S = S + k[:, t, :, :, None] * u[:, :, None]
+        o[:, t] = torch.einsum("nhdv,nhd->nhv", S, q[:, t])
+    return (rms(o, w[p + "norm"](), EPS) * gate.unflatten(-1, (H, v))).flatten(-2)
+
+
+def recurrence(h, w, p, m):
+    y = torch.nn.functional.gelu(linear(h, w[p + "y"]()) + w[p + "y.b"]().to(D), approximate="tanh")
+    u = conv(linear(h, w[p + "x"]()) + w[p + "x.b"]().to(D), w[p + "conv"](), w[p + "conv.b"]())
+    parts = u.unflatten(-1, (m["blocks"], -1))
+    r, i = ((torch.einsum("ntbj,bij->ntbi", parts, w[p + t]().to(D)) + w[p + t + ".b"]().to(D)).sigmoid().flatten(-2) for t in ("ra", "ri"))
+    log_a = -8.0 * r * torch.nn.functional.softplus(w[p + "lam"]().to(D))
+    a, x = log_a.exp(), torch.sqrt(-torch.expm1(2 * log_a)) * i * u
+    S, out = torch.zeros_like(x[:, 0]), torch.empty_like(x)
+    for t in range(x.shape[1]):
+        S = a[:, t] * S + x[:, t]
+        out[:, t] = S
+    return out * y
+
+
+def experts_of(h, w, p, mlp):
+    r = mlp["router"]
+    h = h.flatten(0, 1)
+    s = linear(h, w[p + "router"]()).softmax(-1)
+    top = (s + w[p + "correction"]().to(D)).topk(r["top"], -1).indices
+    share = torch.zeros_like(s).scatter(1, top, s.gather(1, top))
+    out = h * share[:, r["experts"]:].sum(1, keepdim=True)
+    for e in range(r["experts"]):
+        at = share[:, e].nonzero()[:, 0]
+        a = linear(h[at], w["%se%d.up" % (p, e)]()).relu()
+        out[at] += share[at, e, None] * linear(a * a, w["%se%d.down" % (p, e)]())
+    return out
+
+
+def exact_stack(model, tokens, at):
+    cfg, w = config(model), weights(model)
+    razesun = cfg["architecture"] == "Razesun"
+    x = w["embed"]()[tokens].to(D)
+    if razesun:
+        x = rms(x, w["embed.norm"](), EPS)
+    T, kept = tokens.shape[1], {}
+    for i, layer in enumerate(cfg["layers"]):
+        m, n = layer["mixer"], "l%d." % i
+        p = n + "mix."
+        h = rms(x, w[n + "norm1"](), EPS)
+        if layer["type"] == "attention":
+            rot = angles(T, m["rot"]["dims"], m["rot"]["base"])
+            q = rms(linear(h, w[p + "q"]()).unflatten(-1, (m["heads"], -1)), w[p + "q.norm"](), EPS)
+            k = rms(linear(h, w[p + "k"]()).unflatten(-1, (m["kv_heads"], -1)), w[p + "k.norm"](), EPS)
+            v = linear(h, w[p + "v"]()).unflatten(-1, (m["kv_heads"], -1))
+            y = by_sequence(lambda q, k, v: attend(neighbours(q, *rot), neighbours(k, *rot), v, m["scale"], m["mask"]["size"]), q, k, v).flatten(-2)
+        elif layer["type"] == "latent_attention":
+            rot, d, r = angles(T, m["rot_dim"], m["rot"]["base"]), m["dim"], m["kv_rank"]
+            if "kv_from" not in m:
+                z = linear(h, w[p + "dkv"]())
+                kept[i] = rms(z[..., :r], w[p + "dkv.norm"](), EPS), z[..., r:]
+            c, kr = kept[m.get("kv_from", i)]
+            q = linear(rms(linear(h, w[p + "dq"]()), w[p + "dq.norm"](), EPS), w[p + "uq"]()).unflatten(-1, (m["heads"], -1))
+            uk, uv = w[p + "uk"](), w[p + "uv"]()
+
+            def one(q, c, kr):
+                k = linear(c, uk).unflatten(-1, (m["heads"], -1))
+                kr = halves(kr[:, None], *rot).expand(-1, m["heads"], -1)
+                q = torch.cat([q[..., :d], halves(q[..., d:], *rot)], -1)
+                return attend(q, torch.cat([k, kr], -1), linear(c, uv).unflatten(-1, (m["heads"], -1)), m["scale"])
+            y = (by_sequence(one, q, c, kr) * linear(h, w[p + "g"]()).sigmoid()[..., None]).flatten(-2)
+        elif layer["type"] == "rglru":
+            y = recurrence(h, w, p, m)
+        else:
+            y = delta_rule(h, w, p, m, layer["type"] == "channel_delta")
+        y = linear(y, w[p + "o"]())
+        f = n + "mlp."
+        if razesun:
+            h = rms(x, w[n + "norm2"](), EPS)
+            y = y + linear(torch.nn.functional.silu(linear(h, w[f + "gate"]())) * linear(h, w[f + "up"]()), w[f + "down"]())
+            x = x + cfg["residual_mult"] * y
+        else:
+            x = x + rms(y, w[n + "norm1b"](), EPS)
+            y = experts_of(rms(x, w[n + "norm2"](), EPS), w, f, layer["mlp"]).view_as(x)
+            x = x + rms(y, w[n + "norm2b"](), EPS)
+    x = rms(x[torch.arange(len(at), device="cuda"), at], w["final.norm"](), EPS)
+    return linear(x, w["head"]()) * cfg["logit_scale"] if razesun else linear(x, w["embed"]())
+
+
+def exact_qwen(model, expert, tokens, at):
+    cfg, w = config(model), weights(model)
+    eps, nh, nkv, T = cfg["rms_norm_eps"], cfg["num_attention_heads"], cfg["num_key_value_heads"], tokens.shape[1]
+    hd = cfg["hidden_size"] // nh
+    rot = angles(T, hd, cfg["rope_theta"])
+    silu = torch.nn.functional.silu
+    x = w["model.embed_tokens.weight"]()[tokens].to(D)
+    for i in range(cfg["num_hidden_layers"]):
+        p = "model.layers.%d." % i
+        h = rms(x, w[p + "input_layernorm.weight"](), eps)
+        q, k, v = ((linear(h, w[p + "self_attn.%s_proj.weight" % t]()) + w[p + "self_attn.%s_proj.bias" % t]().to(D)).unflatten(-1, (n, hd))
+                   for t, n in (("q", nh), ("k", nkv), ("v", nkv)))
+        y = by_sequence(lambda q, k, v: attend(halves(q, *rot), halves(k, *rot), v, hd ** -0.5), q, k, v).flatten(-2)
+        del q, k, v
+        x = x + linear(y, w[p + "self_attn.o_proj.weight"]())
+        h = rms(x, w[p + "post_attention_layernorm.weight"](), eps)
+        parts = [(1.0, [w[p + "mlp.%s_proj.weight" % t]() for t in ("gate", "up", "down")])]
+        if expert:
+            parts.append((EXPERT_SCALE, [expert_matrix(model, i, j).to(torch.bfloat16) for j in range(3)]))
+        for scale, (gate, up, down) in parts:
+            gate, up, down = gate.to(D), up.to(D), down.to(D)
+            for a in range(len(x)):
+                x[a] += scale * (silu(h[a] @ gate.T) * (h[a] @ up.T) @ down.T)
+    x = rms(x[torch.arange(len(at), device="cuda"), at], w["model.norm.weight"](), eps)
+    return linear(x, w["model.embed_tokens.weight" if cfg["tie_word_embeddings"] else "lm_head.weight"]())
+
+
+def exact(case, seed):
+    if "rows" in case:
+        x = training_rows(case, seed)
+        out = []
+        for layer in range(x.shape[0]):
+            gate, up, down = (expert_matrix(case["model"], layer, j).to(torch.bfloat16).to(D) for j in range(3))
+            h = x[layer].to(D)
+            out.append(EXPERT_SCALE * (torch.nn.functional.silu(h @ gate.T) * (h @ up.T) @ down.T))
+        return {"delta": torch.stack(out)}
+    prompts, fed = request_tokens(case, seed)
+    # shorter sequences are padded behind their last token, which no earlier row sees
+    rows = [np.concatenate([p, f]) for p, f in zip(prompts, fed.T)]
+    tokens = torch.zeros(len(rows), max(map(len, rows)), dtype=torch.long)
+    for i, r in enumerate(rows):
+        tokens[i, : len(r)] = torch.from_numpy(r.astype(np.int64))
+    at = torch.tensor([len(r) - 1 for r in rows], device="cuda")
+    tokens = tokens.cuda()
+    logits = exact_qwen(case["model"], case["expert"], tokens, at) if case["model"] in QWEN else exact_stack(case["model"], tokens, at)
+    return {"picks": None, "logits": logits}
