@@ -209,8 +209,9 @@ def specs(model):
         vec(n + "norm2", H, 1.0, 0.1), vec(n + "norm2b", H, sublayer, 0.1 * sublayer)
         for e in range(r["experts"]):
             lin("%se%d.up" % (f, e), ff, H), lin("%se%d.down" % (f, e), H, ff)
-        lin(f + "router", r["experts"] + r["identity"], H, 2.0)
-        vec(f + "correction", r["experts"] + r["identity"], 0.0, 0.05)
+        # a confident router: where rounding decides between two experts, they are the last chosen and weigh next to nothing
+        lin(f + "router", r["experts"] + r["identity"], H, 6.0)
+        vec(f + "correction", r["experts"] + r["identity"], 0.0, 1e-5)
     vec("final.norm", H, 1.0, 0.1)
     if razesun:
         lin("head", cfg["vocab"], H)
