@@ -848,8 +848,9 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
 
 }  // namespace
 
-bool make_tmap_2d(TmapCache* cache, CUtensorMap* tm, const bf16* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
-    return make_tmap(cache, tm, ptr, rows, cols, ld, box_rows);
+bool make_tmap_2d(TmapCache* cache, CUtensorMap* tm, const bf16* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t batch,
+                  uint32_t batch_ld) {
+    return make_tmap(cache, tm, ptr, rows, cols, ld, box_rows, batch, batch_ld);
 }
 
 int gemm_prepare() {
@@ -863,7 +864,7 @@ int gemm_prepare() {
     if (e != cudaSuccess) return (int)e;
     TFFN_PREP(16) TFFN_PREP(32) TFFN_PREP(64) TFFN_PREP(128) TFFN_PREP(256)
 #undef TFFN_PREP
-    return 0;
+    return gemm_pair_prepare();
 }
 
 // Groups differ in size: a tile of the average size would leave the larger half of the groups a second, nearly
@@ -874,8 +875,47 @@ int gemm_group_tile(int rows) {
     return bn;
 }
 
+// Which launches take the two-CTA tiles of gemm_pair.cu, and how wide (0: none). Measured back to back on one B200 against
+// the tiles of this file (us, here -> there): 4 096 tokens, K 896: q|k|v N 1152 87 -> 23, N 4864 gate|up of base and expert
+// 277 -> 118 (1.21 PFLOP/s); 2 048 tokens, K 3584, N 18944: 1 235 -> 726 (1.53 PFLOP/s).
+//  * gate|up from 65 tokens on (K 896, N 4864: 28 -> 13); other products from 129 on where K is short enough that splitting
+//    it cannot make up for the wider tile (N 4608, K 3584: 160 tokens 50 -> 28, 128 tokens 25 -> 28); very short ones from 65.
+//  * A long K extent with few tiles is split over clusters here: 14 wide tiles of 152 k-blocks 14 -> 50. The wide tiles win
+//    once they are about a quarter of the k-blocks in number, or nearly fill the chip (K 4864, N 896: 768 tokens 39 -> 29,
+//    512 tokens 21 -> 29; two pairs of that K: 1 000 tokens 49 -> 54, 2 048 tokens 80 -> 56).
+//  * One narrow row tile (a router) needs many tokens (K 896: 4 096 tokens 14 -> 8; K 2048: 768 tokens 9 -> 13).
+//  * Width: a k-block costs a pair 0.34 us with 128 weight rows and 0.42 with 256 (0.34 while it has the chip to itself), a
+//    tile about 1 us around them; whole waves of 74 pairs count.
+int pair_width(const GemmCall& c, const GemmWorkspace& ws) {
+    if (c.amax_val || (!c.out && c.mode != GEMM_QKV) || (c.grp && c.grp_bn != 256)) return 0;
+    const bool halves = c.mode == GEMM_SWIGLU, batched = c.batch > 1;
+    // what launch_bn refuses stays with it
+    if (halves && (c.op[0].K != c.op[1].K || c.op[0].X != c.op[1].X)) return 0;
+    if (batched && (c.out2 || c.grp || c.op[1].K > 0 || c.x_batch % 8 || (c.mode != GEMM_STORE_F32 && c.mode != GEMM_STORE_BF16))) return 0;
+    if (c.grp && (c.op[1].K > 0 || c.out2 || halves || c.mode == GEMM_QKV || c.grp_tiles < 1 || c.grp_count < 1)) return 0;
+    if (c.out2 && (c.op2[0].K != c.op[0].K || c.op2[1].K != c.op[1].K)) return 0;
+    if (c.mode == GEMM_QKV && (!c.qkv || c.op[1].K > 0 || c.out2 || (c.qkv->kv.hd != 64 && c.qkv->kv.hd != 128))) return 0;
+    const int kb = (c.op[0].K + BK - 1) / BK + (c.op[1].K > 0 && !halves ? (c.op[1].K + BK - 1) / BK : 0);
+    const long long rows = (c.grp ? (c.grp_rows_hint > 0 ? c.grp_rows_hint : c.grp_tiles) : (c.T + 255) / 256) * (batched ? (long long)c.batch : c.out2 ? 2 : 1);
+    const long long wide = rows * ((c.N + (halves ? 127 : 255)) / (halves ? 128 : 256)), narrow = rows * ((c.N + (halves ? 63 : 127)) / (halves ? 64 : 128));
+    if (!c.grp) {
+        if (c.N <= BM && !batched && !halves) {
+            if (c.T < 2048) return 0;
+        } else if (c.T <= (halves || kb <= 8 ? 64 : 128)) {
+            return 0;
+        } else if (!halves && kb > 56 && narrow * 4 < (kb < 240 ? kb : 240)) {
+            return 0;
+        }
+    }
+    const int pairs = ws.num_sms / 2;
+    auto cost = [&](long long tiles, double us) { return (double)((tiles + pairs - 1) / pairs) * (kb * us + 1.0); };
+    return cost(narrow, 0.34) <= cost(wide, wide < pairs ? 0.34 : 0.42) ? 128 : 256;
+}
+
 int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits) {
     if (c.T <= 0 || c.N <= 0 || c.op[0].K <= 0) return (int)cudaErrorInvalidValue;
+    if (force_splits == 0)
+        if (const int bn = pair_width(c, ws)) return launch_gemm_pair(c, ws, stream, bn);
     if (c.grp) {
         switch (c.grp_bn) {
             case 16: return launch_bn<16>(c, ws, stream, force_splits);

@@ -109,7 +109,9 @@ struct TmapCache;
 TmapCache* tmap_cache_create();
 void tmap_cache_free(TmapCache* c);
 // bf16 tensor [rows, cols] with a row stride of ld elements, boxes of box_rows x 64 columns with the 128-byte swizzle
-bool make_tmap_2d(TmapCache* cache, CUtensorMap* tm, const bf16* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
+// (batch > 1: a 3-D map (column, problem, row) over `batch` such tensors interleaved in a row, batch_ld elements apart)
+bool make_tmap_2d(TmapCache* cache, CUtensorMap* tm, const bf16* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t batch = 1,
+                  uint32_t batch_ld = 0);
 
 struct GemmWorkspace {
     int* status;  // device status word
@@ -120,6 +122,10 @@ struct GemmWorkspace {
 int gemm_prepare();
 // returns cudaError (launch) or -1000 if the tensor maps could not be encoded
 int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits = 0);
+// the same products in tiles of 256 tokens x bn (128 or 256) weight rows over two CTAs; launch_gemm decides (no fused pick,
+// grouped launches with grp_bn 256)
+int gemm_pair_prepare();
+int launch_gemm_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int bn);
 
 // ------------------------------------------------------------------ row kernels of the batched path
 // (pdl: launch with programmatic dependent launch; every kernel here waits before reading its inputs)
