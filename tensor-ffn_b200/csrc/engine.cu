@@ -747,7 +747,7 @@ void Session::gemm(GemmCall& call, int cls, bool pdl) {
     call.trace = (tl_on_ && (int)tl_cls_.size() - 1 == tl_trace_launch_) ? tl_trace_buf_.as<unsigned long long>() : nullptr;
     call.trace_ctas = (int)(tl_trace_buf_.bytes / (64 * 8));
     prof_begin(cls);
-    const int rc = st_ && st_->f32 ? launch_gemm_f32(call, stream_) : launch_gemm(call, gemm_ws(), stream_);
+    const int rc = st_ && st_->f32 ? launch_gemm_f32(call, gemm_ws(), stream_) : launch_gemm(call, gemm_ws(), stream_);
     prof_end();
     if (rc == -1000) throw Error(kErrCuda, "cuTensorMapEncodeTiled failed or is unavailable");
     if (rc != 0) cuda_check((cudaError_t)rc, "GEMM launch", __FILE__, __LINE__);

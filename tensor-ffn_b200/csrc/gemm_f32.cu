@@ -1,7 +1,14 @@
 // The batched path's matrix products in true fp32: out[t, n] = epilogue(sum_k X[t,k] * W[n,k]) with fp32 activations,
 // bf16 weights widened exactly, fp32 FMA on the CUDA cores, the same call structure as the tensor-core GEMM
-// (gemm_tc.cu) so that a session that computes in fp32 runs the same sequence of steps. One CTA = 64 tokens x 64
-// weight rows, K in slices of 16 through shared memory, 4 x 4 outputs per thread.
+// (gemm_tc.cu) so that a session that computes in fp32 runs the same sequence of steps. Two kernels:
+//
+// k_gemm_f32_rows, up to eight tokens, bound by streaming the weights: the threads of a block divide K (16 bytes of a weight
+//   row each), hold eight rows in registers, and the sums meet in shuffles and shared memory. The first weights are
+//   requested ahead of the dependency wait.
+// k_gemm_f32, more tokens, bound by FMA issue: one CTA = 64 tokens x 64 weight rows, 8 x 8 outputs per thread (four 16-byte
+//   shared loads per 64 FMA); the four 64-thread groups of a CTA take a quarter of every K slice each, so that one tile
+//   fills an SM's schedulers. Slices are double-buffered through registers. Where the tiles are fewer than the SMs, K is also
+//   split over a thread-block cluster whose CTAs add their tiles through distributed shared memory in rank order.
 #include "kernels.h"
 #include "ptx.cuh"
 #include "launch.h"
@@ -11,7 +18,12 @@ namespace tffn {
 
 namespace {
 
-constexpr int TB = kGemmF32Tile, NB = 64, KB = 16;
+constexpr int TB = kGemmF32Tile, NB = 64, KB = 32;
+constexpr int kThreads = 256, kGroups = 4, kGroupK = KB / kGroups;
+constexpr int kLd = 68;       // floats of a slice's row in shared memory (64 and a pad; 16-byte aligned)
+constexpr int kMaxSplits = 8; // portable cluster size
+constexpr int kRowTokens = 8;
+constexpr int rows_per_thread(int tokens) { return tokens > 4 ? 4 : 8; }  // 32 sums at most
 
 struct F32Dev {
     const float* X[2];
@@ -21,101 +33,275 @@ struct F32Dev {
     int N, T, K[2], mode, batch, x_batch, out_batch;
     float out_scale, alpha;
     const GroupTile* grp;
+    int splits;   // k_gemm_f32: CTAs of a cluster
+    int lanes;    // k_gemm_f32_rows: threads that divide K
     unsigned long long* tl;
 };
 
-__global__ void __launch_bounds__(256) k_gemm_f32(const F32Dev p) {
-    __shared__ float sx[KB][TB + 4];
-    __shared__ float sw[KB][NB + 4];
+// where a block works: tokens [t0, t_end), its rows of W, its columns of X
+struct Place {
+    int t0, t_end, op0, b;
+    long long w_row0;
+    float* out;
+};
+__device__ __forceinline__ bool place(const F32Dev& p, int tile, int prob, Place& x) {
+    x.t0 = tile * TB;
+    x.t_end = min(p.T, x.t0 + TB);
+    x.w_row0 = 0;
+    if (p.grp) {
+        const int4 g = __ldcg((const int4*)(p.grp + tile));
+        if (g.x < 0) return false;
+        x.t0 = g.y;
+        x.t_end = min(g.z, g.y + TB);
+        x.w_row0 = (long long)g.x * p.N;
+    }
+    x.b = p.batch > 1 ? prob : 0;  // batched: the problems share their operands
+    if (x.b > 0) x.w_row0 = (long long)x.b * p.N;
+    x.op0 = p.batch > 1 ? 0 : prob;
+    x.out = p.batch > 1 ? p.out[0] + (size_t)x.b * p.out_batch : p.out[prob];
+    return true;
+}
+__device__ __forceinline__ float finish(const F32Dev& p, float first, float v) {
+    if (p.K[1] > 0) v = p.mode == GEMM_SWIGLU ? first / (1.f + expf(-first)) * v : first + p.alpha * v;
+    v *= p.out_scale;
+    if (p.mode == GEMM_RELU2) {
+        v = fmaxf(v, 0.f);
+        v *= v;
+    }
+    return v;
+}
+
+// ------------------------------------------------------------------------------------------- few tokens
+// the first `live` of a word's two bf16 values, the others zero
+__device__ __forceinline__ uint32_t keep_low(uint32_t u, int live) { return live >= 2 ? u : live == 1 ? u & 0xffffu : 0u; }
+
+// p.lanes threads (8 .. 256, a power of two) divide K in pieces of 8; the block's kThreads / lanes teams take
+// rows_per_thread weight rows each. TT tokens at a time (the rows' weights are read again, from L2, for the next TT).
+// Measured with k_gemm_f32 below, width 896 and ff 4864, three sequences of up to 150 tokens and eight steps: 88.7 -> 12.4 ms.
+template <int TT>
+__global__ void __launch_bounds__(kThreads, 2) k_gemm_f32_rows(const F32Dev p) {
+    constexpr int R = rows_per_thread(TT);
+    __shared__ float part[kThreads / 32][R * TT];  // per warp
+    __shared__ float keep[kThreads / 32][R * TT];  // per team: the first operand pair's sums
+    if (threadIdx.x == 0) tl_mark(p.tl, 0);
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, team = tid / p.lanes, kl = tid % p.lanes, teams = kThreads / p.lanes;
+    const int n0 = (blockIdx.x * teams + team) * R;
+    // ungrouped weights are older than the previous kernel, and so are all but its own outputs
+    uint4 w[R];
+    auto load_w = [&](const bf16* W, long long ldw, long long row0, int k) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) w[r] = n0 + r < p.N ? __ldg((const uint4*)(W + (size_t)(row0 + n0 + r) * ldw + k)) : make_uint4(0, 0, 0, 0);
+    };
+    bool ahead = false;
+    if (!p.grp && kl * 8 < p.K[0]) {
+        load_w(p.W[p.batch > 1 ? 0 : blockIdx.z], p.ldw[p.batch > 1 ? 0 : blockIdx.z], p.batch > 1 ? (long long)blockIdx.z * p.N : 0, kl * 8);
+        ahead = true;
+    }
+    pdl_wait();
+    if (tid == 0) tl_mark(p.tl, 1);
+    Place at;
+    if (!place(p, blockIdx.y, blockIdx.z, at)) return;
+    const int pairs = p.K[1] > 0 ? 2 : 1;
+    for (int t0 = at.t0; t0 < at.t_end; t0 += TT) {
+        for (int pair = 0; pair < pairs; ++pair) {
+            const int op = at.op0 + pair, K = p.K[pair];
+            const float* X = p.X[op] + (size_t)at.b * p.x_batch;
+            const bf16* W = p.W[op];
+            const long long ldx = p.ldx[op], ldw = p.ldw[op];
+            float acc[R * TT];
+#pragma unroll
+            for (int i = 0; i < R * TT; ++i) acc[i] = 0.f;
+            for (int k = kl * 8; k < K; k += p.lanes * 8) {
+                if (!ahead) load_w(W, ldw, at.w_row0, k);
+                ahead = false;
+                const int live = K - k;  // columns of this piece; what a row's padding holds counts as zero
+                if (live < 8) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) w[r] = make_uint4(keep_low(w[r].x, live), keep_low(w[r].y, live - 2), keep_low(w[r].z, live - 4), keep_low(w[r].w, live - 6));
+                }
+#pragma unroll
+                for (int t = 0; t < TT; ++t) {
+                    const float* xp = X + (size_t)min(t0 + t, at.t_end - 1) * ldx + k;
+                    float x[8];
+                    *(float4*)x = __ldcg((const float4*)xp);
+                    *(float4*)(x + 4) = live > 4 ? __ldcg((const float4*)(xp + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (live < 8) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) x[j] = j < live ? x[j] : 0.f;
+                    }
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const uint32_t u[4] = {w[r].x, w[r].y, w[r].z, w[r].w};
+                        float s = acc[r * TT + t];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) s = fmaf(x[2 * j + 1], bf16_hi(u[j]), fmaf(x[2 * j], bf16_lo(u[j]), s));
+                        acc[r * TT + t] = s;
+                    }
+                }
+            }
+            for (int o = min(p.lanes, 32) >> 1; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < R * TT; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+            if (p.lanes < 32) {  // one pair: every lane of the team holds the sums
+#pragma unroll
+                for (int i = 0; i < R * TT; ++i) {
+                    const int n = n0 + i / TT, t = t0 + i % TT;
+                    if (i % p.lanes == kl && n < p.N && t < at.t_end) at.out[(size_t)t * p.ldo + n] = finish(p, 0.f, acc[i]);
+                }
+                continue;
+            }
+            const int warps = p.lanes / 32, warp0 = team * warps;
+            if ((tid & 31) == 0) {
+#pragma unroll
+                for (int i = 0; i < R * TT; ++i) part[tid >> 5][i] = acc[i];
+            }
+            __syncthreads();
+            for (int i = kl; i < R * TT; i += p.lanes) {
+                float v = 0.f;
+                for (int q = 0; q < warps; ++q) v += part[warp0 + q][i];
+                if (pair == 0 && pairs == 2) {
+                    keep[team][i] = v;  // the same thread reads it
+                    continue;
+                }
+                const int n = n0 + i / TT, t = t0 + i % TT;
+                if (n < p.N && t < at.t_end) at.out[(size_t)t * p.ldo + n] = finish(p, pairs == 2 ? keep[team][i] : 0.f, v);
+            }
+            __syncthreads();
+        }
+    }
+    if (tid == 0) tl_mark(p.tl, 2);
+}
+
+// ------------------------------------------------------------------------------------------- more tokens
+// VEC: 16-byte copies (rows of X and W aligned, see launch_gemm_f32); else element by element.
+template <bool VEC>
+__global__ void __launch_bounds__(kThreads) k_gemm_f32(const F32Dev p) {
+    __shared__ __align__(16) float smem[2 * 2 * KB * kLd];  // two slices of X and W, transposed; then the tile [64][kLd]
     if (threadIdx.x == 0) tl_mark(p.tl, 0);
     pdl_launch_dependents();
     pdl_wait();
     if (threadIdx.x == 0) tl_mark(p.tl, 1);
-    const int prob = blockIdx.z, n0 = blockIdx.x * NB;
-    int t0 = blockIdx.y * TB, t_end = p.T;
-    long long w_row0 = 0;
-    if (p.grp) {
-        const int4 g = __ldcg((const int4*)(p.grp + blockIdx.y));
-        if (g.x < 0) return;
-        t0 = g.y;
-        t_end = min(g.z, g.y + TB);
-        w_row0 = (long long)g.x * p.N;
-    }
-    const int b = p.batch > 1 ? prob : 0;  // batched: the problems share their operands
-    if (b > 0) w_row0 = (long long)b * p.N;
-    const int op0 = p.batch > 1 ? 0 : prob;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;  // tx: weight rows, ty: tokens
-    const int lk = tid & 15, lr = tid >> 4;                     // copies: k within the slice, first row (then + 16 ...)
-    float acc[4][4], first[4][4];  // first: the first operand pair's sums while the second one's are formed
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = first[i][j] = 0.f;
+    const int tid = threadIdx.x;
+    const int rank = (int)blockIdx.x % p.splits, n0 = (int)blockIdx.x / p.splits * NB;
+    Place at;
+    if (!place(p, blockIdx.y, blockIdx.z, at)) return;  // the whole cluster
+    const int grp = tid >> 6, g = tid & 63, tx = g & 7, ty = g >> 3;  // tx: weight rows 4 tx and 32 + 4 tx .., ty: tokens alike
+    const int cr = tid >> 2, ck = (tid & 3) * 8;                      // copies: row, first of 8 columns
+    float first[16];
     const int pairs = p.K[1] > 0 ? 2 : 1;
     for (int pair = 0; pair < pairs; ++pair) {
-        const int op = op0 + pair, K = p.K[pair];
-        const float* X = p.X[op] + (size_t)b * p.x_batch;
-        const bf16* W = p.W[op];
-        const long long ldx = p.ldx[op], ldw = p.ldw[op];
-        if (pair == 1) {
+        const int op = at.op0 + pair, K = p.K[pair];
+        const bool t_on = at.t0 + cr < at.t_end, n_on = n0 + cr < p.N;
+        const float* X = p.X[op] + (size_t)at.b * p.x_batch + (size_t)(t_on ? at.t0 + cr : at.t0) * p.ldx[op];
+        const bf16* W = p.W[op] + (size_t)(at.w_row0 + (n_on ? n0 + cr : 0)) * p.ldw[op];
+        const int slices = (K + KB - 1) / KB, per = (slices + p.splits - 1) / p.splits;
+        const int s0 = rank * per, s1 = min(slices, s0 + per);
+        float xr[8], wr[8];
+        auto fetch = [&](int s) {
+            const int k = s * KB + ck;
+            if (VEC && k + 8 <= K) {
+                const float4 a = t_on ? __ldcg((const float4*)(X + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 b = t_on ? __ldcg((const float4*)(X + k + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const uint4 u = n_on ? __ldg((const uint4*)(W + k)) : make_uint4(0, 0, 0, 0);
+                xr[0] = a.x; xr[1] = a.y; xr[2] = a.z; xr[3] = a.w;
+                xr[4] = b.x; xr[5] = b.y; xr[6] = b.z; xr[7] = b.w;
+                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+                for (int j = 0; j < 4; ++j) { wr[2 * j] = bf16_lo(w[j]); wr[2 * j + 1] = bf16_hi(w[j]); }
+            } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    first[i][j] = acc[i][j];
-                    acc[i][j] = 0.f;
+                for (int j = 0; j < 8; ++j) {
+                    xr[j] = t_on && k + j < K ? __ldcg(X + k + j) : 0.f;
+                    wr[j] = n_on && k + j < K ? __bfloat162float(W[k + j]) : 0.f;
+                }
+            }
+        };
+        float acc[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+        if (s0 < s1) fetch(s0);
+        for (int s = s0; s < s1; ++s) {
+            float* sx = smem + ((s - s0) & 1) * (2 * KB * kLd);
+            float* sw = sx + KB * kLd;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                sx[(ck + j) * kLd + cr] = xr[j];
+                sw[(ck + j) * kLd + cr] = wr[j];
+            }
+            __syncthreads();  // one barrier per slice: the buffer of slice s - 1 is written again only behind the next one
+            if (s + 1 < s1) fetch(s + 1);
+#pragma unroll
+            for (int kk = 0; kk < kGroupK; ++kk) {
+                const float* xk = sx + (grp * kGroupK + kk) * kLd;
+                const float* wk = sw + (grp * kGroupK + kk) * kLd;
+                float a[8], b[8];
+                *(float4*)a = *(const float4*)(xk + 4 * ty);
+                *(float4*)(a + 4) = *(const float4*)(xk + 32 + 4 * ty);
+                *(float4*)b = *(const float4*)(wk + 4 * tx);
+                *(float4*)(b + 4) = *(const float4*)(wk + 32 + 4 * tx);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            }
+        }
+        // the groups' quarters, in order, then the cluster's parts
+#pragma unroll 1
+        for (int q = 0; q < kGroups; ++q) {
+            __syncthreads();
+            if (grp != q) continue;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float4* dst = (float4*)(smem + ((i >> 2) * 32 + 4 * ty + (i & 3)) * kLd + h * 32 + 4 * tx);
+                    float4 v = make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
+                    if (q > 0) {
+                        const float4 o = *dst;
+                        v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
+                    }
+                    *dst = v;
                 }
         }
-        for (int k0 = 0; k0 < K; k0 += KB) {
-            const int k = k0 + lk;
+        if (p.splits > 1) cluster_sync_all();
+        else __syncthreads();
+        // thread: 4 columns from 4 (tid % 16) of rows tid / 16 + 16 i; of a cluster's tile every CTA finishes some rows
+        const uint32_t plane = smem_u32(smem);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int t = t0 + lr + 16 * i, n = n0 + lr + 16 * i;
-                sx[lk][lr + 16 * i] = (t < t_end && k < K) ? __ldcg(X + (size_t)t * ldx + k) : 0.f;
-                sw[lk][lr + 16 * i] = (n < p.N && k < K) ? __bfloat162float(W[(size_t)(w_row0 + n) * ldw + k]) : 0.f;
-            }
-            __syncthreads();
+        for (int i = 0; i < 4; ++i) {
+            const int row = (tid >> 4) + 16 * i, c = 4 * (tid & 15), t = at.t0 + row;
+            if (row % p.splits != rank || t >= at.t_end) continue;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            if (p.splits == 1) {
+                *(float4*)v = *(const float4*)(smem + row * kLd + c);
+            } else {
+                for (int z = 0; z < p.splits; ++z) {
+                    const uint32_t src = map_shared_rank(plane + (uint32_t)(row * kLd + c) * 4, (uint32_t)z);
 #pragma unroll
-            for (int kk = 0; kk < KB; ++kk) {
-                float a[4], b[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    a[i] = sx[kk][ty * 4 + i];
-                    b[i] = sw[kk][tx * 4 + i];
+                    for (int j = 0; j < 4; ++j) v[j] += ld_shared_cluster_f32(src + 4 * j);
                 }
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
             }
-            __syncthreads();
-        }
-    }
-    float* out = p.batch > 1 ? p.out[0] + (size_t)b * p.out_batch : p.out[prob];
+            if (pair == 0 && pairs == 2) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = t0 + ty * 4 + i;
-        if (t >= t_end) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n >= p.N) continue;
-            float v = acc[i][j];
-            if (pairs == 2) v = p.mode == GEMM_SWIGLU ? first[i][j] / (1.f + expf(-first[i][j])) * v : first[i][j] + p.alpha * v;
-            v *= p.out_scale;
-            if (p.mode == GEMM_RELU2) {
-                v = fmaxf(v, 0.f);
-                v *= v;
+                for (int j = 0; j < 4; ++j) first[4 * i + j] = v[j];
+                continue;
             }
-            out[(size_t)t * p.ldo + n] = v;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n0 + c + j < p.N) at.out[(size_t)t * p.ldo + n0 + c + j] = finish(p, pairs == 2 ? first[4 * i + j] : 0.f, v[j]);
         }
+        if (p.splits > 1) cluster_sync_all();  // the peers have read this CTA's tile
+        else __syncthreads();
     }
     if (tid == 0) tl_mark(p.tl, 2);
 }
 
 }  // namespace
 
-int launch_gemm_f32(const GemmCall& c, cudaStream_t stream) {
+int launch_gemm_f32(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream) {
     if (c.T <= 0 || c.N <= 0 || c.op[0].K <= 0 || !c.out) return (int)cudaErrorInvalidValue;
     if (c.mode != GEMM_STORE_F32 && c.mode != GEMM_STORE_BF16 && c.mode != GEMM_RELU2 && c.mode != GEMM_SWIGLU) return (int)cudaErrorInvalidValue;
     if (c.mode == GEMM_SWIGLU ? c.op[1].K != c.op[0].K : c.mode == GEMM_RELU2 && c.op[1].K > 0) return (int)cudaErrorInvalidValue;
@@ -156,8 +342,29 @@ int launch_gemm_f32(const GemmCall& c, cudaStream_t stream) {
     p.out_scale = c.out_scale == 0.f ? 1.f : c.out_scale;
     p.grp = c.grp;
     p.tl = c.tl;
-    const dim3 grid((c.N + NB - 1) / NB, c.grp ? c.grp_tiles : (c.T + TB - 1) / TB, c.out2 ? 2 : p.batch);
-    return (int)launch_k(k_gemm_f32, grid, dim3(256), 0, stream, c.pdl, p);
+    // 16-byte copies need every row of X and W to start on a 16-byte boundary
+    bool vec = c.x_batch % 4 == 0;
+    for (int i = 0; i < 2; ++i)
+        if (p.X[i] && ((uintptr_t)p.X[i] % 16 || (uintptr_t)p.W[i] % 16 || p.ldx[i] % 4 || p.ldw[i] % 8)) vec = false;
+    const int probs = c.out2 ? 2 : p.batch, t_tiles = c.grp ? c.grp_tiles : (c.T + TB - 1) / TB;
+    // A tile of 64 tokens costs the same for one as for 64; streaming the rows costs as much again for every eight.
+    if (vec && c.T <= kRowTokens) {
+        const int K = p.K[0] > p.K[1] ? p.K[0] : p.K[1];
+        p.lanes = p.K[1] > 0 ? 32 : 8;
+        while (p.lanes < kThreads && p.lanes * 8 < K) p.lanes *= 2;
+        const int rows = kThreads / p.lanes * rows_per_thread(c.T);
+        const dim3 grid((c.N + rows - 1) / rows, t_tiles, probs);
+        auto go = [&](auto kern) { return (int)launch_k(kern, grid, dim3(kThreads), 0, stream, c.pdl, p); };
+        return c.T == 1 ? go(k_gemm_f32_rows<1>) : c.T == 2 ? go(k_gemm_f32_rows<2>) : c.T <= 4 ? go(k_gemm_f32_rows<4>) : go(k_gemm_f32_rows<8>);
+    }
+    // splits until the chip is full once, at least four slices each
+    const long long tiles = (long long)((c.N + NB - 1) / NB) * t_tiles * probs;
+    const int slices = (p.K[0] + KB - 1) / KB;
+    p.splits = 1;
+    while (p.splits < kMaxSplits && tiles * p.splits * 2 <= 2 * ws.num_sms && slices >= 8 * p.splits) p.splits *= 2;
+    const dim3 grid((c.N + NB - 1) / NB * p.splits, t_tiles, probs);
+    auto go = [&](auto kern) { return (int)launch_k_cluster(kern, grid, dim3(kThreads), dim3(p.splits, 1, 1), 0, stream, c.pdl, p); };
+    return vec ? go(k_gemm_f32<true>) : go(k_gemm_f32<false>);
 }
 
 }  // namespace tffn

@@ -97,11 +97,7 @@ struct GroupTile {
 };
 // token tile (16 .. 256) of a grouped launch whose groups hold `rows` rows on average
 int gemm_group_tile(int rows);
-// The same products in true fp32 (fp32 X and out, fp32 FMA, weights still bf16): modes STORE_F32, STORE_BF16, RELU2 and
-// SWIGLU (which then store fp32), grouped and batched launches included; two operand pairs only in a plain launch. The operands' X pointers
-// are fp32 arrays behind the bf16 type.
-int launch_gemm_f32(const GemmCall& c, cudaStream_t stream);
-constexpr int kGemmF32Tile = 64;  // its token tile (grp_bn)
+constexpr int kGemmF32Tile = 64;  // token tile (grp_bn) of launch_gemm_f32
 // Encoded tensor maps of the (buffer, shape, box) combinations a caller keeps launching with: encoding one costs
 // microseconds of host time and a decode step needs about 200. Owned by whoever owns the buffers (a session keeps
 // one for its lifetime), so entries die with the buffers they describe.
@@ -122,6 +118,10 @@ struct GemmWorkspace {
 int gemm_prepare();
 // returns cudaError (launch) or -1000 if the tensor maps could not be encoded
 int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits = 0);
+// The same products in true fp32 (fp32 X and out, fp32 FMA, weights still bf16): modes STORE_F32, STORE_BF16, RELU2 and
+// SWIGLU (which then store fp32), grouped and batched launches included; two operand pairs only in a plain launch. The operands' X pointers
+// are fp32 arrays behind the bf16 type.
+int launch_gemm_f32(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream);
 // the same products in tiles of 256 tokens x bn (128 or 256) weight rows over two CTAs; launch_gemm decides (no fused pick,
 // grouped launches with grp_bn 256)
 int gemm_pair_prepare();
