@@ -1,5 +1,4 @@
-// Grouped-query attention of ONE query token over the paged bf16 KV cache (decode; prefill
-// runs it per prompt token with a causal context length).
+// Grouped-query attention of ONE query token over the paged bf16 KV cache (prompts: attn_prompt.cu).
 //
 // Reference arithmetic (inference/src/model/qwen.cu:349-412): scores = (q . k) / sqrt(hd) with
 // q in fp32 and k in bf16, softmax with max-subtraction and exp (cuda_ops.cu:106-126),
@@ -48,13 +47,6 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// (x, y) as two bf16 pairs: hi = bf16(v), lo = bf16(v - hi); x in the low half (the lower k index)
-__device__ __forceinline__ void split_bf16x2(float x, float y, uint32_t& hi, uint32_t& lo) {
-    const __nv_bfloat16 xh = __float2bfloat16_rn(x), yh = __float2bfloat16_rn(y);
-    hi = (uint32_t)__bfloat16_as_ushort(xh) | ((uint32_t)__bfloat16_as_ushort(yh) << 16);
-    lo = (uint32_t)bf16_bits(x - __bfloat162float(xh)) | ((uint32_t)bf16_bits(y - __bfloat162float(yh)) << 16);
-}
-
 constexpr int kAttnCtaThreads = 256;  // 8 warps: each takes 16 keys of a 128-key stage
 constexpr int kAttnWarps = kAttnCtaThreads / 32;
 
@@ -442,138 +434,6 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
 #undef ATTN_TRACE
 }
 
-// Prefill: one CTA per (group of up to 8 consecutive prompt tokens of ONE sequence, kv head). The eight
-// warps are the eight query tokens; the K/V stages (128 keys each, copied by all threads) are shared by
-// them, so the cache is read once per 8 tokens instead of once per token; warp w runs the same 16-key
-// blocks as the decode kernel over keys 0 .. pos_w (causal), owns its token's whole context and writes
-// its output rows itself: no merge.
-template <int HD, bool EXACT>
-__global__ void __launch_bounds__(kAttnCtaThreads) k_attn_prefill(const float* __restrict__ q, KvView kv, int layer,
-                                                               const int* __restrict__ tok_seq,
-                                                               const int* __restrict__ tok_pos,
-                                                               const int* __restrict__ grp_first,
-                                                               const int* __restrict__ grp_count, bf16* __restrict__ ctx,
-                                                               int nh, int G_all, AttnOptions opt, int* status,
-                                                               unsigned long long* tl) {
-    using C = AttnCfg<HD>;
-    extern __shared__ __align__(128) uint8_t smem[];
-    if (threadIdx.x == 0) tl_mark(tl, 0);
-    pdl_launch_dependents();
-    pdl_wait();  // the previous kernel wrote q and the K/V rows of these very tokens
-    if (threadIdx.x == 0) tl_mark(tl, 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nkv = kv.nkv, parts_per_kv = EXACT ? 1 : (G_all + 7) / 8;  // query heads of a kv head in parts of at most 8
-    const int kvh = blockIdx.y / parts_per_kv, part = blockIdx.y % parts_per_kv;
-    const int G = EXACT ? G_all : min(8, G_all - part * 8), head0 = kvh * G_all + part * 8;
-    const int kd = EXACT ? HD : kv.hd, vd = EXACT ? HD : kv.vd;
-    const int chunk = EXACT ? 0 : opt.chunk, vdim = EXACT ? HD : opt.vdim;
-    const int first = __ldcg(grp_first + blockIdx.x), count = __ldcg(grp_count + blockIdx.x);
-    const int seq = __ldcg(tok_seq + first);
-    const int last_len = __ldcg(tok_pos + first + count - 1) + 1;  // positions ascend within a group
-    const bool active = warp < count;
-    const int t = first + (active ? warp : 0);
-    const int my_len = active ? __ldcg(tok_pos + t) + 1 : 0;
-    // first key visible to this warp's token, and the group's first key (page-aligned): a group may cross a chunk's edge
-    const int my_lo = (chunk > 0 && active) ? (my_len - 1) / chunk * chunk : 0;
-    const int grp_lo = chunk > 0 ? (__ldcg(tok_pos + first) / chunk * chunk) / kPageTokens * kPageTokens : 0;
-    const int* bt = kv.block_table + (size_t)seq * kv.max_pages_per_seq;
-    const bf16* kpool = kv.k_pool + (size_t)layer * kv.layer_stride;
-    const bf16* vpool = kv.v_pool + (size_t)layer * kv.layer_stride;
-    const uint32_t smem_base = smem_u32(smem);
-    bool bad = false;
-
-    auto issue_stage = [&](int st) {  // all 256 threads
-        const int s_begin = grp_lo + st * C::STAGE_ROWS;
-        if (s_begin < last_len) {
-            constexpr int PPS = C::STAGE_ROWS / kPageTokens;
-            int pgs[PPS];
-#pragma unroll
-            for (int j = 0; j < PPS; ++j) {
-                const int tok0 = s_begin + j * kPageTokens;
-                const int pg = tok0 < last_len ? __ldg(bt + tok0 / kPageTokens) : -1;
-                if (tok0 < last_len && (pg < 0 || pg >= kv.num_pages)) bad = true;
-                pgs[j] = (pg >= 0 && pg < kv.num_pages) ? pg : -1;
-            }
-            const uint32_t kbuf = smem_base + (uint32_t)((st % C::NST) * C::STAGE_BYTES);
-            const uint32_t vbuf = kbuf + (uint32_t)(C::STAGE_ROWS * C::ROW_BYTES);
-            constexpr int ROWS_PER_IT = kAttnCtaThreads / C::GRAN;
-            const int row0 = tid / C::GRAN, g = tid % C::GRAN;
-#pragma unroll
-            for (int i = 0; i < C::STAGE_ROWS / ROWS_PER_IT; ++i) {
-                const int row = i * ROWS_PER_IT + row0;
-                const int pg = pgs[(i * ROWS_PER_IT) / kPageTokens];
-                const bool valid = s_begin + row < last_len && pg >= 0;
-                const size_t pr = ((size_t)(valid ? pg : 0) * nkv + kvh) * kPageTokens + row % kPageTokens;
-                const uint32_t dst = (uint32_t)(row * C::ROW_BYTES + ((g ^ (row & 7)) << 4));
-                const bool kok = valid && g * 8 < kd, vok = valid && g * 8 < vd;  // zeros past the cached width
-                cp_async16_zfill(kbuf + dst, kpool + (kok ? pr * kd + g * 8 : 0), kok ? 16u : 0u);
-                cp_async16_zfill(vbuf + dst, vpool + (vok ? pr * vd + g * 8 : 0), vok ? 16u : 0u);
-            }
-        }
-        cp_async_commit();
-    };
-    const int n_stages = (last_len - grp_lo + C::STAGE_ROWS - 1) / C::STAGE_ROWS;
-#pragma unroll
-    for (int st = 0; st < C::NST; ++st) issue_stage(st);
-
-    const int hrow = lane >> 2, quad = lane & 3;
-    uint32_t qh[C::KS][2], ql[C::KS][2];
-    {
-        const float* qp = q + ((size_t)t * nh + head0 + hrow) * kd + quad * 2;
-#pragma unroll
-        for (int ks = 0; ks < C::KS; ++ks) {
-            float2 a = make_float2(0.f, 0.f), b = make_float2(0.f, 0.f);
-            if (active && hrow < G) {
-                if (ks * 16 < kd) a = __ldcg((const float2*)(qp + ks * 16));
-                if (ks * 16 + 8 < kd) b = __ldcg((const float2*)(qp + ks * 16 + 8));
-            }
-            split_bf16x2(a.x, a.y, qh[ks][0], ql[ks][0]);
-            split_bf16x2(b.x, b.y, qh[ks][1], ql[ks][1]);
-        }
-    }
-    const float scale = opt.scale;
-    float m_run = kNegBig, l_run = 0.f;
-    float o[C::DT][4];
-#pragma unroll
-    for (int d = 0; d < C::DT; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
-
-    for (int st = 0; st < n_stages; ++st) {
-        cp_async_wait<C::NST - 1>();
-        __syncthreads();  // the stage is complete and visible to every warp
-        const uint32_t kbuf = smem_base + (uint32_t)((st % C::NST) * C::STAGE_BYTES);
-        const uint32_t vbuf = kbuf + (uint32_t)(C::STAGE_ROWS * C::ROW_BYTES);
-#pragma unroll 1
-        for (int blk = 0; blk < C::STAGE_ROWS / 16; ++blk) {
-            const int k0 = grp_lo + st * C::STAGE_ROWS + blk * 16;
-            if (k0 >= my_len) break;  // warp-uniform: causal end of this token
-            if (k0 + 16 <= my_lo) continue;  // before its chunk
-            attn_block16<HD>(kbuf, vbuf, blk * 16, my_lo - k0, my_len - k0, qh, ql, scale, m_run, l_run, o, lane);
-        }
-        __syncthreads();  // every warp is done with this buffer
-        issue_stage(st + C::NST);
-    }
-    cp_async_wait<0>();
-    l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
-    l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-    if (active && hrow < G) {
-        const float inv = 1.f / l_run;  // my_len >= 1: at least one key
-        bf16* dst = ctx + (size_t)t * (EXACT ? (int64_t)nh * HD : opt.ctx_ld) + (size_t)(head0 + hrow) * vdim + quad * 2;
-#pragma unroll
-        for (int d = 0; d < C::DT; ++d) {
-            const float a = (o[d][0] + o[d][2]) * inv, b = (o[d][1] + o[d][3]) * inv;  // P_hi V + P_lo V
-            const int col = d * 8 + quad * 2;
-            if ((vdim & 1) == 0) {
-                if (col < vdim) *(uint32_t*)(dst + d * 8) = (uint32_t)bf16_bits(a) | ((uint32_t)bf16_bits(b) << 16);
-            } else {
-                if (col < vdim) dst[d * 8] = __float2bfloat16_rn(a);
-                if (col + 1 < vdim) dst[d * 8 + 1] = __float2bfloat16_rn(b);
-            }
-        }
-    }
-    if (bad) dev_fail(status, DEV_ERR_BOUNDS);
-    if (tid == 0) tl_mark(tl, 2);
-}
-
 // Attention of one (query head, token) per block without tensor cores, for what the kernels above do not take: fp32
 // caches (a session that computes in fp32) and heads wider than 128. Every warp walks the visible keys with a stride
 // of kSimtWarps; the lanes share the dimensions of a key; exact exponentials; the warps merge at the end.
@@ -660,24 +520,15 @@ void launch_hd(dim3 grid, cudaStream_t s, bool pdl, const float* q, const KvView
              nh, G, splits, early, opt, ws, counters, status, tl, trace);
 }
 
-template <int HD>
-void launch_prefill_hd(dim3 grid, cudaStream_t s, bool pdl, const float* q, const KvView& kv, int layer, const int* tok_seq,
-                       const int* tok_pos, const int* grp_first, const int* grp_count, bf16* ctx, int nh, int G,
-                       const AttnOptions& opt, int* status, unsigned long long* tl) {
-    launch_k(exact(opt, kv, nh, HD) ? k_attn_prefill<HD, true> : k_attn_prefill<HD, false>, grid, dim3(kAttnCtaThreads), (size_t)AttnCfg<HD>::SMEM, s, pdl, q, kv, layer, tok_seq, tok_pos,
-             grp_first, grp_count, ctx, nh, G, opt, status, tl);
-}
+}  // namespace
 
-// options with their defaults filled in
-AttnOptions resolve(AttnOptions o, const KvView& kv, int nh) {
+AttnOptions resolve_attn_options(AttnOptions o, const KvView& kv, int nh) {
     if (o.scale == 0.f) o.scale = 1.f / sqrtf((float)kv.hd);
     if (o.vdim == 0) o.vdim = kv.vd;
     if (o.head_ld == 0) o.head_ld = o.vdim;
     if (o.ctx_ld == 0) o.ctx_ld = (int64_t)nh * o.head_ld;
     return o;
 }
-
-}  // namespace
 
 template <typename Kern>
 static cudaError_t attn_attrs(Kern k, int smem) {
@@ -688,8 +539,6 @@ template <int HD>
 static cudaError_t attn_attrs_hd() {
     cudaError_t e = attn_attrs(k_attn_decode<HD, true>, AttnCfg<HD>::SMEM);
     if (e == cudaSuccess) e = attn_attrs(k_attn_decode<HD, false>, AttnCfg<HD>::SMEM);
-    if (e == cudaSuccess) e = attn_attrs(k_attn_prefill<HD, true>, AttnCfg<HD>::SMEM);
-    if (e == cudaSuccess) e = attn_attrs(k_attn_prefill<HD, false>, AttnCfg<HD>::SMEM);
     return e;
 }
 
@@ -702,7 +551,7 @@ int attn_prepare() {
     if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<bf16, 16>);
     if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<float, 32>);
     if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<bf16, 32>);
-    return (int)e;
+    return e == cudaSuccess ? attn_prompt_prepare() : (int)e;
 }
 
 constexpr int kMinSplitRows = 1024;
@@ -736,7 +585,7 @@ void launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, 
                       bool only_newest_row_fresh, unsigned long long* tl, unsigned long long* trace, int trace_ctas,
                       const AttnOptions& options) {
     const int early = (pdl && only_newest_row_fresh) ? 1 : 0;
-    const AttnOptions opt = resolve(options, kv, nh);
+    const AttnOptions opt = resolve_attn_options(options, kv, nh);
     const int G = nh / kv.nkv;
     const int units = T * kv.nkv * ((G + 7) / 8);
     const int wide = kv.hd > kv.vd ? kv.hd : kv.vd;
@@ -747,20 +596,9 @@ void launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, 
     else if (wide <= 128) launch_hd<128>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, splits, early, opt, ws.partials, ws.counters, status, tl, trace);
 }
 
-void launch_attention_prefill(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, const int* grp_first,
-                              const int* grp_count, int n_groups, bf16* ctx, int nh, int* status, cudaStream_t s, bool pdl,
-                              unsigned long long* tl, const AttnOptions& options) {
-    const AttnOptions opt = resolve(options, kv, nh);
-    const int G = nh / kv.nkv;
-    const int wide = kv.hd > kv.vd ? kv.hd : kv.vd;
-    dim3 grid(n_groups, kv.nkv * ((G + 7) / 8));
-    if (wide <= 64) launch_prefill_hd<64>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, grp_first, grp_count, ctx, nh, G, opt, status, tl);
-    else if (wide <= 128) launch_prefill_hd<128>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, grp_first, grp_count, ctx, nh, G, opt, status, tl);
-}
-
 void launch_attention_simt(const float* q, KvView kv, bool f32, const int* tok_seq, const int* tok_pos, void* ctx, int T, int nh,
                            const AttnOptions& options, int* status, cudaStream_t s, bool pdl, unsigned long long* tl) {
-    const AttnOptions opt = resolve(options, kv, nh);
+    const AttnOptions opt = resolve_attn_options(options, kv, nh);
     const dim3 grid(nh, T), block(kSimtWarps * 32);
     const size_t smem = (size_t)(kv.hd + kSimtWarps * (opt.vdim + 2)) * 4;
     const bool wide = opt.vdim > 512;

@@ -69,35 +69,6 @@ struct LatentDev {
     unsigned long long* tl;
 };
 
-// shared-memory descriptor of an operand whose rows are its K extent: 64 columns (128 swizzled bytes) per row, groups of 64
-// columns block_bytes apart (leading byte offset), groups of 8 rows 1024 bytes apart (stride byte offset)
-__device__ __forceinline__ uint64_t desc_n128(uint32_t smem_addr, int block_bytes) {
-    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(block_bytes >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(v[0]),
-        "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
-        "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ float exp2_fast(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // every lane of an issuing warp waits (acquire), the outcome is made uniform
 __device__ __forceinline__ bool mma_wait(uint64_t* bar, uint32_t parity, int* status, int code) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
@@ -334,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_attn_latent(const __grid_consta
         for (int j = 0; j < tiles; ++j) {
             if (!mma_wait(&p_full[j & 1], (uint32_t)(j >> 1) & 1u, p.status, DEV_ERR_ACC_WAIT)) break;
             tc_fence_after();
-            const uint64_t vd = desc_n128(v_a + (j % p.stages) * stage_bytes, kBlockBytes);
+            const uint64_t vd = umma_desc_n128(v_a + (j % p.stages) * stage_bytes, kBlockBytes);
 #pragma unroll
             for (int half = 0; half < 2; ++half)  // P hi, P lo
 #pragma unroll
@@ -587,8 +558,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_attn_latent_decode(const __grid
             const int j = max(it - warm, 0);
             if (!mma_wait(&p_full[it & 1], (uint32_t)(it >> 1) & 1u, p.status, DEV_ERR_ACC_WAIT)) break;
             tc_fence_after();
-            uint64_t vd = desc_n128(k_a + (j % p.stages) * stage_bytes, k_block);
-            const uint64_t pd = desc_n128(p_a + (it & 1) * p_buf, p_buf);
+            uint64_t vd = umma_desc_n128(k_a + (j % p.stages) * stage_bytes, k_block);
+            const uint64_t pd = umma_desc_n128(p_a + (it & 1) * p_buf, p_buf);
             const uint32_t again = it > 0;
             uint32_t d = tmem + colO;
 #pragma unroll 2

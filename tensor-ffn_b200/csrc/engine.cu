@@ -363,6 +363,7 @@ void Session::alloc_uniform() {
     kv_.layer_stride = layer_stride;
     kv_.nkv = (int)nkv;
     kv_.hd = kv_.vd = (int)hd;
+    attn_group_tokens_ = attention_group_tokens((int)(nh / nkv));
 
     // RoPE tables in float, as the reference builds them on the host (inference/src/model/qwen.cu:120-132)
     {
@@ -739,6 +740,11 @@ int Session::build_groups(const int* seq, const int* pos, int T, int limit, int3
     return n;
 }
 
+void check_launch(int rc, const char* what) {
+    if (rc == -1000) throw Error(kErrCuda, "cuTensorMapEncodeTiled failed or is unavailable");
+    if (rc != 0) cuda_check((cudaError_t)rc, what, __FILE__, __LINE__);
+}
+
 // one GEMM of a step: tensor cores, or true fp32 in a session that computes in fp32
 void Session::gemm(GemmCall& call, int cls, bool pdl) {
     if (ablated(cls)) return;  // timing-only ablation: results are then meaningless
@@ -749,8 +755,7 @@ void Session::gemm(GemmCall& call, int cls, bool pdl) {
     prof_begin(cls);
     const int rc = st_ && st_->f32 ? launch_gemm_f32(call, gemm_ws(), stream_) : launch_gemm(call, gemm_ws(), stream_);
     prof_end();
-    if (rc == -1000) throw Error(kErrCuda, "cuTensorMapEncodeTiled failed or is unavailable");
-    if (rc != 0) cuda_check((cudaError_t)rc, "GEMM launch", __FILE__, __LINE__);
+    check_launch(rc, "GEMM launch");
     launches_++;
 }
 
@@ -759,13 +764,16 @@ Session::Staged Session::stage_rows(const int32_t* tsp, int T) {
     TFFN_CUDA(cudaMemcpyAsync(tokens_.p, tsp, (size_t)T * 4, cudaMemcpyHostToDevice, stream_));
     TFFN_CUDA(cudaMemcpyAsync(tok_seq_.p, seq, (size_t)T * 4, cudaMemcpyHostToDevice, stream_));
     TFFN_CUDA(cudaMemcpyAsync(tok_pos_.p, pos, (size_t)T * 4, cudaMemcpyHostToDevice, stream_));
-    int32_t* runs = h_pinned_runs_.get((size_t)T * 4);
+    int32_t* runs = h_pinned_runs_.get((size_t)T * 6);
     Staged r;
-    r.n_groups = build_groups(seq, pos, T, 8, runs, runs + T);
+    r.n_groups = build_groups(seq, pos, T, attn_group_tokens_, runs, runs + T);
     TFFN_CUDA(cudaMemcpyAsync(grp_first_.p, runs, (size_t)r.n_groups * 4, cudaMemcpyHostToDevice, stream_));
     TFFN_CUDA(cudaMemcpyAsync(grp_count_.p, runs + T, (size_t)r.n_groups * 4, cudaMemcpyHostToDevice, stream_));
-    r.n_segs = 0;
+    r.n_segs = r.n_latent = 0;
     if (st_) {
+        r.n_latent = build_groups(seq, pos, T, 8, runs + 4 * T, runs + 5 * T);
+        TFFN_CUDA(cudaMemcpyAsync(st_->lat_first.p, runs + 4 * T, (size_t)r.n_latent * 4, cudaMemcpyHostToDevice, stream_));
+        TFFN_CUDA(cudaMemcpyAsync(st_->lat_count.p, runs + 5 * T, (size_t)r.n_latent * 4, cudaMemcpyHostToDevice, stream_));
         r.n_segs = build_groups(seq, pos, T, T, runs + 2 * T, runs + 3 * T);
         TFFN_CUDA(cudaMemcpyAsync(st_->seg_first.p, runs + 2 * T, (size_t)r.n_segs * 4, cudaMemcpyHostToDevice, stream_));
         TFFN_CUDA(cudaMemcpyAsync(st_->seg_count.p, runs + 3 * T, (size_t)r.n_segs * 4, cudaMemcpyHostToDevice, stream_));
@@ -836,7 +844,7 @@ void Session::lm_head(const void* x, int64_t ldx, int n_rows, bool decode, bool 
 }
 
 void Session::run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, Staged runs) {
-    if (st_) return run_stack(T, n_logit_rows, logit_rows_are_all, decode, max_ctx, runs.n_groups, runs.n_segs);
+    if (st_) return run_stack(T, n_logit_rows, logit_rows_are_all, decode, max_ctx, runs);
     const int n_groups = runs.n_groups;
     const Config& c = m_->cfg;
     // this rank's slice of the heads, of the intermediate dimension and of the LM head (everything without
@@ -913,10 +921,11 @@ void Session::run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool
         gemm(g, KC_GEMM_QKV, pdl);
         g.qkv = nullptr;
         prof_begin(KC_ATTENTION);
-        if (live(KC_ATTENTION) && n_groups > 0) {
-            // prompt rows: eight consecutive tokens of a sequence share one pass over its cache
-            launch_attention_prefill(q_.as<float>(), kv_, l, tok_seq, tok_pos, grp_first_.as<int>(), grp_count_.as<int>(), n_groups,
-                                     ctx_.as<bf16>(), nh, status, stream_, pdl, tl_next(KC_ATTENTION));
+        if (live(KC_ATTENTION) && n_groups > 0 && !attention_prompt_as_rows(T, nh, nkv, m_->num_sms)) {
+            // prompt rows: consecutive tokens of a sequence share one pass over its cache
+            check_launch(launch_attention_prefill(q_.as<float>(), kv_, l, tok_seq, tok_pos, grp_first_.as<int>(), grp_count_.as<int>(), n_groups,
+                                                  ctx_.as<bf16>(), nh, m_->num_sms, status, tmaps_, stream_, pdl, tl_next(KC_ATTENTION)),
+                         "attention launch");
         } else if (live(KC_ATTENTION)) {
             unsigned long long* tl = tl_next(KC_ATTENTION);
             const bool traced = tl_on_ && (int)tl_cls_.size() - 1 == tl_trace_launch_;

@@ -14,6 +14,7 @@
 namespace tffn {
 
 void cuda_check(cudaError_t e, const char* what, const char* file, int line);
+void check_launch(int rc, const char* what);  // of a launcher that may also fail to encode a tensor map (-1000)
 #define TFFN_CUDA(x) ::tffn::cuda_check((x), #x, __FILE__, __LINE__)
 
 struct DeviceBuffer {
@@ -169,7 +170,7 @@ struct StackState {
     int64_t cq_ld = 0, q_up_ld = 0, u_ld = 0, lru_gate_ld = 0;
     size_t o_lat_cols = 0;
     DeviceBuffer router, counts, pair, pair_w, pair_row, xg, act_e, y, tiles;
-    DeviceBuffer seg_first, seg_count, ones;
+    DeviceBuffer seg_first, seg_count, lat_first, lat_count, ones;
 };
 
 class Session {
@@ -210,7 +211,7 @@ public:
     const Model* model() const { return m_; }
 
 private:
-    struct Staged { int n_groups, n_segs; };  // runs of rows: at most 8 positions of a sequence; all of a sequence
+    struct Staged { int n_groups, n_latent, n_segs; };  // runs of a sequence's rows: at most attn_group_tokens_; at most 8; all
     const Model* m_;
     const Expert* e_;
     TpComm* tp_ = nullptr;  // not owned
@@ -266,7 +267,8 @@ private:
 
     // token metadata and activations of the batched path
     DeviceBuffer tokens_, tok_seq_, tok_pos_, row_idx_, picks_, identity_, dec_tokens_;
-    DeviceBuffer grp_first_, grp_count_;  // prefill attention: groups of up to 8 consecutive rows of one sequence
+    DeviceBuffer grp_first_, grp_count_;  // prompt attention: groups of up to attn_group_tokens_ consecutive rows of one sequence
+    int attn_group_tokens_ = 128;
     DeviceBuffer h_, xn_, q_, ctx_, act_b_, act_e_, xn_last_, logits_;
     size_t logits_rows_ = 0;
     DeviceBuffer attn_partials_, attn_counters_;
@@ -306,7 +308,7 @@ private:
     std::unique_ptr<StackState> st_;
     void alloc_uniform();
     void alloc_stack(bool f32);
-    void run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, int n_groups, int n_segs);
+    void run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, Staged runs);
     int attn_ctx(const LayerSpec& l, int max_ctx) const { return l.chunk > 0 && l.chunk < max_ctx ? l.chunk : max_ctx; }
     int rope_table(const RopeSpec& spec);
     AttnOptions attn_options(const LayerSpec& l) const;
@@ -326,7 +328,7 @@ private:
     void ensure_logits(size_t rows);
     void ensure_ring(int entries);
     // runs T tokens already staged in tokens_/tok_seq_/tok_pos_ (or decode state when decode=true)
-    void run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, Staged runs = {0, 0});
+    void run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, Staged runs = {0, 0, 0});
     // groups for launch_attention_prefill from the rows' (slot, position) lists; fills pin[0..2*n) and returns n
     // (runs of consecutive positions of one sequence, at most `limit` rows each)
     static int build_groups(const int* seq, const int* pos, int T, int limit, int32_t* first, int32_t* count);

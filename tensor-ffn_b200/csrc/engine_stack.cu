@@ -331,6 +331,7 @@ void Session::alloc_stack(bool f32) {
             kv.k_pool = c.k.as<bf16>();
             kv.v_pool = c.v.as<bf16>();
             q_cols = std::max<size_t>(q_cols, (size_t)sp.heads * kv.hd);
+            attn_group_tokens_ = std::min(attn_group_tokens_, attention_group_tokens(sp.heads / sp.kv_heads));
         } else if (sp.mixer == Mixer::LatentAttention) {
             KvView& kv = c.kv;
             if (sp.kv_from >= 0) {
@@ -430,6 +431,8 @@ void Session::alloc_stack(bool f32) {
         s.tiles.alloc((size_t)s.max_tiles * sizeof(GroupTile));
     }
     s.seg_first.alloc(T * 4);
+    s.lat_first.alloc(T * 4);
+    s.lat_count.alloc(T * 4);
     s.seg_count.alloc(T * 4);
     std::vector<int> ones(T, 1);
     upload(s.ones, ones.data(), T * 4);
@@ -488,7 +491,8 @@ int Session::decode_graph_key(int n_seqs, int max_ctx) const {
     return key;
 }
 
-void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, int n_groups, int n_segs) {
+void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, Staged runs) {
+    int n_segs = runs.n_segs;
     StackState& s = *st_;
     const Config& c = m_->cfg;
     const int H = c.hidden_size;
@@ -618,9 +622,10 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
             step(KC_ATTENTION, [&](unsigned long long* tl) {
                 if (f32 || !attention_tc_supported(cache.kv.hd, cache.kv.vd))
                     launch_attention_simt(q_.as<float>(), cache.kv, f32, tok_seq, tok_pos, ctx_.p, T, sp.heads, opt, status, stream_, pdl, tl);
-                else if (n_groups > 0)
-                    launch_attention_prefill(q_.as<float>(), cache.kv, 0, tok_seq, tok_pos, grp_first_.as<int>(), grp_count_.as<int>(),
-                                             n_groups, ctx_.as<bf16>(), sp.heads, status, stream_, pdl, tl, opt);
+                else if (runs.n_groups > 0 && !attention_prompt_as_rows(T, sp.heads, sp.kv_heads, m_->num_sms))
+                    check_launch(launch_attention_prefill(q_.as<float>(), cache.kv, 0, tok_seq, tok_pos, grp_first_.as<int>(), grp_count_.as<int>(),
+                                                          runs.n_groups, ctx_.as<bf16>(), sp.heads, m_->num_sms, status, tmaps_, stream_, pdl, tl, opt),
+                                 "attention launch");
                 else
                     launch_attention(q_.as<float>(), cache.kv, 0, tok_seq, tok_pos, ctx_.as<bf16>(), T, sp.heads, attn_ctx(sp, max_ctx),
                                      attn_ws(), m_->num_sms, status, stream_, pdl, decode, tl, nullptr, 0, opt);
@@ -669,8 +674,8 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
                 at.kv = cache.kv;
                 at.tok_seq = tok_seq;
                 at.tok_pos = tok_pos;
-                at.grp_first = grp_first_.as<int>();
-                at.grp_count = grp_count_.as<int>();
+                at.grp_first = s.lat_first.as<int>();
+                at.grp_count = s.lat_count.as<int>();
                 at.gate = (const bf16*)act_at(s.proj, l.g1_off);
                 at.gate_ld = l.in_rows;
                 at.out = s.o_lat.as<bf16>();
@@ -678,9 +683,8 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
                 at.only_newest_row_fresh = decode;
                 at.status = status;
                 step(KC_ATTENTION, [&](unsigned long long* tl) {
-                    const int rc = launch_attention_latent(at, T, n_groups, max_ctx, attn_ws(), m_->num_sms, tmaps_, stream_, pdl, tl);
-                    if (rc == -1000) throw Error(kErrCuda, "cuTensorMapEncodeTiled failed or is unavailable");
-                    if (rc != 0) cuda_check((cudaError_t)rc, "latent attention launch", __FILE__, __LINE__);
+                    check_launch(launch_attention_latent(at, T, runs.n_latent, max_ctx, attn_ws(), m_->num_sms, tmaps_, stream_, pdl, tl),
+                                 "latent attention launch");
                 });
             } else {
                 batched(KC_GEMM_UK, sp.heads, l.uk.as<bf16>(), dim8, s.q_up.p, s.q_up_ld, dim8, sp.dim, sp.kv_rank, GEMM_STORE_F32, q_.p,

@@ -200,6 +200,8 @@ struct AttnOptions {
     const void* gate = nullptr;  // (launch_attention_simt) optional [T][gate_ld], stored like activations: head h's output times sigmoid(gate[t][h])
     int64_t gate_ld = 0;
 };
+// the options with their defaults filled in
+AttnOptions resolve_attn_options(AttnOptions o, const KvView& kv, int nh);
 // opt the attention kernels into their dynamic shared memory (once per device, outside stream capture)
 int attn_prepare();
 // context splits launch_attention will use (a CUDA-graph key: the grid depends on it)
@@ -220,11 +222,18 @@ void launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, 
                       unsigned long long* trace = nullptr, int trace_ctas = 0,  // trace: 16 u64 per CTA, see attn.cu
                       const AttnOptions& opt = AttnOptions());
 
-// Prompt tokens: rows grp_first[g] .. grp_first[g] + grp_count[g] - 1 (at most 8, consecutive positions of
-// one sequence) share one pass over that sequence's cache; n_groups groups cover the T rows of the call.
-void launch_attention_prefill(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, const int* grp_first,
-                              const int* grp_count, int n_groups, bf16* ctx, int nh, int* status, cudaStream_t s,
-                              bool pdl = false, unsigned long long* tl = nullptr, const AttnOptions& opt = AttnOptions());
+// Prompt tokens: rows grp_first[g] .. grp_first[g] + grp_count[g] - 1 (at most attention_group_tokens of the heads, consecutive
+// positions of one sequence) share one pass over that sequence's cache; n_groups groups cover the T rows of the call.
+// Returns a cudaError (launch) or -1000 if the tensor maps could not be encoded.
+inline int attention_group_tokens(int heads_per_kv) { return heads_per_kv < 128 ? 128 / heads_per_kv : 1; }
+// Prompts whose (token, kv head) units fit the SMs in one wave are better off with a block per unit (launch_attention): it has no
+// chain of products between its warps. 9 tokens of 14 heads and 2 kv heads of 64: about 4 us, in tiles 8; a 60-token continuation
+// of a long context has a fifteenth of the blocks in tiles.
+inline bool attention_prompt_as_rows(int T, int nh, int nkv, int num_sms) { return T * nkv * ((nh / nkv + 7) / 8) <= num_sms; }
+int attn_prompt_prepare();
+int launch_attention_prefill(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, const int* grp_first,
+                             const int* grp_count, int n_groups, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s,
+                             bool pdl = false, unsigned long long* tl = nullptr, const AttnOptions& opt = AttnOptions());
 
 // ------------------------------------------------------------------ layers with an fp32 residual stream
 // "f32" below selects the storage type of activations and cache: fp32 in a session that computes in fp32, else bf16.
@@ -309,7 +318,7 @@ void launch_latent_rope(const void* q_up, int64_t ld, int off, int heads, int ro
                         unsigned long long* tl = nullptr);
 int latent_prepare();
 // The attention itself on the tensor cores (bf16 sessions): the unrotated queries come with the key projections folded in,
-// the rotated parts as projected. Groups as in launch_attention_prefill; n_groups = 0: every row is a token of its own
+// the rotated parts as projected. Groups: at most 8 consecutive positions of a sequence; n_groups = 0: every row is a token of its own
 // (decode), its context possibly in splits (see launch_attention for only_newest_row_fresh).
 struct LatentAttn {
     const bf16* q_lat;        // [rows_alloc][heads][head_ld]
