@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
     uint64_t* acc_full = empty + STAGES;
     uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     int prob = blockIdx.y / p.t_tiles;  // independent problems (base / expert gate-up) share a launch
     const int n0 = blockIdx.x * p.tile_n;
     int t0 = (blockIdx.y % p.t_tiles) * BN, t_end = p.T, w_row0 = n0;
@@ -338,84 +338,83 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
     FinalizePre pre[2];  // epilogue warps, split-K: operands of the columns they will finish
     pre[0].valid = pre[1].valid = false;
 
+    // The two issuing warps pace a CTA's stream, so every lane runs their loops (uniform control flow and operands, stage and
+    // phase carried along) and one is elected per instruction: from a branch of a single lane each costs several times as much.
+    // Inside a decode step: down projections of base and expert, K 2 x 4 864, N 896, 64 tokens 12.0 -> 10.3 us, 13 tokens
+    // 8.7 -> 6.5; q|k|v and gate|up on average 13.0 -> 12.2 (64 tokens, LM head included), 8.5 -> 7.7 (13 tokens).
     if (warp == 0) {
+        const CUtensorMap *const tw = &p.tmW[prob * 2], *const tx = &p.tmX[batched ? 0 : prob * 2];
+        const uint32_t ring = smem_u32(smem), full_0 = smem_u32(full);
         if (lane == 0) {
-            prefetch_tmap(&p.tmW[prob * 2]);
-            prefetch_tmap(&p.tmX[prob * 2]);
-            // Weights do not depend on the previous kernel: the first ring of weight boxes is
-            // requested before griddepcontrol.wait, the activation boxes after it.
-            const int pre = n_iters < STAGES ? n_iters : STAGES;
-            for (int it = 0; it < pre; ++it) {
-                const int i = kb_begin + it;
-                const int seg = i >= p.kblocks[0] ? 1 : 0;
-                const int kb = seg ? i - p.kblocks[0] : i;
-                mbar_arrive_expect_tx(&full[it], Cfg::STAGE_BYTES);
-                if (halves) {
-                    tma_load_2d(smem + it * Cfg::STAGE_BYTES, &p.tmW[prob * 2], kb * BK, w_row0, &full[it]);
-                    tma_load_2d(smem + it * Cfg::STAGE_BYTES + Cfg::A_BYTES / 2, &p.tmW[prob * 2 + 1], kb * BK, w_row0, &full[it]);
-                } else {
-                    tma_load_2d(smem + it * Cfg::STAGE_BYTES, &p.tmW[prob * 2 + seg], kb * BK, w_row0, &full[it]);
-                }
+            prefetch_tmap(tw);
+            prefetch_tmap(tx);
+        }
+        __syncwarp();
+        auto load_w = [&](int i, int s) {
+            const int seg = i >= p.kblocks[0] ? 1 : 0, x = (seg ? i - p.kblocks[0] : i) * BK;
+            const uint32_t a = ring + s * Cfg::STAGE_BYTES, bar = full_0 + s * 8;
+            mbar_arrive_expect_tx_elect(bar, Cfg::STAGE_BYTES);
+            if (halves) {
+                tma_load_2d_elect(a, tw, x, w_row0, bar);
+                tma_load_2d_elect(a + Cfg::A_BYTES / 2, tw + 1, x, w_row0, bar);
+            } else {
+                tma_load_2d_elect(a, tw + seg, x, w_row0, bar);
             }
-            TFFN_TRACE(1);
-            pdl_wait();
+        };
+        auto load_x = [&](int i, int s) {
+            const int seg = i >= p.kblocks[0] ? 1 : 0, x = (seg ? i - p.kblocks[0] : i) * BK;
+            const uint32_t b = ring + s * Cfg::STAGE_BYTES + Cfg::A_BYTES, bar = full_0 + s * 8;
+            if (batched) tma_load_3d_elect(b, tx, x, prob_b, t0, bar);
+            else tma_load_2d_elect(b, tx + seg, x, t0, bar);
+        };
+        // Weights do not depend on the previous kernel: the first ring of weight boxes is
+        // requested before griddepcontrol.wait, the activation boxes after it.
+        const int pre = n_iters < STAGES ? n_iters : STAGES;
+        for (int it = 0; it < pre; ++it) load_w(kb_begin + it, it);
+        if (lane == 0) TFFN_TRACE(1);
+        pdl_wait();
+        if (lane == 0) {
             TFFN_TRACE(2);
             tl_mark(p.tl, 1);
-            for (int it = 0; it < pre; ++it) {
-                const int i = kb_begin + it;
-                const int seg = i >= p.kblocks[0] ? 1 : 0;
-                const int kb = seg ? i - p.kblocks[0] : i;
-                uint8_t* b = smem + it * Cfg::STAGE_BYTES + Cfg::A_BYTES;
-                if (batched) tma_load_3d(b, &p.tmX[0], kb * BK, prob_b, t0, &full[it]);
-                else tma_load_2d(b, &p.tmX[prob * 2 + seg], kb * BK, t0, &full[it]);
-            }
-            for (int it = pre; it < n_iters; ++it) {
-                const int s = it % STAGES;
-                const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-                if (!mbar_wait(&empty[s], ph ^ 1u, p.status, DEV_ERR_EMPTY_WAIT)) break;
-                const int i = kb_begin + it;
-                const int seg = i >= p.kblocks[0] ? 1 : 0;
-                const int kb = seg ? i - p.kblocks[0] : i;
-                uint8_t* a = smem + s * Cfg::STAGE_BYTES;
-                uint8_t* b = a + Cfg::A_BYTES;
-                mbar_arrive_expect_tx(&full[s], Cfg::STAGE_BYTES);
-                if (halves) {
-                    tma_load_2d(a, &p.tmW[prob * 2], kb * BK, w_row0, &full[s]);
-                    tma_load_2d(a + Cfg::A_BYTES / 2, &p.tmW[prob * 2 + 1], kb * BK, w_row0, &full[s]);
-                } else {
-                    tma_load_2d(a, &p.tmW[prob * 2 + seg], kb * BK, w_row0, &full[s]);
-                }
-                if (batched) tma_load_3d(b, &p.tmX[0], kb * BK, prob_b, t0, &full[s]);
-                else tma_load_2d(b, &p.tmX[prob * 2 + seg], kb * BK, t0, &full[s]);
+        }
+        __syncwarp();
+        for (int it = 0; it < pre; ++it) load_x(kb_begin + it, it);
+        int s = 0;
+        uint32_t ph = 0;
+        for (int it = pre; it < n_iters; ++it) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ph, p.status, DEV_ERR_EMPTY_WAIT))) break;
+            load_w(kb_begin + it, s);
+            load_x(kb_begin + it, s);
+            if (++s == STAGES) {
+                s = 0;
+                ph ^= 1;
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(BM, BN);
-            bool started[2] = {false, false};
-            bool ok = true;
-            for (int it = 0; it < n_iters && ok; ++it) {
-                const int s = it % STAGES;
-                const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-                ok = mbar_wait(&full[s], ph, p.status, DEV_ERR_FULL_WAIT);
-                if (!ok) break;
-                if (it < 12) TFFN_TRACE(16 + it);
-                tc_fence_after();
-                const int seg = (kb_begin + it) >= p.kblocks[0] ? 1 : 0;
-                const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
-                const uint32_t b_addr = a_addr + Cfg::A_BYTES;
-                const uint32_t d = tmem_base + (uint32_t)(seg * BN);
+        constexpr uint32_t idesc = umma_idesc_bf16(BM, BN);
+        const uint64_t a_0 = umma_desc_k128(smem_u32(smem)), b_0 = umma_desc_k128(smem_u32(smem) + Cfg::A_BYTES);
+        int s = 0;
+        uint32_t ph = 0;
+        for (int it = 0; it < n_iters; ++it) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, p.status, DEV_ERR_FULL_WAIT))) break;
+            if (lane == 0 && it < 12) TFFN_TRACE(16 + it);
+            __syncwarp();
+            tc_fence_after();
+            const int seg = (kb_begin + it) >= p.kblocks[0] ? 1 : 0;
+            const bool more = it > 0 && kb_begin + it != p.kblocks[0];  // not the first of its accumulator
+            const uint64_t at = (uint64_t)(uint32_t)(s * (Cfg::STAGE_BYTES >> 4));
+            const uint32_t d = tmem_base + (uint32_t)(seg * BN);
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k)
-                    umma_bf16(d, umma_desc_k128(a_addr + k * 32), umma_desc_k128(b_addr + k * 32), idesc,
-                              (started[seg] || k > 0) ? 1u : 0u);
-                started[seg] = true;
-                if (it < 12) TFFN_TRACE(28 + it);
-                umma_commit(&empty[s]);
+            for (int k = 0; k < BK / 16; ++k) umma_bf16_elect(d, a_0 + at + 2 * k, b_0 + at + 2 * k, idesc, (more || k > 0) ? 1u : 0u);
+            umma_commit_elect(&empty[s]);
+            if (++s == STAGES) {
+                s = 0;
+                ph ^= 1;
             }
-            TFFN_TRACE(3);
-            umma_commit(acc_full);  // arrives when every MMA above has finished (also on the error path)
         }
+        if (lane == 0) TFFN_TRACE(3);
+        __syncwarp();
+        umma_commit_elect(acc_full);  // arrives when every MMA above has finished (also on the error path)
     } else {
         // Epilogue warps 2..5 own TMEM lane quarter (warp % 4): thread = one weight row. They combine
         // the two operand pairs (base + alpha * expert) and park ONE fp32 plane [column][row] in the
@@ -766,18 +765,15 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
     // grouped: the grid has room for the worst case, the split policy goes by one tile per group that can have rows
     const int tiles = c.grp && c.grp_rows_hint > 0 ? n_tiles * c.grp_rows_hint : n_tiles * t_tiles * nprob;
     p.t_tiles = t_tiles;
-    // K splits = cluster size (1, 2, 4, 8 or 16). Inside a decode step one CTA takes in roughly one
-    // stage (a 16 KB weight box and its activation box) per 0.5 us whatever the ring depth, about 50 GB/s
-    // per SM (measured with the phase stamps; all SMs together about 7 TB/s), so a weight-streaming launch
-    // needs about as many CTAs as there are SMs: tiles are split along K until the grid fills the SMs,
-    // keeping two k-blocks per split.
+    // K splits = cluster size (1, 2, 4, 8 or 16). A CTA's stream is bound by the latency of its stages (about 50 GB/s per SM,
+    // all SMs together about 7 TB/s), so a weight-streaming launch needs about as many CTAs as there are SMs: tiles are split
+    // along K until the grid fills the SMs.
     int splits = 1;
     if (force_splits > 0) {
         splits = force_splits;
     } else {
         while (splits < kMaxSplits && tiles * splits * 2 <= ws.num_sms + ws.num_sms / 8 && total_kb / (splits * 2) >= 1) splits *= 2;
-        // A long K extent: the stage cadence is a property of the CTA (about 0.45 us per stage), so two
-        // CTAs per SM stream twice as much as one until HBM is the limit; keep splitting while every CTA
+        // A long K extent: two CTAs per SM stream twice as much as one until HBM is the limit; keep splitting while every CTA
         // still gets eight k-blocks and the grid fits two per SM (measured at 16 tokens, N 2048, K 22016:
         // 8 splits 49.5 us, half of the 8-CTA clusters waiting for a second wave; 16 splits 18.0 us).
         // A grouped launch cannot request weights ahead of its dependency wait (the tile table comes from the kernel

@@ -75,15 +75,8 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gsrc, uint3
 __device__ __forceinline__ void bulk_prefetch_l2(const void* gsrc, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gsrc), "r"(bytes) : "memory");
 }
-// 2-D tiled TMA load; x is the innermost coordinate in elements (x * elem_size % 16 == 0)
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, int x, int y, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            smem_u32(smem_dst)),
-        "l"(tmap), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-// the same and the arrival for it, issued by one elected lane of a converged warp with uniform operands
+// 2-D tiled TMA load (x is the innermost coordinate in elements, x * elem_size % 16 == 0) and the arrival for it, issued by one
+// elected lane of a converged warp with uniform operands
 __device__ __forceinline__ void tma_load_2d_elect(uint32_t smem_dst, const void* tmap, int x, int y, uint32_t bar) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
@@ -101,11 +94,12 @@ __device__ __forceinline__ void mbar_arrive_expect_tx_elect(uint32_t bar, uint32
         : "memory");
 }
 // 3-D tiled TMA load
-__device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, int x, int y, int z, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_3d_elect(uint32_t smem_dst, const void* tmap, int x, int y, int z, uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            smem_u32(smem_dst)),
-        "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n\t}" ::"r"(smem_dst),
+        "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
         : "memory");
 }
 __device__ __forceinline__ void prefetch_tmap(const void* tmap) {
@@ -180,20 +174,8 @@ __device__ __forceinline__ uint64_t umma_desc_k128(uint32_t smem_addr) {
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-// D[tmem] (+)= A[smem] * B[smem]; issued by one thread.
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Arrive on an mbarrier once all MMAs issued so far by this thread have completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// The same for a whole warp whose control flow and operands are uniform, one lane elected per instruction. Issued from a
+// D[tmem] (+)= A[smem] * B[smem], and the arrival on an mbarrier once all products issued so far have completed. For a whole warp
+// whose control flow and operands are uniform, one lane elected per instruction. Issued from a
 // branch that a single lane has taken, every instruction costs several times as much (uniform registers are not available).
 __device__ __forceinline__ void umma_bf16_elect(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
