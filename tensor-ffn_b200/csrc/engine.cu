@@ -322,7 +322,6 @@ Session::Session(const Model* m, const Expert* e, int max_batch, int max_seq, cu
     grp_first_.alloc(T * 4);
     grp_count_.alloc(T * 4);
     picks_.alloc(T * 4);
-    dec_tokens_.alloc((size_t)max_batch * 4);
     {
         std::vector<int> id(T);
         for (size_t i = 0; i < T; ++i) id[i] = (int)i;
@@ -333,8 +332,10 @@ Session::Session(const Model* m, const Expert* e, int max_batch, int max_seq, cu
     ensure_logits(std::max<size_t>(256, max_batch));
     attn_partials_.alloc((size_t)32 << 20);
     attn_counters_.alloc(16384 * 4);
-    status_.alloc(4);
-    step_counter_.alloc(4);
+    step_io_.alloc((size_t)(kIoTokens + max_batch) * 4);
+    status_.view(step_io_.p, 4);
+    step_counter_.view(step_io_.as<int>() + kIoCounter, 4);
+    dec_tokens_.view(step_io_.as<int>() + kIoTokens, (size_t)max_batch * 4);
     TFFN_CUDA(cudaMallocHost(&h_status_, 4));
     *h_status_ = 0;
 
@@ -561,12 +562,11 @@ void Session::ensure_pages(int slot, int new_len) {
 }
 void Session::flush_tables() {
     if (!table_dirty_) return;
-    // the host vector may change again before the copy runs, so stage it in pinned memory
-    int32_t* pin = pinned_i32(h_block_table_.size());
-    TFFN_CUDA(cudaStreamSynchronize(stream_));
+    // the host vector may change again before the copy runs, so it is staged in pinned memory of its own
+    int32_t* pin = h_pinned_table_.get(h_block_table_.size());
+    TFFN_CUDA(cudaStreamSynchronize(stream_));  // an earlier copy out of it is done
     memcpy(pin, h_block_table_.data(), h_block_table_.size() * 4);
     TFFN_CUDA(cudaMemcpyAsync(block_table_.p, pin, h_block_table_.size() * 4, cudaMemcpyHostToDevice, stream_));
-    TFFN_CUDA(cudaStreamSynchronize(stream_));
     table_dirty_ = false;
 }
 
@@ -650,8 +650,8 @@ int Session::status() {
     TFFN_CUDA(cudaStreamSynchronize(stream_));
     return *h_status_;
 }
-void Session::check_status() {
-    const int st = status();
+void Session::check_status() { fail_on_status(status()); }
+void Session::fail_on_status(int st) {
     if (st != 0) {
         TFFN_CUDA(cudaMemsetAsync(status_.p, 0, 4, stream_));
         char buf[128];
@@ -1278,9 +1278,11 @@ void Session::prefill(const int32_t* tokens, const int32_t* seq_lens, int n_seqs
         if (sampling() && !last_rows.empty()) upload_draws(last_rows.size());  // one draw per sequence, slot order
         run_batched(T, (int)last_rows.size(), false, false, max_ctx, runs);
         if (!last_rows.empty()) {
-            std::vector<int> picks(last_rows.size());
+            int32_t* picks = pin + 3 * T;  // its row indices have been copied
             std::vector<float> rows_host;
-            TFFN_CUDA(cudaMemcpyAsync(picks.data(), picks_.p, picks.size() * 4, cudaMemcpyDeviceToHost, stream_));
+            TFFN_CUDA(cudaMemcpyAsync(picks, picks_.p, last_rows.size() * 4, cudaMemcpyDeviceToHost, stream_));
+            // prompts end in slot order, so those that end in a chunk are neighbours
+            TFFN_CUDA(cudaMemcpyAsync(dec_tokens_.as<int>() + last_slots[0], picks_.p, last_rows.size() * 4, cudaMemcpyDeviceToDevice, stream_));
             if (logits_last) {
                 rows_host.resize(last_rows.size() * (size_t)V);
                 copy_logits_to_host(rows_host.data(), last_rows.size());
@@ -1288,11 +1290,7 @@ void Session::prefill(const int32_t* tokens, const int32_t* seq_lens, int n_seqs
             TFFN_CUDA(cudaStreamSynchronize(stream_));
             for (size_t i = 0; i < last_rows.size(); ++i) {
                 if (next_tokens) next_tokens[last_slots[i]] = picks[i];
-                int32_t* one = pinned_i32(4);
-                one[0] = picks[i];
-                TFFN_CUDA(cudaMemcpyAsync(dec_tokens_.as<int>() + last_slots[i], one, 4, cudaMemcpyHostToDevice, stream_));
                 if (logits_last) memcpy(logits_last + (size_t)last_slots[i] * V, rows_host.data() + i * (size_t)V, (size_t)V * 4);
-                TFFN_CUDA(cudaStreamSynchronize(stream_));
             }
         } else {
             TFFN_CUDA(cudaStreamSynchronize(stream_));
@@ -1300,8 +1298,7 @@ void Session::prefill(const int32_t* tokens, const int32_t* seq_lens, int n_seqs
     }
     for (int s = 0; s < n_seqs; ++s) h_seq_len_[s] += seq_lens[s];
     TFFN_CUDA(cudaMemcpyAsync(seq_len_dev_.p, h_seq_len_.data(), (size_t)max_batch_ * 4, cudaMemcpyHostToDevice, stream_));
-    TFFN_CUDA(cudaStreamSynchronize(stream_));
-    check_status();
+    check_status();  // waits for the stream
 }
 
 void Session::forward(int slot, const int32_t* tokens, int T, float* logits) {
@@ -1367,15 +1364,18 @@ void Session::decode_step(const int32_t* tokens_in, int n_seqs, int32_t* next_to
     const int V = m_->cfg.vocab_size;
     for (int s = 0; s < n_seqs; ++s) ensure_pages(s, h_seq_len_[s] + 1);
     flush_tables();
-    int32_t* pin = pinned_i32((size_t)std::max(n_seqs, 4));
+    int32_t* pin = pinned_i32((size_t)kIoTokens + n_seqs);
     if (tokens_in) {
         for (int s = 0; s < n_seqs; ++s) {
             if (tokens_in[s] < 0 || tokens_in[s] >= V) throw Error(kErrInvalid, "token id out of range");
-            pin[s] = tokens_in[s];
+            pin[kIoTokens + s] = tokens_in[s];
         }
-        TFFN_CUDA(cudaMemcpyAsync(dec_tokens_.p, pin, (size_t)n_seqs * 4, cudaMemcpyHostToDevice, stream_));
+        for (int i = kIoCounter; i < kIoTokens; ++i) pin[i] = 0;
+        TFFN_CUDA(cudaMemcpyAsync(step_io_.as<int>() + kIoCounter, pin + kIoCounter, (size_t)(kIoTokens - kIoCounter + n_seqs) * 4,
+                                  cudaMemcpyHostToDevice, stream_));
+    } else {
+        TFFN_CUDA(cudaMemsetAsync(step_counter_.p, 0, 4, stream_));
     }
-    TFFN_CUDA(cudaMemsetAsync(step_counter_.p, 0, 4, stream_));
     ensure_ring(n_seqs);
     if (logits) ensure_logits(std::max<size_t>(256, n_seqs));
     if (sampling()) upload_draws((size_t)n_seqs);
@@ -1388,13 +1388,13 @@ void Session::decode_step(const int32_t* tokens_in, int n_seqs, int32_t* next_to
         store_logits_ = logits != nullptr || sampling();
         run_decode_batched(n_seqs, max_ctx);
     }
-    TFFN_CUDA(cudaMemcpyAsync(pin, dec_tokens_.p, (size_t)n_seqs * 4, cudaMemcpyDeviceToHost, stream_));
+    TFFN_CUDA(cudaMemcpyAsync(pin, step_io_.p, (size_t)(kIoTokens + n_seqs) * 4, cudaMemcpyDeviceToHost, stream_));
     if (logits) copy_logits_to_host(logits, (size_t)n_seqs);
     TFFN_CUDA(cudaStreamSynchronize(stream_));
     if (next_tokens)
-        for (int s = 0; s < n_seqs; ++s) next_tokens[s] = pin[s];
+        for (int s = 0; s < n_seqs; ++s) next_tokens[s] = pin[kIoTokens + s];
     for (int s = 0; s < n_seqs; ++s) h_seq_len_[s] += 1;
-    check_status();
+    fail_on_status(pin[0]);
 }
 
 void Session::decode_run(int n_seqs, int steps, int32_t* tokens_out) {

@@ -266,18 +266,23 @@ private:
     DeviceBuffer rope_cos_, rope_sin_;
 
     // token metadata and activations of the batched path
-    DeviceBuffer tokens_, tok_seq_, tok_pos_, row_idx_, picks_, identity_, dec_tokens_;
+    DeviceBuffer tokens_, tok_seq_, tok_pos_, row_idx_, picks_, identity_;
     DeviceBuffer grp_first_, grp_count_;  // prompt attention: groups of up to attn_group_tokens_ consecutive rows of one sequence
     int attn_group_tokens_ = 128;
     DeviceBuffer h_, xn_, q_, ctx_, act_b_, act_e_, xn_last_, logits_;
     size_t logits_rows_ = 0;
     DeviceBuffer attn_partials_, attn_counters_;
-    DeviceBuffer status_, out_ring_, step_counter_;
+    DeviceBuffer out_ring_;
+    // What the host gives a decode step and takes from it, side by side so that each way is one copy: status, step counter,
+    // tokens. The named buffers are views.
+    static constexpr int kIoCounter = 4, kIoTokens = 8;
+    DeviceBuffer step_io_, status_, step_counter_, dec_tokens_;
     int out_ring_cap_ = 0;
     int* h_status_ = nullptr;  // pinned
     int32_t* h_pinned_i32_ = nullptr;
     size_t h_pinned_cap_ = 0;
     PinnedI32 h_pinned_runs_;
+    PinnedI32 h_pinned_table_;  // the block tables on their way to the device
 
     // batch-1 path
     DeviceBuffer bs1_h_, bs1_acc_, bs1_q_, bs1_ctx_, bs1_tickets_, bs1_lm_val_, bs1_lm_idx_;
@@ -336,6 +341,7 @@ private:
     void launch_bs1_step(bool want_logits, bool pdl);
     Bs1Ctx bs1_ctx(bool want_logits) const;
     void check_status();
+    void fail_on_status(int st);
     int32_t* pinned_i32(size_t n);
 };
 
