@@ -14,8 +14,9 @@
 // latency of its loads, not by tensor throughput. q and P are fp32 in the reference; each enters the
 // MMA as a bf16 pair (hi + lo, 16 mantissa bits): hi in tile rows 0-7, lo in rows 8-15, so one MMA
 // yields both partial products in the same thread, which adds them. The softmax is the
-// online form in fp32, per 32- or 16-key block of a warp. Splits are merged by the last split to finish
-// (a ticket, no spinning), always in split order, so the result does not depend on scheduling.
+// online form in fp32, per 32- or 16-key block of a warp. Up to eight splits are a thread-block cluster and are merged through
+// distributed shared memory; more leave partial results and the last one to finish (a ticket, no spinning) merges them. Both in
+// split order, so the result does not depend on scheduling.
 #include "kernels.h"
 #include "ptx.cuh"
 #include "launch.h"
@@ -49,6 +50,7 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 }
 constexpr int kAttnCtaThreads = 256;  // 8 warps: each takes 16 keys of a 128-key stage
 constexpr int kAttnWarps = kAttnCtaThreads / 32;
+constexpr int kClusterSplits = 8;  // portable cluster size
 
 template <int HD>
 struct AttnCfg {
@@ -330,7 +332,10 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
     }
     __syncthreads();
     const int G_part = EXACT ? G_all : min(8, G_all);  // heads of a full part: the stride of the partial results
-    float* partial = ws + ((size_t)unit * splits + split) * (size_t)(G_part * (HD + 2));
+    // a split's merged result [head][HD + 2] = (max, sum, O): in the second stage buffer for the cluster, or in the workspace
+    const bool cluster = splits > 1 && splits <= kClusterSplits;
+    float* const mine = (float*)(smem + C::STAGE_BYTES);
+    float* partial = cluster ? mine : ws + ((size_t)unit * splits + split) * (size_t)(G_part * (HD + 2));
     bf16* ctx_tok = ctx + (size_t)t * (EXACT ? (int64_t)nh * HD : opt.ctx_ld) + (size_t)head0 * vdim;
     for (int idx = tid; idx < G * HD; idx += kAttnCtaThreads) {
         const int g = idx / HD, d = idx % HD;
@@ -355,6 +360,36 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
     if (bad) dev_fail(status, DEV_ERR_BOUNDS);
     ATTN_TRACE(6);
     if (splits == 1) {
+        if (tid == 0) tl_mark(tl, 2);
+        return;
+    }
+
+    if (cluster) {
+        cluster_sync_all();
+        // the outputs are shared out between the ranks; a split without keys has maximum kNegBig and weighs zero
+        for (int idx = split * kAttnCtaThreads + tid; idx < G * HD; idx += splits * kAttnCtaThreads) {
+            const int g = idx / HD, d = idx % HD;
+            const uint32_t row = smem_u32(mine) + (uint32_t)(g * (HD + 2)) * 4;
+            float mz[kClusterSplits], lz[kClusterSplits], az[kClusterSplits];
+#pragma unroll
+            for (int z = 0; z < kClusterSplits; ++z) {
+                const uint32_t from = map_shared_rank(row, (uint32_t)(z < splits ? z : 0));
+                mz[z] = z < splits ? ld_shared_cluster_f32(from) : kNegBig;
+                lz[z] = z < splits ? ld_shared_cluster_f32(from + 4) : 0.f;
+                az[z] = z < splits ? ld_shared_cluster_f32(from + 8 + 4 * d) : 0.f;
+            }
+            float M = kNegBig, L = 0.f, A = 0.f;
+#pragma unroll
+            for (int z = 0; z < kClusterSplits; ++z) M = fmaxf(M, mz[z]);
+#pragma unroll
+            for (int z = 0; z < kClusterSplits; ++z) {
+                const float w = __expf(mz[z] - M);
+                L += lz[z] * w;
+                A += az[z] * w;
+            }
+            if (d < vdim) ctx_tok[(size_t)g * vdim + d] = __float2bfloat16_rn(A / L);
+        }
+        cluster_sync_all();  // no rank leaves while its result is read
         if (tid == 0) tl_mark(tl, 2);
         return;
     }
@@ -516,8 +551,8 @@ template <int HD>
 void launch_hd(dim3 grid, cudaStream_t s, bool pdl, const float* q, const KvView& kv, int layer, const int* tok_seq,
                const int* tok_pos, bf16* ctx, int nh, int G, int splits, int early, const AttnOptions& opt, float* ws,
                int* counters, int* status, unsigned long long* tl, unsigned long long* trace) {
-    launch_k(exact(opt, kv, nh, HD) ? k_attn_decode<HD, true> : k_attn_decode<HD, false>, grid, dim3(kAttnCtaThreads), (size_t)AttnCfg<HD>::SMEM, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx,
-             nh, G, splits, early, opt, ws, counters, status, tl, trace);
+    launch_k_cluster(exact(opt, kv, nh, HD) ? k_attn_decode<HD, true> : k_attn_decode<HD, false>, grid, dim3(kAttnCtaThreads),
+             dim3(1, splits <= kClusterSplits ? splits : 1, 1), (size_t)AttnCfg<HD>::SMEM, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, splits, early, opt, ws, counters, status, tl, trace);
 }
 
 }  // namespace
@@ -554,28 +589,32 @@ int attn_prepare() {
     return e == cudaSuccess ? attn_prompt_prepare() : (int)e;
 }
 
-constexpr int kMinSplitRows = 1024;
+// fewest keys of a context split: of those merged within a cluster, and of more than eight
+constexpr int kMinClusterRows = 256, kMinSplitRows = 1024;
 
 int attention_splits(int T, int nh, int nkv, int hd, int max_ctx, const AttnWorkspace& ws, int num_sms) {
     // One CTA per SM is the target: a CTA holds 128 KB of K/V in flight and its eight warps keep up with
-    // what one SM can take in, and a launch without splits needs no merge (a partial write, a ticket and a
-    // second read-back cost 4 to 6 us per launch, measured with two and three splits). Splits are used only
-    // when there are fewer (token, kv head) units than half the SMs and the context is long: a split
-    // must save more key-loop time (about 0.5 us per 128-key stage) than the merge costs, so each split
-    // gets at least 1024 keys (batch 1 at a few hundred keys of context: 0.94 -> 0.82 ms per token
-    // without splits; halving the minimum for 128-wide heads gained 1.4 us per launch for 32 sequences on a
-    // quarter of the 7B shape's heads and cost batch 1 on the 1.5B shape 16 %: 576 -> 483 tok/s).
+    // what one SM can take in. Splits are used only when there are fewer (token, kv head) units than half the SMs. Up to
+    // eight are merged inside a cluster for about a microsecond, so they pay from two key-loop stages each (128 keys, about
+    // 0.5 us) on; more go through the workspace (a partial write, a ticket and a second read-back: 4 to 6 us), which pays
+    // only where eight splits would be very long.
     const int G = nh / nkv < 8 ? nh / nkv : 8;
     const int units = T * nkv * ((nh / nkv + 7) / 8);
     hd = hd <= 64 ? 64 : 128;  // columns of a partial result
     int splits = 1;
     if (units * 2 <= num_sms) {
-        splits = num_sms / units;
-        const int max_splits = (max_ctx + kMinSplitRows - 1) / kMinSplitRows;
-        if (splits > max_splits) splits = max_splits;
-        if (splits < 1) splits = 1;
-        while (splits > 1 && ((size_t)units * splits * G * (hd + 2) > ws.partial_floats || units > ws.num_counters))
-            --splits;
+        const int room = num_sms / units, parts = (max_ctx + kMinSplitRows - 1) / kMinSplitRows, many = room < parts ? room : parts;
+        if (many >= 2 * kClusterSplits && units <= ws.num_counters) {
+            splits = many;
+            while (splits > kClusterSplits && (size_t)units * splits * G * (hd + 2) > ws.partial_floats) --splits;
+        } else {
+            // A cluster lies within one GPC, whose last SMs it may leave over: 16 clusters of 8 ran in two waves (8 sequences of
+            // 2 048 tokens, 2 kv heads of 128: 19.3 us, 16 clusters of 4 12.4). So the larger ones get half of the chip, the
+            // others three quarters.
+            while (splits < kClusterSplits && splits * 2 * units <= (splits * 2 < kClusterSplits ? num_sms * 3 / 4 : num_sms / 2) &&
+                   max_ctx >= splits * 2 * kMinClusterRows)
+                splits *= 2;
+        }
     }
     return splits;
 }

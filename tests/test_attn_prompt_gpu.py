@@ -53,3 +53,19 @@ def test_pages_of_an_earlier_request(model_dirs):
     assert (got == want).all()
     for s in (used, fresh):
         s.free()
+
+
+# context splits that are a cluster: 2, 4 and 8 of them, sequences that leave most of them empty, chunks that end inside one
+@pytest.mark.parametrize("lens,chunk", [((511, 1), 0), ((1030, 1, 517), 0), ((2047, 2100), 700), ((300, 2049), 0)])
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (72, 128)])
+def test_decode_over_split_contexts(tmp_path_factory, lens, chunk, dim, vdim):
+    c = Case(tmp_path_factory.mktemp("m"), rafilix_config(64, 97, [attention_layer(14, 2, dim, vdim, chunk=chunk or 4096)]), qk_norm=2.0)
+    rows = [c.tokens(n + 2, seed=n) for n in lens]
+    s = c.session("bfloat16", max_batch=len(lens), max_seq=2112)
+    s.prefill([r[:-2] for r in rows])
+    got = [s.decode_step([r[k] for r in rows], want_logits=True)[1] for k in (-2, -1)]
+    for i, r in enumerate(rows):
+        want = c.expect(r)[0][-2:]
+        assert error(np.stack([g[i] for g in got]), want).max() <= LIMIT["bfloat16"], i
+    assert s.status() == 0
+    s.free()
