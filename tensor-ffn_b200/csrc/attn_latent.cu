@@ -15,7 +15,7 @@
 // Decoding (k_attn_latent_decode): one token's heads would leave most of those rows empty, so keys and value columns take
 // the long side instead, S^T[key, head] = K . Q^T and O^T[column, head] += K^T . P^T: all value columns in one CTA. P^T is
 // written to shared memory next to its lo part (twice the columns of one product). One CTA = 16 or 32 heads of a token x
-// one context split, the same seven warps (thread = key). Up to eight splits are a thread-block cluster and add up their rows through
+// one context split, the same seven warps (thread = key). Up to eight splits, or sixteen, are a thread-block cluster and add up their rows through
 // distributed shared memory; more leave partial rows and the last one to finish (a ticket, no waiting) adds them up. Both in
 // split order.
 //
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_attn_latent(const __grid_consta
 
 // ---------------------------------------------------------------------------------------------- decoding
 constexpr int kDecSoftmax = 128;           // threads of the softmax warps
-constexpr int kDecMaxSplits = 64, kClusterSplits = 8;
+constexpr int kDecMaxSplits = 64, kClusterSplits = 16;
 __host__ __device__ inline int partial_ld(int rank) { return (rank + 3) / 4 * 4 + 4; }  // floats of a split's partial row
 __device__ __forceinline__ void softmax_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ bool softmax_any(bool x) {
@@ -437,9 +437,10 @@ __device__ __forceinline__ bool softmax_any(bool x) {
 }
 
 // HP: heads of a tile (16 or 32). KEYS: keys of a tile, 64, or 32 (one page; half of the rows of S^T are not used) where rows
-// are so wide that the ring would hold too few tiles of 64.
+// are so wide that the ring would hold too few tiles of 64. With 16 heads half of an SM's registers are enough (a few spills),
+// so that a block fits beside one of the kernel before and starts under it.
 template <int HP, int KEYS>
-__global__ void __launch_bounds__(kThreads, 1) k_attn_latent_decode(const __grid_constant__ LatentDev p, uint32_t tmem_cols) {
+__global__ void __launch_bounds__(kThreads, HP == 16 ? 2 : 1) k_attn_latent_decode(const __grid_constant__ LatentDev p, uint32_t tmem_cols) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t k_full[kMaxStages], k_empty[kMaxStages], s_full[2], p_full[2], pv_done[2], q_full;
@@ -897,6 +898,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_attn_latent_decode(const __grid
 // how a launch is cut into tiles; stages == 0: does not fit
 struct LatentPlan {
     int part_heads, parts, tile_tokens, q_rows, slices, slice_cols, stages, smem, tmem_cols, keys;
+    int fixed, stage, out;  // decoding: bytes beside the ring, of a stage, that O^T needs in the ring's place
 };
 constexpr int kStaticSmem = 3072;  // room for the kernels' static shared memory
 
@@ -937,10 +939,11 @@ LatentPlan plan_decode(int rank, int rot, int heads) {
         if (l.tmem_cols > 512) continue;
         for (l.keys = TK; l.keys >= kPageTokens; l.keys /= 2) {
             // S^T always has 64 rows: with 32 keys its operand reaches a block past its own
-            const int stage = blocks * l.keys * 128, fixed = 1024 + blocks * hp * 128 + 2 * l.keys * 128 + (TK - l.keys) * 128;
-            l.stages = std::min(kMaxStages, (kSmemLimit - kStaticSmem - fixed) / stage);
-            const int out = hp * ((rank + 127) / 128 * 128 + 4) * 4;  // O^T passes through the ring
-            l.smem = fixed + std::max(l.stages * stage, out);
+            l.stage = blocks * l.keys * 128;
+            l.fixed = 1024 + blocks * hp * 128 + 2 * l.keys * 128 + (TK - l.keys) * 128;
+            l.stages = std::min(kMaxStages, (kSmemLimit - kStaticSmem - l.fixed) / l.stage);
+            l.out = hp * ((rank + 127) / 128 * 128 + 4) * 4;  // O^T passes through the ring
+            l.smem = l.fixed + std::max(l.stages * l.stage, l.out);
             if (l.stages >= (l.keys == TK ? 3 : 1) && l.smem <= kSmemLimit - kStaticSmem) return l;
         }
     }
@@ -954,17 +957,21 @@ bool attention_latent_supported(int rank, int rot, int heads) {
     return heads >= 1 && plan_decode(rank, rot, heads).stages >= 1 && plan_prompt(rank, rot, heads).stages >= 1;
 }
 
+// A cluster of sixteen needs nearly a whole GPC, so only one or two of them are asked for (one context of 3 000 rows of 576
+// columns, 16 heads: 33.0 us in eight splits, 30.2 in sixteen).
+static int widest_cluster(int units, int num_sms) { return units * kClusterSplits * 4 <= num_sms ? kClusterSplits : 8; }
+
 int attention_latent_splits(int rows, int rank, int rot, int heads, int max_ctx, const AttnWorkspace& ws, int num_sms) {
     const LatentPlan l = plan_decode(rank, rot, heads);
     const int units = rows * l.parts;
     int splits = 1;
     if (units * 2 <= num_sms) {
-        const int room = num_sms / units, many = std::min(std::min(room, max_ctx / kLatentSplitKeys), kDecMaxSplits);
-        if (many > kClusterSplits) {
+        const int room = num_sms / units, many = std::min(std::min(room, max_ctx / kLatentSplitKeys), kDecMaxSplits), widest = widest_cluster(units, num_sms);
+        if (many > widest) {
             splits = many;
-            while (splits > kClusterSplits && ((size_t)units * splits * l.part_heads * partial_ld(rank) > ws.partial_floats || units > ws.num_counters)) --splits;
+            while (splits > widest && ((size_t)units * splits * l.part_heads * partial_ld(rank) > ws.partial_floats || units > ws.num_counters)) --splits;
         } else {
-            while (splits < kClusterSplits && splits * 2 <= room && max_ctx / (splits * 2) >= kLatentClusterKeys) splits *= 2;
+            while (splits < widest && splits * 2 <= room && max_ctx / (splits * 2) >= kLatentClusterKeys) splits *= 2;
         }
     }
     return splits;
@@ -1016,11 +1023,20 @@ int launch_attention_latent(const LatentAttn& a, int T, int n_groups, int max_ct
     }
     p.splits = attention_latent_splits(T, a.rank, a.rot, a.heads, max_ctx, ws, num_sms);
     p.early = pdl && a.only_newest_row_fresh;
-    p.cluster = p.splits > 1 && p.splits <= kClusterSplits;
+    // A cluster starts once every CTA of it finds room, and what it fetches ahead of the previous kernel's end only helps if that
+    // is early: where a split has few tiles, a ring of three and half of the registers (see the kernel) leave room beside the
+    // blocks of the kernels before (one context of 3 000 rows of 576 columns: 30.2 us, with both 21.5; the ring alone gave nothing).
+    const int tiles = (max_ctx + p.splits * l.keys - 1) / (p.splits * l.keys);
+    int smem = l.smem;
+    if (tiles <= 8 && p.stages > 3) {
+        p.stages = 3;
+        smem = l.fixed + std::max(3 * l.stage, l.out);
+    }
+    p.cluster = p.splits > 1 && p.splits <= widest_cluster(T * l.parts, num_sms);
     const dim3 grid(T * l.parts, p.splits);
     const auto kernel = l.q_rows == 16 ? (l.keys == TK ? k_attn_latent_decode<16, TK> : k_attn_latent_decode<16, kPageTokens>)
                                        : (l.keys == TK ? k_attn_latent_decode<32, TK> : k_attn_latent_decode<32, kPageTokens>);
-    return (int)launch_k_cluster(kernel, grid, dim3(kThreads), dim3(1, p.cluster ? p.splits : 1), (size_t)l.smem, s, pdl, p, (uint32_t)l.tmem_cols);
+    return (int)launch_k_cluster(kernel, grid, dim3(kThreads), dim3(1, p.cluster ? p.splits : 1), (size_t)smem, s, pdl, p, (uint32_t)l.tmem_cols);
 }
 
 template <typename Kern>
@@ -1028,12 +1044,17 @@ static cudaError_t latent_attr(Kern k) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit - kStaticSmem);
     return e == cudaSuccess ? prefer_max_shared(k) : e;
 }
+template <typename Kern>
+static cudaError_t latent_decode_attr(Kern k) {
+    const cudaError_t e = latent_attr(k);
+    return e == cudaSuccess ? cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : e;
+}
 int attention_latent_prepare() {
     cudaError_t e = latent_attr(k_attn_latent);
-    if (e == cudaSuccess) e = latent_attr(k_attn_latent_decode<16, TK>);
-    if (e == cudaSuccess) e = latent_attr(k_attn_latent_decode<16, kPageTokens>);
-    if (e == cudaSuccess) e = latent_attr(k_attn_latent_decode<32, TK>);
-    if (e == cudaSuccess) e = latent_attr(k_attn_latent_decode<32, kPageTokens>);
+    if (e == cudaSuccess) e = latent_decode_attr(k_attn_latent_decode<16, TK>);
+    if (e == cudaSuccess) e = latent_decode_attr(k_attn_latent_decode<16, kPageTokens>);
+    if (e == cudaSuccess) e = latent_decode_attr(k_attn_latent_decode<32, TK>);
+    if (e == cudaSuccess) e = latent_decode_attr(k_attn_latent_decode<32, kPageTokens>);
     return (int)e;
 }
 
