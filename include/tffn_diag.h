@@ -47,6 +47,12 @@ int tffn_op_gemm_trace(int device, const uint16_t* X, const uint16_t* W, float* 
 int tffn_op_swiglu_bs1_trace(int device, const uint16_t* h_in, const uint16_t* norm_w, const uint16_t* packed_base,
                              const uint16_t* packed_expert, float expert_scale, float eps, int H, int I, uint16_t* h_out,
                              uint64_t* trace, int trace_ctas);
+/* How a decode step of n_seqs sequences, the longest with max_ctx tokens, cuts the contexts of its attention on a device of
+ * num_sms SMs (host arithmetic, no GPU): out[0] = blocks per (sequence, kv head), out[1] = 1 if they merge inside a
+ * thread-block cluster, 0 if through scratch_floats of workspace. resident[n], n = 1..8: clusters of n blocks that the device
+ * holds at once. No counterpart in the reference. */
+int tffn_attention_cut(int n_seqs, int heads, int kv_heads, int head_dim, int max_ctx, int num_sms, const int32_t* resident,
+                       int64_t scratch_floats, int32_t* out);
 
 #ifdef __cplusplus
 }

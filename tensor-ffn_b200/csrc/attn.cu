@@ -14,9 +14,9 @@
 // latency of its loads, not by tensor throughput. q and P are fp32 in the reference; each enters the
 // MMA as a bf16 pair (hi + lo, 16 mantissa bits): hi in tile rows 0-7, lo in rows 8-15, so one MMA
 // yields both partial products in the same thread, which adds them. The softmax is the
-// online form in fp32, per 32- or 16-key block of a warp. Up to eight splits are a thread-block cluster and are merged through
-// distributed shared memory; more leave partial results and the last one to finish (a ticket, no spinning) merges them. Both in
-// split order, so the result does not depend on scheduling.
+// online form in fp32, per 32- or 16-key block of a warp. Splits that are a thread-block cluster are merged through distributed
+// shared memory; others leave partial results and the last one to finish (a ticket, no spinning) merges them. Both in split order,
+// so the result does not depend on scheduling.
 #include "kernels.h"
 #include "ptx.cuh"
 #include "launch.h"
@@ -50,7 +50,6 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 }
 constexpr int kAttnCtaThreads = 256;  // 8 warps: each takes 16 keys of a 128-key stage
 constexpr int kAttnWarps = kAttnCtaThreads / 32;
-constexpr int kClusterSplits = 8;  // portable cluster size
 
 template <int HD>
 struct AttnCfg {
@@ -144,7 +143,7 @@ template <int HD, bool EXACT>
 __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __restrict__ q, KvView kv, int layer,
                                                               const int* __restrict__ tok_seq,
                                                               const int* __restrict__ tok_pos, bf16* __restrict__ ctx,
-                                                              int nh, int G_all, int splits, int early, AttnOptions opt,
+                                                              int nh, int G_all, int splits, int cluster, int early, AttnOptions opt,
                                                               float* __restrict__ ws, int* __restrict__ counters,
                                                               int* status, unsigned long long* tl,
                                                               unsigned long long* trace) {
@@ -333,7 +332,6 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
     __syncthreads();
     const int G_part = EXACT ? G_all : min(8, G_all);  // heads of a full part: the stride of the partial results
     // a split's merged result [head][HD + 2] = (max, sum, O): in the second stage buffer for the cluster, or in the workspace
-    const bool cluster = splits > 1 && splits <= kClusterSplits;
     float* const mine = (float*)(smem + C::STAGE_BYTES);
     float* partial = cluster ? mine : ws + ((size_t)unit * splits + split) * (size_t)(G_part * (HD + 2));
     bf16* ctx_tok = ctx + (size_t)t * (EXACT ? (int64_t)nh * HD : opt.ctx_ld) + (size_t)head0 * vdim;
@@ -370,9 +368,9 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
         for (int idx = split * kAttnCtaThreads + tid; idx < G * HD; idx += splits * kAttnCtaThreads) {
             const int g = idx / HD, d = idx % HD;
             const uint32_t row = smem_u32(mine) + (uint32_t)(g * (HD + 2)) * 4;
-            float mz[kClusterSplits], lz[kClusterSplits], az[kClusterSplits];
+            float mz[kAttnClusterSplits], lz[kAttnClusterSplits], az[kAttnClusterSplits];
 #pragma unroll
-            for (int z = 0; z < kClusterSplits; ++z) {
+            for (int z = 0; z < kAttnClusterSplits; ++z) {
                 const uint32_t from = map_shared_rank(row, (uint32_t)(z < splits ? z : 0));
                 mz[z] = z < splits ? ld_shared_cluster_f32(from) : kNegBig;
                 lz[z] = z < splits ? ld_shared_cluster_f32(from + 4) : 0.f;
@@ -380,9 +378,9 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
             }
             float M = kNegBig, L = 0.f, A = 0.f;
 #pragma unroll
-            for (int z = 0; z < kClusterSplits; ++z) M = fmaxf(M, mz[z]);
+            for (int z = 0; z < kAttnClusterSplits; ++z) M = fmaxf(M, mz[z]);
 #pragma unroll
-            for (int z = 0; z < kClusterSplits; ++z) {
+            for (int z = 0; z < kAttnClusterSplits; ++z) {
                 const float w = __expf(mz[z] - M);
                 L += lz[z] * w;
                 A += az[z] * w;
@@ -549,10 +547,11 @@ bool exact(const AttnOptions& o, const KvView& kv, int nh, int hd) {
 
 template <int HD>
 void launch_hd(dim3 grid, cudaStream_t s, bool pdl, const float* q, const KvView& kv, int layer, const int* tok_seq,
-               const int* tok_pos, bf16* ctx, int nh, int G, int splits, int early, const AttnOptions& opt, float* ws,
+               const int* tok_pos, bf16* ctx, int nh, int G, AttnCut cut, int early, const AttnOptions& opt, float* ws,
                int* counters, int* status, unsigned long long* tl, unsigned long long* trace) {
     launch_k_cluster(exact(opt, kv, nh, HD) ? k_attn_decode<HD, true> : k_attn_decode<HD, false>, grid, dim3(kAttnCtaThreads),
-             dim3(1, splits <= kClusterSplits ? splits : 1, 1), (size_t)AttnCfg<HD>::SMEM, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, splits, early, opt, ws, counters, status, tl, trace);
+             dim3(1, cut.cluster ? cut.splits : 1, 1), (size_t)AttnCfg<HD>::SMEM, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, cut.splits,
+             cut.cluster ? 1 : 0, early, opt, ws, counters, status, tl, trace);
 }
 
 }  // namespace
@@ -589,34 +588,59 @@ int attn_prepare() {
     return e == cudaSuccess ? attn_prompt_prepare() : (int)e;
 }
 
-// fewest keys of a context split: of those merged within a cluster, and of more than eight
-constexpr int kMinClusterRows = 256, kMinSplitRows = 1024;
-
-int attention_splits(int T, int nh, int nkv, int hd, int max_ctx, const AttnWorkspace& ws, int num_sms) {
-    // One CTA per SM is the target: a CTA holds 128 KB of K/V in flight and its eight warps keep up with
-    // what one SM can take in. Splits are used only when there are fewer (token, kv head) units than half the SMs. Up to
-    // eight are merged inside a cluster for about a microsecond, so they pay from two key-loop stages each (128 keys, about
-    // 0.5 us) on; more go through the workspace (a partial write, a ticket and a second read-back: 4 to 6 us), which pays
-    // only where eight splits would be very long.
-    const int G = nh / nkv < 8 ? nh / nkv : 8;
-    const int units = T * nkv * ((nh / nkv + 7) / 8);
-    hd = hd <= 64 ? 64 : 128;  // columns of a partial result
-    int splits = 1;
-    if (units * 2 <= num_sms) {
-        const int room = num_sms / units, parts = (max_ctx + kMinSplitRows - 1) / kMinSplitRows, many = room < parts ? room : parts;
-        if (many >= 2 * kClusterSplits && units <= ws.num_counters) {
-            splits = many;
-            while (splits > kClusterSplits && (size_t)units * splits * G * (hd + 2) > ws.partial_floats) --splits;
-        } else {
-            // A cluster lies within one GPC, whose last SMs it may leave over: 16 clusters of 8 ran in two waves (8 sequences of
-            // 2 048 tokens, 2 kv heads of 128: 19.3 us, 16 clusters of 4 12.4). So the larger ones get half of the chip, the
-            // others three quarters.
-            while (splits < kClusterSplits && splits * 2 * units <= (splits * 2 < kClusterSplits ? num_sms * 3 / 4 : num_sms / 2) &&
-                   max_ctx >= splits * 2 * kMinClusterRows)
-                splits *= 2;
-        }
+int attn_resident_clusters(int (&resident)[kAttnClusterSplits + 1]) {
+    for (int n = 1; n <= kAttnClusterSplits; ++n) {
+        cudaLaunchConfig_t cfg = cudaLaunchConfig_t{};
+        cfg.gridDim = dim3(1, n);
+        cfg.blockDim = dim3(kAttnCtaThreads);
+        cfg.dynamicSmemBytes = AttnCfg<64>::SMEM;  // the same for both widths
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.z = 1;
+        attr[0].val.clusterDim.y = n;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&resident[n], k_attn_decode<64, true>, &cfg);
+        if (e != cudaSuccess) return (int)e;
     }
-    return splits;
+    resident[0] = 0;
+    return 0;
+}
+
+// One CTA per SM: a CTA holds 128 KB of K/V in flight and its eight warps keep up with what one SM can take in. So a cut has to
+// fit the chip in one wave: clusters lie within one GPC and leave SMs over (16 units of eight splits where 15 such clusters fit:
+// 45 us a layer at 8 192 keys, six splits 37), which ws.resident knows; the workspace needs only SMs. Among those that fit, the
+// one of least time by what a sweep measured (2 to 74 units, 130 to 30 000 keys, both widths; microseconds): a stage of 128 keys
+// 0.75 (64 columns) or 1.0, a merge in a cluster 1.5 + 0.25 per split, a merge through the workspace (a partial write, a ticket
+// and a second read-back) 6.7 + 0.2 per split. More than 24 workspace splits gained nothing (2 units, 30 000 keys: 24 splits 39 us
+// a layer, 37 splits 41). The choice is at most 4 % off the fastest cut of any point of the sweep, 0.4 % on average. Power-of-two
+// clusters on three quarters of the chip were up to 66 % off (us a layer before and after, 128 columns: 10 units of 30 000 keys
+// 104 -> 68, 32 units 179 -> 108, 64 units of 8 192 keys 115 -> 79), the workspace alone 20 % (32 units of 2 048 keys 47 -> 39).
+AttnCut attention_cut(int T, int nh, int nkv, int hd, int max_ctx, const AttnWorkspace& ws, int num_sms) {
+    constexpr int kMaxWorkspaceSplits = 24, kStageRows = AttnCfg<64>::STAGE_ROWS;
+    const int G = nh / nkv < 8 ? nh / nkv : 8;
+    const long long units = (long long)T * nkv * ((nh / nkv + 7) / 8);
+    hd = hd <= 64 ? 64 : 128;  // columns of a partial result
+    AttnCut best{1, false};
+    if (units * 2 > num_sms) return best;
+    auto keys = [&](int splits) {  // what the stages of the longest split cost
+        int rows = (max_ctx + splits - 1) / splits;
+        rows = (rows + kPageTokens - 1) / kPageTokens * kPageTokens;
+        return (rows + kStageRows - 1) / kStageRows * (hd == 64 ? 0.75 : 1.0);
+    };
+    double least = keys(1);
+    auto consider = [&](int splits, bool cluster, double merge) {
+        const double us = keys(splits) + merge;
+        if (us < least) {
+            least = us;
+            best = {splits, cluster};
+        }
+    };
+    for (int n = 2; n <= kAttnClusterSplits; ++n)
+        if (units <= ws.resident[n]) consider(n, true, 1.5 + 0.25 * n);
+    const int n = (int)(num_sms / units < kMaxWorkspaceSplits ? num_sms / units : kMaxWorkspaceSplits);
+    if (units <= ws.num_counters && (size_t)units * n * G * (hd + 2) <= ws.partial_floats) consider(n, false, 6.7 + 0.2 * n);
+    return best;
 }
 
 void launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, bf16* ctx, int T,
@@ -628,11 +652,11 @@ void launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, 
     const int G = nh / kv.nkv;
     const int units = T * kv.nkv * ((G + 7) / 8);
     const int wide = kv.hd > kv.vd ? kv.hd : kv.vd;
-    const int splits = attention_splits(T, nh, kv.nkv, wide, max_ctx, ws, num_sms);
-    dim3 grid(units, splits);
-    if ((long long)units * splits > trace_ctas) trace = nullptr;
-    if (wide <= 64) launch_hd<64>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, splits, early, opt, ws.partials, ws.counters, status, tl, trace);
-    else if (wide <= 128) launch_hd<128>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, splits, early, opt, ws.partials, ws.counters, status, tl, trace);
+    const AttnCut cut = attention_cut(T, nh, kv.nkv, wide, max_ctx, ws, num_sms);
+    dim3 grid(units, cut.splits);
+    if ((long long)units * cut.splits > trace_ctas) trace = nullptr;
+    if (wide <= 64) launch_hd<64>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, cut, early, opt, ws.partials, ws.counters, status, tl, trace);
+    else if (wide <= 128) launch_hd<128>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, cut, early, opt, ws.partials, ws.counters, status, tl, trace);
 }
 
 void launch_attention_simt(const float* q, KvView kv, bool f32, const int* tok_seq, const int* tok_pos, void* ctx, int T, int nh,

@@ -532,6 +532,19 @@ int tffn_op_swiglu_bs1_trace(int device, const uint16_t* h_in, const uint16_t* n
     });
 }
 
+int tffn_attention_cut(int n_seqs, int heads, int kv_heads, int head_dim, int max_ctx, int num_sms, const int32_t* resident,
+                       int64_t scratch_floats, int32_t* out) {
+    return guard([&] {
+        need(n_seqs > 0 && kv_heads > 0 && heads >= kv_heads && head_dim > 0 && max_ctx > 0 && num_sms > 0 && resident && scratch_floats >= 0 && out,
+             "bad attention_cut arguments");
+        AttnWorkspace ws{nullptr, (size_t)scratch_floats, nullptr, 1 << 30, {}};
+        for (int n = 1; n <= kAttnClusterSplits; ++n) ws.resident[n] = resident[n];
+        const AttnCut cut = attention_cut(n_seqs, heads, kv_heads, head_dim, max_ctx, ws, num_sms);
+        out[0] = cut.splits;
+        out[1] = cut.cluster ? 1 : 0;
+    });
+}
+
 int tffn_op_wait_selftest(int device) {
     int st = 0;
     int rc = guard([&] {

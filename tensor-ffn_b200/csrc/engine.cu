@@ -341,6 +341,7 @@ Session::Session(const Model* m, const Expert* e, int max_batch, int max_seq, cu
 
     cuda_check((cudaError_t)gemm_prepare(), "gemm_prepare", __FILE__, __LINE__);
     cuda_check((cudaError_t)attn_prepare(), "attn_prepare", __FILE__, __LINE__);
+    cuda_check((cudaError_t)attn_resident_clusters(attn_resident_), "attn_resident_clusters", __FILE__, __LINE__);
     cuda_check((cudaError_t)rows_prepare(), "rows_prepare", __FILE__, __LINE__);
     cuda_check(prefer_max_shared(k_decode_advance), "carveout", __FILE__, __LINE__);
 }
@@ -487,6 +488,7 @@ AttnWorkspace Session::attn_ws() const {
     w.partial_floats = attn_partials_.bytes / 4;
     w.counters = attn_counters_.as<int>();
     w.num_counters = (int)(attn_counters_.bytes / 4);
+    memcpy(w.resident, attn_resident_, sizeof w.resident);
     return w;
 }
 

@@ -272,6 +272,7 @@ private:
     DeviceBuffer h_, xn_, q_, ctx_, act_b_, act_e_, xn_last_, logits_;
     size_t logits_rows_ = 0;
     DeviceBuffer attn_partials_, attn_counters_;
+    int attn_resident_[kAttnClusterSplits + 1] = {};
     DeviceBuffer out_ring_;
     // What the host gives a decode step and takes from it, side by side so that each way is one copy: status, step counter,
     // tokens. The named buffers are views.

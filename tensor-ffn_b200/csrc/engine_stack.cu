@@ -475,15 +475,14 @@ AttnOptions Session::attn_options(const LayerSpec& l) const {
 
 int Session::decode_graph_key(int n_seqs, int max_ctx) const {
     if (!st_) {
-        const Config& c = m_->cfg;
-        return attention_splits(n_seqs, c.num_heads, c.num_kv_heads, c.head_dim, max_ctx, attn_ws(), m_->num_sms);
+        return attention_cut(n_seqs, m_->nh, m_->nkv, m_->cfg.head_dim, max_ctx, attn_ws(), m_->num_sms).key();
     }
     int key = 0;  // at most 64 splits per layer; layers that see the same context agree, so one digit per distinct choice
     std::vector<int> seen;
     for (size_t i = 0; i < m_->stack.size(); ++i) {
         const LayerSpec& l = m_->stack[i].spec;
         if (l.mixer == Mixer::Attention)
-            seen.push_back(attention_splits(n_seqs, l.heads, l.kv_heads, (int)pad8(std::max(l.dim, l.vdim)), attn_ctx(l, max_ctx), attn_ws(), m_->num_sms));
+            seen.push_back(attention_cut(n_seqs, l.heads, l.kv_heads, (int)pad8(std::max(l.dim, l.vdim)), attn_ctx(l, max_ctx), attn_ws(), m_->num_sms).key());
         else if (l.mixer == Mixer::LatentAttention && st_->layers[i].tc)
             seen.push_back(attention_latent_splits(n_seqs, l.kv_rank, l.rot_dim, l.heads, max_ctx, attn_ws(), m_->num_sms));
     }

@@ -183,11 +183,13 @@ void launch_argmax(const float* logits, int R, int V, int* out, float* scratch, 
                    int num_counters, int num_sms, cudaStream_t s, bool pdl = false, unsigned long long* tl = nullptr);
 
 // ------------------------------------------------------------------ attention over the paged cache
+constexpr int kAttnClusterSplits = 8;  // portable cluster size
 struct AttnWorkspace {
     float* partials;  // [T*nkv][splits][G*(hd+2)]
     size_t partial_floats;
     int* counters;    // [T*nkv]
     int num_counters;
+    int resident[kAttnClusterSplits + 1];  // [n]: clusters of n decode attention blocks that the chip holds at once
 };
 // Which keys a query sees and how the scores are scaled, when it differs from the uniform layers' causal attention
 // over 1 / sqrt(hd).
@@ -204,8 +206,14 @@ struct AttnOptions {
 AttnOptions resolve_attn_options(AttnOptions o, const KvView& kv, int nh);
 // opt the attention kernels into their dynamic shared memory (once per device, outside stream capture)
 int attn_prepare();
-// context splits launch_attention will use (a CUDA-graph key: the grid depends on it)
-int attention_splits(int T, int nh, int nkv, int hd, int max_ctx, const AttnWorkspace& ws, int num_sms);
+int attn_resident_clusters(int (&resident)[kAttnClusterSplits + 1]);  // of the current device; after attn_prepare
+// how launch_attention cuts contexts: blocks per (token, kv head), merged inside a cluster or through the workspace
+struct AttnCut {
+    int splits;
+    bool cluster;
+    int key() const { return splits * 2 + (cluster ? 1 : 0); }  // of a captured step: the grid depends on it
+};
+AttnCut attention_cut(int T, int nh, int nkv, int hd, int max_ctx, const AttnWorkspace& ws, int num_sms);
 // whether the tensor-core kernels take this head geometry (else launch_attention_simt)
 inline bool attention_tc_supported(int hd, int vd) { return hd <= 128 && vd <= 128; }
 // One warp-per-key-group attention without tensor cores: any key size up to 2048 and value size up to 1024, bf16 or (f32) fp32 cache and

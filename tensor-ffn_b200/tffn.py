@@ -107,6 +107,7 @@ _SIGS = {
     "tffn_op_swiglu_bs1": (_i, [_i, _vp, _vp, _vp, _vp, _f, _f, _i, _i, _vp]),
     "tffn_op_swiglu_bs1_trace": (_i, [_i, _vp, _vp, _vp, _vp, _f, _f, _i, _i, _vp, _vp, _i]),
     "tffn_op_swiglu_bs1_noalloc": (_i, [_i, _vp, _vp, _vp, _vp, _f, _f, _i, _i, _vp]),
+    "tffn_attention_cut": (_i, [_i, _i, _i, _i, _i, _i, _vp, ctypes.c_int64, _vp]),
     "tffn_op_wait_selftest": (_i, [_i]),
     "tffn_op_tp_wait_selftest": (_i, [_i, _i]),
 }
@@ -475,6 +476,16 @@ class Session:
 
     def stream(self) -> int:
         return int(_L.tffn_session_stream(self._h) or 0)
+
+
+def attention_cut(n_seqs: int, heads: int, kv_heads: int, head_dim: int, max_ctx: int, num_sms: int, resident, scratch_floats: int = 8 << 20):
+    """blocks per (sequence, kv head) of a decode step's attention, and whether they merge inside a cluster (host arithmetic);
+    resident[n]: clusters of n blocks that the device holds at once"""
+    r = np.ascontiguousarray(resident, dtype=np.int32)
+    assert r.size == 9
+    out = np.zeros(2, dtype=np.int32)
+    _check(_L.tffn_attention_cut(n_seqs, heads, kv_heads, head_dim, max_ctx, num_sms, r.ctypes.data, scratch_floats, out.ctypes.data))
+    return int(out[0]), bool(out[1])
 
 
 def op_gemm(X: np.ndarray, W: np.ndarray, splits: int = 0, device: int = 0) -> np.ndarray:
