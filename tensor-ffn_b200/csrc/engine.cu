@@ -1052,7 +1052,7 @@ Bs1Ctx Session::bs1_ctx(bool want_logits) const {
     return x;
 }
 
-void Session::launch_bs1_step(bool want_logits, bool pdl) {
+void Session::launch_bs1_step(bool want_logits, int max_ctx, bool pdl) {
     const Config& c = m_->cfg;
     Bs1Ctx x = bs1_ctx(want_logits);
     const size_t acc_words = bs1_acc_words(c.hidden_size);
@@ -1080,7 +1080,7 @@ void Session::launch_bs1_step(bool want_logits, bool pdl) {
         launch_bs1_qkv(x, ly, m_->embed.as<bf16>(), kv_, l, l == 0, stream_, pdl && l > 0);
         prof_end();
         prof_begin(KC_ATTENTION);
-        launch_attention(x.q, kv_, l, identity_.as<int>(), seq_len_dev_.as<int>(), x.ctx, 1, c.num_heads, max_seq_, attn_ws(),
+        launch_attention(x.q, kv_, l, identity_.as<int>(), seq_len_dev_.as<int>(), x.ctx, 1, c.num_heads, max_ctx, attn_ws(),
                          m_->num_sms, status_.as<int>(), stream_, pdl, true, tl_next(KC_ATTENTION));
         prof_end();
         x.tl = tl_next(KC_BS1_OPROJ);
@@ -1105,29 +1105,11 @@ void Session::launch_bs1_step(bool want_logits, bool pdl) {
     launches_ += (uint64_t)c.num_layers * 4 + 1;
 }
 
-void Session::run_bs1(bool want_logits) {
-    if (launch_mode_ == 2 && !profile_) {
-        if (!bs1_graph_ || bs1_graph_logits_ != want_logits) {
-            if (bs1_graph_) {
-                cudaGraphExecDestroy(bs1_graph_);
-                bs1_graph_ = nullptr;
-            }
-            cudaGraph_t graph = nullptr;
-            const uint64_t before = launches_;
-            TFFN_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-            launch_bs1_step(want_logits, true);
-            cudaError_t ce = cudaStreamEndCapture(stream_, &graph);
-            launches_ = before;
-            TFFN_CUDA(ce);
-            TFFN_CUDA(cudaGraphInstantiate(&bs1_graph_, graph, 0));
-            cudaGraphDestroy(graph);
-            bs1_graph_logits_ = want_logits;
-        }
-        TFFN_CUDA(cudaGraphLaunch(bs1_graph_, stream_));
-        launches_ += (uint64_t)m_->cfg.num_layers * 4 + 1;
-    } else {
-        launch_bs1_step(want_logits, launch_mode_ >= 1);
-    }
+void Session::run_bs1(bool want_logits, int max_ctx) {
+    if (launch_mode_ == 2 && !profile_)
+        run_captured({0, decode_graph_key(1, max_ctx) * 2 + (want_logits ? 1 : 0)}, [&] { launch_bs1_step(want_logits, max_ctx, true); });
+    else
+        launch_bs1_step(want_logits, max_ctx, launch_mode_ >= 1);
     TFFN_CUDA(cudaGetLastError());
 }
 
@@ -1184,8 +1166,6 @@ int Session::timeline(int n_seqs, uint64_t* out, int max_launches, int trace_lau
 }
 
 void Session::drop_graphs() {
-    if (bs1_graph_) cudaGraphExecDestroy(bs1_graph_);
-    bs1_graph_ = nullptr;
     for (auto& kv : dec_graphs_) cudaGraphExecDestroy(kv.second.exec);
     dec_graphs_.clear();
 }
@@ -1204,7 +1184,11 @@ void Session::run_decode_batched(int n_seqs, int max_ctx) {
         body();
         return;
     }
-    const auto key = std::make_pair(n_seqs, decode_graph_key(n_seqs, max_ctx) * 2 + (store_logits_ ? 1 : 0));
+    run_captured({n_seqs, decode_graph_key(n_seqs, max_ctx) * 2 + (store_logits_ ? 1 : 0)}, body);
+}
+
+// the launches of `body` as a graph, captured when its key is new
+void Session::run_captured(std::pair<int, int> key, const std::function<void()>& body) {
     auto it = dec_graphs_.find(key);
     if (it == dec_graphs_.end()) {
         cudaGraph_t graph = nullptr;
@@ -1383,7 +1367,7 @@ void Session::decode_step(const int32_t* tokens_in, int n_seqs, int32_t* next_to
     if (sampling()) upload_draws((size_t)n_seqs);
     const bool bs1 = n_seqs == 1 && use_bs1_ && m_->bs1_ok && !sampling();  // the fused batch-1 LM head picks greedily
     if (bs1) {
-        run_bs1(logits != nullptr);
+        run_bs1(logits != nullptr, h_seq_len_[0] + 1);
     } else {
         int max_ctx = 1;
         for (int s = 0; s < n_seqs; ++s) max_ctx = std::max(max_ctx, h_seq_len_[s] + 1);
@@ -1412,7 +1396,7 @@ void Session::decode_run(int n_seqs, int steps, int32_t* tokens_out) {
     for (int s = 0; s < n_seqs; ++s) max_ctx = std::max(max_ctx, h_seq_len_[s] + steps);
     for (int it = 0; it < steps; ++it) {
         if (bs1) {
-            run_bs1(false);
+            run_bs1(false, h_seq_len_[0] + it + 1);
         } else {
             store_logits_ = sampling();  // a device-resident loop hands out tokens only; sampling reads the logits
             run_decode_batched(n_seqs, max_ctx);

@@ -5,6 +5,7 @@
 #include "host_io.h"
 #include "kernels.h"
 #include <cstdint>
+#include <functional>
 #include <map>
 #include <memory>
 #include <string>
@@ -287,9 +288,7 @@ private:
 
     // batch-1 path
     DeviceBuffer bs1_h_, bs1_acc_, bs1_q_, bs1_ctx_, bs1_tickets_, bs1_lm_val_, bs1_lm_idx_;
-    cudaGraphExec_t bs1_graph_ = nullptr;
-    bool bs1_graph_logits_ = false;
-    // batched decode steps captured per (sequences, attention splits)
+    // decode steps captured per (sequences, 0: the batch-1 path; attention splits and whether logits are stored)
     struct DecGraph { cudaGraphExec_t exec; uint64_t launches; };
     std::map<std::pair<int, int>, DecGraph> dec_graphs_;
     void run_decode_batched(int n_seqs, int max_ctx);
@@ -338,8 +337,9 @@ private:
     // groups for launch_attention_prefill from the rows' (slot, position) lists; fills pin[0..2*n) and returns n
     // (runs of consecutive positions of one sequence, at most `limit` rows each)
     static int build_groups(const int* seq, const int* pos, int T, int limit, int32_t* first, int32_t* count);
-    void run_bs1(bool want_logits);
-    void launch_bs1_step(bool want_logits, bool pdl);
+    void run_bs1(bool want_logits, int max_ctx);
+    void launch_bs1_step(bool want_logits, int max_ctx, bool pdl);
+    void run_captured(std::pair<int, int> key, const std::function<void()>& body);
     Bs1Ctx bs1_ctx(bool want_logits) const;
     void check_status();
     void fail_on_status(int st);

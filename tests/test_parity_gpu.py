@@ -249,6 +249,32 @@ def test_long_context_attention_splits(model_dirs):
     assert rel_err(got["batched"], got["3 splits"]) <= KERNEL_TOL
 
 
+def test_step_does_not_depend_on_the_session_limit(model_dirs):
+    """a batch-1 step cuts its context by the context, not by what the session could hold: the same bits and picks"""
+    import synth
+    import tffn
+    d, ep, cfg = model_dirs["tiny"]
+    m = tffn.qwen_load(d)
+    e = tffn.checkpoint_load(ep, m, 0.1)
+    prompt = synth.prompts(1, 600, 5, cfg["vocab_size"])[0]
+    runs = {}
+    for mode in (1, 2):
+        for limit in (1024, 20480):
+            s = tffn.Session(m, e, max_batch=1, max_seq=limit)
+            s.set_launch_mode(mode)
+            s.prefill([prompt[:130]])
+            short = s.decode_step(prompt[130:131], want_logits=True)[1][0].copy()
+            s.prefill([prompt[131:500]])
+            picks = s.decode_run(1, 40)  # over the context at which a second cut is chosen
+            last = s.decode_step(prompt[599:], want_logits=True)[1][0].copy()
+            assert s.status() == 0 and s.seq_len(0) == 541
+            runs[mode, limit] = short, picks, last
+            s.free()
+    want = runs[1, 1024]
+    for key, got in runs.items():
+        assert all(np.array_equal(a, b) for a, b in zip(got, want)), key
+
+
 def test_forward_without_logits_leaves_the_greedy_pick(model_dirs):
     """tffn_forward(logits = NULL) followed by tffn_decode_step(tokens_in = NULL) feeds the greedy pick
     of the last forwarded row, exactly as when the logits were asked for"""
