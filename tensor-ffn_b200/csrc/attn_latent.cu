@@ -961,20 +961,29 @@ bool attention_latent_supported(int rank, int rot, int heads) {
 // columns, 16 heads: 33.0 us in eight splits, 30.2 in sixteen).
 static int widest_cluster(int units, int num_sms) { return units * kClusterSplits * 4 <= num_sms ? kClusterSplits : 8; }
 
-int attention_latent_splits(int rows, int rank, int rot, int heads, int max_ctx, const AttnWorkspace& ws, int num_sms) {
+LatentCut attention_latent_cut(int rows, int rank, int rot, int heads, int max_ctx, const AttnWorkspace& ws, int num_sms) {
     const LatentPlan l = plan_decode(rank, rot, heads);
+    LatentCut c{1, false, l.stages};
+    if (l.stages < 1) return c;
     const int units = rows * l.parts;
-    int splits = 1;
     if (units * 2 <= num_sms) {
         const int room = num_sms / units, many = std::min(std::min(room, max_ctx / kLatentSplitKeys), kDecMaxSplits), widest = widest_cluster(units, num_sms);
         if (many > widest) {
-            splits = many;
-            while (splits > widest && ((size_t)units * splits * l.part_heads * partial_ld(rank) > ws.partial_floats || units > ws.num_counters)) --splits;
+            c.splits = many;
+            while (c.splits > widest && ((size_t)units * c.splits * l.part_heads * partial_ld(rank) > ws.partial_floats || units > ws.num_counters)) --c.splits;
         } else {
-            while (splits < widest && splits * 2 <= room && max_ctx / (splits * 2) >= kLatentClusterKeys) splits *= 2;
+            while (c.splits < widest && c.splits * 2 <= room && max_ctx / (c.splits * 2) >= kLatentClusterKeys) c.splits *= 2;
         }
+        c.cluster = c.splits > 1 && c.splits <= widest;
     }
-    return splits;
+    // A cluster starts once every CTA of it finds room, and what it fetches ahead of the previous kernel's end only helps if that
+    // is early: where a split has few tiles, a ring of three and half of the registers (see the kernel) leave room beside the
+    // blocks of the kernels before (one context of 3 000 rows of 576 columns: 30.2 us, with both 21.5; the ring alone gave nothing;
+    // a step of four such layers and one context of 8 400 rows, nine tiles a split: 564 -> 534 us). Many tiles want the deep ring
+    // (64 sequences of 3 000 rows of 288 columns, 24 tiles: 611 -> 587 us a step).
+    const int tiles = (max_ctx + c.splits * l.keys - 1) / (c.splits * l.keys);
+    if (tiles <= 8 || c.splits == kClusterSplits) c.stages = std::min(c.stages, 3);
+    return c;
 }
 
 int launch_attention_latent(const LatentAttn& a, int T, int n_groups, int max_ctx, const AttnWorkspace& ws, int num_sms, TmapCache* tmaps,
@@ -1021,18 +1030,12 @@ int launch_attention_latent(const LatentAttn& a, int T, int n_groups, int max_ct
         p.subs = (8 + l.tile_tokens - 1) / l.tile_tokens;
         return (int)launch_k(k_attn_latent, dim3(n_groups * p.subs * l.parts * l.slices), dim3(kThreads), (size_t)l.smem, s, pdl, p);
     }
-    p.splits = attention_latent_splits(T, a.rank, a.rot, a.heads, max_ctx, ws, num_sms);
+    const LatentCut cut = attention_latent_cut(T, a.rank, a.rot, a.heads, max_ctx, ws, num_sms);
+    p.splits = cut.splits;
+    p.cluster = cut.cluster;
+    p.stages = cut.stages;
     p.early = pdl && a.only_newest_row_fresh;
-    // A cluster starts once every CTA of it finds room, and what it fetches ahead of the previous kernel's end only helps if that
-    // is early: where a split has few tiles, a ring of three and half of the registers (see the kernel) leave room beside the
-    // blocks of the kernels before (one context of 3 000 rows of 576 columns: 30.2 us, with both 21.5; the ring alone gave nothing).
-    const int tiles = (max_ctx + p.splits * l.keys - 1) / (p.splits * l.keys);
-    int smem = l.smem;
-    if (tiles <= 8 && p.stages > 3) {
-        p.stages = 3;
-        smem = l.fixed + std::max(3 * l.stage, l.out);
-    }
-    p.cluster = p.splits > 1 && p.splits <= widest_cluster(T * l.parts, num_sms);
+    const int smem = l.fixed + std::max(p.stages * l.stage, l.out);
     const dim3 grid(T * l.parts, p.splits);
     const auto kernel = l.q_rows == 16 ? (l.keys == TK ? k_attn_latent_decode<16, TK> : k_attn_latent_decode<16, kPageTokens>)
                                        : (l.keys == TK ? k_attn_latent_decode<32, TK> : k_attn_latent_decode<32, kPageTokens>);

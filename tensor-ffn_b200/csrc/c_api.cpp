@@ -545,6 +545,19 @@ int tffn_attention_cut(int n_seqs, int heads, int kv_heads, int head_dim, int ma
     });
 }
 
+int tffn_latent_attention_cut(int n_seqs, int heads, int kv_rank, int rot, int max_ctx, int num_sms, int64_t scratch_floats, int32_t* out) {
+    return guard([&] {
+        need(n_seqs > 0 && heads > 0 && kv_rank > 0 && rot > 0 && max_ctx > 0 && num_sms > 0 && scratch_floats >= 0 && out, "bad latent_attention_cut arguments");
+        if (!attention_latent_supported(kv_rank, rot, heads)) throw Error(kErrUnsupported, "rows too wide for the latent attention kernels");
+        const AttnWorkspace ws{nullptr, (size_t)scratch_floats, nullptr, 1 << 30, {}};
+        const LatentCut cut = attention_latent_cut(n_seqs, kv_rank, rot, heads, max_ctx, ws, num_sms);
+        out[0] = cut.splits;
+        out[1] = cut.cluster ? 1 : 0;
+        out[2] = cut.stages;
+        out[3] = cut.key();
+    });
+}
+
 int tffn_op_wait_selftest(int device) {
     int st = 0;
     int rc = guard([&] {

@@ -1107,7 +1107,7 @@ void Session::launch_bs1_step(bool want_logits, int max_ctx, bool pdl) {
 
 void Session::run_bs1(bool want_logits, int max_ctx) {
     if (launch_mode_ == 2 && !profile_)
-        run_captured({0, decode_graph_key(1, max_ctx) * 2 + (want_logits ? 1 : 0)}, [&] { launch_bs1_step(want_logits, max_ctx, true); });
+        run_captured(0, want_logits, max_ctx, [&] { launch_bs1_step(want_logits, max_ctx, true); });
     else
         launch_bs1_step(want_logits, max_ctx, launch_mode_ >= 1);
     TFFN_CUDA(cudaGetLastError());
@@ -1184,11 +1184,13 @@ void Session::run_decode_batched(int n_seqs, int max_ctx) {
         body();
         return;
     }
-    run_captured({n_seqs, decode_graph_key(n_seqs, max_ctx) * 2 + (store_logits_ ? 1 : 0)}, body);
+    run_captured(n_seqs, store_logits_, max_ctx, body);
 }
 
 // the launches of `body` as a graph, captured when its key is new
-void Session::run_captured(std::pair<int, int> key, const std::function<void()>& body) {
+void Session::run_captured(int n_seqs, bool logits, int max_ctx, const std::function<void()>& body) {
+    std::vector<int> key = decode_cuts(std::max(n_seqs, 1), max_ctx);
+    key.push_back(n_seqs * 2 + (logits ? 1 : 0));
     auto it = dec_graphs_.find(key);
     if (it == dec_graphs_.end()) {
         cudaGraph_t graph = nullptr;

@@ -288,9 +288,9 @@ private:
 
     // batch-1 path
     DeviceBuffer bs1_h_, bs1_acc_, bs1_q_, bs1_ctx_, bs1_tickets_, bs1_lm_val_, bs1_lm_idx_;
-    // decode steps captured per (sequences, 0: the batch-1 path; attention splits and whether logits are stored)
+    // decode steps captured per sequences (0: the batch-1 path), whether logits are stored, and the cuts of the attention layers
     struct DecGraph { cudaGraphExec_t exec; uint64_t launches; };
-    std::map<std::pair<int, int>, DecGraph> dec_graphs_;
+    std::map<std::vector<int>, DecGraph> dec_graphs_;
     void run_decode_batched(int n_seqs, int max_ctx);
     void drop_graphs();
 
@@ -318,7 +318,7 @@ private:
     int rope_table(const RopeSpec& spec);
     AttnOptions attn_options(const LayerSpec& l) const;
     // everything in a captured decode step's grids that depends on the context
-    int decode_graph_key(int n_seqs, int max_ctx) const;
+    std::vector<int> decode_cuts(int n_seqs, int max_ctx) const;  // keys of the attention layers' cuts
 
     void gemm(GemmCall& call, int cls, bool pdl);
     void lm_head(const void* x, int64_t ldx, int n_rows, bool decode, bool pdl);
@@ -339,7 +339,7 @@ private:
     static int build_groups(const int* seq, const int* pos, int T, int limit, int32_t* first, int32_t* count);
     void run_bs1(bool want_logits, int max_ctx);
     void launch_bs1_step(bool want_logits, int max_ctx, bool pdl);
-    void run_captured(std::pair<int, int> key, const std::function<void()>& body);
+    void run_captured(int n_seqs, bool logits, int max_ctx, const std::function<void()>& body);
     Bs1Ctx bs1_ctx(bool want_logits) const;
     void check_status();
     void fail_on_status(int st);

@@ -473,21 +473,17 @@ AttnOptions Session::attn_options(const LayerSpec& l) const {
     return o;
 }
 
-int Session::decode_graph_key(int n_seqs, int max_ctx) const {
-    if (!st_) {
-        return attention_cut(n_seqs, m_->nh, m_->nkv, m_->cfg.head_dim, max_ctx, attn_ws(), m_->num_sms).key();
-    }
-    int key = 0;  // at most 64 splits per layer; layers that see the same context agree, so one digit per distinct choice
-    std::vector<int> seen;
+std::vector<int> Session::decode_cuts(int n_seqs, int max_ctx) const {
+    if (!st_) return {attention_cut(n_seqs, m_->nh, m_->nkv, m_->cfg.head_dim, max_ctx, attn_ws(), m_->num_sms).key()};
+    std::vector<int> cuts;
     for (size_t i = 0; i < m_->stack.size(); ++i) {
         const LayerSpec& l = m_->stack[i].spec;
         if (l.mixer == Mixer::Attention)
-            seen.push_back(attention_cut(n_seqs, l.heads, l.kv_heads, (int)pad8(std::max(l.dim, l.vdim)), attn_ctx(l, max_ctx), attn_ws(), m_->num_sms).key());
+            cuts.push_back(attention_cut(n_seqs, l.heads, l.kv_heads, (int)pad8(std::max(l.dim, l.vdim)), attn_ctx(l, max_ctx), attn_ws(), m_->num_sms).key());
         else if (l.mixer == Mixer::LatentAttention && st_->layers[i].tc)
-            seen.push_back(attention_latent_splits(n_seqs, l.kv_rank, l.rot_dim, l.heads, max_ctx, attn_ws(), m_->num_sms));
+            cuts.push_back(attention_latent_cut(n_seqs, l.kv_rank, l.rot_dim, l.heads, max_ctx, attn_ws(), m_->num_sms).key());
     }
-    for (int sp : seen) key = (int)(((uint32_t)key * 257u + (uint32_t)sp) & 0x3fffffffu);
-    return key;
+    return cuts;
 }
 
 void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, Staged runs) {

@@ -349,7 +349,14 @@ struct LatentAttn {
 // fewest keys of a context split: of those that add up within a cluster, and of more than eight
 constexpr int kLatentClusterKeys = 128, kLatentSplitKeys = 512;
 bool attention_latent_supported(int rank, int rot, int heads);  // otherwise launch_attention_simt
-int attention_latent_splits(int rows, int rank, int rot, int heads, int max_ctx, const AttnWorkspace& ws, int num_sms);
+// how a decode launch cuts contexts: splits, merged inside a cluster or through the workspace, and stages of a block's ring
+struct LatentCut {
+    int splits;
+    bool cluster;
+    int stages;
+    int key() const { return (splits * 2 + (cluster ? 1 : 0)) * 16 + stages; }  // of a captured step: the launch depends on all three
+};
+LatentCut attention_latent_cut(int rows, int rank, int rot, int heads, int max_ctx, const AttnWorkspace& ws, int num_sms);
 // returns cudaError (launch) or -1000 if the tensor maps could not be encoded
 int launch_attention_latent(const LatentAttn& a, int T, int n_groups, int max_ctx, const AttnWorkspace& ws, int num_sms, TmapCache* tmaps,
                             cudaStream_t s, bool pdl, unsigned long long* tl = nullptr);

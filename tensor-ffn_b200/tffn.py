@@ -108,6 +108,7 @@ _SIGS = {
     "tffn_op_swiglu_bs1_trace": (_i, [_i, _vp, _vp, _vp, _vp, _f, _f, _i, _i, _vp, _vp, _i]),
     "tffn_op_swiglu_bs1_noalloc": (_i, [_i, _vp, _vp, _vp, _vp, _f, _f, _i, _i, _vp]),
     "tffn_attention_cut": (_i, [_i, _i, _i, _i, _i, _i, _vp, ctypes.c_int64, _vp]),
+    "tffn_latent_attention_cut": (_i, [_i, _i, _i, _i, _i, _i, ctypes.c_int64, _vp]),
     "tffn_op_wait_selftest": (_i, [_i]),
     "tffn_op_tp_wait_selftest": (_i, [_i, _i]),
 }
@@ -486,6 +487,13 @@ def attention_cut(n_seqs: int, heads: int, kv_heads: int, head_dim: int, max_ctx
     out = np.zeros(2, dtype=np.int32)
     _check(_L.tffn_attention_cut(n_seqs, heads, kv_heads, head_dim, max_ctx, num_sms, r.ctypes.data, scratch_floats, out.ctypes.data))
     return int(out[0]), bool(out[1])
+
+
+def latent_attention_cut(n_seqs: int, heads: int, kv_rank: int, rot: int, max_ctx: int, num_sms: int, scratch_floats: int = 8 << 20):
+    """(splits, whether they merge inside a cluster, ring stages, key of a captured step) of latent attention in a decode step"""
+    out = np.zeros(4, dtype=np.int32)
+    _check(_L.tffn_latent_attention_cut(n_seqs, heads, kv_rank, rot, max_ctx, num_sms, scratch_floats, out.ctypes.data))
+    return int(out[0]), bool(out[1]), int(out[2]), int(out[3])
 
 
 def op_gemm(X: np.ndarray, W: np.ndarray, splits: int = 0, device: int = 0) -> np.ndarray:

@@ -57,3 +57,13 @@ def test_cut_fits_the_device_and_its_scratch(units, ctx, scratch):
             assert 2 <= n <= 8 and units * parts <= RESIDENT[n]
         elif n > 1:
             assert units * parts * n * min(heads, 8) * (width + 2) <= scratch
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 16, 40, 64, 80])
+@pytest.mark.parametrize("heads,rank,rot", [(16, 512, 64), (14, 256, 32), (5, 72, 16), (40, 320, 32)])
+def test_latent_steps_are_keyed_by_all_that_their_launch_depends_on(n, heads, rank, rot):
+    """a step captured with one ring depth is not replayed where the rule asks for the other"""
+    import tffn
+    cuts = {tffn.latent_attention_cut(n, heads, rank, rot, ctx, 148) for ctx in list(range(1, 12000, 61)) + [32768]}
+    assert len({c[3] for c in cuts}) == len({c[:3] for c in cuts}) == len(cuts)
+    assert all(c[2] >= 1 and c[0] >= 1 and (not c[1] or c[0] in (2, 4, 8, 16)) for c in cuts)
