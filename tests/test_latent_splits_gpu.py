@@ -1,9 +1,9 @@
 """-m gpu: latent attention decode at the context lengths where its splits change: 2, 4, 8 and 16 of a cluster, the short ring of few
-tiles and the deep one, one and several sequences."""
+tiles and the deep one, one and several sequences; and where they go through the workspace."""
 import numpy as np
 import pytest
 
-from razesun_cases import LIMIT, Case, error, latent_layer, razesun_config
+from razesun_cases import LIMIT, Case, error, latent_layer, plant_key, razesun_config
 
 pytestmark = pytest.mark.gpu
 
@@ -18,5 +18,30 @@ def test_decode_over_split_contexts(tmp_path_factory, lens, rank, rot, heads):
     got = [s.decode_step([r[k] for r in rows], want_logits=True)[1] for k in (-2, -1)]
     for i, r in enumerate(rows):
         assert error(np.stack([g[i] for g in got]), c.expect(r, last=2)[0]).max() <= LIMIT["bfloat16"], i
+    assert s.status() == 0
+    s.free()
+
+
+# splits through the workspace: more than sixteen of one context, more than eight of four sequences' longest; a cluster of sixteen
+@pytest.mark.parametrize("lens,splits,cluster", [((9300,), 18, False), ((4750, 1, 1, 1), 9, False), ((4750,), 16, True)])
+def test_one_key_in_any_split(tmp_path, lens, splits, cluster):
+    """a key in the first, in a middle and in the last split that the last query alone asks for"""
+    import tffn
+    c, key, ask, other = plant_key(tmp_path)
+    for m in (layer["mixer"] for layer in c.cfg["layers"]):
+        assert tffn.latent_attention_cut(len(lens), m["heads"], m["kv_rank"], m["rot_dim"], lens[0], 148)[:2] == (splits, cluster)
+    filler = c.tokens(lens[0], seed=6)
+    filler[np.isin(filler, [key, ask])] = other
+    s = c.session("bfloat16", max_batch=len(lens), max_seq=lens[0] + 20)
+    for kpos in (3, lens[0] // 2, lens[0] - 50):
+        t = filler.copy()
+        t[kpos], t[-1] = key, ask
+        want = c.expect(t, last=1)[0]
+        s.qwen_reset()
+        s.prefill([t[:-1]] + [t[:1]] * (len(lens) - 1))
+        got = s.decode_step([t[-1]] + [other] * (len(lens) - 1), want_logits=True)[1][:1]
+        assert error(got, want).max() <= LIMIT["bfloat16"], kpos
+        t[kpos] = other
+        assert error(c.expect(t, last=1)[0], want)[0] > 3 * LIMIT["bfloat16"]  # the plant is seen
     assert s.status() == 0
     s.free()
