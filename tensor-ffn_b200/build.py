@@ -20,7 +20,7 @@ LIB_SOURCES = ["host_io.cpp", "c_api.cpp", "tp_comm.cpp", "engine.cu", "engine_s
                "rows.cu", "stack_rows.cu", "attn.cu", "attn_prompt.cu", "attn_latent.cu", "latent.cu", "delta.cu", "rglru.cu", "moe.cu", "decode_bs1.cu", "noalloc.cu"]
 CLI_SOURCES = ["cli_main.cpp"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-Xcompiler", "-fPIC,-Wall,-Wno-unused-function", "--expt-relaxed-constexpr"]
+              "-Xcompiler", "-fPIC,-Wall,-Wno-unused-function,-Werror=unused-result", "--expt-relaxed-constexpr"]
 
 
 NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"

@@ -546,10 +546,10 @@ bool exact(const AttnOptions& o, const KvView& kv, int nh, int hd) {
 }
 
 template <int HD>
-void launch_hd(dim3 grid, cudaStream_t s, bool pdl, const float* q, const KvView& kv, int layer, const int* tok_seq,
+cudaError_t launch_hd(dim3 grid, cudaStream_t s, bool pdl, const float* q, const KvView& kv, int layer, const int* tok_seq,
                const int* tok_pos, bf16* ctx, int nh, int G, AttnCut cut, int early, const AttnOptions& opt, float* ws,
                int* counters, int* status, unsigned long long* tl, unsigned long long* trace) {
-    launch_k_cluster(exact(opt, kv, nh, HD) ? k_attn_decode<HD, true> : k_attn_decode<HD, false>, grid, dim3(kAttnCtaThreads),
+    return launch_k_cluster(exact(opt, kv, nh, HD) ? k_attn_decode<HD, true> : k_attn_decode<HD, false>, grid, dim3(kAttnCtaThreads),
              dim3(1, cut.cluster ? cut.splits : 1, 1), (size_t)AttnCfg<HD>::SMEM, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, cut.splits,
              cut.cluster ? 1 : 0, early, opt, ws, counters, status, tl, trace);
 }
@@ -643,7 +643,7 @@ AttnCut attention_cut(int T, int nh, int nkv, int hd, int max_ctx, const AttnWor
     return best;
 }
 
-void launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, bf16* ctx, int T,
+int launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, bf16* ctx, int T,
                       int nh, int max_ctx, AttnWorkspace ws, int num_sms, int* status, cudaStream_t s, bool pdl,
                       bool only_newest_row_fresh, unsigned long long* tl, unsigned long long* trace, int trace_ctas,
                       const AttnOptions& options) {
@@ -655,8 +655,9 @@ void launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, 
     const AttnCut cut = attention_cut(T, nh, kv.nkv, wide, max_ctx, ws, num_sms);
     dim3 grid(units, cut.splits);
     if ((long long)units * cut.splits > trace_ctas) trace = nullptr;
-    if (wide <= 64) launch_hd<64>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, cut, early, opt, ws.partials, ws.counters, status, tl, trace);
-    else if (wide <= 128) launch_hd<128>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, cut, early, opt, ws.partials, ws.counters, status, tl, trace);
+    if (wide <= 64) return (int)launch_hd<64>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, cut, early, opt, ws.partials, ws.counters, status, tl, trace);
+    if (wide <= 128) return (int)launch_hd<128>(grid, s, pdl, q, kv, layer, tok_seq, tok_pos, ctx, nh, G, cut, early, opt, ws.partials, ws.counters, status, tl, trace);
+    return (int)cudaErrorInvalidValue;
 }
 
 void launch_attention_simt(const float* q, KvView kv, bool f32, const int* tok_seq, const int* tok_pos, void* ctx, int T, int nh,

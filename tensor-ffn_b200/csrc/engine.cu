@@ -931,9 +931,10 @@ void Session::run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool
         } else if (live(KC_ATTENTION)) {
             unsigned long long* tl = tl_next(KC_ATTENTION);
             const bool traced = tl_on_ && (int)tl_cls_.size() - 1 == tl_trace_launch_;
-            launch_attention(q_.as<float>(), kv_, l, tok_seq, tok_pos, ctx_.as<bf16>(), T, nh, max_ctx, attn_ws(), m_->num_sms,
-                             status, stream_, pdl, decode /* the step's first kernel (embed) is a full dependency */, tl,
-                             traced ? tl_trace_buf_.as<unsigned long long>() : nullptr, (int)(tl_trace_buf_.bytes / (16 * 8)));
+            check_launch(launch_attention(q_.as<float>(), kv_, l, tok_seq, tok_pos, ctx_.as<bf16>(), T, nh, max_ctx, attn_ws(), m_->num_sms,
+                                          status, stream_, pdl, decode /* the step's first kernel (embed) is a full dependency */, tl,
+                                          traced ? tl_trace_buf_.as<unsigned long long>() : nullptr, (int)(tl_trace_buf_.bytes / (16 * 8))),
+                         "attention launch");
         }
         prof_end();
         // o_proj + residual
@@ -1080,8 +1081,9 @@ void Session::launch_bs1_step(bool want_logits, int max_ctx, bool pdl) {
         launch_bs1_qkv(x, ly, m_->embed.as<bf16>(), kv_, l, l == 0, stream_, pdl && l > 0);
         prof_end();
         prof_begin(KC_ATTENTION);
-        launch_attention(x.q, kv_, l, identity_.as<int>(), seq_len_dev_.as<int>(), x.ctx, 1, c.num_heads, max_ctx, attn_ws(),
-                         m_->num_sms, status_.as<int>(), stream_, pdl, true, tl_next(KC_ATTENTION));
+        check_launch(launch_attention(x.q, kv_, l, identity_.as<int>(), seq_len_dev_.as<int>(), x.ctx, 1, c.num_heads, max_ctx, attn_ws(),
+                                      m_->num_sms, status_.as<int>(), stream_, pdl, true, tl_next(KC_ATTENTION)),
+                     "attention launch");
         prof_end();
         x.tl = tl_next(KC_BS1_OPROJ);
         prof_begin(KC_BS1_OPROJ);

@@ -622,8 +622,9 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
                                                           runs.n_groups, ctx_.as<bf16>(), sp.heads, m_->num_sms, status, tmaps_, stream_, pdl, tl, opt),
                                  "attention launch");
                 else
-                    launch_attention(q_.as<float>(), cache.kv, 0, tok_seq, tok_pos, ctx_.as<bf16>(), T, sp.heads, attn_ctx(sp, max_ctx),
-                                     attn_ws(), m_->num_sms, status, stream_, pdl, decode, tl, nullptr, 0, opt);
+                    check_launch(launch_attention(q_.as<float>(), cache.kv, 0, tok_seq, tok_pos, ctx_.as<bf16>(), T, sp.heads, attn_ctx(sp, max_ctx),
+                                                  attn_ws(), m_->num_sms, status, stream_, pdl, decode, tl, nullptr, 0, opt),
+                                 "attention launch");
             });
         } else if (sp.mixer == Mixer::LatentAttention) {
             const int kd = cache.kv.hd, rot_col = latent_rot_col(sp.kv_rank), dim8 = (int)pad8(sp.dim), rank8 = (int)pad8(sp.kv_rank);

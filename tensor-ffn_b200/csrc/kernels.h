@@ -117,15 +117,15 @@ struct GemmWorkspace {
 // opt the kernels into their dynamic shared memory sizes (once per device, outside stream capture)
 int gemm_prepare();
 // returns cudaError (launch) or -1000 if the tensor maps could not be encoded
-int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits = 0);
+[[nodiscard]] int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits = 0);
 // The same products in true fp32 (fp32 X and out, fp32 FMA, weights still bf16): modes STORE_F32, STORE_BF16, RELU2 and
 // SWIGLU (which then store fp32), grouped and batched launches included; two operand pairs only in a plain launch. The operands' X pointers
 // are fp32 arrays behind the bf16 type.
-int launch_gemm_f32(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream);
+[[nodiscard]] int launch_gemm_f32(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream);
 // the same products in tiles of 256 tokens x bn (128 or 256) weight rows over two CTAs; launch_gemm decides (no fused pick,
 // grouped launches with grp_bn 256)
 int gemm_pair_prepare();
-int launch_gemm_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int bn);
+[[nodiscard]] int launch_gemm_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int bn);
 
 // ------------------------------------------------------------------ row kernels of the batched path
 // (pdl: launch with programmatic dependent launch; every kernel here waits before reading its inputs)
@@ -224,7 +224,7 @@ void launch_attention_simt(const float* q, KvView kv, bool f32, const int* tok_s
 // only_newest_row_fresh (decode): of everything the kernel reads, only q and the cached row at
 // tok_pos[t] were written since the last kernel of the stream that was launched WITHOUT programmatic
 // dependent launch; the rest may then be fetched before the previous kernel has finished.
-void launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, bf16* ctx, int T,
+[[nodiscard]] int launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, bf16* ctx, int T,
                       int nh, int max_ctx, AttnWorkspace ws, int num_sms, int* status, cudaStream_t s, bool pdl = false,
                       bool only_newest_row_fresh = false, unsigned long long* tl = nullptr,
                       unsigned long long* trace = nullptr, int trace_ctas = 0,  // trace: 16 u64 per CTA, see attn.cu
@@ -239,7 +239,7 @@ inline int attention_group_tokens(int heads_per_kv) { return heads_per_kv < 128 
 // of a long context has a fifteenth of the blocks in tiles.
 inline bool attention_prompt_as_rows(int T, int nh, int nkv, int num_sms) { return T * nkv * ((nh / nkv + 7) / 8) <= num_sms; }
 int attn_prompt_prepare();
-int launch_attention_prefill(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, const int* grp_first,
+[[nodiscard]] int launch_attention_prefill(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, const int* grp_first,
                              const int* grp_count, int n_groups, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s,
                              bool pdl = false, unsigned long long* tl = nullptr, const AttnOptions& opt = AttnOptions());
 
@@ -358,7 +358,7 @@ struct LatentCut {
 };
 LatentCut attention_latent_cut(int rows, int rank, int rot, int heads, int max_ctx, const AttnWorkspace& ws, int num_sms);
 // returns cudaError (launch) or -1000 if the tensor maps could not be encoded
-int launch_attention_latent(const LatentAttn& a, int T, int n_groups, int max_ctx, const AttnWorkspace& ws, int num_sms, TmapCache* tmaps,
+[[nodiscard]] int launch_attention_latent(const LatentAttn& a, int T, int n_groups, int max_ctx, const AttnWorkspace& ws, int num_sms, TmapCache* tmaps,
                             cudaStream_t s, bool pdl, unsigned long long* tl = nullptr);
 int attention_latent_prepare();
 
