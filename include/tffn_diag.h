@@ -36,8 +36,10 @@ int tffn_session_timeline(tffn_session* s, int n_seqs, uint64_t* out, int max_la
 /* tffn_op_gemm, and additionally returns 64 device timestamps (globaltimer, ns) per CTA in trace[trace_ctas*64]
  * (CTA order: split-major, then token tile, then row tile): 0 start, 1 weight boxes requested,
  * 2 dependency wait over, 3 last MMA issued, 4 accumulator complete, 5 epilogue done, 6 cluster
- * barrier passed, 7 cluster reduction done, 8 end, 16+i pipeline stage i arrived. A profiling aid with
- * no counterpart in the reference. */
+ * barrier passed, 7 cluster reduction done, 8 end, 16+i pipeline stage i arrived. Launches of the two-CTA
+ * tiles (many tokens, splits 0) have the CTAs of a persistent grid of at most one per SM and stamps 0 to 5 and 8:
+ * 3 in the leading CTA of a pair, 4 for its first tile, 5 for its last. A profiling aid with no counterpart
+ * in the reference. */
 int tffn_op_gemm_trace(int device, const uint16_t* X, const uint16_t* W, float* out, int T, int N, int K, int splits,
                        uint64_t* trace, int trace_ctas);
 /* tffn_op_swiglu_bs1, and additionally returns 16 device timestamps (globaltimer, ns) per CTA of a second, warm

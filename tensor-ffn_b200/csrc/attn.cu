@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
     using C = AttnCfg<HD>;
     // optional per-CTA phase stamps (globaltimer ns), 16 per CTA: 0 entry, 1 token data read, 2 first
     // stages requested, 3 grid wait over, 4 first stage landed, 5 all keys processed, 6 partial result
-    // written, 7 ticket taken, 8 exit
+    // written, 7 ticket taken or the cluster's results there, 8 exit
 #define ATTN_TRACE(slot)                                                                              \
     do {                                                                                              \
         if (trace && threadIdx.x == 0) {                                                              \
@@ -364,6 +364,7 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
 
     if (cluster) {
         cluster_sync_all();
+        ATTN_TRACE(7);
         // the outputs are shared out between the ranks; a split without keys has maximum kNegBig and weighs zero
         for (int idx = split * kAttnCtaThreads + tid; idx < G * HD; idx += splits * kAttnCtaThreads) {
             const int g = idx / HD, d = idx % HD;
@@ -388,6 +389,7 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
             if (d < vdim) ctx_tok[(size_t)g * vdim + d] = __float2bfloat16_rn(A / L);
         }
         cluster_sync_all();  // no rank leaves while its result is read
+        ATTN_TRACE(8);
         if (tid == 0) tl_mark(tl, 2);
         return;
     }

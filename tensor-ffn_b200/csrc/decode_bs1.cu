@@ -29,11 +29,6 @@ using namespace bs1;
 
 constexpr int kRowWarps = 4;
 
-__device__ __forceinline__ unsigned long long gtime_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 // optional per-CTA phase timestamps (Bs1Ctx::trace, 16 u64 per CTA)
 #define BS1_TRACE(c, slot)                                                         \
     do {                                                                           \

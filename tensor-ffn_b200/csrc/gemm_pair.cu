@@ -47,9 +47,14 @@ struct PairDev {
     int* status;
     GemmQkvEpilogue qkv;
     unsigned long long* tl;
+    unsigned long long* trace;  // 64 phase stamps per CTA, as those of gemm_tc.cu
     int batch, out_batch;
     const GroupTile* grp;
 };
+#define TFFN_TRACE(slot)                                                       \
+    do {                                                                       \
+        if (p.trace) p.trace[(size_t)blockIdx.x * 64 + (slot)] = gtime_ns();   \
+    } while (0)
 
 // ------------------------------------------------------------------------------------------- cta_group::2 forms
 __device__ __forceinline__ void tmem_alloc2(uint32_t* smem_slot, uint32_t ncols) {
@@ -273,6 +278,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)cluster_ctarank();
     if (threadIdx.x == 0) {
+        TFFN_TRACE(0);
         tl_mark(p.tl, 0);
         for (int s = 0; s < Cfg::STAGES; ++s) {
             mbar_init(&full[s], 1);
@@ -289,6 +295,10 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
     if (p.grp) {  // an earlier kernel wrote the table; its unused entries are at the end
         pdl_wait();
         if (warp == 0) {
+            if (lane == 0) {
+                TFFN_TRACE(2);
+                tl_mark(p.tl, 1);
+            }
             int used = 0;
             for (int i = lane; i < p.m_tiles; i += 32) used += __ldcg(&p.grp[i].group) >= 0 ? 1 : 0;
             for (int o = 16; o > 0; o >>= 1) used += __shfl_xor_sync(0xffffffffu, used, o);
@@ -358,8 +368,13 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
                     if (rank == 0) mbar_arrive_expect_tx_elect(full_0 + kb * 8, 2 * Cfg::STAGE_BYTES);
                     load_w(w_map[seg], (kb - seg * p.kblocks[0]) * BK, kb);
                 }
+                if (lane == 0) TFFN_TRACE(1);
                 pdl_wait();
-                if (lane == 0) tl_mark(p.tl, 1);
+                if (lane == 0) {
+                    TFFN_TRACE(2);
+                    tl_mark(p.tl, 1);
+                }
+                __syncwarp();
                 waited = true;
             }
             int kb = 0;
@@ -413,6 +428,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
                 }
                 umma2_commit_elect(&acc_full[buf]);
             }
+            if (lane == 0) TFFN_TRACE(3);
         }
     } else {
         pdl_wait();
@@ -426,6 +442,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
             int pos = -1, pg = -1;
             if (MODE == GEMM_QKV) qkv_token(p, t0 + lane, x.t_end, pos, pg);
             if (!warp_wait(&acc_full[buf], (uint32_t)use & 1u, p.status, DEV_ERR_ACC_WAIT)) break;
+            if (threadIdx.x == 64 && n == 0) TFFN_TRACE(4);
+            __syncwarp();
             tc_fence_after();
             const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(dual ? 0 : buf * BN);
             if (t0 < x.t_end) {
@@ -485,11 +503,17 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(map_shared_rank(smem_u32(&acc_empty[buf]), 0));
         }
+        if (threadIdx.x == 64) TFFN_TRACE(5);
+        __syncwarp();
     }
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();  // no barrier or operand of the peer is needed any more
-    if (threadIdx.x == 64) tl_mark(p.tl, 2);
+    if (threadIdx.x == 64) {
+        TFFN_TRACE(8);
+        tl_mark(p.tl, 2);
+    }
+    __syncwarp();
     if (warp == 1) tmem_dealloc2(tmem_base, Cfg::TMEM_COLS);
 }
 
@@ -535,6 +559,7 @@ int launch_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream)
     if (c.mode == GEMM_QKV) p.qkv = *c.qkv;
     const long long tiles = (long long)p.m_tiles * p.n_tiles * p.nprob;
     const int pairs = (int)(tiles < ws.num_sms / 2 ? tiles : ws.num_sms / 2);
+    p.trace = 2 * pairs <= c.trace_ctas ? c.trace : nullptr;
     auto go = [&](auto kern) { return (int)launch_k_cluster(kern, dim3(2 * pairs), dim3(kPairThreads), dim3(2, 1, 1), PairCfg<BN>::SMEM, stream, c.pdl, p); };
     switch (c.mode) {
         case GEMM_STORE_F32: return go(k_gemm_pair<BN, GEMM_STORE_F32>);

@@ -6,7 +6,7 @@
 //
 // One CTA = one 128-row x BN-token output tile (optionally one K split of it), 6 warps:
 //   warp 0   TMA producer: 128x64 weight box + BNx64 activation box per stage, 128-byte swizzle
-//   warp 1   allocates TMEM, issues tcgen05.mma (one thread), commits stages back to the producer
+//   warp 1   allocates TMEM, issues tcgen05.mma (one elected lane), commits stages back to the producer
 //   warps 2-5 epilogue: tcgen05.ld the fp32 accumulators (lane = weight row, column = token),
 //            apply the epilogue and store. With split-K the splits of a tile are one thread-block
 //            cluster: partial tiles stay in shared memory and are summed across the cluster over
@@ -55,11 +55,6 @@ struct GemmDev {
     int* amax_idx;
 };
 
-__device__ __forceinline__ unsigned long long gtime_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 #define TFFN_TRACE(slot)                                                                                            \
     do {                                                                                                            \
         if (p.trace) p.trace[(size_t)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * 64 + (slot)] = gtime_ns(); \

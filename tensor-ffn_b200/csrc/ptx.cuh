@@ -135,12 +135,16 @@ __device__ __forceinline__ float ld_shared_cluster_f32(uint32_t addr) {
 }
 
 // ---------------------------------------------------------------- programmatic dependent launch
+__device__ __forceinline__ unsigned long long gtime_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
 // Step timeline (a diagnostic): six timestamps per launch — minimum and maximum over the CTAs of
 // kernel entry (which = 0), return from the grid-dependency wait (1) and exit (2). tl = nullptr: off.
 __device__ __forceinline__ void tl_mark(unsigned long long* tl, int which) {
     if (tl) {
-        unsigned long long t;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        const unsigned long long t = gtime_ns();
         atomicMin(tl + 2 * which, t);
         atomicMax(tl + 2 * which + 1, t);
     }

@@ -47,6 +47,23 @@ def test_timeline_reports_every_launch_in_order(model_dirs, mode):
     assert s.status() == 0
 
 
+@pytest.mark.parametrize("T,N,K", [(64, 1152, 896), (300, 1152, 896), (513, 4000, 200)])
+def test_gemm_trace_of_both_kinds_of_tiles(T, N, K):
+    """the stamps of a launch in single-CTA tiles (64 tokens) and in two-CTA tiles, and the product itself"""
+    import synth
+    import tffn
+    rng = np.random.default_rng(T)
+    X, W = (synth.f32_to_bf16(rng.standard_normal(n, dtype=np.float32)).reshape(n) for n in ((T, K), (N, K)))
+    got, tr = tffn.op_gemm_trace(X, W)
+    want = synth.bf16_to_f32(X).astype(np.float64) @ synth.bf16_to_f32(W).astype(np.float64).T
+    assert np.abs(got - want).max() <= 1e-4 * np.abs(want).max()  # fp32 sums of exact products
+    t = tr[tr[:, 0] > 0].astype(np.int64)
+    assert len(t) >= 2
+    for a, b in ((0, 1), (1, 2), (0, 4), (4, 5), (5, 8)):
+        live = (t[:, a] > 0) & (t[:, b] > 0)
+        assert live.any() and (t[live, a] <= t[live, b]).all(), (a, b)
+
+
 def test_ablation_is_timing_only_and_restores(model_dirs):
     m, e, s, prompts, cfg = _session(model_dirs)
     s.set_launch_mode(2)
