@@ -219,9 +219,9 @@ def test_peer_handshake_gives_up_when_the_peer_never_signals():
 
 
 def test_long_context_attention_splits(model_dirs):
-    """Contexts beyond 1024 keys make the batch-1 attention split the context over several CTAs and merge
-    the parts: 3 splits (single-pass merge) against the oracle, then 20 splits (generic merge) and the
-    batched tensor-core path (same attention kernel, one token) against the 3-split result."""
+    """A context of 2 100 keys makes the batch-1 attention split it over the CTAs of a cluster and merge the parts:
+    against the oracle, then in a session that could hold ten times as much and on the batched tensor-core path
+    (same attention kernel, one token) against that result. Merges through the workspace: test_attention_cut_gpu.py."""
     import synth
     import tffn
     import oracle
@@ -235,7 +235,7 @@ def test_long_context_attention_splits(model_dirs):
     m = tffn.qwen_load(d)
     e = tffn.checkpoint_load(ep, m, 0.1)
     got = {}
-    for label, max_seq, bs1 in (("3 splits", 2304, True), ("20 splits", 20480, True), ("batched", 2304, False)):
+    for label, max_seq, bs1 in (("batch 1", 2304, True), ("larger session", 20480, True), ("batched", 2304, False)):
         s = tffn.Session(m, e, max_batch=1, max_seq=max_seq)
         s.set_launch_mode(2)
         s.set_bs1_path(bs1)
@@ -244,9 +244,9 @@ def test_long_context_attention_splits(model_dirs):
         assert s.status() == 0, label
         assert s.seq_len(0) == P + steps
         s.free()
-    assert rel_err(got["3 splits"], ref) <= KERNEL_TOL
-    assert rel_err(got["20 splits"], got["3 splits"]) <= KERNEL_TOL
-    assert rel_err(got["batched"], got["3 splits"]) <= KERNEL_TOL
+    assert rel_err(got["batch 1"], ref) <= KERNEL_TOL
+    assert rel_err(got["larger session"], got["batch 1"]) <= KERNEL_TOL
+    assert rel_err(got["batched"], got["batch 1"]) <= KERNEL_TOL
 
 
 def test_step_does_not_depend_on_the_session_limit(model_dirs):
@@ -273,6 +273,29 @@ def test_step_does_not_depend_on_the_session_limit(model_dirs):
     want = runs[1, 1024]
     for key, got in runs.items():
         assert all(np.array_equal(a, b) for a, b in zip(got, want)), key
+
+
+def test_batch1_step_through_the_workspace(model_dirs):
+    """a context whose splits merge through the workspace, twice over the same counters: batch-1 path against the batched one"""
+    import synth
+    import tffn
+    from test_attention_cut_cpu import RESIDENT
+    d, ep, cfg = model_dirs["tiny"]
+    P = 20000
+    assert tffn.attention_cut(1, cfg["num_attention_heads"], cfg["num_key_value_heads"], 64, P, 148, RESIDENT) == (24, False)
+    toks = synth.prompts(1, P + 2, 78, cfg["vocab_size"])[0]
+    m = tffn.qwen_load(d)
+    e = tffn.checkpoint_load(ep, m, 0.1)
+    got = []
+    for bs1 in (True, False):
+        s = tffn.Session(m, e, max_batch=1, max_seq=P + 32)
+        s.set_launch_mode(2)
+        s.set_bs1_path(bs1)
+        s.prefill([toks[:P]])
+        got.append(np.array([s.decode_step([int(t)], want_logits=True)[1][0].copy() for t in toks[P:]]))
+        assert s.status() == 0
+        s.free()
+    assert rel_err(got[0], got[1]) <= KERNEL_TOL
 
 
 def test_forward_without_logits_leaves_the_greedy_pick(model_dirs):

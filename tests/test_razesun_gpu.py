@@ -160,8 +160,8 @@ def test_one_far_key(tmp_path, decoded, compute):
 
 
 def test_one_key_among_thousands(tmp_path):
-    """a context of more splits than a cluster holds: their rows go through the workspace; a key in the first, in the middle
-    and in the last of them"""
+    """a context in the sixteen splits of one cluster (more, through the workspace: test_latent_splits_gpu.py); a key in the first,
+    in the middle and in the last of them"""
     c, key, ask, other = plant_key(tmp_path)
     filler = c.tokens(4750, seed=6)
     filler[np.isin(filler, [key, ask])] = other
