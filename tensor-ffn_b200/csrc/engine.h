@@ -8,6 +8,7 @@
 #include <functional>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <random>
 #include <vector>
@@ -127,11 +128,26 @@ struct Expert {
     DeviceBuffer slab;  // the one allocation the layers' buffers are views of
     std::vector<FfnWeights> layers;
     uint64_t weight_bytes = 0;
+    Expert() = default;
+    Expert(const Expert&) = delete;
+    Expert& operator=(const Expert&) = delete;
+    ~Expert();
     static Expert* load(const Model* m, const std::string& path, float scale);
     // The trainer's expert_forward (trainer/src/model/ffn_expert.cu:151-175) on the inference kernels:
     // d_x device bf16 [layers][T][hidden] (the normalised FFN inputs of every layer), d_out device fp32
     // [layers][T][hidden] = scale * down(silu(gate x) * up x), scale = this expert's output scale.
     void forward_layers(const void* d_x, float* d_out, int T, cudaStream_t stream) const;
+
+private:
+    // what one forward_layers call works in; up to kKept of them stay with the expert between calls, one per thread that runs one
+    struct Scratch {
+        DeviceBuffer act, status;
+        int* h_status = nullptr;  // pinned
+        ~Scratch();
+    };
+    static constexpr size_t kKept = 2, kKeptBytes = (size_t)256 << 20;
+    mutable std::mutex mu_;
+    mutable std::vector<std::unique_ptr<Scratch>> kept_;
 };
 
 // kernel classes of the per-launch profile (tffn_session_profile_*)

@@ -49,6 +49,7 @@ struct PairDev {
     unsigned long long* tl;
     unsigned long long* trace;  // 64 phase stamps per CTA, as those of gemm_tc.cu
     int batch, out_batch;
+    int layers;  // > 1: problems are layers (GemmCall::layers), tmW 3-D (column, layer, row)
     const GroupTile* grp;
 };
 #define TFFN_TRACE(slot)                                                       \
@@ -350,10 +351,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
         bool waited = p.grp != nullptr, ok = true;
         for (int i = first; i < tiles && ok; i += stride) {
             const Tile x = tile_at(i);
-            const int map = p.batch > 1 ? 0 : x.prob * 2;
-            const int t = x.t0 + rank * kHalf, wr = halves ? x.w_row0 : x.w_row0 + rank * (BN / 2);
+            const bool layered = p.layers > 1;
+            const int map = p.batch > 1 || layered ? 0 : x.prob * 2;
+            const int t = x.t0 + rank * kHalf + (layered ? x.prob * p.T : 0), wr = halves ? x.w_row0 : x.w_row0 + rank * (BN / 2);
             auto load_w = [&](const CUtensorMap* tm, int k, int st) {
-                tma2_load_2d_elect(a_0 + st * Cfg::STAGE_BYTES + Cfg::A_BYTES, tm, k, wr, lead_0 + st * 8);
+                if (layered) tma2_load_3d_elect(a_0 + st * Cfg::STAGE_BYTES + Cfg::A_BYTES, tm, k, x.prob, wr, lead_0 + st * 8);
+                else tma2_load_2d_elect(a_0 + st * Cfg::STAGE_BYTES + Cfg::A_BYTES, tm, k, wr, lead_0 + st * 8);
             };
             auto load_x = [&](const CUtensorMap* tm, int k, int st) {
                 if (p.batch > 1) tma2_load_3d_elect(a_0 + st * Cfg::STAGE_BYTES, tm, k, x.prob, t, lead_0 + st * 8);
@@ -459,10 +462,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
                         qkv_pair(p, buf32, lane, t0, x.t_end, x.n0 + c, pos, pg, a, b);
                     }
                 } else {
-                    void* out = p.out[p.batch > 1 ? 0 : x.prob];
-                    if (p.batch > 1) {
-                        if (MODE == GEMM_STORE_F32) out = (float*)out + (size_t)x.prob * p.out_batch;
-                        else out = (bf16*)out + (size_t)x.prob * p.out_batch;
+                    const bool one_out = p.batch > 1 || p.layers > 1;
+                    void* out = p.out[one_out ? 0 : x.prob];
+                    if (one_out) {
+                        const size_t at = (size_t)x.prob * (p.batch > 1 ? (size_t)p.out_batch : (size_t)p.T * (size_t)p.ldo);
+                        if (MODE == GEMM_STORE_F32) out = (float*)out + at;
+                        else out = (bf16*)out + at;
                     }
                     const int cols = tile_n / 2;  // of this warp
 #pragma unroll 1
@@ -521,7 +526,10 @@ template <int BN>
 int launch_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream) {
     PairDev p;
     memset(&p, 0, sizeof p);
-    const bool halves = c.mode == GEMM_SWIGLU, batched = c.batch > 1;
+    const bool halves = c.mode == GEMM_SWIGLU, batched = c.batch > 1, layered = c.layers > 1;
+    if (layered && (batched || c.grp || c.out2 || c.mode == GEMM_QKV || c.mode == GEMM_RESIDUAL || c.w_layer % 8 || c.w_layer >> 32 ||
+                    (!halves && c.op[1].K > 0)))
+        return (int)cudaErrorInvalidValue;
     const int maps = c.out2 ? 2 : 1;
     for (int pr = 0; pr < maps; ++pr)
         for (int i = 0; i < 2; ++i) {
@@ -529,7 +537,9 @@ int launch_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream)
             if (pr == 0) p.kblocks[i] = o.K > 0 ? (o.K + BK - 1) / BK : 0;
             if (o.K <= 0) continue;
             const uint64_t w_rows = (uint64_t)c.N * (c.grp ? c.grp_count : batched ? c.batch : 1);
-            if (!make_tmap_2d(ws.tmaps, &p.tmW[pr * 2 + i], o.W, w_rows, (uint64_t)o.K, (uint64_t)o.ldw, BN / 2)) return -1000;
+            if (!make_tmap_2d(ws.tmaps, &p.tmW[pr * 2 + i], o.W, w_rows, (uint64_t)o.K, (uint64_t)o.ldw, BN / 2, layered ? (uint32_t)c.layers : 1u,
+                              (uint32_t)c.w_layer))
+                return -1000;
             if (!make_tmap_2d(ws.tmaps, &p.tmX[pr * 2 + i], o.X, (uint64_t)(c.x_rows_alloc > c.T ? c.x_rows_alloc : c.T), (uint64_t)o.K,
                               (uint64_t)o.ldx, kHalf, batched ? (uint32_t)c.batch : 1u, (uint32_t)c.x_batch))
                 return -1000;
@@ -543,7 +553,8 @@ int launch_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream)
     const int tile_n = halves ? BN / 2 : BN;
     p.batch = batched ? c.batch : 1;
     p.out_batch = batched ? c.out_batch : 0;
-    p.nprob = batched ? c.batch : maps;
+    p.layers = layered ? c.layers : 1;
+    p.nprob = batched ? c.batch : layered ? c.layers : maps;
     p.N = c.N;
     p.T = c.T;
     p.m_tiles = c.grp ? c.grp_tiles : (c.T + kPairTokens - 1) / kPairTokens;

@@ -866,6 +866,13 @@ int gemm_group_tile(int rows) {
     return bn;
 }
 
+// Width: a k-block costs a pair 0.34 us with 128 weight rows and 0.42 with 256 (0.34 while it has the chip to itself), a
+// tile about 1 us around them; whole waves of 74 pairs count.
+int cheaper_width(long long narrow, long long wide, int kb, int num_sms) {
+    const int pairs = num_sms / 2;
+    auto cost = [&](long long tiles, double us) { return (double)((tiles + pairs - 1) / pairs) * (kb * us + 1.0); };
+    return cost(narrow, 0.34) <= cost(wide, wide < pairs ? 0.34 : 0.42) ? 128 : 256;
+}
 // Which launches take the two-CTA tiles of gemm_pair.cu, and how wide (0: none). Measured back to back on one B200 against
 // the tiles of this file (us, here -> there): 4 096 tokens, K 896: q|k|v N 1152 87 -> 23, N 4864 gate|up of base and expert
 // 277 -> 118 (1.21 PFLOP/s); 2 048 tokens, K 3584, N 18944: 1 235 -> 726 (1.53 PFLOP/s).
@@ -875,8 +882,6 @@ int gemm_group_tile(int rows) {
 //    once they are about a quarter of the k-blocks in number, or nearly fill the chip (K 4864, N 896: 768 tokens 39 -> 29,
 //    512 tokens 21 -> 29; two pairs of that K: 1 000 tokens 49 -> 54, 2 048 tokens 80 -> 56).
 //  * One narrow row tile (a router) needs many tokens (K 896: 4 096 tokens 14 -> 8; K 2048: 768 tokens 9 -> 13).
-//  * Width: a k-block costs a pair 0.34 us with 128 weight rows and 0.42 with 256 (0.34 while it has the chip to itself), a
-//    tile about 1 us around them; whole waves of 74 pairs count.
 int pair_width(const GemmCall& c, const GemmWorkspace& ws) {
     if (c.amax_val || (!c.out && c.mode != GEMM_QKV) || (c.grp && c.grp_bn != 256)) return 0;
     const bool halves = c.mode == GEMM_SWIGLU, batched = c.batch > 1;
@@ -898,9 +903,16 @@ int pair_width(const GemmCall& c, const GemmWorkspace& ws) {
             return 0;
         }
     }
-    const int pairs = ws.num_sms / 2;
-    auto cost = [&](long long tiles, double us) { return (double)((tiles + pairs - 1) / pairs) * (kb * us + 1.0); };
-    return cost(narrow, 0.34) <= cost(wide, wide < pairs ? 0.34 : 0.42) ? 128 : 256;
+    return cheaper_width(narrow, wide, kb, ws.num_sms);
+}
+
+int launch_gemm_layers(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream) {
+    const bool halves = c.mode == GEMM_SWIGLU;
+    if (c.T <= 0 || c.N <= 0 || c.op[0].K <= 0 || !c.out || (halves && (c.op[0].K != c.op[1].K || c.op[0].X != c.op[1].X))) return (int)cudaErrorInvalidValue;
+    const long long rows = (long long)((c.T + 255) / 256) * (c.layers > 1 ? c.layers : 1);
+    const int wide_n = halves ? 128 : 256;
+    const int bn = cheaper_width(rows * ((c.N + wide_n / 2 - 1) / (wide_n / 2)), rows * ((c.N + wide_n - 1) / wide_n), (c.op[0].K + BK - 1) / BK, ws.num_sms);
+    return launch_gemm_pair(c, ws, stream, bn);
 }
 
 int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits) {

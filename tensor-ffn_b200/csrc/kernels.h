@@ -89,6 +89,10 @@ struct GemmCall {
     // N rows of W each (back to back in W), problem b reading columns [b * x_batch, b * x_batch + K) of X and writing
     // columns [b * out_batch, b * out_batch + N) of out. Modes STORE_F32 and STORE_BF16, op[0] only; x_batch a multiple of 8.
     int batch, x_batch, out_batch;
+    // The same product of `layers` > 1 layers whose matrices lie w_layer elements apart (launch_gemm_layers only): layer l reads
+    // rows [l * T, (l + 1) * T) of X and writes the same rows of out.
+    int layers;
+    int64_t w_layer;
 };
 struct GroupTile {
     int group;           // -1: this tile and all later ones are unused
@@ -118,6 +122,8 @@ struct GemmWorkspace {
 int gemm_prepare();
 // returns cudaError (launch) or -1000 if the tensor maps could not be encoded
 [[nodiscard]] int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits = 0);
+// one launch over independent layers: modes STORE_F32, STORE_BF16, SWIGLU, one operand pair
+[[nodiscard]] int launch_gemm_layers(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream);
 // The same products in true fp32 (fp32 X and out, fp32 FMA, weights still bf16): modes STORE_F32, STORE_BF16, RELU2 and
 // SWIGLU (which then store fp32), grouped and batched launches included; two operand pairs only in a plain launch. The operands' X pointers
 // are fp32 arrays behind the bf16 type.

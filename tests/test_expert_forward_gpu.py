@@ -40,3 +40,48 @@ def test_expert_forward_training_shaped(model_dirs, name, T):
     dout2 = torch.empty_like(dout)
     e.expert_forward(dx.data_ptr(), dout2.data_ptr(), T)
     assert torch.equal(dout, dout2)
+
+
+@pytest.mark.parametrize("name,T", [("tiny128", 1), ("mini05", 255), ("tiny", 257), ("mini05", 40000), ("mini05", 110500)])
+def test_expert_forward_layers_of_one_launch(model_dirs, name, T):
+    """the layers share launches, as many as their activations allow (here all of 2 or 3, then 2, then 1): rows around the tiles'
+    and the layers' ends against numpy; a second thread's call at the same time gives the same bits"""
+    import threading
+    import torch
+    import oracle
+    import synth
+    import tffn
+    d, ep, cfg = model_dirs[name]
+    H, I, L = cfg["hidden_size"], cfg["intermediate_size"], cfg["num_hidden_layers"]
+    m = tffn.qwen_load(d)
+    e = tffn.checkpoint_load(ep, m, 0.1)
+    g = torch.Generator("cuda").manual_seed(T)
+    dx = torch.randn((L, T, H), generator=g, device="cuda").to(torch.bfloat16)
+    outs = [torch.full((L, T, H), float("nan"), dtype=torch.float32, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    errors = []
+
+    def call(out):
+        try:
+            s = torch.cuda.Stream()
+            e.expert_forward(dx.data_ptr(), out.data_ptr(), T, s.cuda_stream)
+        except Exception as ex:  # noqa: BLE001
+            errors.append(ex)
+
+    threads = [threading.Thread(target=call, args=(o,)) for o in outs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    assert torch.equal(outs[0], outs[1])
+    rows = sorted({r for r in (0, 1, 127, 128, 254, 255, 256, T // 2, T - 2, T - 1) if 0 <= r < T})
+    x = dx.view(torch.int16)[:, rows].cpu().numpy().view(np.uint16)
+    got = outs[0][:, rows].cpu().numpy()
+    _, _, _, data = oracle.read_expert(ep)
+    for l in range(L):
+        w = [synth.f32_to_bf16(np.ascontiguousarray(data[l, k])) for k in range(3)]
+        ref = oracle.expert_forward_ref(x[l], w[0].reshape(I, H), w[1].reshape(I, H), w[2].reshape(H, I), 0.1)
+        scale = np.abs(ref).max()
+        assert np.abs(got[l] - ref).max() / scale <= 2e-2, (name, l)   # the bounds of the test above
+        assert np.abs(got[l] - ref).mean() / scale <= 1e-3, (name, l)
