@@ -213,10 +213,15 @@ __device__ __forceinline__ void mma_rows_dot(const uint8_t* row_lo, const uint8_
     d_hi = par ? (c[0][3] + c[1][3]) + (c[2][3] + c[3][3]) : (c[0][2] + c[1][2]) + (c[2][2] + c[3][2]);
 }
 
-// acc (two fp32 in one 64-bit register) += a * (lo, hi of a packed bf16 pair): one packed FMA
-__device__ __forceinline__ void axpy_bf16x2(unsigned long long& acc, unsigned long long a2, uint32_t w) {
+// a packed bf16 pair as two fp32 in one 64-bit register
+__device__ __forceinline__ unsigned long long unpack_bf16x2(uint32_t w) {
     unsigned long long v;
     asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(w << 16), "r"(w & 0xffff0000u));
+    return v;
+}
+// acc (two fp32 in one 64-bit register) += a * (lo, hi of a packed bf16 pair): one packed FMA
+__device__ __forceinline__ void axpy_bf16x2(unsigned long long& acc, unsigned long long a2, uint32_t w) {
+    const unsigned long long v = unpack_bf16x2(w);
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a2), "l"(v));
 }
 __device__ __forceinline__ unsigned long long splat_f32x2(float a) {

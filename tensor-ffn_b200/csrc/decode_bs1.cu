@@ -164,41 +164,42 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_bs1_oproj(Bs1Ctx c, Bs1Layer
 }
 
 // ------------------------------------------------------------------------------------------ fused SwiGLU
-// Consumer warps; warp kFfnWarps is the copy producer. A warp takes a chunk of up to four records at a time
-// (fewer when the ring is short, see the kernel).
-constexpr int kFfnWarps = 9;
-constexpr int kFfnThreads = (kFfnWarps + 1) * 32;
+// Warps of a CTA. Twelve at 120 registers (hidden 896) leave each SM sub-partition room for a warp of the next layer's q|k|v and
+// one of its o_proj kernel, which fetch their weights while this one runs.
+__host__ __device__ constexpr int ffn_warps(int nch) { return nch <= 4 ? 12 : 9; }
 constexpr int kSmsLeftToAttention = 4;
+// Measured per token, 0.5B shape with expert, us: ring at once 663, with 192 KB more per SM requested into L2 671; 86 KB at once and
+// the rest 7 000 cycles later 610 (5 000: 622, 9 000: 622; nothing at once and the rest after 5 000: 626). Without the expert 547, 515.
+constexpr size_t kAtOnceBytes = 86016;
+constexpr long long kPauseCycles = 6000;
 
 struct FfnSmem {
     int stages;
     size_t stage_bytes;
-    size_t ring_off, part_off, xs_off, bar_off, total;
+    size_t ring_off, part_off, bar_off, total;
 };
-// One stage holds one record of the base FFN and, next to it, the same record of the expert. Stages
-// are not tied to warps: the producer publishes how many records it has issued, and a consumer polls a
-// stage's barrier only once its record has been issued (see item_ready). The per-warp partial sums
-// reuse the ring once every record has been consumed.
+// One stage holds one record of the base FFN and, next to it, the same record of the expert. Record r goes to stage r % stages;
+// the first round is requested up front, each later record by the warp that has just read its stage's previous one. The per-warp
+// partial sums reuse the ring once every record has been consumed.
 __host__ __device__ inline FfnSmem ffn_smem_layout(int H, bool expert) {
     FfnSmem s;
     s.stage_bytes = (size_t)H * 2 * 3 * (expert ? 2 : 1);
-    const size_t part = (size_t)kFfnWarps * H * 4;
-    const size_t budget = 200 * 1024;
+    const size_t part = (size_t)ffn_warps((H / 8 + 31) / 32) * H * 4;
+    const size_t budget = 211 * 1024;
     int st = (int)(budget / s.stage_bytes);
-    if (st > 32) st = 32;
+    if (st > 40) st = 40;
     if (st < 8) st = 8;
     s.stages = st;
     s.ring_off = 0;
     s.part_off = 0;
     size_t ring = s.stage_bytes * st;
     if (ring < part) ring = part;
-    s.xs_off = (ring + 127) / 128 * 128;
-    s.bar_off = s.xs_off + ((size_t)H * 2 + 127) / 128 * 128;
-    s.total = s.bar_off + (size_t)st * 16 + 64;
+    s.bar_off = (ring + 127) / 128 * 128;
+    s.total = s.bar_off + (size_t)st * 12 + 64;
     return s;
 }
 
-// Bounded wait until the producer has issued item `q` (it publishes the count in shared memory). Only
+// Bounded wait until more than `q` items have been issued (whoever issues them publishes the count in shared memory). Only
 // then may a consumer poll the stage's barrier: a parity wait started before the stage's previous
 // occupant has even landed would see the phase before that one and report "complete".
 __device__ __forceinline__ bool item_issued(const int* s_issued, int q, int* status) {
@@ -213,81 +214,71 @@ __device__ __forceinline__ bool item_issued(const int* s_issued, int q, int* sta
 // act = bf16(silu(bf16(x.Wg)) * bf16(x.Wu)); out = act.Wd (fp32); expert identical, its fp32
 // result scaled by output_scale; ffn = base + expert in fp32; h = bf16(float(h) + ffn)
 // (inference/src/model/qwen.cu:422-447, inference/src/model/expert.cu:44-59).
-// A warp takes four records at a time: their gate and up rows (16 with the expert, 8 without) are the
-// rows of one tensor-core GEMV against the normalised activations; the down columns are then added with
-// packed fp32 FMAs into the warp's running sums for all H outputs.
-template <int NCH>
-__global__ void __launch_bounds__(kFfnThreads, 1) k_bs1_ffn(Bs1Ctx c, Bs1Layer ly) {
+// A warp takes one stage at a time: the dot products of its two (with the expert four) gate and up rows with the normalised
+// activations, which the lanes keep in registers, then the down columns added into the warp's running sums for all H outputs,
+// both as packed fp32 FMAs: as matrix x vector products of mma.sync
+// (half of whose rows stayed empty) the dots alone took 2.4 us of a layer's launch, 13.4 us in all; now 10.2.
+template <int NCH, bool EXPERT>
+__global__ void __launch_bounds__(ffn_warps(NCH) * 32, 1) k_bs1_ffn(Bs1Ctx c, Bs1Layer ly) {
+    constexpr int WARPS = ffn_warps(NCH), ROWS = EXPERT ? 4 : 2;
     extern __shared__ __align__(128) uint8_t smem[];
     const int H = c.H, I = c.I;
-    const bool expert = ly.ffn_expert != nullptr;
-    const FfnSmem L = ffn_smem_layout(H, expert);
+    const FfnSmem L = ffn_smem_layout(H, EXPERT);
     uint8_t* ring = smem + L.ring_off;
     float* part = (float*)(smem + L.part_off);
-    uint8_t* xs = smem + L.xs_off;
     uint64_t* full = (uint64_t*)(smem + L.bar_off);
-    uint64_t* empty = full + L.stages;
-    int* s_flag = (int*)(empty + L.stages);
-    int* s_issued = s_flag + 1;
+    int* s_round = (int*)(full + L.stages);  // per stage: how many records have been requested into it
+    int* s_go = s_round + L.stages;          // the dependency wait is over
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = gridDim.x;
     const int i0 = (int)(((long long)I * blockIdx.x) / G), i1 = (int)(((long long)I * (blockIdx.x + 1)) / G);
     const int nrec = i1 - i0;
-    const size_t rec_bytes = (size_t)H * 6;
+    const uint32_t rec_bytes = (uint32_t)H * 6;
     const int S = L.stages;
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < S; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
-        }
-        *s_issued = 0;
+    if (threadIdx.x < S) {
+        mbar_init(&full[threadIdx.x], 1);
+        s_round[threadIdx.x] = 1;
         fence_mbar_init();
     }
+    if (threadIdx.x == 0) *s_go = 0;
     __syncthreads();
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
         BS1_TRACE(c, 0);
         tl_mark(c.tl, 0);
     }
-
-    if (warp == kFfnWarps) {
-        // producer: the weights do not depend on the previous kernel, so no griddepcontrol.wait here
-        if (lane == 0) {
-            for (int r = 0; r < nrec; ++r) {
-                const int s = r % S;
-                const uint32_t ph = (uint32_t)(r / S) & 1u;
-                if (!mbar_wait(&empty[s], ph ^ 1u, c.status, DEV_ERR_EMPTY_WAIT)) break;
-                uint8_t* dst = ring + (size_t)s * L.stage_bytes;
-                mbar_arrive_expect_tx(&full[s], (uint32_t)L.stage_bytes);
-                __threadfence_block();
-                *(volatile int*)s_issued = r + 1;
-                bulk_g2s(dst, (const uint8_t*)ly.ffn_base + (size_t)(i0 + r) * rec_bytes, (uint32_t)rec_bytes, &full[s]);
-                if (expert)
-                    bulk_g2s(dst + rec_bytes, (const uint8_t*)ly.ffn_expert + (size_t)(i0 + r) * rec_bytes,
-                             (uint32_t)rec_bytes, &full[s]);
-            }
-        }
-        return;
-    }
-
-    // consumers: one warp waits for the previous kernel, the others follow through the CTA barrier
-    constexpr int NT = kFfnWarps * 32;
-    if (warp == 0) pdl_wait();
-    asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
-    {
-        RowRegs<NCH> xn;
-        rmsnorm_regs<NCH>(xn, c.h, ly.ffn_norm, H, c.eps, lane);
-        if (warp == 0) {
-#pragma unroll
-            for (int j = 0; j < NCH; ++j) {
-                const int ch = lane + 32 * j;
-                if (ch < (H >> 3)) ((uint4*)xs)[ch] = xn.v[j];
-            }
+    const uint8_t *base = (const uint8_t*)ly.ffn_base + (size_t)i0 * rec_bytes, *expert = (const uint8_t*)ly.ffn_expert + (size_t)i0 * rec_bytes;
+    auto request = [&](int r, int s) {  // one lane
+        uint8_t* dst = ring + (size_t)s * L.stage_bytes;
+        mbar_arrive_expect_tx(&full[s], (uint32_t)L.stage_bytes);
+        bulk_g2s(dst, base + (size_t)r * rec_bytes, rec_bytes, &full[s]);
+        if (EXPERT) bulk_g2s(dst + rec_bytes, expert + (size_t)r * rec_bytes, rec_bytes, &full[s]);
+    };
+    // The weights do not depend on the previous kernel, so no griddepcontrol.wait here. In a running step this block starts when
+    // the previous layer's leaves, just as the q|k|v kernel between them reads the activations: a whole ring (200 KB per SM)
+    // requested at once keeps it waiting, so all but the first records follow kPauseCycles later, or when they are needed.
+    if (lane == 0) {
+        const int round = min(S, nrec), now = c.paced ? min(round, (int)(kAtOnceBytes / L.stage_bytes)) : round;
+        const long long start = clock64();
+        for (int r = warp; r < now; r += WARPS) request(r, r);
+        if (warp > 0 && now + warp - 1 < round) {
+            while (clock64() - start < kPauseCycles && *(volatile int*)s_go == 0) __nanosleep(100);
+            for (int r = now + warp - 1; r < round; r += WARPS - 1) request(r, r);
         }
     }
+    __syncwarp();
+
+    // one warp waits for the previous kernel, the others follow through the CTA barrier
+    constexpr int NT = WARPS * 32;
+    if (warp == 0) {
+        pdl_wait();
+        if (lane == 0) *(volatile int*)s_go = 1;
+    }
     asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+    RowRegs<NCH> xn;
+    rmsnorm_regs<NCH>(xn, c.h, ly.ffn_norm, H, c.eps, lane);
     if (threadIdx.x == 0) {
         BS1_TRACE(c, 1);
         tl_mark(c.tl, 1);
@@ -295,92 +286,85 @@ __global__ void __launch_bounds__(kFfnThreads, 1) k_bs1_ffn(Bs1Ctx c, Bs1Layer l
     unsigned long long acc[NCH * 4];
 #pragma unroll
     for (int j = 0; j < NCH * 4; ++j) acc[j] = 0ull;
-    const size_t row_bytes = (size_t)H * 2;
-    const int g = lane >> 2;
-    // the MMA rows this lane loads: with the expert, row g = (record g / 4, {gate_b, up_b, gate_e, up_e}[g % 4])
-    // and row g + 8 the same of record 2 + g / 4; without it, row g = (record g / 2, {gate, up}[g % 2])
-    const int j_lo = expert ? (g >> 2) : (g >> 1), j_hi = 2 + (g >> 2);
-    const size_t koff = expert ? (size_t)(g & 1) * row_bytes + (size_t)((g >> 1) & 1) * rec_bytes : (size_t)(g & 1) * row_bytes;
-    // Records per chunk. The ring holds S consecutive records, so only S / CH chunks can be worked on at a
-    // time: with four records per chunk a ring of 19 stages (hidden 896) keeps fewer than five of the nine
-    // warps busy, one of 8 (hidden 2048) two. Smaller chunks use a part of the 16 MMA rows only (the unused
-    // rows repeat the chunk's last record and are dropped), which costs less than idle warps.
-    const int CH = S >= 4 * kFfnWarps ? 4 : (S >= 2 * kFfnWarps ? 2 : 1);
-    const int nchunks = (nrec + CH - 1) / CH;
+    const uint32_t row_bytes = (uint32_t)H * 2;
     const int nchunk16 = H >> 3;
-    bool ok = true;
-    for (int ch = warp; ch < nchunks && ok; ch += kFfnWarps) {
-        const int r0 = ch * CH, nr = min(CH, nrec - r0);
-        for (int j = 0; j < nr && ok; ++j) {
-            const int r = r0 + j;
-            ok = item_issued(s_issued, r, c.status) && mbar_wait(&full[r % S], (uint32_t)(r / S) & 1u, c.status, DEV_ERR_FULL_WAIT);
-        }
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        if (threadIdx.x == 0 && ch == 0) BS1_TRACE(c, 2);
-        // records past the end of this CTA's slice stand in as copies of the last one; their results are dropped
-        auto stage_of = [&](int j) { return ring + (size_t)((r0 + min(j, nr - 1)) % S) * L.stage_bytes; };
-        float v_lo, v_hi = 0.f;
-        // with the expert, chunks of one or two records fill the lower eight MMA rows only: the upper half then
-        // stays empty instead of loading copies
-        if (expert && CH > 2) mma_rows_dot<true>(stage_of(j_lo) + koff, stage_of(j_hi) + koff, H, xs, lane, v_lo, v_hi);
-        else mma_rows_dot<false>(stage_of(j_lo) + koff, nullptr, H, xs, lane, v_lo, v_hi);
-        // a gate row and its up row are neighbours in g: lane ^ 4
-        const float p_lo = __shfl_xor_sync(0xffffffffu, v_lo, 4), p_hi = __shfl_xor_sync(0xffffffffu, v_hi, 4);
-        const float a_lo = silu_mul_bf16(v_lo, p_lo), a_hi = silu_mul_bf16(v_hi, p_hi);  // meaningful where g is even
-        float act_b[4], act_e[4];
-        if (expert) {
-            act_b[0] = __shfl_sync(0xffffffffu, a_lo, 0);
-            act_e[0] = __shfl_sync(0xffffffffu, a_lo, 8);
-            act_b[1] = __shfl_sync(0xffffffffu, a_lo, 16);
-            act_e[1] = __shfl_sync(0xffffffffu, a_lo, 24);
-            act_b[2] = __shfl_sync(0xffffffffu, a_hi, 0);
-            act_e[2] = __shfl_sync(0xffffffffu, a_hi, 8);
-            act_b[3] = __shfl_sync(0xffffffffu, a_hi, 16);
-            act_e[3] = __shfl_sync(0xffffffffu, a_hi, 24);
-        } else {
+    int s = warp % S;
+    for (int r = warp; r < nrec; r += WARPS) {
+        const int round = r / S;
+        const bool ok = (round == 0 || item_issued(s_round + s, round, c.status)) && mbar_wait(&full[s], (uint32_t)round & 1u, c.status, DEV_ERR_FULL_WAIT);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        if (threadIdx.x == 0 && r == 0) BS1_TRACE(c, 2);
+        const uint8_t* st = ring + (size_t)s * L.stage_bytes;
+        unsigned long long dot[ROWS];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                act_b[j] = __shfl_sync(0xffffffffu, a_lo, 8 * j);
-                act_e[j] = 0.f;
+        for (int k = 0; k < ROWS; ++k) dot[k] = 0ull;
+#pragma unroll
+        for (int j = 0; j < NCH; ++j) {
+            const int c16 = lane + 32 * j;
+            if (c16 < nchunk16) {
+                uint4 w[ROWS];
+#pragma unroll
+                for (int k = 0; k < ROWS; ++k) w[k] = *(const uint4*)(st + (k >> 1) * rec_bytes + (k & 1) * row_bytes + c16 * 16);
+                const uint32_t x[4] = {xn.v[j].x, xn.v[j].y, xn.v[j].z, xn.v[j].w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const unsigned long long x2 = unpack_bf16x2(x[u]);
+#pragma unroll
+                    for (int k = 0; k < ROWS; ++k) axpy_bf16x2(dot[k], x2, u == 0 ? w[k].x : u == 1 ? w[k].y : u == 2 ? w[k].z : w[k].w);
+                }
             }
         }
+        // each half of the warp sums the rows of one record, each quarter one row: a gate row's sum ends up 8 lanes from its up row's
+        float v[ROWS];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (j < nr) {
-                const uint8_t* st = ring + (size_t)((r0 + j) % S) * L.stage_bytes;
-                const unsigned long long ab = splat_f32x2(act_b[j]);
-                const uint4* db = (const uint4*)(st + 2 * row_bytes);
+        for (int k = 0; k < ROWS; ++k) {
+            const float2 t = unpack_f32x2(dot[k]);
+            v[k] = t.x + t.y;
+        }
+        float g = v[0], u = v[1];
+        if (EXPERT) {
+            const bool up_half = lane & 16;
+            const float give_g = up_half ? v[0] : v[ROWS - 2], give_u = up_half ? v[1] : v[ROWS - 1];
+            g = (up_half ? v[ROWS - 2] : v[0]) + __shfl_xor_sync(0xffffffffu, give_g, 16);
+            u = (up_half ? v[ROWS - 1] : v[1]) + __shfl_xor_sync(0xffffffffu, give_u, 16);
+        } else {
+            g += __shfl_xor_sync(0xffffffffu, g, 16);
+            u += __shfl_xor_sync(0xffffffffu, u, 16);
+        }
+        float t = (lane & 8 ? u : g) + __shfl_xor_sync(0xffffffffu, lane & 8 ? g : u, 8);
+        t += __shfl_xor_sync(0xffffffffu, t, 4);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        const float other = __shfl_xor_sync(0xffffffffu, t, 8);
+        const float act = silu_mul_bf16(lane & 8 ? other : t, lane & 8 ? t : other);
+        const unsigned long long ab = splat_f32x2(__shfl_sync(0xffffffffu, act, 0));
+        const unsigned long long ae = splat_f32x2(EXPERT ? __shfl_sync(0xffffffffu, act, 16) * c.expert_scale : 0.f);
 #pragma unroll
-                for (int jj = 0; jj < NCH; ++jj) {
-                    const int c16 = lane + 32 * jj;
-                    if (c16 < nchunk16) {
-                        const uint4 d = db[c16];
-                        axpy_bf16x2(acc[jj * 4 + 0], ab, d.x);
-                        axpy_bf16x2(acc[jj * 4 + 1], ab, d.y);
-                        axpy_bf16x2(acc[jj * 4 + 2], ab, d.z);
-                        axpy_bf16x2(acc[jj * 4 + 3], ab, d.w);
-                    }
-                }
-                if (expert) {
-                    const unsigned long long ae = splat_f32x2(act_e[j] * c.expert_scale);
-                    const uint4* de = (const uint4*)(st + rec_bytes + 2 * row_bytes);
-#pragma unroll
-                    for (int jj = 0; jj < NCH; ++jj) {
-                        const int c16 = lane + 32 * jj;
-                        if (c16 < nchunk16) {
-                            const uint4 d = de[c16];
-                            axpy_bf16x2(acc[jj * 4 + 0], ae, d.x);
-                            axpy_bf16x2(acc[jj * 4 + 1], ae, d.y);
-                            axpy_bf16x2(acc[jj * 4 + 2], ae, d.z);
-                            axpy_bf16x2(acc[jj * 4 + 3], ae, d.w);
-                        }
-                    }
+        for (int j = 0; j < NCH; ++j) {
+            const int c16 = lane + 32 * j;
+            if (c16 < nchunk16) {
+                const uint4 d = *(const uint4*)(st + 2 * row_bytes + c16 * 16);
+                axpy_bf16x2(acc[j * 4 + 0], ab, d.x);
+                axpy_bf16x2(acc[j * 4 + 1], ab, d.y);
+                axpy_bf16x2(acc[j * 4 + 2], ab, d.z);
+                axpy_bf16x2(acc[j * 4 + 3], ab, d.w);
+                if (EXPERT) {
+                    const uint4 e = *(const uint4*)(st + rec_bytes + 2 * row_bytes + c16 * 16);
+                    axpy_bf16x2(acc[j * 4 + 0], ae, e.x);
+                    axpy_bf16x2(acc[j * 4 + 1], ae, e.y);
+                    axpy_bf16x2(acc[j * 4 + 2], ae, e.z);
+                    axpy_bf16x2(acc[j * 4 + 3], ae, e.w);
                 }
             }
         }
         __syncwarp();
-        if (lane < nr) mbar_arrive(&empty[(r0 + lane) % S]);
+        if (lane == 0 && r + S < nrec) {
+            request(r + S, s);
+            __threadfence_block();
+            *(volatile int*)(s_round + s) = round + 2;
+        }
+        s += WARPS;
+        while (s >= S) s -= S;
     }
     if (threadIdx.x == 0) BS1_TRACE(c, 3);
     // fold the consumer warps of this CTA (fixed order); the partial sums reuse the ring, so
@@ -404,10 +388,10 @@ __global__ void __launch_bounds__(kFfnThreads, 1) k_bs1_ffn(Bs1Ctx c, Bs1Layer l
     // next (the q|k|v kernel of the next layer, the LM head) adds the total in.
     unsigned long long* acc_out = (unsigned long long*)c.acc_out + (size_t)(blockIdx.x % kAccReplicas) * H;
     for (int col = threadIdx.x; col < H; col += NT) {
-        float s = 0.f;
+        float sum = 0.f;
 #pragma unroll
-        for (int w = 0; w < kFfnWarps; ++w) s += part[(size_t)w * H + col];
-        atomicAdd(acc_out + col, (unsigned long long)__float2ll_rn(s * kAccScale));
+        for (int w = 0; w < WARPS; ++w) sum += part[(size_t)w * H + col];
+        atomicAdd(acc_out + col, (unsigned long long)__float2ll_rn(sum * kAccScale));
     }
     if (threadIdx.x == 0) {
         BS1_TRACE(c, 4);
@@ -607,10 +591,12 @@ int bs1_prepare(int H, bool expert) {
     const size_t lm = lm_smem_layout(H).total;
     cudaError_t e1 = cudaSuccess, e2 = cudaSuccess;
     TFFN_NCH_SWITCH(H, {
-        e1 = cudaFuncSetAttribute(k_bs1_ffn<NCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ffn);
+        e1 = cudaFuncSetAttribute(k_bs1_ffn<NCH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ffn);
+        if (e1 == cudaSuccess) e1 = cudaFuncSetAttribute(k_bs1_ffn<NCH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ffn);
         e2 = cudaFuncSetAttribute(k_bs1_lmhead<NCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lm);
         // one carveout for every kernel of the step, so that they can be resident together
-        if (e1 == cudaSuccess) e1 = prefer_max_shared(k_bs1_ffn<NCH>);
+        if (e1 == cudaSuccess) e1 = prefer_max_shared(k_bs1_ffn<NCH, false>);
+        if (e1 == cudaSuccess) e1 = prefer_max_shared(k_bs1_ffn<NCH, true>);
         if (e1 == cudaSuccess) e1 = prefer_max_shared(k_bs1_qkv<NCH>);
         if (e1 == cudaSuccess) e1 = prefer_max_shared(k_bs1_oproj<NCH>);
         if (e2 == cudaSuccess) e2 = prefer_max_shared(k_bs1_lmhead<NCH>);
@@ -628,15 +614,18 @@ void launch_bs1_oproj(const Bs1Ctx& c, const Bs1Layer& ly, cudaStream_t s, bool 
     dim3 grid((c.H + kRowWarps * 2 - 1) / (kRowWarps * 2)), block(kRowWarps * 32);
     TFFN_NCH_SWITCH(c.H, launch_k(k_bs1_oproj<NCH>, grid, block, 0, s, pdl, c, ly));
 }
-void launch_bs1_ffn(const Bs1Ctx& c, const Bs1Layer& ly, cudaStream_t s, bool pdl) {
+void launch_bs1_ffn(const Bs1Ctx& ctx, const Bs1Layer& ly, cudaStream_t s, bool pdl) {
+    Bs1Ctx c = ctx;
+    c.paced = pdl ? 1 : 0;  // else it starts when the previous kernel has finished
     const FfnSmem L = ffn_smem_layout(c.H, ly.ffn_expert != nullptr);
     // Every kernel of a layer is resident at once (dependent launches). An attention CTA and an FFN CTA do
     // not fit on one SM together, so a grid of one CTA per SM would leave the CTAs that land behind the
     // attention's without their head start on the weight stream: keep a few SMs out of the grid.
     int G = c.num_sms > 32 ? c.num_sms - kSmsLeftToAttention : c.num_sms;
     if (G > c.I) G = c.I;
-    dim3 grid(G), block(kFfnThreads);
-    TFFN_NCH_SWITCH(c.H, launch_k(k_bs1_ffn<NCH>, grid, block, L.total, s, pdl, c, ly));
+    dim3 grid(G), block(ffn_warps(nch_of(c.H)) * 32);
+    if (ly.ffn_expert) TFFN_NCH_SWITCH(c.H, launch_k(k_bs1_ffn<NCH, true>, grid, block, L.total, s, pdl, c, ly))
+    else TFFN_NCH_SWITCH(c.H, launch_k(k_bs1_ffn<NCH, false>, grid, block, L.total, s, pdl, c, ly));
 }
 void launch_bs1_lmhead(const Bs1Ctx& c, const bf16* final_norm, const bf16* lm_head, cudaStream_t s, bool pdl) {
     const LmSmem L = lm_smem_layout(c.H);

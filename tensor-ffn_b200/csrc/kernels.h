@@ -518,6 +518,7 @@ struct Bs1Ctx {
     // 2 first record arrived, 3 last record consumed, 4 this CTA's sums added to acc_out
     unsigned long long* trace;
     unsigned long long* tl;  // optional 6 u64 of the step timeline for this launch (see tl_mark)
+    int paced;  // k_bs1_ffn: its weights are requested in two portions (see there)
 };
 bool bs1_supported(int H, int I, int hd, int nh, int nkv);
 // 64-bit words of one FFN accumulator: a few replicas (CTAs spread over them to thin out same-address

@@ -76,3 +76,25 @@ def test_fused_bs1_ffn_kernel(H, I, expert):
     assert np.abs(out - ref).mean() / scale <= 1.5e-3
     again = synth.bf16_to_f32(tffn.op_swiglu_bs1(h, w, pb, pe if expert else None, 0.1, 1e-6))
     assert (again == out).all()  # fixed reduction order
+
+
+# widths around what a lane holds (256 columns per piece; 12 warps up to 1 024, then 9), records around a ring's and a warp round's ends
+@pytest.mark.parametrize("H,I,expert", [(64, 3, True), (64, 7001, False), (1024, 1730, True), (1088, 1297, False), (1280, 1300, True),
+                                        (1792, 1153, False), (1920, 2000, True), (2048, 145, False)])
+def test_fused_bs1_ffn_kernel_edges(H, I, expert):
+    import synth
+    import tffn
+    rng = np.random.default_rng([H, I])
+    h = _rand_bf16(rng, (H,))
+    w = synth.f32_to_bf16(1.0 + 0.1 * rng.standard_normal(H, dtype=np.float32))
+    mats = [[_rand_bf16(rng, s, 0.02) for s in ((I, H), (I, H), (H, I))] for _ in range(2)]
+    pb, pe = tffn.pack_ffn(*mats[0]), tffn.pack_ffn(*mats[1])
+    out = synth.bf16_to_f32(tffn.op_swiglu_bs1(h, w, pb, pe if expert else None, 0.1, 1e-6))
+    ref = synth.bf16_to_f32(h).astype(np.float64) + _ffn_ref(h, w, *mats[0], 1e-6)
+    if expert:
+        ref = ref + 0.1 * _ffn_ref(h, w, *mats[1], 1e-6)
+    scale = np.abs(ref).max()
+    assert np.abs(out - ref).max() / scale <= 1e-2   # one bf16 ulp of the largest element is 0.8 %
+    assert np.abs(out - ref).mean() / scale <= 1.5e-3
+    again = synth.bf16_to_f32(tffn.op_swiglu_bs1(h, w, pb, pe if expert else None, 0.1, 1e-6))
+    assert (again == out).all()  # fixed reduction order
