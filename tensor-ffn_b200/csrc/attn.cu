@@ -21,6 +21,7 @@
 #include "ptx.cuh"
 #include "launch.h"
 #include "attn_core.cuh"
+#include <type_traits>
 
 namespace tffn {
 
@@ -470,8 +471,11 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
 }
 
 // Attention of one (query head, token) per block without tensor cores, for what the kernels above do not take: fp32
-// caches (a session that computes in fp32) and heads wider than 128. Every warp walks the visible keys with a stride
-// of kSimtWarps; the lanes share the dimensions of a key; exact exponentials; the warps merge at the end.
+// caches (a session that computes in fp32) and heads wider than 128. The lanes share the dimensions of a key; exact
+// exponentials; the warps merge at the end. Bound by the latency of a key's loads and sums, so k_attn_simt4 has KEYS
+// neighbouring keys (of one page) of a warp in flight at once, four columns per lane and load (14 heads on rows of
+// 320 columns, three sequences of about 155 keys: 34.6 -> 8.3 us a launch inside a step; 450 prompt rows 228 -> 128).
+// k_attn_simt, a key at a time, is for rows of more than 1 024 columns.
 constexpr int kSimtWarps = 8;
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(bf16 v) { return __bfloat162float(v); }
@@ -543,6 +547,130 @@ __global__ void __launch_bounds__(kSimtWarps * 32) k_attn_simt(const float* __re
     if (tid == 0) tl_mark(tl, 2);
 }
 
+__device__ __forceinline__ void load_cols4(const float* p, float (&v)[4]) {
+    const float4 q = __ldcg((const float4*)p);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void load_cols4(const bf16* p, float (&v)[4]) {
+    const uint2 q = __ldcg((const uint2*)p);
+    v[0] = bf16_lo(q.x); v[1] = bf16_hi(q.x); v[2] = bf16_lo(q.y); v[3] = bf16_hi(q.y);
+}
+// N: groups of four columns per lane, for rows (multiples of four wide) of up to 128 N columns. SAME: a key's row is its value as well
+constexpr int simt_keys(int n, bool same) { return n == 1 ? 8 : n == 4 ? (same ? 4 : 2) : same ? 2 : 1; }
+constexpr int simt_warps(int n) { return n <= 4 ? 16 : 8; }  // at most
+template <typename C, int N, bool SAME>
+__global__ void __launch_bounds__(simt_warps(N) * 32) k_attn_simt4(const float* __restrict__ q, KvView kv, const int* __restrict__ tok_seq,
+                                                                  const int* __restrict__ tok_pos, C* __restrict__ ctx, int nh, AttnOptions opt,
+                                                                  int* status, unsigned long long* tl) {
+    constexpr int KEYS = simt_keys(N, SAME);
+    static_assert(kPageTokens % KEYS == 0, "a group of keys lies in one page");
+    extern __shared__ float simt_smem[];  // [warp][vdim + 2]
+    if (threadIdx.x == 0) tl_mark(tl, 0);
+    pdl_launch_dependents();
+    pdl_wait();
+    if (threadIdx.x == 0) tl_mark(tl, 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    const int head = blockIdx.x, t = blockIdx.y;
+    const int kvh = head / (nh / kv.nkv), kd = kv.hd, vd = kv.vd, vdim = opt.vdim;
+    const int seq = __ldcg(tok_seq + t), last = __ldcg(tok_pos + t);
+    float qr[N][4], acc[N][4];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const int d = 4 * (lane + 32 * j);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) qr[j][c] = acc[j][c] = 0.f;
+        if (d < kd) load_cols4(q + ((size_t)t * nh + head) * kd + d, qr[j]);
+    }
+    const int lo = opt.chunk > 0 ? last / opt.chunk * opt.chunk : 0;
+    const int* bt = kv.block_table + (size_t)seq * kv.max_pages_per_seq;
+    const C* kpool = (const C*)kv.k_pool;
+    const C* vpool = (const C*)kv.v_pool;
+    float m = kNegBig, l = 0.f;
+    bool bad = false;
+    for (int key0 = (lo / KEYS + warp) * KEYS; key0 <= last; key0 += warps * KEYS) {
+        const int pg = __ldcg(bt + key0 / kPageTokens);
+        if (pg < 0 || pg >= kv.num_pages) { bad = true; continue; }
+        const size_t row = ((size_t)pg * kv.nkv + kvh) * kPageTokens + key0 % kPageTokens;
+        float k[KEYS][N][4], v[SAME ? 1 : KEYS][N][4];
+#pragma unroll
+        for (int i = 0; i < KEYS; ++i) {
+            const bool on = key0 + i >= lo && key0 + i <= last;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const int d = 4 * (lane + 32 * j);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    k[i][j][c] = 0.f;
+                    if constexpr (!SAME) v[i][j][c] = 0.f;
+                }
+                if (on && d < kd) load_cols4(kpool + (row + i) * kd + d, k[i][j]);
+                if constexpr (!SAME)
+                    if (on && d < vd) load_cols4(vpool + (row + i) * vd + d, v[i][j]);
+            }
+        }
+        float s[KEYS], mx = kNegBig;
+#pragma unroll
+        for (int i = 0; i < KEYS; ++i) {
+            s[i] = 0.f;
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s[i] = fmaf(qr[j][c], k[i][j][c], s[i]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < KEYS; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
+#pragma unroll
+        for (int i = 0; i < KEYS; ++i) {
+            s[i] *= opt.scale;
+            if (key0 + i >= lo && key0 + i <= last) mx = fmaxf(mx, s[i]);
+        }
+        const float mn = fmaxf(m, mx), corr = expf(m - mn);
+        m = mn;
+        l *= corr;
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[j][c] *= corr;
+#pragma unroll
+        for (int i = 0; i < KEYS; ++i) {
+            if (key0 + i < lo || key0 + i > last) continue;
+            const float p = expf(s[i] - mn);
+            l += p;
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(p, SAME ? k[i][j][c] : v[SAME ? 0 : i][j][c], acc[j][c]);
+        }
+    }
+    float* mw = simt_smem + warp * (vdim + 2);
+    if (lane == 0) { mw[0] = m; mw[1] = l; }
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int d = 4 * (lane + 32 * j) + c;
+            if (d < vdim) mw[2 + d] = acc[j][c];
+        }
+    float gate = 1.f;
+    if (opt.gate) {
+        const float z = to_f32(((const C*)opt.gate)[(size_t)t * opt.gate_ld + head]);
+        gate = 1.f / (1.f + expf(-z));
+    }
+    __syncthreads();
+    float M = kNegBig, L = 0.f;
+    for (int w = 0; w < warps; ++w) M = fmaxf(M, simt_smem[w * (vdim + 2)]);
+    for (int w = 0; w < warps; ++w) L += simt_smem[w * (vdim + 2) + 1] * expf(simt_smem[w * (vdim + 2)] - M);
+    for (int d = tid; d < vdim; d += blockDim.x) {
+        float A = 0.f;
+        for (int w = 0; w < warps; ++w) A += simt_smem[w * (vdim + 2) + 2 + d] * expf(simt_smem[w * (vdim + 2)] - M);
+        store_as(ctx + (size_t)t * opt.ctx_ld + (size_t)head * opt.head_ld + d, A / L * gate);
+    }
+    if (bad && lane == 0) dev_fail(status, DEV_ERR_BOUNDS);
+    if (tid == 0) tl_mark(tl, 2);
+}
+
 bool exact(const AttnOptions& o, const KvView& kv, int nh, int hd) {
     return kv.hd == hd && kv.vd == hd && o.vdim == hd && o.ctx_ld == (int64_t)nh * hd && o.chunk == 0 && !o.gate && nh / kv.nkv <= 8;
 }
@@ -587,6 +715,13 @@ int attn_prepare() {
     if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<bf16, 16>);
     if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<float, 32>);
     if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<bf16, 32>);
+    auto simt4 = [&](auto kern) {
+        if (e == cudaSuccess) e = prefer_max_shared(kern);
+    };
+    simt4(k_attn_simt4<float, 1, false>), simt4(k_attn_simt4<float, 4, false>), simt4(k_attn_simt4<float, 8, false>);
+    simt4(k_attn_simt4<float, 1, true>), simt4(k_attn_simt4<float, 4, true>), simt4(k_attn_simt4<float, 8, true>);
+    simt4(k_attn_simt4<bf16, 1, false>), simt4(k_attn_simt4<bf16, 4, false>), simt4(k_attn_simt4<bf16, 8, false>);
+    simt4(k_attn_simt4<bf16, 1, true>), simt4(k_attn_simt4<bf16, 4, true>), simt4(k_attn_simt4<bf16, 8, true>);
     return e == cudaSuccess ? attn_prompt_prepare() : (int)e;
 }
 
@@ -665,7 +800,31 @@ int launch_attention(const float* q, KvView kv, int layer, const int* tok_seq, c
 void launch_attention_simt(const float* q, KvView kv, bool f32, const int* tok_seq, const int* tok_pos, void* ctx, int T, int nh,
                            const AttnOptions& options, int* status, cudaStream_t s, bool pdl, unsigned long long* tl) {
     const AttnOptions opt = resolve_attn_options(options, kv, nh);
-    const dim3 grid(nh, T), block(kSimtWarps * 32);
+    const dim3 grid(nh, T);
+    const int cols = kv.hd > kv.vd ? kv.hd : kv.vd;
+    if (cols <= 1024 && kv.hd % 4 == 0 && kv.vd % 4 == 0) {
+        const bool same = kv.k_pool == kv.v_pool && kv.hd == kv.vd;
+        auto go = [&](auto kern, auto* out, int most) {
+            // few blocks (decoding): more warps share the keys of one
+            const int warps = (long long)T * nh <= 256 ? most : kSimtWarps;
+            launch_k(kern, grid, dim3(warps * 32), (size_t)warps * (opt.vdim + 2) * 4, s, pdl, q, kv, tok_seq, tok_pos, out, nh, opt, status, tl);
+        };
+        auto widths = [&](auto* out, auto same_c) {
+            using C = std::remove_pointer_t<decltype(out)>;
+            constexpr bool SAME = decltype(same_c)::value;
+            if (cols <= 128) go(k_attn_simt4<C, 1, SAME>, out, simt_warps(1));
+            else if (cols <= 512) go(k_attn_simt4<C, 4, SAME>, out, simt_warps(4));
+            else go(k_attn_simt4<C, 8, SAME>, out, simt_warps(8));
+        };
+        auto types = [&](auto same_c) {
+            if (f32) widths((float*)ctx, same_c);
+            else widths((bf16*)ctx, same_c);
+        };
+        if (same) types(std::true_type());
+        else types(std::false_type());
+        return;
+    }
+    const dim3 block(kSimtWarps * 32);
     const size_t smem = (size_t)(kv.hd + kSimtWarps * (opt.vdim + 2)) * 4;
     const bool wide = opt.vdim > 512;
     if (f32) launch_k(wide ? k_attn_simt<float, 32> : k_attn_simt<float, 16>, grid, block, smem, s, pdl, q, kv, tok_seq, tok_pos, (float*)ctx, nh, opt, status, tl);
