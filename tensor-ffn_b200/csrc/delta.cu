@@ -363,9 +363,17 @@ __global__ void __launch_bounds__(NT) k_delta_scan(const DeltaRule a, int cols, 
         // The token's vectors in registers; with room for them, the next token's are requested before this token's sums
         // are exchanged, so that the exchange hides the shared-memory latency.
         constexpr bool AHEAD = !FUSED && J <= 2;
+        constexpr bool SCALARS = AHEAD && C == 1;  // v, beta, k . q and the head's decay as well
         ulonglong2 q4[J], k4[J], g4[J];
+        float vc = 0.f, gc = 0.f;
+        float2 bc = make_float2(0.f, 0.f);
         auto vectors = [&](int k) {
             const float* tok = buf + (size_t)k * tokf;
+            if constexpr (SCALARS) {
+                vc = c0 - cb < ncols ? tok[vOff + (c0 - cb)] : 0.f;
+                bc = *(const float2*)(tok + vOff + cols);
+                if constexpr (HEAD_DECAY) gc = tok[vOff + cols + 2];
+            }
 #pragma unroll
             for (int j = 0; j < J; ++j) {
                 const int d = 4 * (r + 8 * j);
@@ -383,7 +391,7 @@ __global__ void __launch_bounds__(NT) k_delta_scan(const DeltaRule a, int cols, 
             for (int c = 0; c < C; ++c) t2[c] = w2[c] = 0ull;
             f32x2 gh = 0ull;
             if constexpr (HEAD_DECAY) {
-                const float g = tok[vOff + cols + 2];
+                const float g = SCALARS ? gc : tok[vOff + cols + 2];
                 gh = pack2(g, g);
             }
 #pragma unroll
@@ -399,16 +407,42 @@ __global__ void __launch_bounds__(NT) k_delta_scan(const DeltaRule a, int cols, 
                 }
             }
             ulonglong2 kk[J];  // this token's key for the update
+            const float v0 = vc;
+            float2 bk = bc;
             if (AHEAD) {
 #pragma unroll
                 for (int j = 0; j < J; ++j) kk[j] = k4[j];
                 vectors(min(k + 1, n - 1));
             }
-            const float2 bk = *(const float2*)(tok + vOff + cols);
+            if constexpr (!SCALARS) bk = *(const float2*)(tok + vOff + cols);
             // Sums over the eight lanes by halving exchange (partners 4, 2, 1 lanes away): lane r ends with S^T k and
             // S^T q of column r (C = 8), or of column r & 3 with S^T k in lanes 0-3 and S^T q in lanes 4-7 (C = 4).
+            // With one or two columns every lane gets S^T k of all of them (the sums are formed in the same order).
             float uc[C];
-            if constexpr (C == 8) {
+            if constexpr (C <= 2) {
+                float ts[C], ws[C];
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    ts[c] = sum2(t2[c]);
+                    ws[c] = sum2(w2[c]);
+                }
+#pragma unroll
+                for (int x = 4; x > 0; x >>= 1)
+#pragma unroll
+                    for (int c = 0; c < C; ++c) ts[c] += __shfl_xor_sync(0xffffffffu, ts[c], x);
+#pragma unroll
+                for (int c = 0; c < C; ++c) uc[c] = bk.x * ((SCALARS ? v0 : c0 + c - cb < ncols ? tok[vOff + (c0 + c - cb)] : 0.f) - ts[c]);
+#pragma unroll
+                for (int x = 4; x > 0; x >>= 1)
+#pragma unroll
+                    for (int c = 0; c < C; ++c) ws[c] += __shfl_xor_sync(0xffffffffu, ws[c], x);
+                const int col = c0 + (r & (C - 1));
+                if (r < C && col - cb < ncols) {
+                    const float o = (C == 2 && r == 1 ? ws[C - 1] : ws[0]) + (C == 2 && r == 1 ? uc[C - 1] : uc[0]) * bk.y;
+                    if constexpr (FUSED) o_s[k * cols + (col - cb)] = o;
+                    else a.o[((size_t)(first + tile * kScanTokens + k) * H + h) * vdimP + col] = o;
+                }
+            } else if constexpr (C == 8) {
                 float tx[4], wx[4], ty[2], wy[2];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -534,6 +568,9 @@ cudaError_t scan_attrs_hd() {
         if (e == cudaSuccess) e = scan_attr<A, J, 8, false, 128, HD>();
     }
     if (e == cudaSuccess) e = scan_attr<A, J, 4, false, 128, HD>();
+    if (e == cudaSuccess) e = scan_attr<A, J, 2, false, 128, HD>();
+    if constexpr (HD)
+        if (e == cudaSuccess) e = scan_attr<A, J, 1, false, 128, HD>();
     return e;
 }
 template <typename A, int J>
@@ -563,6 +600,14 @@ void launch_scan_hd(const DeltaRule& a, int n_segs, bool fused, int num_sms, cud
         launch_k(kernel, dim3(a.heads, n_segs, (a.vdimP + cols - 1) / cols), dim3(threads), scan_smem(32 * J, cols, f, HD), s, pdl, a, cols, tl);
     };
     const int whole = (a.vdimP + 7) / 8 * 8;
+    // Few sequences leave schedulers idle and a token's chain of sums is what counts: fewer columns per lane, more warps. us a token
+    // with 4, 2 and 1 columns: 64-wide heads with a decay per channel, 14 of one sequence 0.333, 0.289, 0.324, of eight 0.338, 0.364,
+    // 0.521; with a decay per head, one sequence 0.365, 0.340, 0.273, four 0.367, 0.341, 0.371; 16 heads 128 wide, one sequence
+    // 0.422, 0.321, 0.296, two 0.420, 0.321, 0.357, four 0.425, 0.417, 0.513.
+    const long long quads = (long long)a.heads * n_segs * ((a.vdimP + 15) / 16);  // warps with four columns per lane
+    if constexpr (HD)
+        if (!fused && quads <= num_sms) return go(k_delta_scan<A, J, 1, false, 128, HD>, 1, 16, false);
+    if (!fused && quads <= 2ll * num_sms) return go(k_delta_scan<A, J, 2, false, 128, HD>, 2, 32, false);
     if constexpr (J <= 4) {
         if (fused && a.heads * n_segs < num_sms && whole <= 128) return go(k_delta_scan<A, J, 4, true, 256, HD>, 4, whole, true);
         if (fused) return go(k_delta_scan<A, J, 8, true, 256, HD>, 8, whole, true);
