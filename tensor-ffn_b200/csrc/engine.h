@@ -286,6 +286,7 @@ private:
     DeviceBuffer tokens_, tok_seq_, tok_pos_, row_idx_, picks_, identity_;
     DeviceBuffer grp_first_, grp_count_;  // prompt attention: groups of up to attn_group_tokens_ consecutive rows of one sequence
     int attn_group_tokens_ = 128;
+    DeviceBuffer ssq_;  // sums of squares that the folded norms pass on, see GemmCall::norm_w
     DeviceBuffer h_, xn_, q_, ctx_, act_b_, act_e_, xn_last_, logits_;
     size_t logits_rows_ = 0;
     DeviceBuffer attn_partials_, attn_counters_;

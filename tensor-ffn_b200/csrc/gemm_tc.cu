@@ -51,6 +51,12 @@ struct GemmDev {
     unsigned long long* tl;     // optional: step timeline of this launch
     int batch, out_batch;       // batched launch (GemmCall::batch): X is a 3-D map (column, problem, row)
     const GroupTile* grp;       // grouped launch: one entry per token tile (blockIdx.y), see GemmCall::grp
+    const bf16* norm_w;         // GemmCall::norm_w and what follows
+    bf16* norm_out;
+    float* norm_ssq;
+    const float* rms_ssq;
+    int rms_tiles, rms_n;
+    float rms_eps;
     float* amax_val;            // GEMM_STORE_F32: per (token, tile) maximum and its index, or nullptr
     int* amax_idx;
 };
@@ -73,7 +79,7 @@ struct GemmCfg {
     static constexpr int SHARED_STAGES = (BN <= 64) ? 4 : MAX_STAGES;
     // the epilogue parks one fp32 plane [BN][128] in the (by then idle) stage memory
     static_assert(BN * BM * 4 + BN * 8 <= SHARED_STAGES * STAGE_BYTES, "plane (+ per-token maxima) must fit the smallest ring");
-    static constexpr int smem_bytes(int stages) { return stages * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/; }
+    static constexpr int smem_bytes(int stages) { return stages * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + BN * 4 /*factors of the rows*/; }
     static constexpr int TMEM_COLS = (2 * BN < 32) ? 32 : 2 * BN;  // two accumulators, power of two
 };
 
@@ -172,6 +178,21 @@ __device__ __forceinline__ void prefetch_residual(const GemmDev& p, const void* 
     if (f.valid) f.residual = __ldcg((const uint2*)((const bf16*)out + (size_t)t * (size_t)p.ldo + n));
 }
 
+// GEMM_RESIDUAL with norm_w: h = bf16(float(h) + sum), the normed row up to its factor, and this tile's share of the factor. The
+// whole warp calls it.
+__device__ __forceinline__ void finalize_residual_norm(const GemmDev& p, void* out, int n, int t, float4 v, const FinalizePre& pre, uint2 nw, int lane) {
+    const size_t o = (size_t)t * (size_t)p.ldo + n;
+    bf16* h = (bf16*)out;
+    const uint2 old = pre.valid ? pre.residual : __ldcg((const uint2*)(h + o));
+    const uint2 now = pack_bf16x4(bf16_lo(old.x) + v.x, bf16_hi(old.x) + v.y, bf16_lo(old.y) + v.z, bf16_hi(old.y) + v.w);
+    *(uint2*)(h + o) = now;
+    const float a = bf16_lo(now.x), b = bf16_hi(now.x), c = bf16_lo(now.y), d = bf16_hi(now.y);
+    *(uint2*)(p.norm_out + o) = pack_bf16x4(a * bf16_lo(nw.x), b * bf16_hi(nw.x), c * bf16_lo(nw.y), d * bf16_hi(nw.y));
+    float ss = (a * a + b * b) + (c * c + d * d);
+    ss = warp_sum(ss);
+    if (lane == 0) p.norm_ssq[(size_t)t * gridDim.x + blockIdx.x] = ss;
+}
+
 // STORE / RESIDUAL / SWIGLU (the SwiGLU value was formed before the call)
 __device__ __forceinline__ void finalize_plain(const GemmDev& p, void* out, int n, int t, float4 v, FinalizePre pre) {
     if (n >= p.N) return;
@@ -265,7 +286,8 @@ __device__ __forceinline__ void add4(float4& a, const float4& b) {
     a.w += b.w;
 }
 
-template <int BN>
+// FOLD: a launch that passes a norm on or takes one (GemmCall::norm_w, rms_ssq)
+template <int BN, bool FOLD>
 __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(const __grid_constant__ GemmDev p) {
     using Cfg = GemmCfg<BN>;
     extern __shared__ uint8_t smem_raw[];
@@ -275,6 +297,7 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;
     uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
+    float* row_factor = (float*)(smem + STAGES * Cfg::STAGE_BYTES + 256);  // per token of the tile, with rms_ssq
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     int prob = blockIdx.y / p.t_tiles;  // independent problems (base / expert gate-up) share a launch
@@ -330,6 +353,7 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
+    const uint2 norm_w4 = FOLD && p.norm_w && warp >= 2 ? __ldg((const uint2*)(p.norm_w + n0 + lane * 4)) : make_uint2(0u, 0u);
     FinalizePre pre[2];  // epilogue warps, split-K: operands of the columns they will finish
     pre[0].valid = pre[1].valid = false;
 
@@ -417,6 +441,24 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
         const int q = warp & 3;
         const int row = q * 32 + lane;
         pdl_wait();  // later phases read and write buffers of earlier kernels
+        if (FOLD && p.rms_ssq) {
+            // 128 / BN neighbouring lanes per token, their loads in flight together
+            constexpr int L = (kGemmThreads - 64) / BN < 1 ? 1 : (kGemmThreads - 64) / BN;
+            const int j = ((int)threadIdx.x - 64) / L, sub = (int)threadIdx.x % L;
+            float ss = 0.f;
+            if (t0 + j < t_end) {
+                const float* from = p.rms_ssq + (size_t)(t0 + j) * p.rms_tiles;
+                for (int i0 = sub; i0 < p.rms_tiles; i0 += 4 * L) {
+                    float v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = i0 + u * L < p.rms_tiles ? __ldcg(from + i0 + u * L) : 0.f;
+                    ss += (v[0] + v[1]) + (v[2] + v[3]);
+                }
+            }
+#pragma unroll
+            for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (sub == 0) row_factor[j] = rsqrtf(ss / (float)p.rms_n + p.rms_eps);
+        }
         if (p.splits > 1) {
             // split-K: the (at most two) columns this warp will finish are known; fetch their operands now
             const int S = p.splits, cps = BN / S, rank = (int)cluster_ctarank();
@@ -490,7 +532,8 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
             for (int c = w; c < ncols; c += kWarps) {
                 const float2 g = *(const float2*)(plane + (size_t)c * BM + 2 * lane);
                 const float2 u = *(const float2*)(plane + (size_t)c * BM + 64 + 2 * lane);
-                const float a0 = silu_mul_bf16(g.x, u.x), a1 = silu_mul_bf16(g.y, u.y);
+                const float f = FOLD && p.rms_ssq ? row_factor[c] : 1.f;
+                const float a0 = silu_mul_bf16(g.x * f, u.x * f), a1 = silu_mul_bf16(g.y * f, u.y * f);
                 bf16* dst = o + (size_t)(t0 + c) * (size_t)p.ldo + nn;
                 if (pair) {
                     *(uint32_t*)dst = (uint32_t)bf16_bits(a0) | ((uint32_t)bf16_bits(a1) << 16);
@@ -503,7 +546,12 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
             const int n = n0 + lane * 4;
             FinalizePre none;
             none.valid = false;
-            if (!p.amax_val) {
+            if (FOLD && p.norm_w) {
+                if (warp >= 2)
+#pragma unroll 2
+                    for (int c = w - 2; c < ncols; c += kWarps - 2)
+                        finalize_residual_norm(p, out, n, t0 + c, *(const float4*)(plane + (size_t)c * BM + lane * 4), none, norm_w4, lane);
+            } else if (!p.amax_val) {
 #pragma unroll 4
                 for (int c = w; c < ncols; c += kWarps)
                     finalize_plain(p, out, n, t0 + c, *(const float4*)(plane + (size_t)c * BM + lane * 4), none);
@@ -553,7 +601,14 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
             return acc;
         };
         auto finish = [&](int t, float4 acc, float4 up, const FinalizePre& f) {
-            if (p.mode == GEMM_QKV) {
+            if (FOLD && p.rms_ssq) {
+                const float r = row_factor[t - t0];
+                acc = make_float4(acc.x * r, acc.y * r, acc.z * r, acc.w * r);
+                up = make_float4(up.x * r, up.y * r, up.z * r, up.w * r);
+            }
+            if (FOLD && p.norm_w) {
+                finalize_residual_norm(p, out, n, t, acc, f, norm_w4, lane);
+            } else if (p.mode == GEMM_QKV) {
                 finalize_qkv(p, n, t, acc, f);
             } else if (halves) {
                 // rows 0..63 of the tile hold gate, rows 64..127 up, for the same 64 output indices
@@ -694,7 +749,7 @@ int max_active_clusters(const cudaLaunchConfig_t& cfg, int stages, int splits) {
     int n = 0;
     cudaLaunchConfig_t q = cfg;
     q.dynamicSmemBytes = GemmCfg<BN>::smem_bytes(stages);
-    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<BN>, &q) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<BN, false>, &q) != cudaSuccess) {
         cudaGetLastError();
         n = 1 << 30;  // unknown: keep the configuration
     }
@@ -745,6 +800,17 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
     p.status = ws.status;
     p.trace = c.trace;
     p.tl = c.tl;
+    if ((c.norm_w && (c.mode != GEMM_RESIDUAL || !c.norm_out || !c.norm_ssq || c.N % BM || c.ldo % 4)) ||
+        (c.rms_ssq && ((c.mode != GEMM_QKV && c.mode != GEMM_SWIGLU) || c.rms_tiles < 1 || c.rms_n < 1)) ||
+        ((c.norm_w || c.rms_ssq) && (c.T > kFoldTokens || batched || c.grp)))
+        return (int)cudaErrorInvalidValue;
+    p.norm_w = c.norm_w;
+    p.norm_out = c.norm_out;
+    p.norm_ssq = c.norm_ssq;
+    p.rms_ssq = c.rms_ssq;
+    p.rms_tiles = c.rms_tiles;
+    p.rms_n = c.rms_n;
+    p.rms_eps = c.rms_eps;
     p.amax_val = c.mode == GEMM_STORE_F32 ? c.amax_val : nullptr;
     p.amax_idx = c.amax_idx;
     if (!c.out && !(c.mode == GEMM_STORE_F32 && c.amax_val && c.amax_idx) && c.mode != GEMM_QKV) return (int)cudaErrorInvalidValue;
@@ -834,7 +900,9 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
             cfg.dynamicSmemBytes = Cfg::smem_bytes(p.stages);
         }
     }
-    return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN>, p);
+    if constexpr (BN <= kFoldTokens)
+        if (p.norm_w || p.rms_ssq) return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, true>, p);
+    return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, false>, p);
 }
 
 }  // namespace
@@ -846,14 +914,15 @@ bool make_tmap_2d(TmapCache* cache, CUtensorMap* tm, const bf16* ptr, uint64_t r
 
 int gemm_prepare() {
     cudaError_t e;
-#define TFFN_PREP(BN)                                                                                                 \
-    e = cudaFuncSetAttribute(k_gemm_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem); \
+#define TFFN_PREP(BN, FOLD)                                                                                                 \
+    e = cudaFuncSetAttribute(k_gemm_tc<BN, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem); \
     if (e != cudaSuccess) return (int)e;                                                                             \
-    e = cudaFuncSetAttribute(k_gemm_tc<BN>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);                     \
+    e = cudaFuncSetAttribute(k_gemm_tc<BN, FOLD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);                     \
     if (e != cudaSuccess) return (int)e;                                                                             \
-    e = prefer_max_shared(k_gemm_tc<BN>);                                                                            \
+    e = prefer_max_shared(k_gemm_tc<BN, FOLD>);                                                                            \
     if (e != cudaSuccess) return (int)e;
-    TFFN_PREP(16) TFFN_PREP(32) TFFN_PREP(64) TFFN_PREP(128) TFFN_PREP(256)
+    TFFN_PREP(16, false) TFFN_PREP(32, false) TFFN_PREP(64, false) TFFN_PREP(128, false) TFFN_PREP(256, false)
+    TFFN_PREP(16, true) TFFN_PREP(32, true) TFFN_PREP(64, true)
 #undef TFFN_PREP
     return gemm_pair_prepare();
 }
@@ -883,7 +952,7 @@ int cheaper_width(long long narrow, long long wide, int kb, int num_sms) {
 //    512 tokens 21 -> 29; two pairs of that K: 1 000 tokens 49 -> 54, 2 048 tokens 80 -> 56).
 //  * One narrow row tile (a router) needs many tokens (K 896: 4 096 tokens 14 -> 8; K 2048: 768 tokens 9 -> 13).
 int pair_width(const GemmCall& c, const GemmWorkspace& ws) {
-    if (c.amax_val || (!c.out && c.mode != GEMM_QKV) || (c.grp && c.grp_bn != 256)) return 0;
+    if (c.amax_val || c.norm_w || c.rms_ssq || (!c.out && c.mode != GEMM_QKV) || (c.grp && c.grp_bn != 256)) return 0;
     const bool halves = c.mode == GEMM_SWIGLU, batched = c.batch > 1;
     // what launch_bn refuses stays with it
     if (halves && (c.op[0].K != c.op[1].K || c.op[0].X != c.op[1].X)) return 0;

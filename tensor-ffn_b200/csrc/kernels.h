@@ -93,7 +93,19 @@ struct GemmCall {
     // rows [l * T, (l + 1) * T) of X and writes the same rows of out.
     int layers;
     int64_t w_layer;
+    // RMSNorm without a kernel of its own (single-CTA tiles, at most kFoldTokens tokens, N a multiple of 128). A GEMM_RESIDUAL
+    // launch with norm_w also leaves bf16(h * norm_w) in norm_out [T, ldo] and, per token and row tile, the sum of h^2 in
+    // norm_ssq [t * N / 128 + tile]; a GEMM_QKV or GEMM_SWIGLU launch with rms_ssq takes such rows as X and scales every
+    // sum by 1 / sqrt(sum of rms_tiles entries / rms_n + rms_eps). The row's factor commutes with the product, so each
+    // value is rounded to bf16 as often as with the kernel.
+    const bf16* norm_w;
+    bf16* norm_out;
+    float* norm_ssq;
+    const float* rms_ssq;
+    int rms_tiles, rms_n;
+    float rms_eps;
 };
+constexpr int kFoldTokens = 64;
 struct GroupTile {
     int group;           // -1: this tile and all later ones are unused
     int row0, row_end;   // rows [row0, min(row0 + grp_bn, row_end)) of X and out belong to it
