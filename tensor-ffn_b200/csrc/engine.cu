@@ -782,14 +782,18 @@ void check_launch(int rc, const char* what) {
 }
 
 // one GEMM of a step: tensor cores, or true fp32 in a session that computes in fp32
-void Session::gemm(GemmCall& call, int cls, bool pdl) {
+// (beside: an independent one of the same rows in the same launch where that is possible)
+void Session::gemm(GemmCall& call, int cls, bool pdl, GemmCall* beside) {
     if (ablated(cls)) return;  // timing-only ablation: results are then meaningless
     call.pdl = pdl;
     call.tl = tl_next(cls);
     call.trace = (tl_on_ && (int)tl_cls_.size() - 1 == tl_trace_launch_) ? tl_trace_buf_.as<unsigned long long>() : nullptr;
     call.trace_ctas = (int)(tl_trace_buf_.bytes / (64 * 8));
     prof_begin(cls);
-    const int rc = st_ && st_->f32 ? launch_gemm_f32(call, gemm_ws(), stream_) : launch_gemm(call, gemm_ws(), stream_);
+    if (beside) beside->pdl = pdl;
+    const int rc = st_ && st_->f32 ? launch_gemm_f32(call, gemm_ws(), stream_)
+                   : beside        ? launch_gemm_beside(call, *beside, gemm_ws(), stream_)
+                                   : launch_gemm(call, gemm_ws(), stream_);
     prof_end();
     check_launch(rc, "GEMM launch");
     launches_++;

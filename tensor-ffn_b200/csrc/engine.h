@@ -337,7 +337,7 @@ private:
     // everything in a captured decode step's grids that depends on the context
     std::vector<int> decode_cuts(int n_seqs, int max_ctx) const;  // keys of the attention layers' cuts
 
-    void gemm(GemmCall& call, int cls, bool pdl);
+    void gemm(GemmCall& call, int cls, bool pdl, GemmCall* beside = nullptr);
     void lm_head(const void* x, int64_t ldx, int n_rows, bool decode, bool pdl);
     // tokens, slots and positions of T rows (three consecutive lists) to the device, with the runs the kernels need
     Staged stage_rows(const int32_t* tok_seq_pos, int T);

@@ -576,9 +576,13 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
         const int64_t nv = sp.out_cols(), ctx_ld = pad8(nv);
         const bool dense = sp.ff > 0 && sp.experts == 0;
         const int64_t ffp = pad8(sp.ff);
-        auto gate_up = [&](const void* x) {  // the dense feed-forward's gated activations
+        auto gate_up_product = [&](const void* x) {  // the dense feed-forward's gated activations
             GemmCall g = product(l.gate.as<bf16>(), s.h_ld, x, s.h_ld, H, sp.ff, GEMM_SWIGLU, s.ff_act.p, ffp);
             g.op[1] = {l.up.as<bf16>(), s.h_ld, (const bf16*)x, s.h_ld, H};
+            return g;
+        };
+        auto gate_up = [&](const void* x) {
+            GemmCall g = gate_up_product(x);
             gemm(g, KC_GEMM_GATEUP, pdl);
         };
         auto batched = [&](int cls, int batch, const bf16* W, int64_t ldw, const void* X, int64_t ldx, int x_batch, int K, int N, int mode, void* out,
@@ -590,7 +594,17 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
             gemm(g, cls, pdl);
         };
 
-        run_product(KC_GEMM_IN, l.w_in.as<bf16>(), s.h_ld, xn, s.h_ld, H, l.in_rows, GEMM_STORE_BF16, s.proj.p, l.in_rows);
+        // Parallel blocks: the feed-forward's first product reads the same stream as the mixer's, and few rows leave either of them
+        // short of tiles. In one launch: a step of 16 sequences, 12 layers 768 wide 380 -> 322 us, of 4 with 2 048 tokens behind them
+        // 485 -> 475. More than 64 rows run on the two-CTA tiles.
+        const bool beside = c.block == Block::Parallel && dense && !f32 && T <= 64;
+        GemmCall in = product(l.w_in.as<bf16>(), s.h_ld, xn, s.h_ld, H, l.in_rows, GEMM_STORE_BF16, s.proj.p, l.in_rows);
+        if (beside) {
+            GemmCall g = gate_up_product(s.xn2.p);
+            gemm(in, KC_GEMM_IN, pdl, &g);
+        } else {
+            gemm(in, KC_GEMM_IN, pdl);
+        }
         if (sp.mixer == Mixer::Attention) {
             QkNormRope q;
             memset(&q, 0, sizeof q);
@@ -812,7 +826,7 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
         if (c.block == Block::Parallel) {
             // both sublayers' outputs are sums of one launch
             if (dense) {
-                gate_up(s.xn2.p);
+                if (!beside) gate_up(s.xn2.p);
                 o.op[1] = {l.down.as<bf16>(), ffp, s.ff_act.as<bf16>(), ffp, sp.ff};
             }
             gemm(o, dense ? KC_GEMM_OUT_DOWN : KC_GEMM_OPROJ, pdl);

@@ -42,6 +42,9 @@ struct GemmDev {
     int kblocks[2];
     int N, T, splits, mode, t_tiles, stages;
     int tile_n;          // output indices per tile: 128, or 64 for GEMM_SWIGLU (64 gate rows + 64 up rows per tile)
+    int tiles_1;         // with a product beside it (launch_gemm_beside): tiles blockIdx.x >= tiles_1 are its, a GEMM_SWIGLU's, else 0
+    int N_2;
+    long long ldo_2;
     float alpha, out_scale;
     void* out[2];        // per problem
     long long ldo;
@@ -65,6 +68,12 @@ struct GemmDev {
     do {                                                                                                            \
         if (p.trace) p.trace[(size_t)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * 64 + (slot)] = gtime_ns(); \
     } while (0)
+
+// what a CTA writes: the launch's product, or the one beside it
+struct OutView {
+    int N, mode;
+    long long ldo;
+};
 
 template <int BN>
 struct GemmCfg {
@@ -170,12 +179,12 @@ __device__ __forceinline__ void finalize_qkv(const GemmDev& p, int n, int t, flo
     *(uint2*)dst = pack_bf16x4(o[0], o[1], o[2], o[3]);
 }
 
-__device__ __forceinline__ bool plain_is_vector(const GemmDev& p, int n) { return (n + 3 < p.N) && (((p.ldo | p.out_batch) & 3) == 0); }
+__device__ __forceinline__ bool plain_is_vector(const GemmDev& p, const OutView& w, int n) { return (n + 3 < w.N) && (((w.ldo | p.out_batch) & 3) == 0); }
 
 // GEMM_RESIDUAL: the old values of rows n .. n+3 of token t (read through L2)
-__device__ __forceinline__ void prefetch_residual(const GemmDev& p, const void* out, int n, int t, FinalizePre& f) {
-    f.valid = n < p.N && plain_is_vector(p, n);
-    if (f.valid) f.residual = __ldcg((const uint2*)((const bf16*)out + (size_t)t * (size_t)p.ldo + n));
+__device__ __forceinline__ void prefetch_residual(const GemmDev& p, const OutView& w, const void* out, int n, int t, FinalizePre& f) {
+    f.valid = n < w.N && plain_is_vector(p, w, n);
+    if (f.valid) f.residual = __ldcg((const uint2*)((const bf16*)out + (size_t)t * (size_t)w.ldo + n));
 }
 
 // GEMM_RESIDUAL with norm_w: h = bf16(float(h) + sum), the normed row up to its factor, and this tile's share of the factor. The
@@ -194,18 +203,18 @@ __device__ __forceinline__ void finalize_residual_norm(const GemmDev& p, void* o
 }
 
 // STORE / RESIDUAL / SWIGLU (the SwiGLU value was formed before the call)
-__device__ __forceinline__ void finalize_plain(const GemmDev& p, void* out, int n, int t, float4 v, FinalizePre pre) {
-    if (n >= p.N) return;
-    const size_t o = (size_t)t * (size_t)p.ldo + n;
-    const bool vec = plain_is_vector(p, n);
+__device__ __forceinline__ void finalize_plain(const GemmDev& p, const OutView& w, void* out, int n, int t, float4 v, FinalizePre pre) {
+    if (n >= w.N) return;
+    const size_t o = (size_t)t * (size_t)w.ldo + n;
+    const bool vec = plain_is_vector(p, w, n);
     const float f[4] = {v.x, v.y, v.z, v.w};
-    switch (p.mode) {
+    switch (w.mode) {
         case GEMM_STORE_F32:
             if (!out) break;  // only the fused arg-max was asked for
             if (vec) {
                 *(float4*)((float*)out + o) = make_float4(p.out_scale * v.x, p.out_scale * v.y, p.out_scale * v.z, p.out_scale * v.w);
             } else {
-                for (int j = 0; j < 4 && n + j < p.N; ++j) ((float*)out)[o + j] = p.out_scale * f[j];
+                for (int j = 0; j < 4 && n + j < w.N; ++j) ((float*)out)[o + j] = p.out_scale * f[j];
             }
             break;
         case GEMM_RESIDUAL: {
@@ -216,7 +225,7 @@ __device__ __forceinline__ void finalize_plain(const GemmDev& p, void* out, int 
                 *(uint2*)(h + o) = pack_bf16x4(bf16_lo(old.x) + f[0], bf16_hi(old.x) + f[1], bf16_lo(old.y) + f[2],
                                                bf16_hi(old.y) + f[3]);
             } else {
-                for (int j = 0; j < 4 && n + j < p.N; ++j) {
+                for (int j = 0; j < 4 && n + j < w.N; ++j) {
                     const float old = __uint_as_float((uint32_t)__ldcg((const unsigned short*)(h + o + j)) << 16);
                     h[o + j] = __float2bfloat16_rn(old + f[j]);
                 }
@@ -224,7 +233,7 @@ __device__ __forceinline__ void finalize_plain(const GemmDev& p, void* out, int 
             break;
         }
         default:  // GEMM_STORE_BF16, GEMM_SWIGLU, GEMM_RELU2
-            if (p.mode == GEMM_RELU2) {
+            if (w.mode == GEMM_RELU2) {
                 float r[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -234,14 +243,14 @@ __device__ __forceinline__ void finalize_plain(const GemmDev& p, void* out, int 
                 if (vec) {
                     *(uint2*)((bf16*)out + o) = pack_bf16x4(r[0], r[1], r[2], r[3]);
                 } else {
-                    for (int j = 0; j < 4 && n + j < p.N; ++j) ((bf16*)out)[o + j] = __float2bfloat16_rn(r[j]);
+                    for (int j = 0; j < 4 && n + j < w.N; ++j) ((bf16*)out)[o + j] = __float2bfloat16_rn(r[j]);
                 }
                 break;
             }
             if (vec) {
                 *(uint2*)((bf16*)out + o) = pack_bf16x4(f[0], f[1], f[2], f[3]);
             } else {
-                for (int j = 0; j < 4 && n + j < p.N; ++j) ((bf16*)out)[o + j] = __float2bfloat16_rn(f[j]);
+                for (int j = 0; j < 4 && n + j < w.N; ++j) ((bf16*)out)[o + j] = __float2bfloat16_rn(f[j]);
             }
             break;
     }
@@ -301,7 +310,9 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     int prob = blockIdx.y / p.t_tiles;  // independent problems (base / expert gate-up) share a launch
-    const int n0 = blockIdx.x * p.tile_n;
+    const bool beside = p.tiles_1 > 0 && (int)blockIdx.x >= p.tiles_1;
+    const OutView view = beside ? OutView{p.N_2, GEMM_SWIGLU, p.ldo_2} : OutView{p.N, p.mode, p.ldo};
+    const int n0 = beside ? ((int)blockIdx.x - p.tiles_1) * (BM / 2) : (int)blockIdx.x * p.tile_n;
     int t0 = (blockIdx.y % p.t_tiles) * BN, t_end = p.T, w_row0 = n0;
     if (p.grp) {
         // grouped launch: which group's weights and which rows this tile covers was written by an earlier kernel, so
@@ -320,7 +331,8 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
         w_row0 = prob_b * p.N + n0;
         prob = 0;
     }
-    const bool halves = p.mode == GEMM_SWIGLU;  // A tile = 64 gate rows over 64 up rows, one accumulator
+    if (beside) prob = 1;
+    const bool halves = view.mode == GEMM_SWIGLU;  // A tile = 64 gate rows over 64 up rows, one accumulator
     void* out = p.out[prob];
     if (batched) {
         if (p.mode == GEMM_STORE_F32) out = (float*)out + (size_t)prob_b * p.out_batch;
@@ -467,7 +479,7 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
                 const int jj = (warp - 2) + 4 * u, t = t0 + jj * S + rank;
                 if (cps <= 8 && jj < cps && t < t_end) {
                     if (p.mode == GEMM_QKV) prefetch_qkv(p, n0 + lane * 4, t, pre[u]);
-                    else if (p.mode == GEMM_RESIDUAL) prefetch_residual(p, out, n0 + lane * 4, t, pre[u]);
+                    else if (p.mode == GEMM_RESIDUAL) prefetch_residual(p, view, out, n0 + lane * 4, t, pre[u]);
                 }
             }
         }
@@ -527,19 +539,19 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
             // lane l finishes indices n0 + 2l and n0 + 2l + 1
             bf16* o = (bf16*)out;
             const int nn = n0 + 2 * lane;
-            const bool pair = nn + 1 < p.N && (p.ldo & 1) == 0;
+            const bool pair = nn + 1 < view.N && (view.ldo & 1) == 0;
 #pragma unroll 4
             for (int c = w; c < ncols; c += kWarps) {
                 const float2 g = *(const float2*)(plane + (size_t)c * BM + 2 * lane);
                 const float2 u = *(const float2*)(plane + (size_t)c * BM + 64 + 2 * lane);
                 const float f = FOLD && p.rms_ssq ? row_factor[c] : 1.f;
                 const float a0 = silu_mul_bf16(g.x * f, u.x * f), a1 = silu_mul_bf16(g.y * f, u.y * f);
-                bf16* dst = o + (size_t)(t0 + c) * (size_t)p.ldo + nn;
+                bf16* dst = o + (size_t)(t0 + c) * (size_t)view.ldo + nn;
                 if (pair) {
                     *(uint32_t*)dst = (uint32_t)bf16_bits(a0) | ((uint32_t)bf16_bits(a1) << 16);
                 } else {
-                    if (nn < p.N) dst[0] = __float2bfloat16_rn(a0);
-                    if (nn + 1 < p.N) dst[1] = __float2bfloat16_rn(a1);
+                    if (nn < view.N) dst[0] = __float2bfloat16_rn(a0);
+                    if (nn + 1 < view.N) dst[1] = __float2bfloat16_rn(a1);
                 }
             }
         } else {
@@ -554,7 +566,7 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
             } else if (!p.amax_val) {
 #pragma unroll 4
                 for (int c = w; c < ncols; c += kWarps)
-                    finalize_plain(p, out, n, t0 + c, *(const float4*)(plane + (size_t)c * BM + lane * 4), none);
+                    finalize_plain(p, view, out, n, t0 + c, *(const float4*)(plane + (size_t)c * BM + lane * 4), none);
             } else if (warp < 2) {
                 // Fused greedy pick: thread = token column, a plain scan down the 128 parked rows (a warp
                 // reduction per column would put 64 shuffle chains into every CTA's epilogue). The scan
@@ -580,7 +592,7 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
             } else if (out) {
 #pragma unroll 4
                 for (int c = w - 2; c < ncols; c += kWarps - 2)
-                    finalize_plain(p, out, n, t0 + c, *(const float4*)(plane + (size_t)c * BM + lane * 4), none);
+                    finalize_plain(p, view, out, n, t0 + c, *(const float4*)(plane + (size_t)c * BM + lane * 4), none);
             }
         }
     } else if (warp >= 2) {
@@ -613,11 +625,11 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
             } else if (halves) {
                 // rows 0..63 of the tile hold gate, rows 64..127 up, for the same 64 output indices
                 if (lane < 16)
-                    finalize_plain(p, out, n, t,
+                    finalize_plain(p, view, out, n, t,
                                    make_float4(silu_mul_bf16(acc.x, up.x), silu_mul_bf16(acc.y, up.y), silu_mul_bf16(acc.z, up.z),
                                                silu_mul_bf16(acc.w, up.w)), f);
             } else {
-                finalize_plain(p, out, n, t, acc, f);
+                finalize_plain(p, view, out, n, t, acc, f);
                 publish_amax(p, n, t, acc, lane);
             }
         };
@@ -757,8 +769,9 @@ int max_active_clusters(const cudaLaunchConfig_t& cfg, int stages, int splits) {
     return n;
 }
 
+// beside: an independent GEMM_SWIGLU of the same rows and K whose tiles follow those of c, or nullptr
 template <int BN>
-int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits) {
+int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits, const GemmCall* beside = nullptr) {
     using Cfg = GemmCfg<BN>;
     GemmDev p;
     memset(&p, 0, sizeof p);
@@ -782,8 +795,19 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
                 return -1000;
         }
     if (halves) p.kblocks[1] = 0;  // gate and up rows share one accumulator and one pass over K
+    if (beside) {
+        if (batched || c.grp || c.out2 || halves || c.op[1].K > 0 || c.mode == GEMM_QKV || c.norm_w || beside->mode != GEMM_SWIGLU || beside->T != c.T ||
+            beside->op[0].K != c.op[0].K || beside->op[1].K != c.op[0].K || beside->op[1].X != beside->op[0].X || beside->out2 || beside->rms_ssq)
+            return (int)cudaErrorInvalidValue;
+        for (int i = 0; i < 2; ++i) {
+            const GemmOperand& o = beside->op[i];
+            if (!make_tmap(ws.tmaps, &p.tmW[2 + i], o.W, (uint64_t)beside->N, (uint64_t)o.K, (uint64_t)o.ldw, BM / 2)) return -1000;
+            if (!make_tmap(ws.tmaps, &p.tmX[2 + i], o.X, (uint64_t)(beside->x_rows_alloc > c.T ? beside->x_rows_alloc : c.T), (uint64_t)o.K, (uint64_t)o.ldx, BN))
+                return -1000;
+        }
+    }
     for (int i = 1; i < 4; ++i)  // keep unused maps valid
-        if (i >= maps * 2 || (p.kblocks[i & 1] == 0 && !halves)) {
+        if ((!beside || i < 2) && (i >= maps * 2 || (p.kblocks[i & 1] == 0 && !halves))) {
             p.tmW[i] = p.tmW[0];
             p.tmX[i] = p.tmX[0];
         }
@@ -795,7 +819,9 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
     p.alpha = c.alpha;
     p.out_scale = c.out_scale == 0.f ? 1.f : c.out_scale;
     p.out[0] = c.out;
-    p.out[1] = c.out2 ? c.out2 : c.out;
+    p.out[1] = beside ? beside->out : c.out2 ? c.out2 : c.out;
+    p.N_2 = beside ? beside->N : 0;
+    p.ldo_2 = beside ? beside->ldo : 0;
     p.ldo = c.ldo;
     p.status = ws.status;
     p.trace = c.trace;
@@ -818,7 +844,8 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
         if (!c.qkv || c.op[1].K > 0 || c.out2 || (c.qkv->kv.hd != 64 && c.qkv->kv.hd != 128)) return (int)cudaErrorInvalidValue;
         p.qkv = *c.qkv;
     }
-    const int n_tiles = (c.N + p.tile_n - 1) / p.tile_n, t_tiles = c.grp ? c.grp_tiles : (c.T + BN - 1) / BN;
+    p.tiles_1 = beside ? (c.N + BM - 1) / BM : 0;
+    const int n_tiles = (c.N + p.tile_n - 1) / p.tile_n + (beside ? (beside->N + BM / 2 - 1) / (BM / 2) : 0), t_tiles = c.grp ? c.grp_tiles : (c.T + BN - 1) / BN;
     if (c.grp && (c.grp_bn != BN || c.op[1].K > 0 || c.out2 || halves || c.mode == GEMM_QKV || c.grp_tiles < 1 || c.grp_count < 1))
         return (int)cudaErrorInvalidValue;
     p.grp = c.grp;
@@ -1036,6 +1063,17 @@ int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream,
     if (c.T <= 64) return launch_bn<64>(c, ws, stream, force_splits);
     if (c.T <= 128) return launch_bn<128>(c, ws, stream, force_splits);
     return launch_bn<256>(c, ws, stream, force_splits);
+}
+
+int launch_gemm_beside(const GemmCall& a, const GemmCall& b, const GemmWorkspace& ws, cudaStream_t stream) {
+    const bool one = a.T > 0 && a.T <= 64 && b.T == a.T && a.N > 0 && b.N > 0 && a.out && b.out && a.op[0].K > 0 && a.op[0].K == b.op[0].K && b.mode == GEMM_SWIGLU &&
+                     !pair_width(a, ws) && !pair_width(b, ws);
+    if (!one) {
+        const int rc = launch_gemm(a, ws, stream);
+        return rc ? rc : launch_gemm(b, ws, stream);
+    }
+    if (a.T <= 16) return launch_bn<16>(a, ws, stream, 0, &b);
+    return a.T <= 32 ? launch_bn<32>(a, ws, stream, 0, &b) : launch_bn<64>(a, ws, stream, 0, &b);
 }
 
 }  // namespace tffn

@@ -134,6 +134,8 @@ struct GemmWorkspace {
 int gemm_prepare();
 // returns cudaError (launch) or -1000 if the tensor maps could not be encoded
 [[nodiscard]] int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits = 0);
+// Two independent products of the same rows (of X matrices of their own) and K, b a GEMM_SWIGLU: one launch for at most 64 rows, else two.
+[[nodiscard]] int launch_gemm_beside(const GemmCall& a, const GemmCall& b, const GemmWorkspace& ws, cudaStream_t stream);
 // one launch over independent layers: modes STORE_F32, STORE_BF16, SWIGLU, one operand pair
 [[nodiscard]] int launch_gemm_layers(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream);
 // The same products in true fp32 (fp32 X and out, fp32 FMA, weights still bf16): modes STORE_F32, STORE_BF16, RELU2 and
