@@ -53,6 +53,8 @@ struct GemmDev {
     unsigned long long* trace;  // optional: 64 timestamps (ns) per CTA, see GemmCall::trace
     unsigned long long* tl;     // optional: step timeline of this launch
     int batch, out_batch;       // batched launch (GemmCall::batch): X is a 3-D map (column, problem, row)
+    const int* bins;            // grouped launch over bins: GemmCall::bin_counts
+    int bin, bin_groups, bin_ahead;
     const GroupTile* grp;       // grouped launch: one entry per token tile (blockIdx.y), see GemmCall::grp
     const bf16* norm_w;         // GemmCall::norm_w and what follows
     bf16* norm_out;
@@ -306,6 +308,7 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;
     uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
+    int* tile_end = (int*)(tmem_slot + 1);  // bins: for the warps that do not read the count themselves
     float* row_factor = (float*)(smem + STAGES * Cfg::STAGE_BYTES + 256);  // per token of the tile, with rms_ssq
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -324,6 +327,22 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
         t0 = g.y;
         t_end = min(g.z, g.y + BN);
         w_row0 = g.x * p.N + n0;
+    }
+    // bins: which weights this CTA needs does not depend on the counts, only how many rows there are
+    // (the groups' first tiles come first: the others are mostly empty and would hold their places)
+    const int group = p.bins ? (int)blockIdx.y % p.bin_groups : 0, bin0 = group * p.bin;
+    auto bin_end = [&] { return min(bin0 + min(p.bin, __ldcg(p.bins + group)), t0 + BN); };
+    bool count_later = false;
+    if (p.bins) {
+        t0 = bin0 + (int)blockIdx.y / p.bin_groups * BN;
+        w_row0 = group * p.N + n0;
+        prob = 0;
+        count_later = p.bin_ahead && t0 == bin0;
+        if (!count_later) {
+            pdl_wait();
+            t_end = bin_end();
+            if (t_end <= t0) return;  // an empty tile: all CTAs of a cluster alike
+        }
     }
     const bool batched = p.batch > 1;
     const int prob_b = prob;
@@ -453,6 +472,10 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
         const int q = warp & 3;
         const int row = q * 32 + lane;
         pdl_wait();  // later phases read and write buffers of earlier kernels
+        if (count_later) {
+            t_end = bin_end();
+            if (threadIdx.x == 64) *tile_end = t_end;
+        }
         if (FOLD && p.rms_ssq) {
             // 128 / BN neighbouring lanes per token, their loads in flight together
             constexpr int L = (kGemmThreads - 64) / BN < 1 ? 1 : (kGemmThreads - 64) / BN;
@@ -509,6 +532,7 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
     }
     tc_fence_before();
     __syncthreads();
+    if (count_later && warp < 2) t_end = *tile_end;
     if (threadIdx.x == 64) TFFN_TRACE(5);
     // Finalisation is vectorised the other way round from the TMEM layout: a warp takes one column, a
     // lane 4 consecutive rows, so every global access is 8 or 16 bytes per lane and the RoPE partner of
@@ -788,7 +812,7 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
             if (pr == 0) p.kblocks[i] = o.K > 0 ? (o.K + BK - 1) / BK : 0;
             if (o.K <= 0) continue;
             if (pr == 1 && (o.K + BK - 1) / BK != p.kblocks[i]) return (int)cudaErrorInvalidValue;
-            const uint64_t w_rows = (uint64_t)c.N * (c.grp ? c.grp_count : batched ? c.batch : 1);
+            const uint64_t w_rows = (uint64_t)c.N * (c.grp || c.bin_counts ? c.grp_count : batched ? c.batch : 1);
             if (!make_tmap(ws.tmaps, &p.tmW[pr * 2 + i], o.W, w_rows, (uint64_t)o.K, (uint64_t)o.ldw, halves ? BM / 2 : BM)) return -1000;
             if (!make_tmap(ws.tmaps, &p.tmX[pr * 2 + i], o.X, (uint64_t)(c.x_rows_alloc > c.T ? c.x_rows_alloc : c.T), (uint64_t)o.K,
                            (uint64_t)o.ldx, BN, batched ? (uint32_t)c.batch : 1u, (uint32_t)c.x_batch))
@@ -796,7 +820,7 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
         }
     if (halves) p.kblocks[1] = 0;  // gate and up rows share one accumulator and one pass over K
     if (beside) {
-        if (batched || c.grp || c.out2 || halves || c.op[1].K > 0 || c.mode == GEMM_QKV || c.norm_w || beside->mode != GEMM_SWIGLU || beside->T != c.T ||
+        if (batched || c.grp || c.bin_counts || c.out2 || halves || c.op[1].K > 0 || c.mode == GEMM_QKV || c.norm_w || beside->mode != GEMM_SWIGLU || beside->T != c.T ||
             beside->op[0].K != c.op[0].K || beside->op[1].K != c.op[0].K || beside->op[1].X != beside->op[0].X || beside->out2 || beside->rms_ssq)
             return (int)cudaErrorInvalidValue;
         for (int i = 0; i < 2; ++i) {
@@ -828,7 +852,7 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
     p.tl = c.tl;
     if ((c.norm_w && (c.mode != GEMM_RESIDUAL || !c.norm_out || !c.norm_ssq || c.N % BM || c.ldo % 4)) ||
         (c.rms_ssq && ((c.mode != GEMM_QKV && c.mode != GEMM_SWIGLU) || c.rms_tiles < 1 || c.rms_n < 1)) ||
-        ((c.norm_w || c.rms_ssq) && (c.T > kFoldTokens || batched || c.grp)))
+        ((c.norm_w || c.rms_ssq) && (c.T > kFoldTokens || batched || c.grp || c.bin_counts)))
         return (int)cudaErrorInvalidValue;
     p.norm_w = c.norm_w;
     p.norm_out = c.norm_out;
@@ -845,13 +869,20 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
         p.qkv = *c.qkv;
     }
     p.tiles_1 = beside ? (c.N + BM - 1) / BM : 0;
-    const int n_tiles = (c.N + p.tile_n - 1) / p.tile_n + (beside ? (beside->N + BM / 2 - 1) / (BM / 2) : 0), t_tiles = c.grp ? c.grp_tiles : (c.T + BN - 1) / BN;
+    const int n_tiles = (c.N + p.tile_n - 1) / p.tile_n + (beside ? (beside->N + BM / 2 - 1) / (BM / 2) : 0),
+              bin_tiles = (c.bin + BN - 1) / BN, t_tiles = c.bin_counts ? c.grp_count * bin_tiles : c.grp ? c.grp_tiles : (c.T + BN - 1) / BN;
+    if (c.bin_counts && (c.grp || batched || c.grp_bn != BN || BN > 64 || c.op[1].K > 0 || c.out2 || halves || c.mode == GEMM_QKV || c.bin < 1 || c.grp_count < 1))
+        return (int)cudaErrorInvalidValue;
+    p.bins = c.bin_counts;
+    p.bin = c.bin;
+    p.bin_groups = c.grp_count;
+    p.bin_ahead = c.bin_ahead ? 1 : 0;
     if (c.grp && (c.grp_bn != BN || c.op[1].K > 0 || c.out2 || halves || c.mode == GEMM_QKV || c.grp_tiles < 1 || c.grp_count < 1))
         return (int)cudaErrorInvalidValue;
     p.grp = c.grp;
     const int total_kb = p.kblocks[0] + p.kblocks[1];
     // grouped: the grid has room for the worst case, the split policy goes by one tile per group that can have rows
-    const int tiles = c.grp && c.grp_rows_hint > 0 ? n_tiles * c.grp_rows_hint : n_tiles * t_tiles * nprob;
+    const int tiles = (c.grp || c.bin_counts) && c.grp_rows_hint > 0 ? n_tiles * c.grp_rows_hint : n_tiles * t_tiles * nprob;
     p.t_tiles = t_tiles;
     // K splits = cluster size (1, 2, 4, 8 or 16). A CTA's stream is bound by the latency of its stages (about 50 GB/s per SM,
     // all SMs together about 7 TB/s), so a weight-streaming launch needs about as many CTAs as there are SMs: tiles are split
@@ -866,7 +897,7 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
         // 8 splits 49.5 us, half of the 8-CTA clusters waiting for a second wave; 16 splits 18.0 us).
         // A grouped launch cannot request weights ahead of its dependency wait (the tile table comes from the kernel
         // before), so its k-loop is all exposed and shorter splits pay.
-        const int min_kb = c.grp ? 3 : 8;
+        const int min_kb = c.grp || (c.bin_counts && !c.bin_ahead) ? 3 : 8;
         while (splits < kMaxSplits && tiles * splits * 2 <= 2 * ws.num_sms && total_kb / (splits * 2) >= min_kb) splits *= 2;
     }
     if (splits != 1 && splits != 2 && splits != 4 && splits != 8 && splits != 16) return (int)cudaErrorInvalidValue;
@@ -979,7 +1010,7 @@ int cheaper_width(long long narrow, long long wide, int kb, int num_sms) {
 //    512 tokens 21 -> 29; two pairs of that K: 1 000 tokens 49 -> 54, 2 048 tokens 80 -> 56).
 //  * One narrow row tile (a router) needs many tokens (K 896: 4 096 tokens 14 -> 8; K 2048: 768 tokens 9 -> 13).
 int pair_width(const GemmCall& c, const GemmWorkspace& ws) {
-    if (c.amax_val || c.norm_w || c.rms_ssq || (!c.out && c.mode != GEMM_QKV) || (c.grp && c.grp_bn != 256)) return 0;
+    if (c.amax_val || c.norm_w || c.rms_ssq || c.bin_counts || (!c.out && c.mode != GEMM_QKV) || (c.grp && c.grp_bn != 256)) return 0;
     const bool halves = c.mode == GEMM_SWIGLU, batched = c.batch > 1;
     // what launch_bn refuses stays with it
     if (halves && (c.op[0].K != c.op[1].K || c.op[0].X != c.op[1].X)) return 0;
@@ -1015,7 +1046,7 @@ int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream,
     if (c.T <= 0 || c.N <= 0 || c.op[0].K <= 0) return (int)cudaErrorInvalidValue;
     if (force_splits == 0)
         if (const int bn = pair_width(c, ws)) return launch_gemm_pair(c, ws, stream, bn);
-    if (c.grp) {
+    if (c.grp || c.bin_counts) {
         switch (c.grp_bn) {
             case 16: return launch_bn<16>(c, ws, stream, force_splits);
             case 32: return launch_bn<32>(c, ws, stream, force_splits);

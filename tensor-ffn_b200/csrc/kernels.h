@@ -85,6 +85,12 @@ struct GemmCall {
     const struct GroupTile* grp;
     int grp_tiles, grp_bn, grp_count;  // grp_count: groups in W
     int grp_rows_hint;                 // tiles that will be in use, about (0: all)
+    // Grouped launch over bins instead of a table: group g's rows are [g * bin, g * bin + bin_counts[g]) of X and out, counts
+    // written by an earlier kernel. grp_count groups, token tiles of grp_bn (at most 64) rows. With bin_ahead the groups are taken
+    // to be not empty, and the first weights of their first tiles are requested ahead of the dependency wait.
+    const int* bin_counts;
+    int bin;
+    bool bin_ahead;
     // Batched launch (the heads of a per-head projection, the parts of a block-diagonal matrix): `batch` > 1 products of
     // N rows of W each (back to back in W), problem b reading columns [b * x_batch, b * x_batch + K) of X and writing
     // columns [b * out_batch, b * out_batch + N) of out. Modes STORE_F32 and STORE_BF16, op[0] only; x_batch a multiple of 8.
@@ -275,6 +281,12 @@ struct MoeRoute {
     int* counts;              // [experts], zero before the launch
     int2* pair;               // [T][top]: expert (-1: identity) and the pair's place within it
     float* pair_w;            // [T][top] softmax score (without the correction)
+    // Optional (launch_residual_rows): an expert's rows stand in `bin` places of their own, so a pair's row is known at once; the
+    // token's normed row is copied there and pair_row says where (-1: identity).
+    int bin;                  // 0: no bins
+    int* pair_row;            // [T][top]
+    void* xg;                 // [experts * bin][xg_ld], stored like the rows
+    int64_t xg_ld;
 };
 enum RowSource : int { ROWS_KEEP = 0, ROWS_EMBED, ROWS_DELTA, ROWS_MOE };
 // One pass over the residual stream per sublayer: x = table[token] (or its norm * embed_w) | x + norm(delta) * post_w, or

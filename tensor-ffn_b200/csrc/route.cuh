@@ -7,7 +7,7 @@
 namespace tffn {
 
 // s[0 .. n): the token's logits in shared memory, n = experts + identity (overwritten with the softmax scores);
-// choice[0 .. n): scratch. The lanes own strided entries.
+// choice[0 .. n): scratch, with bins afterwards the rows of the pairs. The lanes own strided entries.
 __device__ __forceinline__ void route_token(const MoeRoute& a, int t, float* s, float* choice, int lane) {
     const int n = a.experts + a.identity;
     float mx = -INFINITY;
@@ -21,9 +21,40 @@ __device__ __forceinline__ void route_token(const MoeRoute& a, int t, float* s, 
         sum += e;
     }
     const float inv = 1.f / warp_sum(sum);
-    for (int i = lane; i < n; i += 32) {
-        s[i] *= inv;
-        choice[i] = s[i] + __ldg(a.correction + i);
+    auto put = [&](int j, int bi) {  // place within the expert; the choices' atomics are in flight together
+        int2 p = make_int2(-1, 0);
+        if (bi < a.experts) p = make_int2(bi, atomicAdd(a.counts + bi, 1));
+        a.pair[(size_t)t * a.top + j] = p;
+        a.pair_w[(size_t)t * a.top + j] = s[bi];
+        if (a.bin > 0) {
+            const int row = p.x < 0 ? -1 : p.x * a.bin + p.y;
+            a.pair_row[(size_t)t * a.top + j] = row;
+            ((int*)choice)[j] = row;
+        }
+    };
+    if (n <= 32) {
+        // a lane per entry: its rank is the number of entries chosen before it (larger, or equal and earlier)
+        float c = -INFINITY;
+        if (lane < n) {
+            s[lane] *= inv;
+            c = s[lane] + __ldg(a.correction + lane);
+        }
+        if (__all_sync(0xffffffffu, lane >= n || c > -INFINITY)) {  // else (NaN inputs) as below
+            int rank = 0;
+            for (int j = 0; j < n; ++j) {
+                const float o = __shfl_sync(0xffffffffu, c, j);
+                rank += o > c || (o == c && j < lane) ? 1 : 0;
+            }
+            __syncwarp();
+            if (lane < n && rank < a.top) put(rank, lane);
+            return;
+        }
+        if (lane < n) choice[lane] = c;
+    } else {
+        for (int i = lane; i < n; i += 32) {
+            s[i] *= inv;
+            choice[i] = s[i] + __ldg(a.correction + i);
+        }
     }
     int mine[2] = {-1, -1};  // lane j keeps choices j and 32 + j (top <= 64)
     for (int j = 0; j < a.top; ++j) {
@@ -42,17 +73,10 @@ __device__ __forceinline__ void route_token(const MoeRoute& a, int t, float* s, 
         if ((j & 31) == lane) mine[j >> 5] = bi;
     }
     __syncwarp();  // every lane's scores are visible
-    // places within the experts: the choices' atomics in flight together
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const int j = k * 32 + lane;
-        if (j < a.top) {
-            const int bi = mine[k];
-            int2 p = make_int2(-1, 0);
-            if (bi < a.experts) p = make_int2(bi, atomicAdd(a.counts + bi, 1));
-            a.pair[(size_t)t * a.top + j] = p;
-            a.pair_w[(size_t)t * a.top + j] = s[bi];
-        }
+        if (j < a.top) put(j, mine[k]);
     }
 }
 

@@ -36,6 +36,11 @@ __global__ void __launch_bounds__(512) k_residual_rows4(const ResidualRows a, un
     if (threadIdx.x == 0) tl_mark(tl, 0);
     pdl_launch_dependents();
     const int H = a.H, r = blockIdx.x, n = blockDim.x, tid = threadIdx.x;
+    if (a.router_w) {  // its rows have left L2 since the last step: request them now, one line per thread
+        const char* w = (const char*)a.router_w;
+        const size_t bytes = (size_t)(a.route.experts + a.route.identity) * a.router_ld * sizeof(bf16);
+        for (size_t o = ((size_t)r * n + tid) * 128; o < bytes; o += (size_t)gridDim.x * n * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + o));
+    }
     // norm weights do not depend on earlier kernels
     float pw[IT][4], nw[IT][4];
 #pragma unroll
@@ -208,6 +213,16 @@ __global__ void __launch_bounds__(512) k_residual_rows4(const ResidualRows a, un
         }
         __syncthreads();
         if (warp == 0) route_token(a.route, r, z, z + outs, lane);
+        if (a.route.bin > 0) {
+            __syncthreads();
+            const int* dest = (const int*)(z + outs);
+            for (int i = tid * 4; i < H; i += n * 4) {
+                const float4 q = *(const float4*)(rows4_smem + i);
+                const float v[4] = {q.x, q.y, q.z, q.w};  // as stored: no rounding here
+                for (int j = 0; j < a.route.top; ++j)
+                    if (dest[j] >= 0) store4((A*)a.route.xg + (size_t)dest[j] * a.route.xg_ld + i, v);
+            }
+        }
     }
     if (tid == 0) tl_mark(tl, 2);
 }

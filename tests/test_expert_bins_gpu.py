@@ -1,0 +1,28 @@
+"""-m gpu: launches of few rows whose experts' rows stand in one bin per expert, at the ends of the token tiles and of the bins, with
+every row at the same experts (full bins of several tiles, the others empty), and the launch that no longer uses bins."""
+import numpy as np
+import pytest
+
+from rafilix_cases import LIMIT, Case, attention_layer, error, moe_mlp, rafilix_config
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("experts,top,identity", [(12, 2, 0), (40, 3, 2), (3, 3, 0)])
+def test_full_and_empty_bins(tmp_path, experts, top, identity):
+    def edit(name, x):  # settles every choice
+        if name.endswith("correction"):
+            y = np.zeros_like(x)
+            for i, e in enumerate([1, experts - 1, 0][:top]):
+                y[e] = 8.0 - 2 * i
+            return y
+    c = Case(tmp_path, rafilix_config(64, 97, [attention_layer(2, 1, 16, 16, chunk=20, mlp=moe_mlp(experts, top, 40, identity=identity))]), edit=edit)
+    t = c.tokens(140)
+    want, _ = c.expect(t)
+    s = c.session("bfloat16", max_seq=160)
+    for n in (1, 2, 15, 16, 17, 32, 33, 63, 64, 65, 127, 128, 129, 140):
+        s.qwen_reset()
+        e = error(s.qwen_forward(t[:n]), want[:n])
+        assert e.max() <= LIMIT["bfloat16"], (n, float(e.max()))
+    assert s.status() == 0
+    s.free()
