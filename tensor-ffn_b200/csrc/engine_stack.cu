@@ -436,6 +436,7 @@ void Session::alloc_stack(bool f32) {
     s.seg_count.alloc(T * 4);
     std::vector<int> ones(T, 1);
     upload(s.ones, ones.data(), T * 4);
+    if (s.f32) cuda_check((cudaError_t)gemm_f32_prepare(), "gemm_f32_prepare", __FILE__, __LINE__);
     cuda_check((cudaError_t)stack_rows_prepare(), "stack_rows_prepare", __FILE__, __LINE__);
     cuda_check((cudaError_t)delta_prepare(), "delta_prepare", __FILE__, __LINE__);
     cuda_check((cudaError_t)moe_prepare(), "moe_prepare", __FILE__, __LINE__);

@@ -3,8 +3,8 @@
 // (gemm_tc.cu) so that a session that computes in fp32 runs the same sequence of steps. Two kernels:
 //
 // k_gemm_f32_rows, up to eight tokens, bound by streaming the weights: the threads of a block divide K (16 bytes of a weight
-//   row each), hold eight rows in registers, and the sums meet in shuffles and shared memory. The first weights are
-//   requested ahead of the dependency wait.
+//   row each) for up to eight rows, and the sums meet in shuffles and shared memory. Blocks walk over groups of rows; the weights
+//   of the next pieces are on their way into shared memory, the first ones requested ahead of the dependency wait.
 // k_gemm_f32, more tokens, bound by FMA issue: one CTA = 64 tokens x 64 weight rows, 8 x 8 outputs per thread (four 16-byte
 //   shared loads per 64 FMA); the four 64-thread groups of a CTA take a quarter of every K slice each, so that one tile
 //   fills an SM's schedulers. Slices are double-buffered through registers. Where the tiles are fewer than the SMs, K is also
@@ -23,7 +23,7 @@ constexpr int kThreads = 256, kGroups = 4, kGroupK = KB / kGroups;
 constexpr int kLd = 68;       // floats of a slice's row in shared memory (64 and a pad; 16-byte aligned)
 constexpr int kMaxSplits = 8; // portable cluster size
 constexpr int kRowTokens = 8;
-constexpr int rows_per_thread(int tokens) { return tokens > 4 ? 4 : 8; }  // 32 sums at most
+constexpr int rows_per_thread(int tokens) { return tokens > 2 ? 4 : 8; }  // 32 sums at most
 
 struct F32Dev {
     const float* X[2];
@@ -75,105 +75,204 @@ __device__ __forceinline__ float finish(const F32Dev& p, float first, float v) {
 // the first `live` of a word's two bf16 values, the others zero
 __device__ __forceinline__ uint32_t keep_low(uint32_t u, int live) { return live >= 2 ? u : live == 1 ? u & 0xffffu : 0u; }
 
+// Sums of v[0 .. COUNT) (COUNT a power of two, at most 32) over the warp by halving exchange: lane l returns that of value l % COUNT.
+template <int COUNT>
+__device__ __forceinline__ float warp_sums(float (&v)[COUNT], int lane) {
+#pragma unroll
+    for (int o = 16, n = COUNT; o > 0; o >>= 1) {
+        if (n > 1) {
+            // the lanes with bit (n / 2) of their number keep the upper half of the values, their partners the lower
+            n >>= 1;
+            const int x = n;  // exchange distance: the values left are those of lane % n
+#pragma unroll
+            for (int i = 0; i < COUNT / 2; ++i) {
+                if (i >= n) break;
+                const bool up = lane & x;
+                const float give = up ? v[i] : v[i + n];
+                v[i] = (up ? v[i + n] : v[i]) + __shfl_xor_sync(0xffffffffu, give, x);
+            }
+        }
+    }
+    float r = v[0];
+#pragma unroll
+    for (int o = 16; o >= COUNT; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    return r;
+}
+
 // p.lanes threads (8 .. 256, a power of two) divide K in pieces of 8; the block's kThreads / lanes teams take
 // rows_per_thread weight rows each. TT tokens at a time (the rows' weights are read again, from L2, for the next TT).
-// Measured with k_gemm_f32 below, width 896 and ff 4864, three sequences of up to 150 tokens and eight steps: 88.7 -> 12.4 ms.
-template <int TT>
+// A thread's next DEPTH pieces are on their way into shared memory of its own (no barrier), 96 KB a block: the bytes in flight bound
+// it, and one piece ahead in registers was too few. ONE: K is one piece of every thread and both pairs read the same X, which then
+// stays in registers for all row groups. Inside a step of three sequences, 8 layers 896 wide, us: gate|up 16.8 -> 9.4, out and down
+// 12.5 -> 7.7, LM head (32 768 rows) 41 -> 23; the step 633 -> 375.
+constexpr int rows_depth(int tokens) { return 24 / rows_per_thread(tokens); }
+constexpr size_t rows_smem(int tokens) { return (size_t)rows_depth(tokens) * rows_per_thread(tokens) * kThreads * 16; }
+template <int TT, bool ONE>
 __global__ void __launch_bounds__(kThreads, 2) k_gemm_f32_rows(const F32Dev p) {
-    constexpr int R = rows_per_thread(TT);
-    __shared__ float part[kThreads / 32][R * TT];  // per warp
-    __shared__ float keep[kThreads / 32][R * TT];  // per team: the first operand pair's sums
+    constexpr int R = rows_per_thread(TT), SUMS = R * TT, DEPTH = rows_depth(TT);
+    extern __shared__ __align__(16) uint8_t ring_raw[];  // [DEPTH][R][kThreads] pieces of 16 bytes
+    __shared__ float part[2][kThreads / 32][SUMS];  // per warp; a sum's readers are done before the one after next is written
     if (threadIdx.x == 0) tl_mark(p.tl, 0);
     pdl_launch_dependents();
-    const int tid = threadIdx.x, team = tid / p.lanes, kl = tid % p.lanes, teams = kThreads / p.lanes;
-    const int n0 = (blockIdx.x * teams + team) * R;
-    // ungrouped weights are older than the previous kernel, and so are all but its own outputs
-    uint4 w[R];
-    auto load_w = [&](const bf16* W, long long ldw, long long row0, int k) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) w[r] = n0 + r < p.N ? __ldg((const uint4*)(W + (size_t)(row0 + n0 + r) * ldw + k)) : make_uint4(0, 0, 0, 0);
+    const int tid = threadIdx.x, lane = tid & 31, team = tid / p.lanes, kl = tid % p.lanes, teams = kThreads / p.lanes;
+    const int group_rows = teams * R, groups = (p.N + group_rows - 1) / group_rows, pairs = p.K[1] > 0 ? 2 : 1;
+    const int steps_of[2] = {(p.K[0] + p.lanes * 8 - 1) / (p.lanes * 8), (p.K[1] + p.lanes * 8 - 1) / (p.lanes * 8)};
+    uint4* const ring = (uint4*)ring_raw + tid;
+    Place at{};
+    // what a block works through: row groups, operand pairs, pieces of K
+    struct Piece {
+        int group, pair, step;
     };
-    bool ahead = false;
-    if (!p.grp && kl * 8 < p.K[0]) {
-        load_w(p.W[p.batch > 1 ? 0 : blockIdx.z], p.ldw[p.batch > 1 ? 0 : blockIdx.z], p.batch > 1 ? (long long)blockIdx.z * p.N : 0, kl * 8);
-        ahead = true;
+    const Piece start{(int)blockIdx.x, 0, 0};
+    auto next = [&](Piece x) {
+        if (++x.step < (x.pair ? steps_of[1] : steps_of[0])) return x;
+        x.step = 0;
+        if (++x.pair < pairs) return x;
+        x.pair = 0;
+        x.group += gridDim.x;
+        return x;
+    };
+    auto request = [&](const Piece& x, int slot) {  // rows and columns that do not exist become zeros
+        const int k = (x.step * p.lanes + kl) * 8, n0 = x.group * group_rows + team * R, op = at.op0 + x.pair;
+        const bool k_on = x.group < groups && k < p.K[x.pair];
+        const bf16* W = p.W[op] + (size_t)(at.w_row0 + n0) * p.ldw[op] + k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const bool on = k_on && n0 + r < p.N;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(ring + (slot * R + r) * kThreads)),
+                         "l"(on ? W + (size_t)r * p.ldw[op] : p.W[op]), "r"(on ? 16 : 0)
+                         : "memory");
+        }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    Piece ahead = start;
+    auto fill = [&] {
+        ahead = start;
+        for (int i = 0; i < DEPTH; ++i) {
+            request(ahead, i);
+            commit();
+            ahead = next(ahead);
+        }
+    };
+    // ungrouped weights are older than the previous kernel, and so are all but its own outputs
+    if (!p.grp) {
+        place(p, blockIdx.y, blockIdx.z, at);
+        fill();
     }
     pdl_wait();
     if (tid == 0) tl_mark(p.tl, 1);
-    Place at;
-    if (!place(p, blockIdx.y, blockIdx.z, at)) return;
-    const int pairs = p.K[1] > 0 ? 2 : 1;
+    if (p.grp) {
+        if (!place(p, blockIdx.y, blockIdx.z, at)) return;
+        fill();
+    }
+    int half = 0;
     for (int t0 = at.t0; t0 < at.t_end; t0 += TT) {
-        for (int pair = 0; pair < pairs; ++pair) {
-            const int op = at.op0 + pair, K = p.K[pair];
-            const float* X = p.X[op] + (size_t)at.b * p.x_batch;
-            const bf16* W = p.W[op];
-            const long long ldx = p.ldx[op], ldw = p.ldw[op];
-            float acc[R * TT];
+        if (t0 > at.t0) fill();  // the next tokens start over
+        float acc[SUMS], first = 0.f;
 #pragma unroll
-            for (int i = 0; i < R * TT; ++i) acc[i] = 0.f;
-            for (int k = kl * 8; k < K; k += p.lanes * 8) {
-                if (!ahead) load_w(W, ldw, at.w_row0, k);
-                ahead = false;
-                const int live = K - k;  // columns of this piece; what a row's padding holds counts as zero
-                if (live < 8) {
+        for (int i = 0; i < SUMS; ++i) acc[i] = 0.f;
+        // columns k .. k + 7 of token t0 + t; what a row's padding holds counts as zero
+        auto load_x = [&](int op, int t, int k, int live, float (&v)[8]) {
+            const float* xp = p.X[op] + (size_t)at.b * p.x_batch + k + (size_t)min(t0 + t, at.t_end - 1) * p.ldx[op];
+            *(float4*)v = live > 0 ? __ldcg((const float4*)xp) : make_float4(0.f, 0.f, 0.f, 0.f);
+            *(float4*)(v + 4) = live > 4 ? __ldcg((const float4*)(xp + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live < 8) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = j < live ? v[j] : 0.f;
+            }
+        };
+        float kept[ONE ? TT : 1][8];
+        if constexpr (ONE) {
+#pragma unroll
+            for (int t = 0; t < TT; ++t) load_x(at.op0, t, kl * 8, p.K[0] - kl * 8, kept[t]);
+        }
+        int slot = 0;
+        for (Piece x = start; x.group < groups; x = next(x)) {
+            const int K = p.K[x.pair], k = (x.step * p.lanes + kl) * 8, live = K - k;  // columns of this piece
+            asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH - 1) : "memory");
+            if (live > 0) {
+                uint4 w[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) w[r] = ring[(slot * R + r) * kThreads];
+                if (live < 8) {  // what a row's padding holds counts as zero
 #pragma unroll
                     for (int r = 0; r < R; ++r) w[r] = make_uint4(keep_low(w[r].x, live), keep_low(w[r].y, live - 2), keep_low(w[r].z, live - 4), keep_low(w[r].w, live - 6));
                 }
 #pragma unroll
                 for (int t = 0; t < TT; ++t) {
-                    const float* xp = X + (size_t)min(t0 + t, at.t_end - 1) * ldx + k;
-                    float x[8];
-                    *(float4*)x = __ldcg((const float4*)xp);
-                    *(float4*)(x + 4) = live > 4 ? __ldcg((const float4*)(xp + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (live < 8) {
+                    float xv[8];
+                    if constexpr (ONE) {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) x[j] = j < live ? x[j] : 0.f;
+                        for (int j = 0; j < 8; ++j) xv[j] = kept[t][j];
+                    } else {
+                        load_x(at.op0 + x.pair, t, k, live, xv);
                     }
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         const uint32_t u[4] = {w[r].x, w[r].y, w[r].z, w[r].w};
-                        float s = acc[r * TT + t];
+                        float a = acc[r * TT + t];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) s = fmaf(x[2 * j + 1], bf16_hi(u[j]), fmaf(x[2 * j], bf16_lo(u[j]), s));
-                        acc[r * TT + t] = s;
+                        for (int j = 0; j < 4; ++j) a = fmaf(xv[2 * j + 1], bf16_hi(u[j]), fmaf(xv[2 * j], bf16_lo(u[j]), a));
+                        acc[r * TT + t] = a;
                     }
                 }
             }
-            for (int o = min(p.lanes, 32) >> 1; o > 0; o >>= 1)
-#pragma unroll
-                for (int i = 0; i < R * TT; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-            if (p.lanes < 32) {  // one pair: every lane of the team holds the sums
-#pragma unroll
-                for (int i = 0; i < R * TT; ++i) {
+            request(ahead, slot);
+            commit();
+            ahead = next(ahead);
+            if (++slot == DEPTH) slot = 0;
+            if (x.step + 1 == (x.pair ? steps_of[1] : steps_of[0])) {  // the pair's sums
+                const int n0 = x.group * group_rows + team * R;
+                auto store = [&](int i, float v) {
                     const int n = n0 + i / TT, t = t0 + i % TT;
-                    if (i % p.lanes == kl && n < p.N && t < at.t_end) at.out[(size_t)t * p.ldo + n] = finish(p, 0.f, acc[i]);
-                }
-                continue;
-            }
-            const int warps = p.lanes / 32, warp0 = team * warps;
-            if ((tid & 31) == 0) {
+                    if (n < p.N && t < at.t_end) at.out[(size_t)t * p.ldo + n] = finish(p, first, v);
+                };
+                if (p.lanes < 32) {  // one pair: every lane of the team gets the sums
+                    for (int o = p.lanes >> 1; o > 0; o >>= 1)
 #pragma unroll
-                for (int i = 0; i < R * TT; ++i) part[tid >> 5][i] = acc[i];
-            }
-            __syncthreads();
-            for (int i = kl; i < R * TT; i += p.lanes) {
-                float v = 0.f;
-                for (int q = 0; q < warps; ++q) v += part[warp0 + q][i];
-                if (pair == 0 && pairs == 2) {
-                    keep[team][i] = v;  // the same thread reads it
-                    continue;
+                        for (int i = 0; i < SUMS; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+#pragma unroll
+                    for (int i = 0; i < SUMS; ++i)
+                        if (i % p.lanes == kl) store(i, acc[i]);
+                } else {
+                    const float mine = warp_sums<SUMS>(acc, lane);
+                    half ^= 1;
+                    if (lane < SUMS) part[half][tid >> 5][lane] = mine;
+                    __syncthreads();
+                    if (kl < SUMS) {
+                        const int warp0 = team * (p.lanes / 32);
+                        float v = 0.f;
+                        for (int q = 0; q < p.lanes / 32; ++q) v += part[half][warp0 + q][kl];
+                        if (x.pair + 1 < pairs) first = v;
+                        else store(kl, v);
+                    }
                 }
-                const int n = n0 + i / TT, t = t0 + i % TT;
-                if (n < p.N && t < at.t_end) at.out[(size_t)t * p.ldo + n] = finish(p, pairs == 2 ? keep[team][i] : 0.f, v);
+#pragma unroll
+                for (int i = 0; i < SUMS; ++i) acc[i] = 0.f;
             }
-            __syncthreads();
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     if (tid == 0) tl_mark(p.tl, 2);
 }
 
 // ------------------------------------------------------------------------------------------- more tokens
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 splat2(float x) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+    return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
 // VEC: 16-byte copies (rows of X and W aligned, see launch_gemm_f32); else element by element.
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads) k_gemm_f32(const F32Dev p) {
@@ -217,11 +316,11 @@ __global__ void __launch_bounds__(kThreads) k_gemm_f32(const F32Dev p) {
                 }
             }
         };
-        float acc[8][8];
+        f32x2 acc[8][4];  // pairs of neighbouring weight rows: packed FMA
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
         if (s0 < s1) fetch(s0);
         for (int s = s0; s < s1; ++s) {
             float* sx = smem + ((s - s0) & 1) * (2 * KB * kLd);
@@ -237,15 +336,17 @@ __global__ void __launch_bounds__(kThreads) k_gemm_f32(const F32Dev p) {
             for (int kk = 0; kk < kGroupK; ++kk) {
                 const float* xk = sx + (grp * kGroupK + kk) * kLd;
                 const float* wk = sw + (grp * kGroupK + kk) * kLd;
-                float a[8], b[8];
+                float a[8];
                 *(float4*)a = *(const float4*)(xk + 4 * ty);
                 *(float4*)(a + 4) = *(const float4*)(xk + 32 + 4 * ty);
-                *(float4*)b = *(const float4*)(wk + 4 * tx);
-                *(float4*)(b + 4) = *(const float4*)(wk + 32 + 4 * tx);
+                const ulonglong2 b0 = *(const ulonglong2*)(wk + 4 * tx), b1 = *(const ulonglong2*)(wk + 32 + 4 * tx);
+                const f32x2 b[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
+                for (int i = 0; i < 8; ++i) {
+                    const f32x2 aa = splat2(a[i]);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                    for (int j = 0; j < 4; ++j) acc[i][j] = fma2(aa, b[j], acc[i][j]);
+                }
             }
         }
         // the groups' quarters, in order, then the cluster's parts
@@ -258,7 +359,8 @@ __global__ void __launch_bounds__(kThreads) k_gemm_f32(const F32Dev p) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     float4* dst = (float4*)(smem + ((i >> 2) * 32 + 4 * ty + (i & 3)) * kLd + h * 32 + 4 * tx);
-                    float4 v = make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
+                    const float2 lo = unpack2(acc[i][2 * h]), hi = unpack2(acc[i][2 * h + 1]);
+                    float4 v = make_float4(lo.x, lo.y, hi.x, hi.y);
                     if (q > 0) {
                         const float4 o = *dst;
                         v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
@@ -300,6 +402,17 @@ __global__ void __launch_bounds__(kThreads) k_gemm_f32(const F32Dev p) {
 }
 
 }  // namespace
+
+int gemm_f32_prepare() {
+    cudaError_t e = cudaSuccess;
+    auto prep = [&](auto kern, int tokens) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem(tokens));
+        if (e == cudaSuccess) e = prefer_max_shared(kern);
+    };
+    prep(k_gemm_f32_rows<1, true>, 1), prep(k_gemm_f32_rows<2, true>, 2), prep(k_gemm_f32_rows<4, true>, 4);
+    prep(k_gemm_f32_rows<1, false>, 1), prep(k_gemm_f32_rows<2, false>, 2), prep(k_gemm_f32_rows<4, false>, 4), prep(k_gemm_f32_rows<8, false>, 8);
+    return (int)e;
+}
 
 int launch_gemm_f32(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream) {
     if (c.T <= 0 || c.N <= 0 || c.op[0].K <= 0 || !c.out) return (int)cudaErrorInvalidValue;
@@ -352,10 +465,14 @@ int launch_gemm_f32(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t str
         const int K = p.K[0] > p.K[1] ? p.K[0] : p.K[1];
         p.lanes = p.K[1] > 0 ? 32 : 8;
         while (p.lanes < kThreads && p.lanes * 8 < K) p.lanes *= 2;
-        const int rows = kThreads / p.lanes * rows_per_thread(c.T);
-        const dim3 grid((c.N + rows - 1) / rows, t_tiles, probs);
-        auto go = [&](auto kern) { return (int)launch_k(kern, grid, dim3(kThreads), 0, stream, c.pdl, p); };
-        return c.T == 1 ? go(k_gemm_f32_rows<1>) : c.T == 2 ? go(k_gemm_f32_rows<2>) : c.T <= 4 ? go(k_gemm_f32_rows<4>) : go(k_gemm_f32_rows<8>);
+        const int rows = kThreads / p.lanes * rows_per_thread(c.T), groups = (c.N + rows - 1) / rows;
+        // two blocks per SM; more groups than that are walked over, so that their weights are requested ahead
+        const int most = (2 * ws.num_sms + t_tiles * probs - 1) / (t_tiles * probs);
+        const dim3 grid(c.grp || groups <= most ? groups : most, t_tiles, probs);
+        auto go = [&](auto kern) { return (int)launch_k(kern, grid, dim3(kThreads), rows_smem(c.T == 3 ? 4 : c.T > 4 ? 8 : c.T), stream, c.pdl, p); };
+        if (K <= p.lanes * 8 && !c.grp && (p.K[1] <= 0 || (p.K[1] == p.K[0] && p.X[1] == p.X[0] && p.ldx[1] == p.ldx[0])) && c.T <= 4)
+            return c.T == 1 ? go(k_gemm_f32_rows<1, true>) : c.T == 2 ? go(k_gemm_f32_rows<2, true>) : go(k_gemm_f32_rows<4, true>);
+        return c.T == 1 ? go(k_gemm_f32_rows<1, false>) : c.T == 2 ? go(k_gemm_f32_rows<2, false>) : c.T <= 4 ? go(k_gemm_f32_rows<4, false>) : go(k_gemm_f32_rows<8, false>);
     }
     // splits until the chip is full once, at least four slices each
     const long long tiles = (long long)((c.N + NB - 1) / NB) * t_tiles * probs;

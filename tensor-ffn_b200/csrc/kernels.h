@@ -147,6 +147,7 @@ int gemm_prepare();
 // The same products in true fp32 (fp32 X and out, fp32 FMA, weights still bf16): modes STORE_F32, STORE_BF16, RELU2 and
 // SWIGLU (which then store fp32), grouped and batched launches included; two operand pairs only in a plain launch. The operands' X pointers
 // are fp32 arrays behind the bf16 type.
+int gemm_f32_prepare();  // as gemm_prepare
 [[nodiscard]] int launch_gemm_f32(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream);
 // the same products in tiles of 256 tokens x bn (128 or 256) weight rows over two CTAs; launch_gemm decides (no fused pick,
 // grouped launches with grp_bn 256)
