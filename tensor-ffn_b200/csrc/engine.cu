@@ -2,9 +2,13 @@
 #include "launch.h"
 #include "upload.h"
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <memory>
+#include <system_error>
+#include <thread>
 
 namespace tffn {
 
@@ -534,13 +538,57 @@ void Session::ensure_logits(size_t rows) {
     logits_rows_ = rows;
     drop_graphs();  // captured steps hold the old pointer
 }
+// Device to pageable host memory in chunks through pinned buffers, one per thread: the threads bring the destination's pages in
+// while the device is still busy with the step, then copy out of their buffers side by side. A plain copy of 39 MB (64 rows of the
+// Qwen2 vocabulary) into fresh pages took 8.6 ms behind a step of 1.15 ms, this one 1.7 to 3.2. Returns when the data is there.
+void Session::copy_staged(char* dst, const char* src, size_t bytes) {
+    constexpr size_t kChunk = (size_t)2 << 20, kPage = 4096;
+    const int n = (int)std::min<size_t>(4, std::max(1u, std::thread::hardware_concurrency()));
+    char* pinned = (char*)h_pinned_copy_.get(n * kChunk / 4);
+    const int device = m_->device;
+    std::atomic<int> failed{0};
+    std::promise<int> started;
+    std::shared_future<int> threads_in_all = started.get_future().share();
+    auto run = [&](int t) {  // chunks t, t + threads, ...
+        const size_t step = (size_t)threads_in_all.get() * kChunk;
+        cudaEvent_t done = nullptr;
+        cudaError_t e = cudaSetDevice(device);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+        for (size_t o = t * kChunk; o < bytes && e == cudaSuccess; o += step)
+            for (size_t p = o; p < std::min(bytes, o + kChunk); p += kPage) *(volatile char*)(dst + p) = 0;
+        for (size_t o = t * kChunk; o < bytes && e == cudaSuccess; o += step) {
+            const size_t len = std::min(kChunk, bytes - o);
+            e = cudaMemcpyAsync(pinned + t * kChunk, src + o, len, cudaMemcpyDeviceToHost, stream_);
+            if (e == cudaSuccess) e = cudaEventRecord(done, stream_);
+            if (e == cudaSuccess) e = cudaEventSynchronize(done);
+            if (e == cudaSuccess) memcpy(dst + o, pinned + t * kChunk, len);
+        }
+        if (done) cudaEventDestroy(done);
+        if (e != cudaSuccess) failed = (int)e;
+    };
+    std::vector<std::thread> threads;
+    try {
+        for (int t = 1; t < n; ++t) threads.emplace_back(run, t);
+    } catch (const std::system_error&) {  // fewer threads
+    }
+    started.set_value((int)threads.size() + 1);
+    run(0);
+    for (auto& t : threads) t.join();
+    cuda_check((cudaError_t)failed.load(), "copy of the logits", __FILE__, __LINE__);
+}
+
 // fp32 logits rows [0, rows) of the last LM-head launch -> host [rows, vocab]. With tensor parallelism
 // every rank holds its slice of the vocabulary: the slices are all-gathered on the device and laid out
 // side by side by the copies. Asynchronous on the session's stream.
 void Session::copy_logits_to_host(float* dst, size_t rows) {
     const size_t V = m_->cfg.vocab_size, Vl = m_->V;
     if (!tp_) {
-        TFFN_CUDA(cudaMemcpyAsync(dst, logits_.p, rows * V * 4, cudaMemcpyDeviceToHost, stream_));
+        const size_t bytes = rows * V * 4;
+        cudaPointerAttributes at;
+        const bool pageable = bytes >= kStagedCopyBytes && cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+        cudaGetLastError();
+        if (pageable) copy_staged((char*)dst, (const char*)logits_.p, bytes);
+        else TFFN_CUDA(cudaMemcpyAsync(dst, logits_.p, bytes, cudaMemcpyDeviceToHost, stream_));
         return;
     }
     const int n = m_->tp.tp_size;

@@ -247,6 +247,9 @@ private:
     TpPickParts tp_pick_parts_;
     size_t tp_pick_off_ = 0;  // in bytes: [tp_small_rows_] candidates of 8 bytes
     bool tp_fused_ = true;
+    static constexpr size_t kStagedCopyBytes = (size_t)16 << 20;
+    void copy_staged(char* dst, const char* src, size_t bytes);
+    PinnedI32 h_pinned_copy_;
     void copy_logits_to_host(float* dst, size_t rows);  // rows of logits_ (this rank's vocabulary slice) -> full rows on the host
     int max_batch_, max_seq_, max_pages_per_seq_, num_pages_;
     int cap_tokens_;  // rows of the activation buffers

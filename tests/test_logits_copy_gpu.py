@@ -1,0 +1,38 @@
+"""-m gpu: logits of 16 MB or more for memory that is not pinned are copied in chunks by several threads."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_large_copies_equal_small_ones(tmp_path):
+    import synth
+    import tffn
+    V = 70001
+    synth.write_model(str(tmp_path), dict(hidden_size=128, num_hidden_layers=1, num_attention_heads=2, num_key_value_heads=1, intermediate_size=256,
+                                          vocab_size=V, tie_word_embeddings=True), seed=3)
+    m = tffn.qwen_load(str(tmp_path))
+    t = synth.prompts(1, 60, 3, V)[0]
+    problems = []
+
+    def run():
+        s = tffn.Session(m, None, max_batch=1, max_seq=96)
+        small = s.qwen_forward(t[:58])  # 58 x V x 4 bytes: one plain copy; the same tiles of the same products
+        for _ in range(3):
+            s.qwen_reset()
+            large = s.qwen_forward(t)
+            if not (large[:58] == small).all() or not np.isfinite(large).all():
+                problems.append("rows differ")
+        s.qwen_reset()
+        if not (s.qwen_forward(t[:58]) == small).all():
+            problems.append("plain copy after a staged one")
+        s.free()
+
+    threads = [threading.Thread(target=run) for _ in range(2)]
+    for x in threads:
+        x.start()
+    for x in threads:
+        x.join()
+    assert not problems, problems
