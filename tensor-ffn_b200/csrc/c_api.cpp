@@ -457,6 +457,13 @@ int tffn_op_gemm_trace(int device, const uint16_t* X, const uint16_t* W, float* 
         }
         cuda_check((cudaError_t)gemm_prepare(), "gemm_prepare", __FILE__, __LINE__);
         GemmWorkspace ws{status.as<int>(), prop.multiProcessorCount};
+        DeviceBuffer partials, counters;  // as a session's kernels have them
+        partials.alloc((size_t)32 << 20);
+        counters.alloc(16384 * 4);
+        ws.partials = partials.as<float>();
+        ws.partial_floats = partials.bytes / 4;
+        ws.counters = counters.as<int>();
+        ws.num_counters = 16384;
         int rc = launch_gemm(g, ws, 0, splits);
         if (rc == -1000) throw Error(kErrCuda, "cuTensorMapEncodeTiled failed or is unavailable");
         if (rc != 0) cuda_check((cudaError_t)rc, "tensor-core GEMM launch", __FILE__, __LINE__);

@@ -518,6 +518,11 @@ GemmWorkspace Session::gemm_ws() const {
     w.status = status_.as<int>();
     w.num_sms = m_->num_sms;
     w.tmaps = tmaps_;
+    // the attention's scratch: the stream's kernels use it one after the other
+    w.partials = attn_partials_.as<float>();
+    w.partial_floats = attn_partials_.bytes / 4;
+    w.counters = attn_counters_.as<int>();
+    w.num_counters = (int)(attn_counters_.bytes / 4);
     return w;
 }
 AttnWorkspace Session::attn_ws() const {

@@ -10,6 +10,8 @@
 //   warps 2-9 epilogue: lane = token, registers = consecutive output columns (gate beside up, a rotary pair beside each
 //             other), transposed 32 x 32 through shared memory so that global accesses are 64 to 128 bytes of a row
 // Here the tokens are the MMA's rows (gemm_tc.cu has the weights there, which suits few tokens).
+// Tiles that would be a last wave on less than half of the pairs are split along K where that pays (pair_split): every part leaves its
+// fp32 sums in scratch memory, and per warp the last part to finish (a ticket, no waiting) adds all of them in order and finishes the tile.
 // Two operand pairs of different scale (base and expert down projections) take both TMEM regions as accumulators; their K
 // extent is long, so the exposed epilogue weighs little.
 #include "kernels.h"
@@ -49,6 +51,9 @@ struct PairDev {
     unsigned long long* tl;
     unsigned long long* trace;  // 64 phase stamps per CTA, as those of gemm_tc.cu
     int batch, out_batch;
+    int whole, splits;  // PAIR_SPLIT: tiles worked on as one, the first ones; parts of each of the others
+    float* partials;    // [split tile][part][rank][epilogue warp][column][row]
+    int* tickets;       // [split tile][rank][epilogue warp], zero
     int layers;  // > 1: problems are layers (GemmCall::layers), tmW 3-D (column, layer, row)
     const GroupTile* grp;
 };
@@ -263,7 +268,11 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* s
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
 }
 
-template <int BN, int MODE>
+// What a launch's tiles are: tiles of one or two problems, of a batch or of groups; of several layers (GemmCall::layers); with
+// the last ones in parts. The issuing loops of the first kind carry none of what the others need: a test per k-block there cost a
+// prompt's products 2 to 3 %.
+enum PairKind { PAIR_TILES, PAIR_LAYERS, PAIR_SPLIT };
+template <int BN, int MODE, int KIND>
 __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_constant__ PairDev p) {
     using Cfg = PairCfg<BN>;
     extern __shared__ uint8_t smem_raw[];
@@ -321,9 +330,25 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
     constexpr int tile_n = halves ? BN / 2 : BN;
     struct Tile {
         int m, n0, prob, t0, t_end, w_row0;
+        int kb0, kb1;       // k-blocks of this unit
+        int split, part;    // number of the split tile (-1: a whole one), part of it
     };
-    auto tile_at = [&](int i) {
-        Tile x;
+    constexpr bool SPLIT = KIND == PAIR_SPLIT, LAYERED = KIND == PAIR_LAYERS;
+    // the u-th tile, or part of one, of this pair (false: there are no more)
+    auto tile_at = [&](int u, Tile& x) {
+        int i = first + u * stride;
+        x.kb0 = 0;
+        x.kb1 = total_kb;
+        x.split = -1;
+        x.part = 0;
+        if (SPLIT && i >= p.whole) {
+            x.split = (i - p.whole) / p.splits;
+            x.part = (i - p.whole) % p.splits;
+            x.kb0 = (int)((long long)x.part * total_kb / p.splits);
+            x.kb1 = (int)((long long)(x.part + 1) * total_kb / p.splits);
+            i = p.whole + x.split;
+        }
+        if (i >= tiles) return false;
         x.m = i % m_tiles;
         const int r = i / m_tiles;
         x.n0 = (r % p.n_tiles) * tile_n;
@@ -339,7 +364,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
         } else if (p.batch > 1) {
             x.w_row0 = x.prob * p.N + x.n0;
         }
-        return x;
+        return true;
     };
 
     // The two issuing warps pace the pipeline (a k-block's products take 0.13 to 0.27 us), so their loops carry stage, phase
@@ -349,13 +374,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
         int s = 0, issued = 0;
         uint32_t ph = 1;  // a fresh barrier passes a wait for the phase before its first
         bool waited = p.grp != nullptr, ok = true;
-        for (int i = first; i < tiles && ok; i += stride) {
-            const Tile x = tile_at(i);
-            const bool layered = p.layers > 1;
-            const int map = p.batch > 1 || layered ? 0 : x.prob * 2;
-            const int t = x.t0 + rank * kHalf + (layered ? x.prob * p.T : 0), wr = halves ? x.w_row0 : x.w_row0 + rank * (BN / 2);
+        Tile x;
+        for (int u = 0; ok && tile_at(u, x); ++u) {
+            const int map = p.batch > 1 || LAYERED ? 0 : x.prob * 2;
+            const int t = x.t0 + rank * kHalf + (LAYERED ? x.prob * p.T : 0), wr = halves ? x.w_row0 : x.w_row0 + rank * (BN / 2);
             auto load_w = [&](const CUtensorMap* tm, int k, int st) {
-                if (layered) tma2_load_3d_elect(a_0 + st * Cfg::STAGE_BYTES + Cfg::A_BYTES, tm, k, x.prob, wr, lead_0 + st * 8);
+                if (LAYERED) tma2_load_3d_elect(a_0 + st * Cfg::STAGE_BYTES + Cfg::A_BYTES, tm, k, x.prob, wr, lead_0 + st * 8);
                 else tma2_load_2d_elect(a_0 + st * Cfg::STAGE_BYTES + Cfg::A_BYTES, tm, k, wr, lead_0 + st * 8);
             };
             auto load_x = [&](const CUtensorMap* tm, int k, int st) {
@@ -365,12 +389,14 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
             const CUtensorMap* const w_map[2] = {&p.tmW[map + (halves ? rank : 0)], &p.tmW[map + 1]};
             int ahead = 0;
             if (!waited) {  // weights do not depend on the previous kernel: the first ring is requested ahead of the wait
-                ahead = total_kb < Cfg::STAGES ? total_kb : Cfg::STAGES;
-                for (int kb = 0; kb < ahead; ++kb) {
-                    const int seg = kb >= p.kblocks[0] ? 1 : 0;
-                    if (rank == 0) mbar_arrive_expect_tx_elect(full_0 + kb * 8, 2 * Cfg::STAGE_BYTES);
-                    load_w(w_map[seg], (kb - seg * p.kblocks[0]) * BK, kb);
+                const int kb0 = SPLIT ? x.kb0 : 0, n = SPLIT ? x.kb1 - x.kb0 : total_kb;
+                ahead = n < Cfg::STAGES ? n : Cfg::STAGES;
+                for (int st = 0; st < ahead; ++st) {
+                    const int kb = kb0 + st, seg = kb >= p.kblocks[0] ? 1 : 0;
+                    if (rank == 0) mbar_arrive_expect_tx_elect(full_0 + st * 8, 2 * Cfg::STAGE_BYTES);
+                    load_w(w_map[seg], (kb - seg * p.kblocks[0]) * BK, st);
                 }
+                ahead += kb0;
                 if (lane == 0) TFFN_TRACE(1);
                 pdl_wait();
                 if (lane == 0) {
@@ -380,10 +406,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
                 __syncwarp();
                 waited = true;
             }
-            int kb = 0;
+            int kb = SPLIT ? x.kb0 : 0;
             for (int seg = 0; seg < 2 && ok; ++seg) {
                 const CUtensorMap *const tw = w_map[seg], *const tx = &p.tmX[map + seg];
-                for (int k = 0; k < p.kblocks[seg] * BK; k += BK, ++kb) {
+                const int seg0 = seg ? p.kblocks[0] : 0;
+                const int k_end = SPLIT ? (min(x.kb1, seg0 + p.kblocks[seg]) - seg0) * BK : p.kblocks[seg] * BK;
+                for (int k = SPLIT ? (kb - seg0) * BK : 0; k < k_end; k += BK, ++kb) {
                     if (!(ok = warp_wait(&empty[s], ph, p.status, DEV_ERR_EMPTY_WAIT))) break;
                     if (kb >= ahead) {
                         if (rank == 0) mbar_arrive_expect_tx_elect(full_0 + s * 8, 2 * Cfg::STAGE_BYTES);
@@ -410,18 +438,21 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
             int s = 0, n = 0;
             uint32_t ph = 0;
             bool ok = true;
-            for (int i = first; i < tiles && ok; i += stride, ++n) {
+            Tile x;
+            for (int i = first; ok && (SPLIT ? tile_at(n, x) : i < tiles); i += stride, ++n) {
                 const int buf = dual ? 0 : n & 1, use = dual ? n : n >> 1;
                 if (!(ok = warp_wait(&acc_empty[buf], (uint32_t)(use & 1) ^ 1u, p.status, DEV_ERR_ACC_WAIT))) break;
                 for (int seg = 0; seg < 2 && ok; ++seg) {
                     const uint32_t d = tmem_base + (uint32_t)((dual ? seg : buf) * BN);
-                    for (int kb = 0; kb < p.kblocks[seg]; ++kb) {
+                    const int seg0 = seg ? p.kblocks[0] : 0;
+                    const int kb_first = SPLIT ? max(x.kb0, seg0) : 0, kb_end = SPLIT ? min(x.kb1, seg0 + p.kblocks[seg]) : p.kblocks[seg];
+                    for (int kb = kb_first; kb < kb_end; ++kb) {
                         if (!(ok = warp_wait(&full[s], ph, p.status, DEV_ERR_FULL_WAIT))) break;
                         tc_fence_after();
                         const uint64_t at = (uint64_t)(uint32_t)(s * (Cfg::STAGE_BYTES >> 4));
                         const uint64_t ad = a_0 + at, bd = b_0 + at;
 #pragma unroll
-                        for (int k = 0; k < BK / 16; ++k) umma2_bf16_elect(d, ad + 2 * k, bd + 2 * k, idesc, (kb | k) ? 1u : 0u);
+                        for (int k = 0; k < BK / 16; ++k) umma2_bf16_elect(d, ad + 2 * k, bd + 2 * k, idesc, ((SPLIT ? kb - kb_first : kb) | k) ? 1u : 0u);
                         umma2_commit_elect(&empty[s]);
                         if (++s == Cfg::STAGES) {
                             s = 0;
@@ -438,8 +469,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
         const int q = warp & 3, part = (warp - 2) >> 2;  // TMEM lane quarter, which half of the columns
         float* buf32 = (float*)(epi + (warp - 2) * 32 * kStageRow);
         int n = 0;
-        for (int i = first; i < tiles; i += stride, ++n) {
-            const Tile x = tile_at(i);
+        Tile x;
+        for (; tile_at(n, x); ++n) {
             const int buf = dual ? 0 : n & 1, use = dual ? n : n >> 1;
             const int t0 = x.t0 + rank * kHalf + q * 32;
             int pos = -1, pg = -1;
@@ -462,7 +493,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
                         qkv_pair(p, buf32, lane, t0, x.t_end, x.n0 + c, pos, pg, a, b);
                     }
                 } else {
-                    const bool one_out = p.batch > 1 || p.layers > 1;
+                    const bool one_out = p.batch > 1 || LAYERED;
                     void* out = p.out[one_out ? 0 : x.prob];
                     if (one_out) {
                         const size_t at = (size_t)x.prob * (p.batch > 1 ? (size_t)p.out_batch : (size_t)p.T * (size_t)p.ldo);
@@ -470,8 +501,43 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
                         else out = (bf16*)out + at;
                     }
                     const int cols = tile_n / 2;  // of this warp
+                    // a part's sums: a warp's block of the scratch memory, [column][row]
+                    const size_t block = (size_t)cols * 32, slot = (size_t)2 * kEpiWarps * block;
+                    float* const sums = SPLIT && x.split >= 0 ? p.partials + (size_t)x.split * p.splits * slot + ((size_t)rank * kEpiWarps + (warp - 2)) * block : nullptr;
+                    bool finish = true;
+                    if (SPLIT && x.split >= 0) {
+                        const bool has0 = x.kb0 < p.kblocks[0], has1 = x.kb1 > p.kblocks[0];
+                        float* mine = sums + x.part * slot;
 #pragma unroll 1
-                    for (int c = part * cols; c < (part + 1) * cols; c += 32) {
+                        for (int c = 0; c < cols; c += 32) {
+                            float v[32];
+                            if (dual) {
+                                float w[32];
+                                tmem_ld32(acc + (uint32_t)(part * cols + c), v);
+                                tmem_ld32(acc + (uint32_t)(part * cols + c + BN), w);
+                                tc_wait_ld();
+#pragma unroll
+                                for (int j = 0; j < 32; ++j) v[j] = (has0 ? v[j] : 0.f) + (has1 ? p.alpha * w[j] : 0.f);
+                            } else {
+                                tmem_ld32(acc + (uint32_t)(part * cols + c), v);
+                                tc_wait_ld();
+                            }
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) mine[(c + j) * 32 + lane] = v[j];
+                        }
+                        __threadfence();
+                        __syncwarp();
+                        int* ticket = p.tickets + (x.split * 2 + rank) * kEpiWarps + (warp - 2);
+                        int before = 0;
+                        if (lane == 0) before = atomicAdd(ticket, 1);
+                        finish = __shfl_sync(0xffffffffu, before, 0) == p.splits - 1;
+                        if (finish) {
+                            if (lane == 0) *ticket = 0;
+                            __threadfence();
+                        }
+                    }
+#pragma unroll 1
+                    for (int c = part * cols; finish && c < (part + 1) * cols; c += 32) {
                         if (x.n0 + c >= p.N) break;
                         const int col = x.n0 + c + 4 * (lane & 7);
                         const bool vec = col + 3 < p.N && ((p.ldo | p.out_batch) & 3) == 0;
@@ -484,6 +550,19 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_gemm_pair(const __grid_cons
                             }
                         }
                         float v[32];
+                        if (SPLIT && x.split >= 0) {
+                            const float* from = sums + (size_t)(c - part * cols) * 32 + lane;
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) v[j] = __ldcg(from + j * 32);
+                            for (int z = 1; z < p.splits; ++z) {
+                                from += slot;
+#pragma unroll
+                                for (int j = 0; j < 32; ++j) v[j] += __ldcg(from + j * 32);
+                            }
+                            park(buf32, lane, v);
+                            store_piece<MODE>(p, out, buf32, lane, t0, x.t_end, col, old, vec);
+                            continue;
+                        }
                         tmem_ld32(acc + (uint32_t)c, v);
                         if (halves || dual) {
                             float w[32];
@@ -527,7 +606,7 @@ int launch_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream)
     PairDev p;
     memset(&p, 0, sizeof p);
     const bool halves = c.mode == GEMM_SWIGLU, batched = c.batch > 1, layered = c.layers > 1;
-    if (layered && (batched || c.grp || c.out2 || c.mode == GEMM_QKV || c.mode == GEMM_RESIDUAL || c.w_layer % 8 || c.w_layer >> 32 ||
+    if (layered && ((c.mode != GEMM_SWIGLU && c.mode != GEMM_STORE_F32) || batched || c.grp || c.out2 || c.mode == GEMM_QKV || c.mode == GEMM_RESIDUAL || c.w_layer % 8 || c.w_layer >> 32 ||
                     (!halves && c.op[1].K > 0)))
         return (int)cudaErrorInvalidValue;
     const int maps = c.out2 ? 2 : 1;
@@ -569,16 +648,33 @@ int launch_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream)
     p.grp = c.grp;
     if (c.mode == GEMM_QKV) p.qkv = *c.qkv;
     const long long tiles = (long long)p.m_tiles * p.n_tiles * p.nprob;
-    const int pairs = (int)(tiles < ws.num_sms / 2 ? tiles : ws.num_sms / 2);
+    int pairs = (int)(tiles < ws.num_sms / 2 ? tiles : ws.num_sms / 2);
+    bool split = false;
+    if (!c.grp && !layered && ws.partials && (c.mode == GEMM_STORE_F32 || c.mode == GEMM_STORE_BF16 || c.mode == GEMM_RESIDUAL)) {
+        const PairSplit s = pair_split(tiles, p.kblocks[0] + p.kblocks[1], BN, ws.num_sms);
+        split = s.splits > 1 && (size_t)s.tail * s.splits * kPairTokens * BN <= ws.partial_floats && (long long)s.tail * 2 * kEpiWarps <= ws.num_counters;
+        if (split) {
+            p.whole = (int)(tiles - s.tail);
+            p.splits = s.splits;
+            p.partials = ws.partials;
+            p.tickets = ws.counters;
+            const long long units = p.whole + (long long)s.tail * s.splits;
+            pairs = (int)(units < ws.num_sms / 2 ? units : ws.num_sms / 2);
+        }
+    }
     p.trace = 2 * pairs <= c.trace_ctas ? c.trace : nullptr;
     auto go = [&](auto kern) { return (int)launch_k_cluster(kern, dim3(2 * pairs), dim3(kPairThreads), dim3(2, 1, 1), PairCfg<BN>::SMEM, stream, c.pdl, p); };
+    if (layered) {
+        if (c.mode == GEMM_SWIGLU) return go(k_gemm_pair<BN, GEMM_SWIGLU, PAIR_LAYERS>);
+        return c.mode == GEMM_STORE_F32 ? go(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_LAYERS>) : (int)cudaErrorInvalidValue;
+    }
     switch (c.mode) {
-        case GEMM_STORE_F32: return go(k_gemm_pair<BN, GEMM_STORE_F32>);
-        case GEMM_STORE_BF16: return go(k_gemm_pair<BN, GEMM_STORE_BF16>);
-        case GEMM_RESIDUAL: return go(k_gemm_pair<BN, GEMM_RESIDUAL>);
-        case GEMM_SWIGLU: return go(k_gemm_pair<BN, GEMM_SWIGLU>);
-        case GEMM_RELU2: return go(k_gemm_pair<BN, GEMM_RELU2>);
-        case GEMM_QKV: return go(k_gemm_pair<BN, GEMM_QKV>);
+        case GEMM_STORE_F32: return split ? go(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_SPLIT>) : go(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_TILES>);
+        case GEMM_STORE_BF16: return split ? go(k_gemm_pair<BN, GEMM_STORE_BF16, PAIR_SPLIT>) : go(k_gemm_pair<BN, GEMM_STORE_BF16, PAIR_TILES>);
+        case GEMM_RESIDUAL: return split ? go(k_gemm_pair<BN, GEMM_RESIDUAL, PAIR_SPLIT>) : go(k_gemm_pair<BN, GEMM_RESIDUAL, PAIR_TILES>);
+        case GEMM_SWIGLU: return go(k_gemm_pair<BN, GEMM_SWIGLU, PAIR_TILES>);
+        case GEMM_RELU2: return go(k_gemm_pair<BN, GEMM_RELU2, PAIR_TILES>);
+        case GEMM_QKV: return go(k_gemm_pair<BN, GEMM_QKV, PAIR_TILES>);
     }
     return (int)cudaErrorInvalidValue;
 }
@@ -590,16 +686,38 @@ cudaError_t prepare_pair() {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<BN>::SMEM);
         if (e == cudaSuccess) e = prefer_max_shared(kern);
     };
-    prep(k_gemm_pair<BN, GEMM_STORE_F32>);
-    prep(k_gemm_pair<BN, GEMM_STORE_BF16>);
-    prep(k_gemm_pair<BN, GEMM_RESIDUAL>);
-    prep(k_gemm_pair<BN, GEMM_SWIGLU>);
-    prep(k_gemm_pair<BN, GEMM_RELU2>);
-    prep(k_gemm_pair<BN, GEMM_QKV>);
+    prep(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_TILES>);
+    prep(k_gemm_pair<BN, GEMM_STORE_BF16, PAIR_TILES>);
+    prep(k_gemm_pair<BN, GEMM_RESIDUAL, PAIR_TILES>);
+    prep(k_gemm_pair<BN, GEMM_SWIGLU, PAIR_TILES>);
+    prep(k_gemm_pair<BN, GEMM_RELU2, PAIR_TILES>);
+    prep(k_gemm_pair<BN, GEMM_QKV, PAIR_TILES>);
+    prep(k_gemm_pair<BN, GEMM_SWIGLU, PAIR_LAYERS>);
+    prep(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_LAYERS>);
+    prep(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_SPLIT>);
+    prep(k_gemm_pair<BN, GEMM_STORE_BF16, PAIR_SPLIT>);
+    prep(k_gemm_pair<BN, GEMM_RESIDUAL, PAIR_SPLIT>);
     return e;
 }
 
 }  // namespace
+
+// A k-block costs a pair 0.34 us with 128 weight rows and 0.42 with 256 (0.34 while it has the chip to itself), a tile about 1 us
+// around them; whole waves of 74 pairs count. The tiles of the last wave can be split along K, if it is at most half full: a part's
+// sums cost about 3 us to leave behind and the last part 1.6 us for each of them to add up (4 096 tokens, K 17920 of two operand
+// pairs, N 1536: 96 tiles, the last 22 in three parts, 235 -> 179 us). Shares of equal length for all pairs, across tile borders, were
+// slower than whole tiles (262): the pairs no longer read the same columns at about the same time.
+PairSplit pair_split(long long tiles, int kb, int bn, int num_sms) {
+    const int pairs = num_sms / 2, tail = (int)(tiles % pairs);
+    const double us = bn == 128 || tiles < pairs ? 0.34 : 0.42;
+    const double whole = (double)((tiles + pairs - 1) / pairs) * (kb * us + 1.0);
+    PairSplit best{tail, 1, whole, whole};
+    for (int s = 2; tail > 0 && s * tail <= pairs && s <= 8 && kb >= 8 * s; ++s) {
+        const double cost = (double)(tiles / pairs) * (kb * us + 1.0) + (double)kb / s * us + 1.0 + 3.0 + 1.6 * s;
+        if (cost < best.us) best = PairSplit{tail, s, cost, whole};
+    }
+    return best;
+}
 
 int gemm_pair_prepare() {
     const cudaError_t e = prepare_pair<128>();

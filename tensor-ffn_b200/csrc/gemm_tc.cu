@@ -993,12 +993,12 @@ int gemm_group_tile(int rows) {
     return bn;
 }
 
-// Width: a k-block costs a pair 0.34 us with 128 weight rows and 0.42 with 256 (0.34 while it has the chip to itself), a
-// tile about 1 us around them; whole waves of 74 pairs count.
-int cheaper_width(long long narrow, long long wide, int kb, int num_sms) {
-    const int pairs = num_sms / 2;
-    auto cost = [&](long long tiles, double us) { return (double)((tiles + pairs - 1) / pairs) * (kb * us + 1.0); };
-    return cost(narrow, 0.34) <= cost(wide, wide < pairs ? 0.34 : 0.42) ? 128 : 256;
+int cheaper_width(long long narrow, long long wide, int kb, int num_sms, bool can_split) {
+    auto us = [&](long long tiles, int bn) {
+        const PairSplit s = pair_split(tiles, kb, bn, num_sms);
+        return can_split ? s.us : s.whole_us;
+    };
+    return us(narrow, 128) <= us(wide, 256) ? 128 : 256;
 }
 // Which launches take the two-CTA tiles of gemm_pair.cu, and how wide (0: none). Measured back to back on one B200 against
 // the tiles of this file (us, here -> there): 4 096 tokens, K 896: q|k|v N 1152 87 -> 23, N 4864 gate|up of base and expert
@@ -1030,7 +1030,7 @@ int pair_width(const GemmCall& c, const GemmWorkspace& ws) {
             return 0;
         }
     }
-    return cheaper_width(narrow, wide, kb, ws.num_sms);
+    return cheaper_width(narrow, wide, kb, ws.num_sms, !c.grp && ws.partials && (c.mode == GEMM_STORE_F32 || c.mode == GEMM_STORE_BF16 || c.mode == GEMM_RESIDUAL));
 }
 
 int launch_gemm_layers(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream) {
@@ -1038,7 +1038,7 @@ int launch_gemm_layers(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t 
     if (c.T <= 0 || c.N <= 0 || c.op[0].K <= 0 || !c.out || (halves && (c.op[0].K != c.op[1].K || c.op[0].X != c.op[1].X))) return (int)cudaErrorInvalidValue;
     const long long rows = (long long)((c.T + 255) / 256) * (c.layers > 1 ? c.layers : 1);
     const int wide_n = halves ? 128 : 256;
-    const int bn = cheaper_width(rows * ((c.N + wide_n / 2 - 1) / (wide_n / 2)), rows * ((c.N + wide_n - 1) / wide_n), (c.op[0].K + BK - 1) / BK, ws.num_sms);
+    const int bn = cheaper_width(rows * ((c.N + wide_n / 2 - 1) / (wide_n / 2)), rows * ((c.N + wide_n - 1) / wide_n), (c.op[0].K + BK - 1) / BK, ws.num_sms, false);
     return launch_gemm_pair(c, ws, stream, bn);
 }
 

@@ -135,6 +135,12 @@ struct GemmWorkspace {
     int* status;  // device status word
     int num_sms;
     TmapCache* tmaps = nullptr;  // optional; without it every launch encodes its maps
+    // optional scratch of the stream's kernels (counters zero between launches): tiles that would be a last, mostly empty wave of
+    // the two-CTA tiles are then split along K
+    float* partials = nullptr;
+    size_t partial_floats = 0;
+    int* counters = nullptr;
+    int num_counters = 0;
 };
 // opt the kernels into their dynamic shared memory sizes (once per device, outside stream capture)
 int gemm_prepare();
@@ -142,6 +148,13 @@ int gemm_prepare();
 [[nodiscard]] int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, int force_splits = 0);
 // Two independent products of the same rows (of X matrices of their own) and K, b a GEMM_SWIGLU: one launch for at most 64 rows, else two.
 [[nodiscard]] int launch_gemm_beside(const GemmCall& a, const GemmCall& b, const GemmWorkspace& ws, cudaStream_t stream);
+// How gemm_pair.cu cuts `tiles` tiles of kb k-blocks (bn weight rows): the last `tail` tiles in `splits` parts each; expected time, and
+// that with whole tiles only.
+struct PairSplit {
+    int tail, splits;
+    double us, whole_us;
+};
+PairSplit pair_split(long long tiles, int kb, int bn, int num_sms);
 // one launch over independent layers: modes STORE_F32, STORE_BF16, SWIGLU, one operand pair
 [[nodiscard]] int launch_gemm_layers(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream);
 // The same products in true fp32 (fp32 X and out, fp32 FMA, weights still bf16): modes STORE_F32, STORE_BF16, RELU2 and

@@ -29,6 +29,38 @@ def test_tiles_match_numpy(T, N, K):
     assert (tffn.op_gemm(X, W) == out).all()
 
 
+# tiles in parts of K: all 36 in two, all 22 in three, the last six of 80 in four and three, the last eight of 82 in three; K and
+# N not multiples of a block or a tile
+@pytest.mark.parametrize("T,N,K", [(2300, 896, 4864), (2600, 300, 6000), (5000, 1024, 3000), (4865, 1000, 1800), (10400, 500, 2400)])
+def test_split_tiles_match_numpy(T, N, K):
+    test_tiles_match_numpy(T, N, K)
+
+
+def test_split_tiles_of_two_operand_pairs(tmp_path):
+    """down projections of base and expert in parts that hold the one pair, the other, or both: a prompt of 4 100 rows (16 tiles of
+    128 k-blocks in a launch, four parts each, and one of 4 rows) against the same in small portions"""
+    import synth
+    import tffn
+    shape = dict(hidden_size=256, num_hidden_layers=1, num_attention_heads=4, num_key_value_heads=2, intermediate_size=4096, vocab_size=512,
+                 tie_word_embeddings=True)
+    cfg = synth.write_model(str(tmp_path), shape, seed=21, norm_jitter=0.1)
+    synth.write_expert(str(tmp_path / "expert.bin"), cfg, seed=22)
+    m = tffn.qwen_load(str(tmp_path))
+    e = tffn.checkpoint_load(str(tmp_path / "expert.bin"), m, 0.5)
+    t = synth.prompts(1, 4100, 3, 512)[0]
+    got, want = [], []
+    for out, cuts in ((got, [4100]), (want, [100] * 41)):
+        s = tffn.Session(m, e, max_batch=1, max_seq=4160)
+        at = 0
+        for n in cuts:
+            out.append(s.qwen_forward(t[at:at + n]))
+            at += n
+        s.free()
+    got, want = np.concatenate(got), np.concatenate(want)
+    err = np.abs(got - want) / np.abs(want).max()
+    assert err.max() <= 1.5e-2 and err.mean() <= 2e-3  # as below
+
+
 @pytest.mark.parametrize("name", ["mini05", "tiny128", "mini7"])
 @pytest.mark.parametrize("expert", [False, True])
 def test_prompts_whole_and_in_portions(model_dirs, name, expert):
