@@ -898,7 +898,11 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
         // A grouped launch cannot request weights ahead of its dependency wait (the tile table comes from the kernel
         // before), so its k-loop is all exposed and shorter splits pay.
         const int min_kb = c.grp || (c.bin_counts && !c.bin_ahead) ? 3 : 8;
-        while (splits < kMaxSplits && tiles * splits * 2 <= 2 * ws.num_sms && total_kb / (splits * 2) >= min_kb) splits *= 2;
+        // From 32 tokens on a stage's products weigh more and a second CTA on a third of the SMs is as far as it pays (us a step of
+        // four layers, K 22016, N 2048: 32 tokens 381 with 16 splits, 364 with 8; 64 tokens in 32-wide tiles 462, in 64-wide ones 428
+        // and 406; K 17920, N 1536: 64 tokens 390, 352, 352).
+        const int most = BN < 32 || c.grp || c.bin_counts ? 2 * ws.num_sms : ws.num_sms + ws.num_sms / 3;
+        while (splits < kMaxSplits && tiles * splits * 2 <= most && total_kb / (splits * 2) >= min_kb) splits *= 2;
     }
     if (splits != 1 && splits != 2 && splits != 4 && splits != 8 && splits != 16) return (int)cudaErrorInvalidValue;
     if (splits > total_kb) return (int)cudaErrorInvalidValue;
@@ -1068,16 +1072,11 @@ int launch_gemm(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream,
         if (force_splits == 0 && c.mode != GEMM_SWIGLU && !c.out2 && c.T > 32 && c.T <= 64 && total_kb <= 16 &&
             n_tiles * 8 <= ws.num_sms)
             return launch_bn<32>(c, ws, stream, force_splits);
-        // A long K extent with as few tiles (the down projection): the largest cluster, 16 splits, is
+        // A long K extent with as few tiles (the down projection of the narrowest model): the largest cluster, 16 splits, is
         // not enough to fill the SMs with 64-token tiles; with 32-token tiles twice as many CTAs (two per SM)
-        // stream half as many k-blocks each (measured: 12.6 -> 11.6 us per launch inside a step).
-        if (force_splits == 0 && c.mode != GEMM_SWIGLU && !c.out2 && c.T > 32 && c.T <= 64 && total_kb >= 64 &&
-            n_tiles * 8 <= ws.num_sms) {
-            // 16 splits as long as two CTAs per SM hold them all, else 8 (16 tiles: 28 -> 14 us). The bf16 residual
-            // epilogue keeps its order of summation.
-            const bool second_wave = c.mode == GEMM_STORE_F32 && n_tiles * 2 * kMaxSplits > 2 * ws.num_sms;
-            return launch_bn<32>(c, ws, stream, second_wave ? kMaxSplits / 2 : kMaxSplits);
-        }
+        // stream half as many k-blocks each (measured: 12.6 -> 11.6 us per launch inside a step), as long as the SMs hold them all.
+        if (force_splits == 0 && c.mode != GEMM_SWIGLU && !c.out2 && c.T > 32 && c.T <= 64 && total_kb >= 64 && n_tiles * kMaxSplits <= ws.num_sms)
+            return launch_bn<32>(c, ws, stream, kMaxSplits);
     }
     // One row tile (a router): with wide token tiles a handful of CTAs would carry the whole launch and split it along
     // K, exchanging planes that are mostly padding; narrow token tiles spread it over the SMs instead.

@@ -39,3 +39,16 @@ def test_razesun_rows_of_a_prompt(tmp_path):
         e = error(s.qwen_forward(t[:n]), want[:n])
         assert e.max() <= LIMIT["bfloat16"], (n, float(e.max()))
     s.free()
+
+
+# 33 to 64 tokens and a long K: row tiles that sixteen 32-wide splits hold at once (9), one more (10), many (17), and a ragged K and N
+@pytest.mark.parametrize("T", [33, 48, 64])
+@pytest.mark.parametrize("N,K", [(1152, 4096), (1153, 4096), (2100, 4120), (130, 9000)])
+def test_long_products_match_numpy(T, N, K):
+    import synth
+    import tffn
+    rng = np.random.default_rng([T, N, K])
+    X, W = (synth.f32_to_bf16((rng.standard_normal((n, K), dtype=np.float32) * s).reshape(-1)).reshape(n, K) for n, s in ((T, 1.0), (N, 0.05)))
+    out = tffn.op_gemm(X, W)
+    ref = synth.bf16_to_f32(X).astype(np.float64) @ synth.bf16_to_f32(W).astype(np.float64).T
+    assert np.abs(out - ref).max() / np.abs(ref).max() < 2e-5  # fp32 accumulation of exact bf16 products
