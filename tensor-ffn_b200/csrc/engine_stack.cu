@@ -857,8 +857,10 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
         // and, where the experts' rows may stand in bins of T places (in tiles of up to 64 rows, within the scratch memory), puts them
         // there instead of a kernel of its own; the products find their tiles in the counts. A step of 64 sequences, 8 layers 896 wide
         // with 16 experts and 2 identity ones, four a token: 671 -> 620 us.
+        // Few choices keep the kernel: every expert's tiles are launched and wait for the counts, also those of the many without rows
+        // (a step of two sequences 464 -> 452, but of one 439 -> 487).
         const int pairs = T * sp.top, avg_tile = sp.experts > 0 ? gemm_group_tile((pairs + outs - 1) / outs) : 0;
-        const bool bins = routed && !f32 && avg_tile <= 64 && (int64_t)sp.experts * T <= (int64_t)cap_tokens_ * s.max_top;
+        const bool bins = routed && !f32 && pairs * 3 >= outs && avg_tile <= 64 && (int64_t)sp.experts * T <= (int64_t)cap_tokens_ * s.max_top;
         if (bins) {
             r.bin = T;
             r.pair_row = s.pair_row.as<int>();
