@@ -297,8 +297,11 @@ __device__ __forceinline__ void add4(float4& a, const float4& b) {
     a.w += b.w;
 }
 
-// FOLD: a launch that passes a norm on or takes one (GemmCall::norm_w, rms_ssq)
-template <int BN, bool FOLD>
+// What a launch is beyond tiles of one or two problems, of a batch or of groups: TC_FOLD passes a norm on or takes one
+// (GemmCall::norm_w, rms_ssq), TC_BINS finds its rows in bins, TC_BESIDE has another product's tiles behind its own. Kinds of their own,
+// as their tests on the way to the first load cost every launch 0.2 us (a step of 97 products 687 -> 706 us).
+enum TcKind { TC_PLAIN, TC_FOLD, TC_BINS, TC_BESIDE };
+template <int BN, int KIND>
 __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(const __grid_constant__ GemmDev p) {
     using Cfg = GemmCfg<BN>;
     extern __shared__ uint8_t smem_raw[];
@@ -313,7 +316,8 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     int prob = blockIdx.y / p.t_tiles;  // independent problems (base / expert gate-up) share a launch
-    const bool beside = p.tiles_1 > 0 && (int)blockIdx.x >= p.tiles_1;
+    constexpr bool FOLD = KIND == TC_FOLD, BINS = KIND == TC_BINS;
+    const bool beside = KIND == TC_BESIDE && (int)blockIdx.x >= p.tiles_1;
     const OutView view = beside ? OutView{p.N_2, GEMM_SWIGLU, p.ldo_2} : OutView{p.N, p.mode, p.ldo};
     const int n0 = beside ? ((int)blockIdx.x - p.tiles_1) * (BM / 2) : (int)blockIdx.x * p.tile_n;
     int t0 = (blockIdx.y % p.t_tiles) * BN, t_end = p.T, w_row0 = n0;
@@ -330,10 +334,10 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
     }
     // bins: which weights this CTA needs does not depend on the counts, only how many rows there are
     // (the groups' first tiles come first: the others are mostly empty and would hold their places)
-    const int group = p.bins ? (int)blockIdx.y % p.bin_groups : 0, bin0 = group * p.bin;
+    const int group = BINS ? (int)blockIdx.y % p.bin_groups : 0, bin0 = group * p.bin;
     auto bin_end = [&] { return min(bin0 + min(p.bin, __ldcg(p.bins + group)), t0 + BN); };
     bool count_later = false;
-    if (p.bins) {
+    if constexpr (BINS) {
         t0 = bin0 + (int)blockIdx.y / p.bin_groups * BN;
         w_row0 = group * p.N + n0;
         prob = 0;
@@ -476,23 +480,15 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
             t_end = bin_end();
             if (threadIdx.x == 64) *tile_end = t_end;
         }
-        if (FOLD && p.rms_ssq) {
-            // 128 / BN neighbouring lanes per token, their loads in flight together
-            constexpr int L = (kGemmThreads - 64) / BN < 1 ? 1 : (kGemmThreads - 64) / BN;
-            const int j = ((int)threadIdx.x - 64) / L, sub = (int)threadIdx.x % L;
-            float ss = 0.f;
-            if (t0 + j < t_end) {
-                const float* from = p.rms_ssq + (size_t)(t0 + j) * p.rms_tiles;
-                for (int i0 = sub; i0 < p.rms_tiles; i0 += 4 * L) {
-                    float v[4];
+        // the row factors: 128 / BN neighbouring lanes per token. Their loads are requested here and used behind the requests below.
+        constexpr int L = (kGemmThreads - 64) / BN < 1 ? 1 : (kGemmThreads - 64) / BN;
+        const int rj = ((int)threadIdx.x - 64) / L, sub = (int)threadIdx.x % L;
+        const float* from = p.rms_ssq + (size_t)(t0 + rj) * p.rms_tiles;
+        float part[4] = {0.f, 0.f, 0.f, 0.f};
+        if (FOLD && p.rms_ssq && t0 + rj < t_end) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) v[u] = i0 + u * L < p.rms_tiles ? __ldcg(from + i0 + u * L) : 0.f;
-                    ss += (v[0] + v[1]) + (v[2] + v[3]);
-                }
-            }
-#pragma unroll
-            for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            if (sub == 0) row_factor[j] = rsqrtf(ss / (float)p.rms_n + p.rms_eps);
+            for (int u = 0; u < 4; ++u)
+                if (sub + u * L < p.rms_tiles) part[u] = __ldcg(from + sub + u * L);
         }
         if (p.splits > 1) {
             // split-K: the (at most two) columns this warp will finish are known; fetch their operands now
@@ -505,6 +501,18 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
                     else if (p.mode == GEMM_RESIDUAL) prefetch_residual(p, view, out, n0 + lane * 4, t, pre[u]);
                 }
             }
+        }
+        if (FOLD && p.rms_ssq) {
+            float ss = (part[0] + part[1]) + (part[2] + part[3]);
+            for (int i0 = sub + 4 * L; i0 < p.rms_tiles && t0 + rj < t_end; i0 += 4 * L) {
+                float v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = i0 + u * L < p.rms_tiles ? __ldcg(from + i0 + u * L) : 0.f;
+                ss += (v[0] + v[1]) + (v[2] + v[3]);
+            }
+#pragma unroll
+            for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (sub == 0) row_factor[rj] = rsqrtf(ss / (float)p.rms_n + p.rms_eps);
         }
         // every lane waits (acquire); the outcome is made warp-uniform because tcgen05.ld is .aligned
         bool ok = mbar_wait(acc_full, 0, p.status, DEV_ERR_ACC_WAIT);
@@ -785,7 +793,7 @@ int max_active_clusters(const cudaLaunchConfig_t& cfg, int stages, int splits) {
     int n = 0;
     cudaLaunchConfig_t q = cfg;
     q.dynamicSmemBytes = GemmCfg<BN>::smem_bytes(stages);
-    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<BN, false>, &q) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_tc<BN, TC_PLAIN>, &q) != cudaSuccess) {
         cudaGetLastError();
         n = 1 << 30;  // unknown: keep the configuration
     }
@@ -898,10 +906,10 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
         // A grouped launch cannot request weights ahead of its dependency wait (the tile table comes from the kernel
         // before), so its k-loop is all exposed and shorter splits pay.
         const int min_kb = c.grp || (c.bin_counts && !c.bin_ahead) ? 3 : 8;
-        // From 32 tokens on a stage's products weigh more and a second CTA on a third of the SMs is as far as it pays (us a step of
+        // From 32 to 64 tokens a stage's products weigh more and a second CTA on a third of the SMs is as far as it pays (us a step of
         // four layers, K 22016, N 2048: 32 tokens 381 with 16 splits, 364 with 8; 64 tokens in 32-wide tiles 462, in 64-wide ones 428
         // and 406; K 17920, N 1536: 64 tokens 390, 352, 352).
-        const int most = BN < 32 || c.grp || c.bin_counts ? 2 * ws.num_sms : ws.num_sms + ws.num_sms / 3;
+        const int most = (BN != 32 && BN != 64) || c.grp || c.bin_counts ? 2 * ws.num_sms : ws.num_sms + ws.num_sms / 3;
         while (splits < kMaxSplits && tiles * splits * 2 <= most && total_kb / (splits * 2) >= min_kb) splits *= 2;
     }
     if (splits != 1 && splits != 2 && splits != 4 && splits != 8 && splits != 16) return (int)cudaErrorInvalidValue;
@@ -962,9 +970,12 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
             cfg.dynamicSmemBytes = Cfg::smem_bytes(p.stages);
         }
     }
-    if constexpr (BN <= kFoldTokens)
-        if (p.norm_w || p.rms_ssq) return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, true>, p);
-    return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, false>, p);
+    if constexpr (BN <= kFoldTokens) {
+        if (p.norm_w || p.rms_ssq) return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, TC_FOLD>, p);
+        if (p.bins) return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, TC_BINS>, p);
+        if (beside) return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, TC_BESIDE>, p);
+    }
+    return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, TC_PLAIN>, p);
 }
 
 }  // namespace
@@ -976,15 +987,17 @@ bool make_tmap_2d(TmapCache* cache, CUtensorMap* tm, const bf16* ptr, uint64_t r
 
 int gemm_prepare() {
     cudaError_t e;
-#define TFFN_PREP(BN, FOLD)                                                                                                 \
-    e = cudaFuncSetAttribute(k_gemm_tc<BN, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem); \
+#define TFFN_PREP(BN, KIND)                                                                                                 \
+    e = cudaFuncSetAttribute(k_gemm_tc<BN, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem); \
     if (e != cudaSuccess) return (int)e;                                                                             \
-    e = cudaFuncSetAttribute(k_gemm_tc<BN, FOLD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);                     \
+    e = cudaFuncSetAttribute(k_gemm_tc<BN, KIND>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);                     \
     if (e != cudaSuccess) return (int)e;                                                                             \
-    e = prefer_max_shared(k_gemm_tc<BN, FOLD>);                                                                            \
+    e = prefer_max_shared(k_gemm_tc<BN, KIND>);                                                                            \
     if (e != cudaSuccess) return (int)e;
-    TFFN_PREP(16, false) TFFN_PREP(32, false) TFFN_PREP(64, false) TFFN_PREP(128, false) TFFN_PREP(256, false)
-    TFFN_PREP(16, true) TFFN_PREP(32, true) TFFN_PREP(64, true)
+    TFFN_PREP(16, TC_PLAIN) TFFN_PREP(32, TC_PLAIN) TFFN_PREP(64, TC_PLAIN) TFFN_PREP(128, TC_PLAIN) TFFN_PREP(256, TC_PLAIN)
+    TFFN_PREP(16, TC_FOLD) TFFN_PREP(32, TC_FOLD) TFFN_PREP(64, TC_FOLD)
+    TFFN_PREP(16, TC_BINS) TFFN_PREP(32, TC_BINS) TFFN_PREP(64, TC_BINS)
+    TFFN_PREP(16, TC_BESIDE) TFFN_PREP(32, TC_BESIDE) TFFN_PREP(64, TC_BESIDE)
 #undef TFFN_PREP
     return gemm_pair_prepare();
 }

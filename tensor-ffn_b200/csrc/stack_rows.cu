@@ -28,15 +28,16 @@ __device__ __forceinline__ float as_stored(float v, const float*) { return v; }
 __device__ __forceinline__ float as_stored(float v, const bf16*) { return bf16_round(v); }
 
 // The pass over rows whose width is a multiple of 4: a thread keeps its IT groups of four columns in registers from the
-// first load to the last store, all loads of a phase in flight together.
-template <typename A, int IT>
+// first load to the last store, all loads of a phase in flight together. ROUTE: with a router (a kind of its own: what it needs cost
+// the plain passes of 4 096 rows 896 wide 1.5 to 2 us of 13).
+template <typename A, int IT, bool ROUTE>
 __global__ void __launch_bounds__(512) k_residual_rows4(const ResidualRows a, unsigned long long* tl) {
     extern __shared__ float rows4_smem[];  // with a router: the row as stored [H], logits [n], scratch [n]
     __shared__ float red[32];
     if (threadIdx.x == 0) tl_mark(tl, 0);
     pdl_launch_dependents();
     const int H = a.H, r = blockIdx.x, n = blockDim.x, tid = threadIdx.x;
-    if (a.router_w) {  // its rows have left L2 since the last step: request them now, one line per thread
+    if constexpr (ROUTE) {  // the router's rows have left L2 since the last step: request them now, one line per thread
         const char* w = (const char*)a.router_w;
         const size_t bytes = (size_t)(a.route.experts + a.route.identity) * a.router_ld * sizeof(bf16);
         for (size_t o = ((size_t)r * n + tid) * 128; o < bytes; o += (size_t)gridDim.x * n * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + o));
@@ -178,14 +179,14 @@ __global__ void __launch_bounds__(512) k_residual_rows4(const ResidualRows a, un
                     for (int c = 0; c < 4; ++c) v2[c] = x[k][c] * inv * w2[c];
                     store4((A*)a.out2 + (size_t)r * a.out_ld + i, v2);
                 }
-                if (a.router_w) {
+                if constexpr (ROUTE) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) rows4_smem[i + c] = as_stored(v[c], out);
                 }
             }
         }
     }
-    if (a.router_w) {
+    if constexpr (ROUTE) {
         // logits: one warp per output, the row from shared memory, 16 bytes of weights per lane and step (H % 8 == 0)
         const int warp = tid >> 5, lane = tid & 31, outs = a.route.experts + a.route.identity;
         float* z = rows4_smem + H;
@@ -426,8 +427,9 @@ constexpr int kRowsMaxSmem = 128 * 1024;
 
 template <typename A, int IT>
 cudaError_t rows4_attrs() {
-    cudaError_t e = cudaFuncSetAttribute(k_residual_rows4<A, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsMaxSmem);
-    return e == cudaSuccess ? prefer_max_shared(k_residual_rows4<A, IT>) : e;
+    cudaError_t e = cudaFuncSetAttribute(k_residual_rows4<A, IT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsMaxSmem);
+    if (e == cudaSuccess) e = prefer_max_shared(k_residual_rows4<A, IT, true>);
+    return e == cudaSuccess ? prefer_max_shared(k_residual_rows4<A, IT, false>) : e;
 }
 template <typename A>
 cudaError_t rows4_attrs_all() {
@@ -466,10 +468,14 @@ static void launch_rows(const ResidualRows& a, int rows, cudaStream_t s, bool pd
     const int per = groups <= 256 ? 1 : groups <= 1024 ? 2 : groups <= 2048 ? 4 : 8;
     const int threads = ((groups + per - 1) / per + 31) / 32 * 32;
     const dim3 grid(rows), block(a.router_w ? 512 : threads);  // routing: as many warps for the router's outputs as fit
-    if (per == 1) launch_k(k_residual_rows4<A, 1>, grid, block, smem, s, pdl, a, tl);
-    else if (per == 2) launch_k(k_residual_rows4<A, 2>, grid, block, smem, s, pdl, a, tl);
-    else if (per == 4) launch_k(k_residual_rows4<A, 4>, grid, block, smem, s, pdl, a, tl);
-    else launch_k(k_residual_rows4<A, 8>, grid, block, smem, s, pdl, a, tl);
+    auto go = [&](auto plain, auto route) {
+        if (a.router_w) launch_k(route, grid, block, smem, s, pdl, a, tl);
+        else launch_k(plain, grid, block, smem, s, pdl, a, tl);
+    };
+    if (per == 1) go(k_residual_rows4<A, 1, false>, k_residual_rows4<A, 1, true>);
+    else if (per == 2) go(k_residual_rows4<A, 2, false>, k_residual_rows4<A, 2, true>);
+    else if (per == 4) go(k_residual_rows4<A, 4, false>, k_residual_rows4<A, 4, true>);
+    else go(k_residual_rows4<A, 8, false>, k_residual_rows4<A, 8, true>);
 }
 void launch_residual_rows(const ResidualRows& a, bool f32, int rows, cudaStream_t s, bool pdl, unsigned long long* tl) {
     if (f32) launch_rows<float>(a, rows, s, pdl, tl);
