@@ -460,19 +460,23 @@ int launch_gemm_f32(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t str
     for (int i = 0; i < 2; ++i)
         if (p.X[i] && ((uintptr_t)p.X[i] % 16 || (uintptr_t)p.W[i] % 16 || p.ldx[i] % 4 || p.ldw[i] % 8)) vec = false;
     const int probs = c.out2 ? 2 : p.batch, t_tiles = c.grp ? c.grp_tiles : (c.T + TB - 1) / TB;
-    // A tile of 64 tokens costs the same for one as for 64; streaming the rows costs as much again for every eight.
-    if (vec && c.T <= kRowTokens) {
-        const int K = p.K[0] > p.K[1] ? p.K[0] : p.K[1];
+    // A tile of 64 tokens costs the same for one as for 64; streaming the rows costs as much again for every eight. Groups go by
+    // their average, rounded up to leave room (a group of more rows reads its weights again,
+    // from L2). 16 experts, 896 x 1 792, four a token, us a launch: 4 pairs 13 -> 7, 8 pairs 41 -> 11; in tiles of 64: 16 pairs 110 -> 18.
+    const int live_tiles = !c.grp ? t_tiles : c.grp_rows_hint > 0 && c.grp_rows_hint < t_tiles ? c.grp_rows_hint : t_tiles;
+    const int avg = c.grp ? (c.T + live_tiles - 1) / live_tiles : c.T, at_once = c.grp && avg < c.T ? 2 * avg : avg;
+    if (vec && at_once <= kRowTokens) {
+        const int K = p.K[0] > p.K[1] ? p.K[0] : p.K[1], tokens = at_once <= 2 ? at_once : at_once <= 4 ? 4 : kRowTokens;
         p.lanes = p.K[1] > 0 ? 32 : 8;
         while (p.lanes < kThreads && p.lanes * 8 < K) p.lanes *= 2;
-        const int rows = kThreads / p.lanes * rows_per_thread(c.T), groups = (c.N + rows - 1) / rows;
+        const int rows = kThreads / p.lanes * rows_per_thread(tokens), groups = (c.N + rows - 1) / rows;
         // two blocks per SM; more groups than that are walked over, so that their weights are requested ahead
-        const int most = (2 * ws.num_sms + t_tiles * probs - 1) / (t_tiles * probs);
-        const dim3 grid(c.grp || groups <= most ? groups : most, t_tiles, probs);
-        auto go = [&](auto kern) { return (int)launch_k(kern, grid, dim3(kThreads), rows_smem(c.T == 3 ? 4 : c.T > 4 ? 8 : c.T), stream, c.pdl, p); };
-        if (K <= p.lanes * 8 && !c.grp && (p.K[1] <= 0 || (p.K[1] == p.K[0] && p.X[1] == p.X[0] && p.ldx[1] == p.ldx[0])) && c.T <= 4)
-            return c.T == 1 ? go(k_gemm_f32_rows<1, true>) : c.T == 2 ? go(k_gemm_f32_rows<2, true>) : go(k_gemm_f32_rows<4, true>);
-        return c.T == 1 ? go(k_gemm_f32_rows<1, false>) : c.T == 2 ? go(k_gemm_f32_rows<2, false>) : c.T <= 4 ? go(k_gemm_f32_rows<4, false>) : go(k_gemm_f32_rows<8, false>);
+        const int most = (2 * ws.num_sms + live_tiles * probs - 1) / (live_tiles * probs);
+        const dim3 grid(groups <= most ? groups : most, t_tiles, probs);
+        auto go = [&](auto kern) { return (int)launch_k(kern, grid, dim3(kThreads), rows_smem(tokens), stream, c.pdl, p); };
+        if (K <= p.lanes * 8 && (p.K[1] <= 0 || (p.K[1] == p.K[0] && p.X[1] == p.X[0] && p.ldx[1] == p.ldx[0])) && tokens <= 4)
+            return tokens == 1 ? go(k_gemm_f32_rows<1, true>) : tokens == 2 ? go(k_gemm_f32_rows<2, true>) : go(k_gemm_f32_rows<4, true>);
+        return tokens == 1 ? go(k_gemm_f32_rows<1, false>) : tokens == 2 ? go(k_gemm_f32_rows<2, false>) : tokens == 4 ? go(k_gemm_f32_rows<4, false>) : go(k_gemm_f32_rows<8, false>);
     }
     // splits until the chip is full once, at least four slices each
     const long long tiles = (long long)((c.N + NB - 1) / NB) * t_tiles * probs;
