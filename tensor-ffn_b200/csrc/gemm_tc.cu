@@ -1024,7 +1024,10 @@ int cheaper_width(long long narrow, long long wide, int kb, int num_sms, bool ca
 //    it cannot make up for the wider tile (N 4608, K 3584: 160 tokens 50 -> 28, 128 tokens 25 -> 28); very short ones from 65.
 //  * A long K extent with few tiles is split over clusters here: 14 wide tiles of 152 k-blocks 14 -> 50. The wide tiles win
 //    once they are about a quarter of the k-blocks in number, or nearly fill the chip (K 4864, N 896: 768 tokens 39 -> 29,
-//    512 tokens 21 -> 29; two pairs of that K: 1 000 tokens 49 -> 54, 2 048 tokens 80 -> 56).
+//    512 tokens 21 -> 29; two pairs of that K: 1 000 tokens 49 -> 54, 2 048 tokens 80 -> 56), or, where they can be split too, from
+//    2 700 narrow tiles' k-blocks on (with 6 us of launch: K 11008, N 2048: 130 tokens 55 -> 43, 512 tokens 81 -> 44; K 17920 of two
+//    pairs, N 1536: 130 tokens 46 -> 49, 512 tokens 70 -> 50, 1 000 tokens 109 -> 60; K 37888, N 3584: 130 tokens 95 -> 80; below:
+//    K 9728, N 896: 384 tokens 39 -> 41, 256 tokens 25 -> 30).
 //  * One narrow row tile (a router) needs many tokens (K 896: 4 096 tokens 14 -> 8; K 2048: 768 tokens 9 -> 13).
 int pair_width(const GemmCall& c, const GemmWorkspace& ws) {
     if (c.amax_val || c.norm_w || c.rms_ssq || c.bin_counts || (!c.out && c.mode != GEMM_QKV) || (c.grp && c.grp_bn != 256)) return 0;
@@ -1038,16 +1041,17 @@ int pair_width(const GemmCall& c, const GemmWorkspace& ws) {
     const int kb = (c.op[0].K + BK - 1) / BK + (c.op[1].K > 0 && !halves ? (c.op[1].K + BK - 1) / BK : 0);
     const long long rows = (c.grp ? (c.grp_rows_hint > 0 ? c.grp_rows_hint : c.grp_tiles) : (c.T + 255) / 256) * (batched ? (long long)c.batch : c.out2 ? 2 : 1);
     const long long wide = rows * ((c.N + (halves ? 127 : 255)) / (halves ? 128 : 256)), narrow = rows * ((c.N + (halves ? 63 : 127)) / (halves ? 64 : 128));
+    const bool can_split = !c.grp && ws.partials && (c.mode == GEMM_STORE_F32 || c.mode == GEMM_STORE_BF16 || c.mode == GEMM_RESIDUAL);
     if (!c.grp) {
         if (c.N <= BM && !batched && !halves) {
             if (c.T < 2048) return 0;
         } else if (c.T <= (halves || kb <= 8 ? 64 : 128)) {
             return 0;
-        } else if (!halves && kb > 56 && narrow * 4 < (kb < 240 ? kb : 240)) {
+        } else if (!halves && kb > 56 && narrow * 4 < (kb < 240 ? kb : 240) && (!can_split || narrow * kb < 2700)) {
             return 0;
         }
     }
-    return cheaper_width(narrow, wide, kb, ws.num_sms, !c.grp && ws.partials && (c.mode == GEMM_STORE_F32 || c.mode == GEMM_STORE_BF16 || c.mode == GEMM_RESIDUAL));
+    return cheaper_width(narrow, wide, kb, ws.num_sms, can_split);
 }
 
 int launch_gemm_layers(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream) {

@@ -30,8 +30,9 @@ def test_tiles_match_numpy(T, N, K):
 
 
 # tiles in parts of K: all 36 in two, all 22 in three, the last six of 80 in four and three, the last eight of 82 in three; K and
-# N not multiples of a block or a tile
-@pytest.mark.parametrize("T,N,K", [(2300, 896, 4864), (2600, 300, 6000), (5000, 1024, 3000), (4865, 1000, 1800), (10400, 500, 2400)])
+# N not multiples of a block or a tile; then few tiles of a long K on both sides of where the one-CTA tiles' clusters end
+@pytest.mark.parametrize("T,N,K", [(2300, 896, 4864), (2600, 300, 6000), (5000, 1024, 3000), (4865, 1000, 1800), (10400, 500, 2400),
+                                   (129, 2048, 10800), (131, 2048, 10816), (256, 1500, 17920), (400, 896, 9728), (700, 900, 9728)])
 def test_split_tiles_match_numpy(T, N, K):
     test_tiles_match_numpy(T, N, K)
 
