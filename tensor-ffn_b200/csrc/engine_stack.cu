@@ -753,7 +753,8 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
             step(KC_LRU_PREP, [&](unsigned long long* tl) { launch_lru_prep(u, f32, T, stream_, pdl, tl); });
             batched(KC_GEMM_LRU, sp.lru_blocks, l.lru_gates.as<bf16>(), pad8(n), s.u.p, s.u_ld, u.u_part, n, 2 * n, GEMM_STORE_F32,
                     s.lru_gate.p, s.lru_gate_ld, 2 * n);
-            step(KC_LRU_SCAN, [&](unsigned long long* tl) { launch_lru_scan(u, f32, n_segs, decode, stream_, pdl, tl); });
+            // a prompt's few, long CTAs start when every SM is free (see k_delta_prep): 3 000 tokens 2 048 wide 6 400 -> 6 355 us in all
+            step(KC_LRU_SCAN, [&](unsigned long long* tl) { launch_lru_scan(u, f32, n_segs, decode, stream_, pdl && decode, tl); });
         } else {
             const bool per_head = sp.mixer == Mixer::Delta;  // decay and gate logits are part of the input projection
             if (!per_head) {
@@ -814,6 +815,7 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
             d.seg_first = seg_first;
             d.seg_count = seg_count;
             d.max_slots = max_batch_;
+            d.prompt = !decode;
             d.status = status;
             const bool fuse_out = decode && cache.dimP <= 128;
             step(KC_DELTA_PREP, [&](unsigned long long* tl) { launch_delta_prep(d, f32, T, stream_, pdl, tl); });

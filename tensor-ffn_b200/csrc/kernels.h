@@ -462,6 +462,7 @@ struct DeltaRule {
     const int *tok_seq, *tok_pos;
     const int *seg_first, *seg_count;  // runs of consecutive positions of one sequence among the T rows
     int max_slots;
+    bool prompt;  // the preparation lets the scan start at its end, not its beginning
     int* status;
 };
 void launch_delta_prep(const DeltaRule& a, bool f32, int T, cudaStream_t s, bool pdl, unsigned long long* tl = nullptr);
