@@ -8,8 +8,8 @@
 //           as records [gate row | up row | down column] of the base FFN and of the expert
 //           FFN side by side (bulk copies into a shared-memory ring, mbarrier-tracked),
 //           forms act = silu(g)*u for both, accumulates act_b*down_b + scale*act_e*down_e for
-//           all H outputs in registers, and the per-CTA partial sums are folded by a two-level
-//           ticket (last CTA of a group, then last group) in a fixed order into the residual
+//           all H outputs in registers, and the per-CTA sums are added to the layer's fixed-point
+//           accumulator, which the next kernel folds into the residual
 //   lmhead  final RMSNorm + tied LM-head rows streamed through the same kind of ring +
 //           arg-max (lowest index among maxima); the last CTA publishes the next token
 //
