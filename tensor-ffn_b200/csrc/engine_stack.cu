@@ -519,6 +519,7 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
         g.mode = mode;
         g.out = out;
         g.ldo = ldo;
+        g.mixed = true;
         return g;
     };
     auto run_product = [&](int cls, const bf16* W, int64_t ldw, const void* X, int64_t ldx, int K, int N, int mode, void* out, int64_t ldo) {

@@ -297,10 +297,12 @@ __device__ __forceinline__ void add4(float4& a, const float4& b) {
     a.w += b.w;
 }
 
-// What a launch is beyond tiles of one or two problems, of a batch or of groups: TC_FOLD passes a norm on or takes one
-// (GemmCall::norm_w, rms_ssq), TC_BINS finds its rows in bins, TC_BESIDE has another product's tiles behind its own. Kinds of their own,
-// as their tests on the way to the first load cost every launch 0.2 us (a step of 97 products 687 -> 706 us).
-enum TcKind { TC_PLAIN, TC_FOLD, TC_BINS, TC_BESIDE };
+// What a launch can be beyond tiles of one or two problems, of a batch or of groups: TC_FOLD passes a norm on or takes one
+// (GemmCall::norm_w, rms_ssq), TC_MIXED finds its rows in bins or has another product's tiles behind its own. The tests for the latter on the
+// way to the first load cost every launch 0.2 us (a step of 97 products 687 -> 706 us), but the steps that have such launches run all of
+// theirs as one kind (GemmCall::mixed): a kernel of its own for some of them was not in the SMs' instruction caches when its turn came
+// (16 sequences, parallel blocks, first products 6.5 -> 7.8 us, step 322 -> 342).
+enum TcKind { TC_PLAIN, TC_FOLD, TC_MIXED };
 template <int BN, int KIND>
 __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(const __grid_constant__ GemmDev p) {
     using Cfg = GemmCfg<BN>;
@@ -316,8 +318,8 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     int prob = blockIdx.y / p.t_tiles;  // independent problems (base / expert gate-up) share a launch
-    constexpr bool FOLD = KIND == TC_FOLD, BINS = KIND == TC_BINS;
-    const bool beside = KIND == TC_BESIDE && (int)blockIdx.x >= p.tiles_1;
+    constexpr bool FOLD = KIND == TC_FOLD;
+    const bool bins = KIND == TC_MIXED && p.bins, beside = KIND == TC_MIXED && p.tiles_1 > 0 && (int)blockIdx.x >= p.tiles_1;
     const OutView view = beside ? OutView{p.N_2, GEMM_SWIGLU, p.ldo_2} : OutView{p.N, p.mode, p.ldo};
     const int n0 = beside ? ((int)blockIdx.x - p.tiles_1) * (BM / 2) : (int)blockIdx.x * p.tile_n;
     int t0 = (blockIdx.y % p.t_tiles) * BN, t_end = p.T, w_row0 = n0;
@@ -334,10 +336,10 @@ __global__ void __launch_bounds__(kGemmThreads, (BN <= 64) ? 2 : 1) k_gemm_tc(co
     }
     // bins: which weights this CTA needs does not depend on the counts, only how many rows there are
     // (the groups' first tiles come first: the others are mostly empty and would hold their places)
-    const int group = BINS ? (int)blockIdx.y % p.bin_groups : 0, bin0 = group * p.bin;
+    const int group = bins ? (int)blockIdx.y % p.bin_groups : 0, bin0 = group * p.bin;
     auto bin_end = [&] { return min(bin0 + min(p.bin, __ldcg(p.bins + group)), t0 + BN); };
     bool count_later = false;
-    if constexpr (BINS) {
+    if (bins) {
         t0 = bin0 + (int)blockIdx.y / p.bin_groups * BN;
         w_row0 = group * p.N + n0;
         prob = 0;
@@ -972,8 +974,7 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
     }
     if constexpr (BN <= kFoldTokens) {
         if (p.norm_w || p.rms_ssq) return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, TC_FOLD>, p);
-        if (p.bins) return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, TC_BINS>, p);
-        if (beside) return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, TC_BESIDE>, p);
+        if (p.bins || beside || c.mixed) return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, TC_MIXED>, p);
     }
     return (int)cudaLaunchKernelEx(&cfg, k_gemm_tc<BN, TC_PLAIN>, p);
 }
@@ -996,8 +997,7 @@ int gemm_prepare() {
     if (e != cudaSuccess) return (int)e;
     TFFN_PREP(16, TC_PLAIN) TFFN_PREP(32, TC_PLAIN) TFFN_PREP(64, TC_PLAIN) TFFN_PREP(128, TC_PLAIN) TFFN_PREP(256, TC_PLAIN)
     TFFN_PREP(16, TC_FOLD) TFFN_PREP(32, TC_FOLD) TFFN_PREP(64, TC_FOLD)
-    TFFN_PREP(16, TC_BINS) TFFN_PREP(32, TC_BINS) TFFN_PREP(64, TC_BINS)
-    TFFN_PREP(16, TC_BESIDE) TFFN_PREP(32, TC_BESIDE) TFFN_PREP(64, TC_BESIDE)
+    TFFN_PREP(16, TC_MIXED) TFFN_PREP(32, TC_MIXED) TFFN_PREP(64, TC_MIXED)
 #undef TFFN_PREP
     return gemm_pair_prepare();
 }

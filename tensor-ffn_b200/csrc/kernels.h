@@ -85,6 +85,7 @@ struct GemmCall {
     const struct GroupTile* grp;
     int grp_tiles, grp_bn, grp_count;  // grp_count: groups in W
     int grp_rows_hint;                 // tiles that will be in use, about (0: all)
+    bool mixed;  // one of a step's launches some of which use bins or have a product beside them: runs the same kernel (k_gemm_tc)
     // Grouped launch over bins instead of a table: group g's rows are [g * bin, g * bin + bin_counts[g]) of X and out, counts
     // written by an earlier kernel. grp_count groups, token tiles of grp_bn (at most 64) rows. With bin_ahead the groups are taken
     // to be not empty, and the first weights of their first tiles are requested ahead of the dependency wait.
