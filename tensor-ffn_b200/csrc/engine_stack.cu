@@ -861,10 +861,14 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
         // there instead of a kernel of its own; the products find their tiles in the counts. A step of 64 sequences, 8 layers 896 wide
         // with 16 experts and 2 identity ones, four a token: 671 -> 620 us.
         // Few choices keep the kernel: every expert's tiles are launched and wait for the counts, also those of the many without rows
-        // (a step of two sequences 464 -> 452, but of one 439 -> 487).
-        const int pairs = T * sp.top, avg_tile = sp.experts > 0 ? gemm_group_tile((pairs + outs - 1) / outs) : 0;
-        const bool bins = routed && !f32 && pairs * 3 >= outs && avg_tile <= 64 && (int64_t)sp.experts * T <= (int64_t)cap_tokens_ * s.max_top;
+        // (a step of two sequences 464 -> 452, but of one 439 -> 487). So do more tiles than two an SM: the bins' empty tiles come behind them
+        // (32 experts of 1 536, 2 048 wide, 64 sequences: 36 -> 45 us a launch).
+        const int pairs = T * sp.top;
+        int avg_tile = sp.experts > 0 ? gemm_group_tile((pairs + outs - 1) / outs) : 0;
+        const int64_t expert_tiles = (int64_t)sp.experts * ((std::max(sp.ff, H) + 127) / 128);
+        const bool bins = routed && !f32 && pairs * 3 >= outs && expert_tiles <= 2 * m_->num_sms && avg_tile <= 64 && (int64_t)sp.experts * T <= (int64_t)cap_tokens_ * s.max_top;
         if (bins) {
+            while (avg_tile * 2 < T) avg_tile *= 2;  // two tiles a bin: all are launched, and more would mostly be empty (48 -> 45 us there)
             r.bin = T;
             r.pair_row = s.pair_row.as<int>();
             r.xg = s.xg.p;
