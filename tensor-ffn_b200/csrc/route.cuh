@@ -3,6 +3,7 @@
 #pragma once
 #include "act.cuh"
 #include "ptx.cuh"
+#include <cfloat>
 
 namespace tffn {
 
@@ -32,29 +33,28 @@ __device__ __forceinline__ void route_token(const MoeRoute& a, int t, float* s, 
             ((int*)choice)[j] = row;
         }
     };
+    // What can be chosen is at least -FLT_MAX (a correction of -inf retires an entry; NaN inputs), what has been chosen is -inf: a token
+    // never chooses an entry twice, so an expert has at most T rows, as many as a bin holds.
+    auto score = [&](int i) { return fmaxf(s[i] + __ldg(a.correction + i), -FLT_MAX); };
     if (n <= 32) {
         // a lane per entry: its rank is the number of entries chosen before it (larger, or equal and earlier)
         float c = -INFINITY;
         if (lane < n) {
             s[lane] *= inv;
-            c = s[lane] + __ldg(a.correction + lane);
+            c = score(lane);
         }
-        if (__all_sync(0xffffffffu, lane >= n || c > -INFINITY)) {  // else (NaN inputs) as below
-            int rank = 0;
-            for (int j = 0; j < n; ++j) {
-                const float o = __shfl_sync(0xffffffffu, c, j);
-                rank += o > c || (o == c && j < lane) ? 1 : 0;
-            }
-            __syncwarp();
-            if (lane < n && rank < a.top) put(rank, lane);
-            return;
+        int rank = 0;
+        for (int j = 0; j < n; ++j) {
+            const float o = __shfl_sync(0xffffffffu, c, j);
+            rank += o > c || (o == c && j < lane) ? 1 : 0;
         }
-        if (lane < n) choice[lane] = c;
-    } else {
-        for (int i = lane; i < n; i += 32) {
-            s[i] *= inv;
-            choice[i] = s[i] + __ldg(a.correction + i);
-        }
+        __syncwarp();
+        if (lane < n && rank < a.top) put(rank, lane);
+        return;
+    }
+    for (int i = lane; i < n; i += 32) {
+        s[i] *= inv;
+        choice[i] = score(i);
     }
     int mine[2] = {-1, -1};  // lane j keeps choices j and 32 + j (top <= 64)
     for (int j = 0; j < a.top; ++j) {
@@ -68,7 +68,6 @@ __device__ __forceinline__ void route_token(const MoeRoute& a, int t, float* s, 
             const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
             if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
         }
-        if (bi >= n) bi = j;  // no finite score is left (NaN inputs): stay in range
         if ((bi & 31) == lane) choice[bi] = -INFINITY;
         if ((j & 31) == lane) mine[j >> 5] = bi;
     }

@@ -28,3 +28,24 @@ def test_full_and_empty_bins(tmp_path, experts, top, identity, compute):
         assert e.max() <= LIMIT[compute], (n, float(e.max()))
     assert s.status() == 0
     s.free()
+
+
+@pytest.mark.parametrize("compute", ["bfloat16", "float32"])
+@pytest.mark.parametrize("experts,top,identity,live", [(12, 3, 0, [7]), (3, 3, 0, [2]), (5, 2, 1, []), (40, 4, 2, [5, 39]), (70, 6, 6, [69, 70])])
+def test_fewer_live_experts_than_choices(tmp_path, experts, top, identity, live, compute):
+    """corrections of -inf (retired experts) leave fewer entries than a token chooses: the first of the others are taken, each once"""
+    def edit(name, x):
+        if name.endswith("correction"):
+            y = np.full_like(x, -np.inf)
+            y[live] = x[live]
+            return y
+    c = Case(tmp_path, rafilix_config(64, 97, [attention_layer(2, 1, 16, 16, chunk=20, mlp=moe_mlp(experts, top, 40, identity=identity))]), edit=edit)
+    t = c.tokens(130)
+    want, _ = c.expect(t)
+    s = c.session(compute, max_seq=160)
+    for n in (1, 2, 3, 16, 17, 64, 65, 128, 130):
+        s.qwen_reset()
+        e = error(s.qwen_forward(t[:n]), want[:n])
+        assert e.max() <= LIMIT[compute], (n, float(e.max()))
+    assert s.status() == 0
+    s.free()
