@@ -2,12 +2,10 @@
 #include "launch.h"
 #include "upload.h"
 #include <algorithm>
-#include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
-#include <future>
 #include <memory>
-#include <system_error>
 #include <thread>
 
 namespace tffn {
@@ -543,48 +541,96 @@ void Session::ensure_logits(size_t rows) {
     logits_rows_ = rows;
     drop_graphs();  // captured steps hold the old pointer
 }
-// Device to pageable host memory in chunks through pinned buffers, one per thread: the threads bring the destination's pages in
-// while the device is still busy with the step, then copy out of their buffers side by side. A plain copy of 39 MB (64 rows of the
-// Qwen2 vocabulary) into fresh pages took 8.6 ms behind a step of 1.15 ms, this one 1.7 to 3.2. Returns when the data is there.
+// Device to pageable host memory in chunks through a ring of pinned buffers. The calling thread enqueues every copy: the session's stream
+// may be the per-thread default stream, which is another stream in every thread. The other threads bring the destination's pages in while
+// the device is still busy with the step, then copy the chunks out of the ring side by side. A plain copy of 39 MB (64 rows of the Qwen2
+// vocabulary) into fresh pages took 8.6 ms behind a step of 1.15 ms, this one 1.4 to 1.9. Returns when the data is there.
 void Session::copy_staged(char* dst, const char* src, size_t bytes) {
-    constexpr size_t kChunk = (size_t)2 << 20, kPage = 4096;
-    const int n = (int)std::min<size_t>(4, std::max(1u, std::thread::hardware_concurrency()));
-    char* pinned = (char*)h_pinned_copy_.get(n * kChunk / 4);
-    const int device = m_->device;
-    std::atomic<int> failed{0};
-    std::promise<int> started;
-    std::shared_future<int> threads_in_all = started.get_future().share();
-    auto run = [&](int t) {  // chunks t, t + threads, ...
-        const size_t step = (size_t)threads_in_all.get() * kChunk;
-        cudaEvent_t done = nullptr;
-        cudaError_t e = cudaSetDevice(device);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
-        for (size_t o = t * kChunk; o < bytes && e == cudaSuccess; o += step)
-            for (size_t p = o; p < std::min(bytes, o + kChunk); p += kPage) *(volatile char*)(dst + p) = 0;
-        for (size_t o = t * kChunk; o < bytes && e == cudaSuccess; o += step) {
-            const size_t len = std::min(kChunk, bytes - o);
-            e = cudaMemcpyAsync(pinned + t * kChunk, src + o, len, cudaMemcpyDeviceToHost, stream_);
-            if (e == cudaSuccess) e = cudaEventRecord(done, stream_);
-            if (e == cudaSuccess) e = cudaEventSynchronize(done);
-            if (e == cudaSuccess) memcpy(dst + o, pinned + t * kChunk, len);
+    constexpr size_t kChunk = (size_t)1 << 20, kPage = 4096;
+    constexpr int kSlots = 8, kThreads = 4;
+    char* const ring = (char*)h_pinned_copy_.get(kSlots * kChunk / 4);
+    const int device = m_->device, chunks = (int)((bytes + kChunk - 1) / kChunk);
+    struct Events {
+        cudaEvent_t e[kSlots] = {};
+        ~Events() {
+            for (cudaEvent_t x : e)
+                if (x) cudaEventDestroy(x);
         }
-        if (done) cudaEventDestroy(done);
-        if (e != cudaSuccess) failed = (int)e;
+    } there;  // per slot: its chunk has arrived
+    for (cudaEvent_t& x : there.e) TFFN_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+
+    std::mutex mu;
+    std::condition_variable changed;
+    int workers = 0, sent = 0;  // workers: how many share the chunks (0: not known yet)
+    int out_of[kSlots] = {};    // per slot: chunks copied out of it
+    cudaError_t error = cudaSuccess;
+    auto fail = [&](cudaError_t e) {
+        std::lock_guard<std::mutex> lock(mu);
+        error = e;
+        changed.notify_all();
+    };
+    auto work = [&](int t) {  // chunks t, t + workers, ...
+        {
+            std::unique_lock<std::mutex> lock(mu);
+            changed.wait(lock, [&] { return workers > 0; });
+        }
+        for (int c = t; c < chunks; c += workers)
+            for (size_t o = c * kChunk; o < std::min(bytes, (c + 1) * kChunk); o += kPage) *(volatile char*)(dst + o) = 0;
+        cudaError_t e = cudaSetDevice(device);
+        for (int c = t; c < chunks && e == cudaSuccess; c += workers) {
+            {
+                std::unique_lock<std::mutex> lock(mu);
+                changed.wait(lock, [&] { return sent > c || error != cudaSuccess; });
+                if (error != cudaSuccess) return;
+            }
+            e = cudaEventSynchronize(there.e[c % kSlots]);
+            if (e != cudaSuccess) break;
+            memcpy(dst + c * kChunk, ring + c % kSlots * kChunk, std::min(kChunk, bytes - c * kChunk));
+            std::lock_guard<std::mutex> lock(mu);
+            ++out_of[c % kSlots];
+            changed.notify_all();
+        }
+        if (e != cudaSuccess) fail(e);
     };
     std::vector<std::thread> threads;
+    threads.reserve(kThreads);
     try {
-        for (int t = 1; t < n; ++t) threads.emplace_back(run, t);
-    } catch (const std::system_error&) {  // fewer threads
+        while (threads.size() < kThreads) threads.emplace_back(work, (int)threads.size());
+    } catch (...) {  // fewer threads
     }
-    started.set_value((int)threads.size() + 1);
-    run(0);
+    if (threads.empty()) {
+        TFFN_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream_));
+        return;
+    }
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        workers = (int)threads.size();
+        changed.notify_all();
+    }
+    for (int c = 0; c < chunks; ++c) {
+        const int slot = c % kSlots;
+        {
+            std::unique_lock<std::mutex> lock(mu);
+            changed.wait(lock, [&] { return out_of[slot] == c / kSlots || error != cudaSuccess; });
+            if (error != cudaSuccess) break;
+        }
+        cudaError_t e = cudaMemcpyAsync(ring + slot * kChunk, src + c * kChunk, std::min(kChunk, bytes - c * kChunk), cudaMemcpyDeviceToHost, stream_);
+        if (e == cudaSuccess) e = cudaEventRecord(there.e[slot], stream_);
+        if (e != cudaSuccess) {
+            fail(e);
+            break;
+        }
+        std::lock_guard<std::mutex> lock(mu);
+        sent = c + 1;
+        changed.notify_all();
+    }
     for (auto& t : threads) t.join();
-    cuda_check((cudaError_t)failed.load(), "copy of the logits", __FILE__, __LINE__);
+    cuda_check(error, "copy of the logits", __FILE__, __LINE__);
 }
 
 // fp32 logits rows [0, rows) of the last LM-head launch -> host [rows, vocab]. With tensor parallelism
 // every rank holds its slice of the vocabulary: the slices are all-gathered on the device and laid out
-// side by side by the copies. Asynchronous on the session's stream.
+// side by side by the copies. Asynchronous on the session's stream, or (large copies to pageable memory) finished on return.
 void Session::copy_logits_to_host(float* dst, size_t rows) {
     const size_t V = m_->cfg.vocab_size, Vl = m_->V;
     if (!tp_) {

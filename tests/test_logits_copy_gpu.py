@@ -36,3 +36,28 @@ def test_large_copies_equal_small_ones(tmp_path):
     for x in threads:
         x.join()
     assert not problems, problems
+
+
+PER_THREAD = 2  # the handle of CUDA's per-thread default stream: another stream in every thread that uses it
+
+
+def test_per_thread_default_stream(tmp_path):
+    """the same logits as on a stream of the session's own, of prompts and of steps that are not much shorter than their copy"""
+    import synth
+    import tffn
+    V = 70001
+    synth.write_model(str(tmp_path), dict(hidden_size=128, num_hidden_layers=12, num_attention_heads=2, num_key_value_heads=1, intermediate_size=1024,
+                                          vocab_size=V, tie_word_embeddings=True), seed=4)
+    m = tffn.qwen_load(str(tmp_path))
+    prompts = [synth.prompts(1, 20, i, V)[0] for i in range(64)]
+    got = []
+    for stream in (None, PER_THREAD):
+        s = tffn.Session(m, None, max_batch=64, max_seq=64, stream=stream)
+        rows = [s.prefill(prompts, want_logits=True)[1].copy()]
+        for k in range(6):
+            rows.append(s.decode_step([(997 * i + 31 * k) % V for i in range(64)], want_logits=True)[1].copy())
+        got.append(rows)
+        assert s.status() == 0
+        s.free()
+    for a, b in zip(*got):
+        assert (a == b).all()
