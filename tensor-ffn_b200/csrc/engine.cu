@@ -1094,6 +1094,7 @@ void Session::run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool
                          "attention launch");
         }
         prof_end();
+        launches_++;
         // o_proj + residual
         g.op[0] = {ly.wo.as<bf16>(), nh * hd, ctx_.as<bf16>(), nh * hd, nh * hd};
         g.N = H;
@@ -1103,25 +1104,20 @@ void Session::run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool
         if (fold) leave_norm(g, ly.ffn_norm.as<bf16>());
         gemm(g, KC_GEMM_OPROJ, pdl);
         g.norm_w = nullptr;
-        if (!fold) launches_++;
-        prof_begin(KC_RMSNORM);
-        if (fold) {
-        } else if (fused) {
-            prof_end();
+        if (fused) {
             reduce_fused(0, ly.ffn_norm.as<bf16>());
+        } else if (!fold) {
+            if (tp) all_reduce_delta(T);
             prof_begin(KC_RMSNORM);
-        } else if (tp) {
+            if (tp)
+                launch_residual_norm(h_.as<bf16>(), delta_.as<float>(), ly.ffn_norm.as<bf16>(), xn_.as<bf16>(), T, H, c.rms_norm_eps,
+                                     stream_, pdl);
+            else if (live(KC_RMSNORM))
+                launch_rmsnorm(h_.as<bf16>(), ly.ffn_norm.as<bf16>(), xn_.as<bf16>(), T, H, c.rms_norm_eps, nullptr, stream_, pdl,
+                               tl_next(KC_RMSNORM));
             prof_end();
-            all_reduce_delta(T);
-            prof_begin(KC_RMSNORM);
-            launch_residual_norm(h_.as<bf16>(), delta_.as<float>(), ly.ffn_norm.as<bf16>(), xn_.as<bf16>(), T, H, c.rms_norm_eps,
-                                 stream_, pdl);
-        } else if (live(KC_RMSNORM)) {
-            launch_rmsnorm(h_.as<bf16>(), ly.ffn_norm.as<bf16>(), xn_.as<bf16>(), T, H, c.rms_norm_eps, nullptr, stream_, pdl,
-                           tl_next(KC_RMSNORM));
+            launches_++;
         }
-        prof_end();
-        launches_++;
         // gate|up with the SwiGLU epilogue: strided views of the [I][3][H] records; the expert's
         // gate|up rides in the same launch as a second, independent problem
         {

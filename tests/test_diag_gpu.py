@@ -47,6 +47,24 @@ def test_timeline_reports_every_launch_in_order(model_dirs, mode):
     assert s.status() == 0
 
 
+@pytest.mark.parametrize("name,norms", [("mini05", 7), ("mini7", 2)])
+def test_profile_counts_the_launches_of_a_step(model_dirs, name, norms):
+    """as many launches per class as the timeline of such a step has; a norm that rides in the products around it has none"""
+    import collections
+    m, e, s, prompts, cfg = _session(model_dirs, name)
+    s.set_launch_mode(1)
+    nxt = s.prefill(prompts)[0]
+    s.profile(True)
+    for _ in range(2):
+        nxt = s.decode_step(nxt)[0]
+    counts = {k: n for k, (_, n) in s.profile_read().items()}
+    s.profile(False)
+    names, _ = s.timeline(4)
+    want = collections.Counter(names)
+    assert want["rmsnorm_rows"] == norms  # two a layer and the last, or the first layer's and the last
+    assert all(counts[k] == 2 * n for k, n in want.items()), (counts, want)
+
+
 @pytest.mark.parametrize("T,N,K", [(64, 1152, 896), (300, 1152, 896), (513, 4000, 200)])
 def test_gemm_trace_of_both_kinds_of_tiles(T, N, K):
     """the stamps of a launch in single-CTA tiles (64 tokens) and in two-CTA tiles, and the product itself"""
