@@ -55,7 +55,10 @@ int tffn_op_swiglu_bs1_trace(int device, const uint16_t* h_in, const uint16_t* n
  * holds at once. No counterpart in the reference. */
 int tffn_attention_cut(int n_seqs, int heads, int kv_heads, int head_dim, int max_ctx, int num_sms, const int32_t* resident,
                        int64_t scratch_floats, int32_t* out);
-/* The same for latent attention of `heads` heads over cached rows of kv_rank latent and rot rotated columns: out[0] splits, out[1]
+/* 1 if a prompt launch of n_seqs sequences of lens[i] tokens starts its attention only when the kernel before has left every
+ * SM, 0 if ahead of that (host arithmetic, no GPU). No counterpart in the reference. */
+int tffn_prompt_attention_waits(const int32_t* lens, int n_seqs, int heads, int kv_heads, int num_sms);
+/* The cut of a decode step (tffn_attention_cut) for latent attention of `heads` heads over cached rows of kv_rank latent and rot rotated columns: out[0] splits, out[1]
  * 1 if they merge inside a cluster, out[2] stages of a block's ring, out[3] what a captured step is keyed by. */
 int tffn_latent_attention_cut(int n_seqs, int heads, int kv_rank, int rot, int max_ctx, int num_sms, int64_t scratch_floats, int32_t* out);
 

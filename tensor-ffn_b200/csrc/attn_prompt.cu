@@ -379,7 +379,7 @@ int attn_prompt_prepare() {
 }
 
 int launch_attention_prefill(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, const int* grp_first,
-                             const int* grp_count, int n_groups, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s, bool pdl,
+                             const int* grp_count, int n_groups, int key_spread, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s, bool pdl,
                              unsigned long long* tl, const AttnOptions& options) {
     const AttnOptions opt = resolve_attn_options(options, kv, nh);
     PromptDev p;
@@ -410,13 +410,8 @@ int launch_attention_prefill(const float* q, KvView kv, int layer, const int* to
     p.status = status;
     p.tl = tl;
     const dim3 grid((unsigned)n_groups * kv.nkv * p.parts), block(kThreads);
-    // Up to half as many CTAs again as SMs: those of the most keys come first and should have an SM each. Started ahead of the kernel
-    // before, they would go two to the SMs that are free first. Whole prompts, us: 0.5B widths 1 700 tokens (190 CTAs) 3 610 -> 3 425, 2 000
-    // (224) 3 945 -> 3 715, 1.5B 2 000 (192) 1 604 -> 1 565; the rest keeps the early start: 1 200 tokens (134) 2 930 -> 3 065, three of 700
-    // (234) 3 325 -> 3 390, 2 700 (300) 4 595 -> 4 640.
-    const unsigned sms = (unsigned)num_sms;
-    if (grid.x > sms + sms / 16 && grid.x <= sms + sms * 11 / 20) pdl = false;
-    p.warm = pdl && grid.x <= sms;
+    if (attention_prompt_waits(grid.x, num_sms, key_spread)) pdl = false;
+    p.warm = pdl && grid.x <= (unsigned)num_sms;
     if (kv.hd <= 64 && kv.vd <= 64) return (int)launch_k(k_attn_prompt<64>, grid, block, (size_t)PromptCfg<64>::SMEM, s, pdl, p);
     if (kv.hd <= 128 && kv.vd <= 128) return (int)launch_k(k_attn_prompt<128>, grid, block, (size_t)PromptCfg<128>::SMEM, s, pdl, p);
     return (int)cudaErrorInvalidValue;

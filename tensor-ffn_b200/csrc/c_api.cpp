@@ -552,6 +552,25 @@ int tffn_attention_cut(int n_seqs, int heads, int kv_heads, int head_dim, int ma
     });
 }
 
+int tffn_prompt_attention_waits(const int32_t* lens, int n_seqs, int heads, int kv_heads, int num_sms) {
+    int waits = 0;
+    const int rc = guard([&] {
+        need(lens && n_seqs > 0 && kv_heads > 0 && heads >= kv_heads && num_sms > 0, "bad prompt_attention_waits arguments");
+        std::vector<int32_t> seq, pos;
+        for (int i = 0; i < n_seqs; ++i)
+            for (int t = 0; t < lens[i]; ++t) {
+                seq.push_back(i);
+                pos.push_back(t);
+            }
+        const int T = (int)seq.size(), G = heads / kv_heads;
+        std::vector<int32_t> first(T), count(T);
+        const int n = Session::build_groups(seq.data(), pos.data(), T, attention_group_tokens(G), first.data(), count.data());
+        const int parts = (G + 127) / 128;  // heads of a tile: at most 128
+        waits = attention_prompt_waits((unsigned)n * kv_heads * parts, num_sms, prompt_key_spread(pos.data(), first.data(), count.data(), n)) ? 1 : 0;
+    });
+    return rc == TFFN_OK ? waits : rc;
+}
+
 int tffn_latent_attention_cut(int n_seqs, int heads, int kv_rank, int rot, int max_ctx, int num_sms, int64_t scratch_floats, int32_t* out) {
     return guard([&] {
         need(n_seqs > 0 && heads > 0 && kv_rank > 0 && rot > 0 && max_ctx > 0 && num_sms > 0 && scratch_floats >= 0 && out, "bad latent_attention_cut arguments");

@@ -906,6 +906,7 @@ Session::Staged Session::stage_rows(const int32_t* tsp, int T) {
     int32_t* runs = h_pinned_runs_.get((size_t)T * 6);
     Staged r;
     r.n_groups = build_groups(seq, pos, T, attn_group_tokens_, runs, runs + T);
+    r.key_spread = prompt_key_spread(pos, runs, runs + T, r.n_groups);
     TFFN_CUDA(cudaMemcpyAsync(grp_first_.p, runs, (size_t)r.n_groups * 4, cudaMemcpyHostToDevice, stream_));
     TFFN_CUDA(cudaMemcpyAsync(grp_count_.p, runs + T, (size_t)r.n_groups * 4, cudaMemcpyHostToDevice, stream_));
     r.n_segs = r.n_latent = 0;
@@ -1082,7 +1083,7 @@ void Session::run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool
         prof_begin(KC_ATTENTION);
         if (live(KC_ATTENTION) && n_groups > 0 && !attention_prompt_as_rows(T, nh, nkv, m_->num_sms)) {
             // prompt rows: consecutive tokens of a sequence share one pass over its cache
-            check_launch(launch_attention_prefill(q_.as<float>(), kv_, l, tok_seq, tok_pos, grp_first_.as<int>(), grp_count_.as<int>(), n_groups,
+            check_launch(launch_attention_prefill(q_.as<float>(), kv_, l, tok_seq, tok_pos, grp_first_.as<int>(), grp_count_.as<int>(), n_groups, runs.key_spread,
                                                   ctx_.as<bf16>(), nh, m_->num_sms, status, tmaps_, stream_, pdl, tl_next(KC_ATTENTION)),
                          "attention launch");
         } else if (live(KC_ATTENTION)) {

@@ -226,9 +226,12 @@ public:
     uint64_t launch_count() const { return launches_; }
     cudaStream_t stream() const { return stream_; }
     const Model* model() const { return m_; }
+    // groups for launch_attention_prefill from the rows' (slot, position) lists: returns how many
+    // (runs of consecutive positions of one sequence, at most `limit` rows each)
+    static int build_groups(const int* seq, const int* pos, int T, int limit, int32_t* first, int32_t* count);
 
 private:
-    struct Staged { int n_groups, n_latent, n_segs; };  // runs of a sequence's rows: at most attn_group_tokens_; at most 8; all
+    struct Staged { int n_groups, n_latent, n_segs, key_spread; };  // runs of a sequence's rows: at most attn_group_tokens_; at most 8; all
     const Model* m_;
     const Expert* e_;
     TpComm* tp_ = nullptr;  // not owned
@@ -353,10 +356,7 @@ private:
     void ensure_logits(size_t rows);
     void ensure_ring(int entries);
     // runs T tokens already staged in tokens_/tok_seq_/tok_pos_ (or decode state when decode=true)
-    void run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, Staged runs = {0, 0, 0});
-    // groups for launch_attention_prefill from the rows' (slot, position) lists; fills pin[0..2*n) and returns n
-    // (runs of consecutive positions of one sequence, at most `limit` rows each)
-    static int build_groups(const int* seq, const int* pos, int T, int limit, int32_t* first, int32_t* count);
+    void run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool decode, int max_ctx, Staged runs = {0, 0, 0, 0});
     void run_bs1(bool want_logits, int max_ctx);
     void launch_bs1_step(bool want_logits, int max_ctx, bool pdl);
     void run_captured(int n_seqs, bool logits, int max_ctx, const std::function<void()>& body);

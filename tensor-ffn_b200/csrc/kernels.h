@@ -272,16 +272,38 @@ void launch_attention_simt(const float* q, KvView kv, bool f32, const int* tok_s
                       const AttnOptions& opt = AttnOptions());
 
 // Prompt tokens: rows grp_first[g] .. grp_first[g] + grp_count[g] - 1 (at most attention_group_tokens of the heads, consecutive
-// positions of one sequence) share one pass over that sequence's cache; n_groups groups cover the T rows of the call.
+// positions of one sequence) share one pass over that sequence's cache; n_groups groups cover the T rows of the call (key_spread:
+// prompt_key_spread of them, 0 where a chunk keeps the groups alike).
 // Returns a cudaError (launch) or -1000 if the tensor maps could not be encoded.
 inline int attention_group_tokens(int heads_per_kv) { return heads_per_kv < 128 ? 128 / heads_per_kv : 1; }
 // Prompts whose (token, kv head) units fit the SMs in one wave are better off with a block per unit (launch_attention): it has no
 // chain of products between its warps. 9 tokens of 14 heads and 2 kv heads of 64: about 4 us, in tiles 8; a 60-token continuation
 // of a long context has a fifteenth of the blocks in tiles.
 inline bool attention_prompt_as_rows(int T, int nh, int nkv, int num_sms) { return T * nkv * ((nh / nkv + 7) / 8) <= num_sms; }
+// Keys that the group with the most sees beyond the average of all groups; positions of the rows, the groups of them
+inline int prompt_key_spread(const int32_t* pos, const int32_t* first, const int32_t* count, int n_groups) {
+    long long sum = 0;
+    int most = 0;
+    for (int g = 0; g < n_groups; ++g) {
+        const int keys = pos[first[g]] + count[g];
+        sum += keys;
+        most = keys > most ? keys : most;
+    }
+    return n_groups > 0 ? most - (int)(sum / n_groups) : 0;
+}
+// Whether a prompt's attention starts when the kernel before has left every SM, not ahead of that. Two of its CTAs fit an SM; where there
+// are more than SMs, those that start ahead go two to the SMs that are free first, and those of the most keys, which come first, share
+// one. Keeping them apart is worth it where they outlast the others by much; what it costs is the overlap, about 4 us a launch.
+// Whole prompts, early -> full start: 0.5B widths, 24 layers, one prompt of 1 440 tokens (160 CTAs, spread 720) 3 253 -> 3 206 us,
+// 1 800 3 720 -> 3 621, 2 340 (260 CTAs) 4 205 -> 4 170, 2 700 (300) 4 669 -> 4 644; one of 1 500 beside three of 100 (spread 870) 3 537 -> 3 507,
+// 1 200 and 600 (700) 3 354 -> 3 355; two of 900 (450) 3 279 -> 3 256, but two of 1 170 (585) 3 671 -> 3 749, 1 000, 400, 200, 100
+// and 50 (650) 3 108 -> 3 163, four of 450 (225) 3 123 -> 3 149, twenty of 90 2 842 -> 2 944. 1.5B widths: 2 000 tokens 1 629 -> 1 578, eight of 250 1 406 -> 1 427.
+inline bool attention_prompt_waits(unsigned ctas, int num_sms, int key_spread) {
+    return ctas > (unsigned)num_sms && ctas <= 2 * (unsigned)num_sms && key_spread >= 700;
+}
 int attn_prompt_prepare();
 [[nodiscard]] int launch_attention_prefill(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, const int* grp_first,
-                             const int* grp_count, int n_groups, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s,
+                             const int* grp_count, int n_groups, int key_spread, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s,
                              bool pdl = false, unsigned long long* tl = nullptr, const AttnOptions& opt = AttnOptions());
 
 // ------------------------------------------------------------------ layers with an fp32 residual stream

@@ -108,6 +108,7 @@ _SIGS = {
     "tffn_op_swiglu_bs1_trace": (_i, [_i, _vp, _vp, _vp, _vp, _f, _f, _i, _i, _vp, _vp, _i]),
     "tffn_op_swiglu_bs1_noalloc": (_i, [_i, _vp, _vp, _vp, _vp, _f, _f, _i, _i, _vp]),
     "tffn_attention_cut": (_i, [_i, _i, _i, _i, _i, _i, _vp, ctypes.c_int64, _vp]),
+    "tffn_prompt_attention_waits": (_i, [_vp, _i, _i, _i, _i]),
     "tffn_latent_attention_cut": (_i, [_i, _i, _i, _i, _i, _i, ctypes.c_int64, _vp]),
     "tffn_op_wait_selftest": (_i, [_i]),
     "tffn_op_tp_wait_selftest": (_i, [_i, _i]),
@@ -487,6 +488,12 @@ def attention_cut(n_seqs: int, heads: int, kv_heads: int, head_dim: int, max_ctx
     out = np.zeros(2, dtype=np.int32)
     _check(_L.tffn_attention_cut(n_seqs, heads, kv_heads, head_dim, max_ctx, num_sms, r.ctypes.data, scratch_floats, out.ctypes.data))
     return int(out[0]), bool(out[1])
+
+
+def prompt_attention_waits(lens, heads: int, kv_heads: int, num_sms: int) -> bool:
+    """whether the attention of a prompt launch of these lengths waits for the kernel before to leave every SM (host arithmetic)"""
+    n = np.ascontiguousarray(lens, dtype=np.int32)
+    return bool(_check(_L.tffn_prompt_attention_waits(n.ctypes.data, n.size, heads, kv_heads, num_sms)))
 
 
 def latent_attention_cut(n_seqs: int, heads: int, kv_rank: int, rot: int, max_ctx: int, num_sms: int, scratch_floats: int = 8 << 20):

@@ -1,5 +1,5 @@
 """How a decode step's attention is cut over the chip, against times measured for every cut. The cut is host arithmetic; what the
-two ways of merging compute is tested on the GPU (test_parity_gpu.py)."""
+two ways of merging compute is tested on the GPU (test_parity_gpu.py). At the end the same for when a prompt's attention starts."""
 import pytest
 
 # clusters of 1 .. 8 blocks of the decode attention kernel that a B200 of 148 SMs holds at once
@@ -67,3 +67,27 @@ def test_latent_steps_are_keyed_by_all_that_their_launch_depends_on(n, heads, ra
     cuts = {tffn.latent_attention_cut(n, heads, rank, rot, ctx, 148) for ctx in list(range(1, 12000, 61)) + [32768]}
     assert len({c[3] for c in cuts}) == len({c[:3] for c in cuts}) == len(cuts)
     assert all(c[2] >= 1 and c[0] >= 1 and (not c[1] or c[0] in (2, 4, 8, 16)) for c in cuts)
+
+
+# whole prompts, us: heads, kv heads, lengths, with the attention started ahead of the kernel before it and behind it
+PROMPTS = [
+    (14, 2, [1332], 3145, 3144), (14, 2, [1440], 3253, 3206), (14, 2, [720] * 2, 2904, 2921), (14, 2, [360] * 4, 2745, 2782),
+    (14, 2, [144] * 10, 2686, 2700), (14, 2, [36] * 40, 2637, 2710), (14, 2, [1600], 3425, 3382), (14, 2, [800] * 2, 3038, 3053),
+    (14, 2, [400] * 4, 2872, 2920), (14, 2, [200] * 8, 2815, 2864), (14, 2, [160] * 10, 2793, 2844), (14, 2, [1800], 3720, 3621),
+    (14, 2, [900] * 2, 3279, 3256), (14, 2, [600] * 3, 3171, 3157), (14, 2, [450] * 4, 3123, 3149), (14, 2, [300] * 6, 3025, 3069),
+    (14, 2, [180] * 10, 2901, 2976), (14, 2, [90] * 20, 2842, 2944), (14, 2, [36] * 50, 2858, 2961), (14, 2, [2016], 3814, 3707),
+    (14, 2, [1008] * 2, 3311, 3295), (14, 2, [666] * 3, 3182, 3229), (14, 2, [504] * 4, 3089, 3148), (14, 2, [252] * 8, 2915, 3022),
+    (14, 2, [126] * 16, 2867, 2973), (14, 2, [2100], 3963, 3899), (14, 2, [2340], 4205, 4170), (14, 2, [1170] * 2, 3671, 3749),
+    (14, 2, [2700], 4669, 4644), (14, 2, [1500, 100, 100, 100], 3537, 3507), (14, 2, [1000, 400, 200, 100, 50], 3108, 3163),
+    (14, 2, [1300, 450], 3291, 3281), (14, 2, [700, 500, 300, 200], 2997, 3027), (14, 2, [50, 100, 200, 1400], 3381, 3348),
+    (14, 2, [1000, 800], 3290, 3274), (14, 2, [1200, 600], 3354, 3355),
+    (12, 2, [1600], 1481, 1465), (12, 2, [2000], 1629, 1578), (12, 2, [1000] * 2, 1491, 1494), (12, 2, [500] * 4, 1429, 1452),
+    (12, 2, [250] * 8, 1406, 1427), (12, 2, [126] * 16, 1386, 1408), (12, 2, [2300], 1739, 1699),
+]
+
+
+@pytest.mark.parametrize("heads,kv,lens,ahead,behind", PROMPTS)
+def test_prompt_attention_starts_where_it_is_faster(heads, kv, lens, ahead, behind):
+    import tffn
+    chosen = behind if tffn.prompt_attention_waits(lens, heads, kv, 148) else ahead
+    assert chosen <= 1.01 * min(ahead, behind)  # repeated measurements differ by about as much
