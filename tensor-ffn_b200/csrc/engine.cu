@@ -81,7 +81,6 @@ void Expert::forward_layers(const void* d_x, float* d_out, int T, cudaStream_t s
     TFFN_CUDA(cudaSetDevice(model->device));
     // the layers of the slab are equally far apart
     const int64_t layer_elems = L > 1 ? layers[1].packed.as<bf16>() - layers[0].packed.as<bf16>() : 0;
-    constexpr size_t kActBytes = (size_t)128 << 20;
     const size_t act_bytes = (size_t)T * I * 2;
     const int per_launch = (int)std::min<size_t>((size_t)L, std::max<size_t>(1, kActBytes / act_bytes));
 
@@ -91,6 +90,7 @@ void Expert::forward_layers(const void* d_x, float* d_out, int T, cudaStream_t s
         if (!kept_.empty()) {
             s = std::move(kept_.back());
             kept_.pop_back();
+            kept_bytes_ -= s->act.bytes;
         }
     }
     if (!s) {
@@ -140,9 +140,13 @@ void Expert::forward_layers(const void* d_x, float* d_out, int T, cudaStream_t s
     TFFN_CUDA(cudaMemcpyAsync(s->h_status, s->status.p, 4, cudaMemcpyDeviceToHost, stream));
     TFFN_CUDA(cudaStreamSynchronize(stream));
     const int st = *s->h_status;
-    if (s->act.bytes <= kKeptBytes) {
+    {
         std::lock_guard<std::mutex> lock(mu_);
-        if (kept_.size() < kKept) kept_.push_back(std::move(s));
+        const size_t bytes = s->act.bytes;
+        if (kept_.size() < kKept && kept_bytes_ + bytes <= kActBytes) {
+            kept_.push_back(std::move(s));
+            kept_bytes_ += bytes;
+        }
     }
     if (st != 0) throw Error(kErrDevice, "device status " + std::to_string(st) + " in expert_forward");
 }

@@ -139,15 +139,17 @@ struct Expert {
     void forward_layers(const void* d_x, float* d_out, int T, cudaStream_t stream) const;
 
 private:
-    // what one forward_layers call works in; up to kKept of them stay with the expert between calls, one per thread that runs one
+    // What one forward_layers call works in. Those of one or several threads' calls stay with the expert between calls, up to
+    // kActBytes in all: as much as a call that shares launches among layers takes.
     struct Scratch {
         DeviceBuffer act, status;
         int* h_status = nullptr;  // pinned
         ~Scratch();
     };
-    static constexpr size_t kKept = 2, kKeptBytes = (size_t)256 << 20;
+    static constexpr size_t kActBytes = (size_t)128 << 20, kKept = 8;
     mutable std::mutex mu_;
     mutable std::vector<std::unique_ptr<Scratch>> kept_;
+    mutable size_t kept_bytes_ = 0;
 };
 
 // kernel classes of the per-launch profile (tffn_session_profile_*)

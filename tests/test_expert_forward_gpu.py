@@ -85,3 +85,35 @@ def test_expert_forward_layers_of_one_launch(model_dirs, name, T):
         scale = np.abs(ref).max()
         assert np.abs(got[l] - ref).max() / scale <= 2e-2, (name, l)   # the bounds of the test above
         assert np.abs(got[l] - ref).mean() / scale <= 1e-3, (name, l)
+
+
+def test_memory_kept_between_calls(model_dirs):
+    """calls of several threads at once leave at most 128 MB of device memory with the expert, which go with it"""
+    import threading
+    import torch
+    import tffn
+    d, ep, cfg = model_dirs["mini05"]
+    H, L, T = cfg["hidden_size"], cfg["num_hidden_layers"], 40000  # a call works in 97 MB
+    m = tffn.qwen_load(d)
+    e = tffn.checkpoint_load(ep, m, 0.1)
+    dx = torch.zeros((L, T, H), dtype=torch.bfloat16, device="cuda")
+    outs = [torch.empty((L, T, H), dtype=torch.float32, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    free = lambda: torch.cuda.mem_get_info()[0]  # noqa: E731
+    before = free()
+    gate = threading.Barrier(len(outs))
+
+    def call(out):
+        stream = torch.cuda.Stream()
+        gate.wait()
+        for _ in range(3):
+            e.expert_forward(dx.data_ptr(), out.data_ptr(), T, stream.cuda_stream)
+
+    threads = [threading.Thread(target=call, args=(o,)) for o in outs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert before - free() <= (128 + 16) << 20  # 16 MB for the streams' own
+    e.free()
+    assert before - free() <= 16 << 20
