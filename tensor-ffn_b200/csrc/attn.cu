@@ -475,15 +475,15 @@ __global__ void __launch_bounds__(kAttnCtaThreads) k_attn_decode(const float* __
 // exponentials; the warps merge at the end. Bound by the latency of a key's loads and sums, so k_attn_simt4 has KEYS
 // neighbouring keys (of one page) of a warp in flight at once, four columns per lane and load (14 heads on rows of
 // 320 columns, three sequences of about 155 keys: 34.6 -> 8.3 us a launch inside a step; 450 prompt rows 228 -> 128).
-// k_attn_simt, a key at a time, is for rows of more than 1 024 columns.
-constexpr int kSimtWarps = 8;
+// k_attn_simt, a key at a time, is for rows of more than 1 024 columns: latent ones of up to kLatentMaxRank value columns, which leave
+// no registers for a second key.
+constexpr int kSimtWarps = 8, kSimtCols = kLatentMaxRank / 32;  // value columns per lane
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(bf16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ void store_as(float* p, float v) { *p = v; }
 __device__ __forceinline__ void store_as(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
-// ML: value columns per lane, for heads of up to 32 ML value columns
-template <typename C, int ML>
+template <typename C>
 __global__ void __launch_bounds__(kSimtWarps * 32) k_attn_simt(const float* __restrict__ q, KvView kv, const int* __restrict__ tok_seq,
                                                                const int* __restrict__ tok_pos, C* __restrict__ ctx, int nh,
                                                                AttnOptions opt, int* status, unsigned long long* tl) {
@@ -504,9 +504,9 @@ __global__ void __launch_bounds__(kSimtWarps * 32) k_attn_simt(const float* __re
     const int* bt = kv.block_table + (size_t)seq * kv.max_pages_per_seq;
     const C* kpool = (const C*)kv.k_pool;
     const C* vpool = (const C*)kv.v_pool;
-    float m = kNegBig, l = 0.f, acc[ML];
+    float m = kNegBig, l = 0.f, acc[kSimtCols];
 #pragma unroll
-    for (int j = 0; j < ML; ++j) acc[j] = 0.f;
+    for (int j = 0; j < kSimtCols; ++j) acc[j] = 0.f;
     bool bad = false;
     for (int key = lo + warp; key <= last; key += kSimtWarps) {
         const int pg = __ldcg(bt + key / kPageTokens);
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(kSimtWarps * 32) k_attn_simt(const float* __re
         m = mn;
         l = l * corr + p;
 #pragma unroll
-        for (int j = 0; j < ML; ++j) {
+        for (int j = 0; j < kSimtCols; ++j) {
             const int d = j * 32 + lane;
             if (d < vdim) acc[j] = acc[j] * corr + p * to_f32(vpool[row * vd + d]);
         }
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(kSimtWarps * 32) k_attn_simt(const float* __re
     float* mw = merge + warp * (vdim + 2);
     if (lane == 0) { mw[0] = m; mw[1] = l; }
 #pragma unroll
-    for (int j = 0; j < ML; ++j)
+    for (int j = 0; j < kSimtCols; ++j)
         if (j * 32 + lane < vdim) mw[2 + j * 32 + lane] = acc[j];
     __syncthreads();
     float M = kNegBig, L = 0.f;
@@ -711,10 +711,8 @@ static cudaError_t attn_attrs_hd() {
 int attn_prepare() {
     cudaError_t e = attn_attrs_hd<64>();
     if (e == cudaSuccess) e = attn_attrs_hd<128>();
-    if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<float, 16>);
-    if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<bf16, 16>);
-    if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<float, 32>);
-    if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<bf16, 32>);
+    if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<float>);
+    if (e == cudaSuccess) e = prefer_max_shared(k_attn_simt<bf16>);
     auto simt4 = [&](auto kern) {
         if (e == cudaSuccess) e = prefer_max_shared(kern);
     };
@@ -826,9 +824,8 @@ void launch_attention_simt(const float* q, KvView kv, bool f32, const int* tok_s
     }
     const dim3 block(kSimtWarps * 32);
     const size_t smem = (size_t)(kv.hd + kSimtWarps * (opt.vdim + 2)) * 4;
-    const bool wide = opt.vdim > 512;
-    if (f32) launch_k(wide ? k_attn_simt<float, 32> : k_attn_simt<float, 16>, grid, block, smem, s, pdl, q, kv, tok_seq, tok_pos, (float*)ctx, nh, opt, status, tl);
-    else launch_k(wide ? k_attn_simt<bf16, 32> : k_attn_simt<bf16, 16>, grid, block, smem, s, pdl, q, kv, tok_seq, tok_pos, (bf16*)ctx, nh, opt, status, tl);
+    if (f32) launch_k(k_attn_simt<float>, grid, block, smem, s, pdl, q, kv, tok_seq, tok_pos, (float*)ctx, nh, opt, status, tl);
+    else launch_k(k_attn_simt<bf16>, grid, block, smem, s, pdl, q, kv, tok_seq, tok_pos, (bf16*)ctx, nh, opt, status, tl);
 }
 
 }  // namespace tffn

@@ -567,6 +567,7 @@ __global__ void __launch_bounds__(NT) k_delta_scan(const DeltaRule a, int cols, 
             // With one or two columns every lane gets S^T k of all of them (the sums are formed in the same order).
             float uc[C];
             if constexpr (C <= 2) {
+                static_assert(!FUSED, "");
                 float ts[C], ws[C];
 #pragma unroll
                 for (int c = 0; c < C; ++c) {
@@ -586,8 +587,7 @@ __global__ void __launch_bounds__(NT) k_delta_scan(const DeltaRule a, int cols, 
                 const int col = c0 + (r & (C - 1));
                 if (r < C && col - cb < ncols) {
                     const float o = (C == 2 && r == 1 ? ws[C - 1] : ws[0]) + (C == 2 && r == 1 ? uc[C - 1] : uc[0]) * bk.y;
-                    if constexpr (FUSED) o_s[k * cols + (col - cb)] = o;
-                    else a.o[((size_t)(first + tile * kScanTokens + k) * H + h) * vdimP + col] = o;
+                    a.o[((size_t)(first + tile * kScanTokens + k) * H + h) * vdimP + col] = o;
                 }
             } else if constexpr (C == 8) {
                 float tx[4], wx[4], ty[2], wy[2];

@@ -13,6 +13,7 @@ LATENT = {
     "one_head": (48, latent_layer(1, 24, 8, 40, 40, 24), 4.0),
     "wide_rank": (64, latent_layer(3, 32, 32, 16, 320, 40, scale=0.2), 2.0),
     "widest_rank": (64, latent_layer(2, 48, 64, 64, 512, 64), 3.0),
+    "beyond_1024_columns": (48, latent_layer(3, 16, 64, 24, 1000, 32), 2.0),
     "very_wide_rank": (48, latent_layer(2, 16, 16, 24, 712, 32), 2.0),
     "wide_rotation": (72, latent_layer(5, 16, 80, 24, 96, 56, base=500.0), 3.0),
     "many_heads": (64, latent_layer(20, 16, 8, 16, 48, 32), 3.0),
