@@ -38,6 +38,32 @@ def test_large_copies_equal_small_ones(tmp_path):
     assert not problems, problems
 
 
+# bytes: 16 MB; 25 MB; 18 MB and 4 bytes; 16 MB and a chunk of 23 KB. Destinations at the start of a page and inside one
+@pytest.mark.parametrize("V,rows,offset", [(65536, 64, 0), (65536, 100, 1), (44099, 107, 0), (44099, 107, 777), (70001, 60, 5)])
+def test_every_byte(tmp_path, V, rows, offset):
+    """the same rows through a plain copy into pinned memory; a poisoned destination with guards around it"""
+    import synth
+    import tffn
+    import torch
+    synth.write_model(str(tmp_path), dict(hidden_size=128, num_hidden_layers=1, num_attention_heads=2, num_key_value_heads=1, intermediate_size=256,
+                                          vocab_size=V, tie_word_embeddings=True), seed=5)
+    m = tffn.qwen_load(str(tmp_path))
+    s = tffn.Session(m, None, max_batch=1, max_seq=128)
+    t = np.ascontiguousarray(synth.prompts(1, rows, 9, V)[0], dtype=np.int32)
+    n, poison, guard = rows * V, np.float32(-12345.5), 1024
+    pinned = torch.empty(n, dtype=torch.float32, pin_memory=True).numpy()
+    pages = np.full(n + 3 * guard + 1024, poison, dtype=np.float32)
+    skip = -pages.ctypes.data % 4096 // 4 + guard + offset  # guard: a page
+    out = pages[skip:skip + n]
+    for dst in (pinned, out):
+        s.qwen_reset()
+        tffn._check(tffn._L.tffn_forward(s._h, 0, t.ctypes.data, rows, dst.ctypes.data))
+    assert np.isfinite(pinned).all() and not (pinned == poison).any()
+    assert (out == pinned).all()
+    assert (pages[:skip] == poison).all() and (pages[skip + n:] == poison).all()
+    s.free()
+
+
 PER_THREAD = 2  # the handle of CUDA's per-thread default stream: another stream in every thread that uses it
 
 
