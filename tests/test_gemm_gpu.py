@@ -98,3 +98,32 @@ def test_fused_bs1_ffn_kernel_edges(H, I, expert):
     assert np.abs(out - ref).mean() / scale <= 1.5e-3
     again = synth.bf16_to_f32(tffn.op_swiglu_bs1(h, w, pb, pe if expert else None, 0.1, 1e-6))
     assert (again == out).all()  # fixed reduction order
+
+
+# The same kernel inside a step, where its weights are requested in two portions (14 336 / H records at once, half as many with the
+# expert): the rest of a ring short and long, ring rounds and rest, nothing left for the second portion, 9 and 12 warps
+@pytest.mark.parametrize("H,heads,kv,I,expert", [(896, 14, 2, 4864, True), (896, 14, 2, 1160, True), (1024, 16, 4, 4328, False), (1088, 17, 17, 2600, True),
+                                                 (1536, 12, 2, 1600, False), (2048, 16, 2, 648, True), (2048, 16, 2, 1184, False), (128, 2, 1, 17000, False)])
+def test_bs1_ffn_in_two_portions(tmp_path, H, heads, kv, I, expert):
+    """early starts (portions) and full dependencies (everything requested at once) give the same bits"""
+    import synth
+    import tffn
+    shape = dict(hidden_size=H, num_hidden_layers=3, num_attention_heads=heads, num_key_value_heads=kv, intermediate_size=I, vocab_size=512,
+                 tie_word_embeddings=True)
+    cfg = synth.write_model(str(tmp_path), shape, seed=31, norm_jitter=0.1)
+    e = None
+    m = tffn.qwen_load(str(tmp_path))
+    if expert:
+        synth.write_expert(str(tmp_path / "expert.bin"), cfg, seed=32)
+        e = tffn.checkpoint_load(str(tmp_path / "expert.bin"), m, 0.5)
+    t = synth.prompts(1, 24, 3, 512)[0]
+    rows = {}
+    for mode in (0, 1, 2):
+        s = tffn.Session(m, e, max_batch=1, max_seq=64)
+        s.set_launch_mode(mode)
+        s.prefill([t[:8]])
+        rows[mode] = np.concatenate([s.decode_step(t[i:i + 1], want_logits=True)[1] for i in range(8, 24)])
+        assert s.status() == 0
+        s.free()
+    assert np.isfinite(rows[0]).all()
+    assert (rows[1] == rows[0]).all() and (rows[2] == rows[0]).all()
