@@ -379,8 +379,8 @@ int attn_prompt_prepare() {
 }
 
 int launch_attention_prefill(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, const int* grp_first,
-                             const int* grp_count, int n_groups, int key_spread, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s, bool pdl,
-                             unsigned long long* tl, const AttnOptions& options) {
+                             const int* grp_count, int n_groups, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s, bool pdl,
+                             unsigned long long* tl, const AttnOptions& options, int key_spread) {
     const AttnOptions opt = resolve_attn_options(options, kv, nh);
     PromptDev p;
     memset(&p, 0, sizeof p);

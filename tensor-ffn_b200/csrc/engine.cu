@@ -1087,8 +1087,8 @@ void Session::run_batched(int T, int n_logit_rows, bool logit_rows_are_all, bool
         prof_begin(KC_ATTENTION);
         if (live(KC_ATTENTION) && n_groups > 0 && !attention_prompt_as_rows(T, nh, nkv, m_->num_sms)) {
             // prompt rows: consecutive tokens of a sequence share one pass over its cache
-            check_launch(launch_attention_prefill(q_.as<float>(), kv_, l, tok_seq, tok_pos, grp_first_.as<int>(), grp_count_.as<int>(), n_groups, runs.key_spread,
-                                                  ctx_.as<bf16>(), nh, m_->num_sms, status, tmaps_, stream_, pdl, tl_next(KC_ATTENTION)),
+            check_launch(launch_attention_prefill(q_.as<float>(), kv_, l, tok_seq, tok_pos, grp_first_.as<int>(), grp_count_.as<int>(), n_groups,
+                                                  ctx_.as<bf16>(), nh, m_->num_sms, status, tmaps_, stream_, pdl, tl_next(KC_ATTENTION), AttnOptions(), runs.key_spread),
                          "attention launch");
         } else if (live(KC_ATTENTION)) {
             unsigned long long* tl = tl_next(KC_ATTENTION);

@@ -635,7 +635,8 @@ void Session::run_stack(int T, int n_logit_rows, bool logit_rows_are_all, bool d
                     launch_attention_simt(q_.as<float>(), cache.kv, f32, tok_seq, tok_pos, ctx_.p, T, sp.heads, opt, status, stream_, pdl, tl);
                 else if (runs.n_groups > 0 && !attention_prompt_as_rows(T, sp.heads, sp.kv_heads, m_->num_sms))
                     check_launch(launch_attention_prefill(q_.as<float>(), cache.kv, 0, tok_seq, tok_pos, grp_first_.as<int>(), grp_count_.as<int>(),
-                                                          runs.n_groups, sp.chunk > 0 && sp.chunk < max_ctx ? 0 : runs.key_spread, ctx_.as<bf16>(), sp.heads, m_->num_sms, status, tmaps_, stream_, pdl, tl, opt),
+                                                          runs.n_groups, ctx_.as<bf16>(), sp.heads, m_->num_sms, status, tmaps_, stream_, pdl, tl, opt,
+                                                          sp.chunk > 0 && sp.chunk < max_ctx ? 0 : runs.key_spread),
                                  "attention launch");
                 else
                     check_launch(launch_attention(q_.as<float>(), cache.kv, 0, tok_seq, tok_pos, ctx_.as<bf16>(), T, sp.heads, attn_ctx(sp, max_ctx),

@@ -303,8 +303,8 @@ inline bool attention_prompt_waits(unsigned ctas, int num_sms, int key_spread) {
 }
 int attn_prompt_prepare();
 [[nodiscard]] int launch_attention_prefill(const float* q, KvView kv, int layer, const int* tok_seq, const int* tok_pos, const int* grp_first,
-                             const int* grp_count, int n_groups, int key_spread, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s,
-                             bool pdl = false, unsigned long long* tl = nullptr, const AttnOptions& opt = AttnOptions());
+                             const int* grp_count, int n_groups, bf16* ctx, int nh, int num_sms, int* status, TmapCache* tmaps, cudaStream_t s,
+                             bool pdl = false, unsigned long long* tl = nullptr, const AttnOptions& opt = AttnOptions(), int key_spread = 0);
 
 // ------------------------------------------------------------------ layers with an fp32 residual stream
 // "f32" below selects the storage type of activations and cache: fp32 in a session that computes in fp32, else bf16.
