@@ -44,8 +44,8 @@ int tffn_op_gemm_trace(int device, const uint16_t* X, const uint16_t* W, float* 
                        uint64_t* trace, int trace_ctas);
 /* tffn_op_swiglu_bs1, and additionally returns 16 device timestamps (globaltimer, ns) per CTA of a second, warm
  * launch in trace[trace_ctas*16] (trace_ctas >= SM count): 0 start, 1 RMSNorm done, 2 first record
- * arrived, 3 last record consumed, 4 CTA partial written, 5 group ticket taken, 6 group fold done,
- * 7 residual updated. A profiling aid with no counterpart in the reference. */
+ * arrived, 3 last record consumed, 4 this CTA's sums added to the layer's accumulator (the others stay zero). A profiling aid with no
+ * counterpart in the reference. */
 int tffn_op_swiglu_bs1_trace(int device, const uint16_t* h_in, const uint16_t* norm_w, const uint16_t* packed_base,
                              const uint16_t* packed_expert, float expert_scale, float eps, int H, int I, uint16_t* h_out,
                              uint64_t* trace, int trace_ctas);

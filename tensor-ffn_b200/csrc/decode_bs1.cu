@@ -164,12 +164,17 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_bs1_oproj(Bs1Ctx c, Bs1Layer
 }
 
 // ------------------------------------------------------------------------------------------ fused SwiGLU
-// Warps of a CTA. Twelve at 120 registers (hidden 896) leave each SM sub-partition room for a warp of the next layer's q|k|v and
-// one of its o_proj kernel, which fetch their weights while this one runs.
+// Warps of a CTA. Three per SM sub-partition at 110 registers (hidden 769 to 1 024 without the expert) leave it room for a warp of the
+// next layer's q|k|v kernel (88) and one of its o_proj kernel (64), at 126 (with the expert) for one of them; these fetch their weights while this
+// one runs. Wider rows take 128 to 168 registers.
 __host__ __device__ constexpr int ffn_warps(int nch) { return nch <= 4 ? 12 : 9; }
 constexpr int kSmsLeftToAttention = 4;
-// Measured per token, 0.5B shape with expert, us: ring at once 663, with 192 KB more per SM requested into L2 671; 86 KB at once and
-// the rest 7 000 cycles later 610 (5 000: 622, 9 000: 622; nothing at once and the rest after 5 000: 626). Without the expert 547, 515.
+// Measured per token (sessions in turn; two of the same setting differ by about 1 %), us: the ring at once, then kAtOnceBytes at once and
+// the rest 3 000, 4 000 ... 9 000 cycles later: 0.5B shape with expert 627, 603 607 613 607 609 613 615, without 551, 543 541 535 526 532
+// 539 537; 1 536 wide, 8 layers 450, 442 443 444 445 441 445 445, without 350, 343 345 347 349 344 349 350; 2 048 wide, 8 layers 635, 636 633
+// 630 630 630 626 628, without 481, 488 480 476 477 475 475 475. 6 000 cycles later with 48 and 126 KB at once: 612 and 614, 535 and
+// 530; 440 and 443, 348 and 344; 627 and 629, 482 and 482. 6 000 is the best on the 0.5B shape without the expert, which gains most, and
+// within 2 % of the best elsewhere. With 192 KB more per SM requested into L2: 671 against 663 at once (0.5B with expert, earlier kernel).
 constexpr size_t kAtOnceBytes = 86016;
 constexpr long long kPauseCycles = 6000;
 

@@ -54,7 +54,6 @@ struct PairDev {
     int whole, splits;  // PAIR_SPLIT: tiles worked on as one, the first ones; parts of each of the others
     float* partials;    // [split tile][part][rank][epilogue warp][column][row]
     int* tickets;       // [split tile][rank][epilogue warp], zero
-    int layers;  // > 1: problems are layers (GemmCall::layers), tmW 3-D (column, layer, row)
     const GroupTile* grp;
 };
 #define TFFN_TRACE(slot)                                                       \
@@ -268,8 +267,8 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* s
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
 }
 
-// What a launch's tiles are: tiles of one or two problems, of a batch or of groups; of several layers (GemmCall::layers); with
-// the last ones in parts. The issuing loops of the first kind carry none of what the others need: a test per k-block there cost a
+// What a launch's tiles are: tiles of one or two problems, of a batch or of groups; of several layers (GemmCall::layers: a problem is a
+// layer, tmW is 3-D: column, layer, row); with the last ones in parts. The issuing loops of the first kind carry none of what the others need: a test per k-block there cost a
 // prompt's products 2 to 3 %.
 enum PairKind { PAIR_TILES, PAIR_LAYERS, PAIR_SPLIT };
 template <int BN, int MODE, int KIND>
@@ -606,8 +605,7 @@ int launch_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream)
     PairDev p;
     memset(&p, 0, sizeof p);
     const bool halves = c.mode == GEMM_SWIGLU, batched = c.batch > 1, layered = c.layers > 1;
-    if (layered && ((c.mode != GEMM_SWIGLU && c.mode != GEMM_STORE_F32) || batched || c.grp || c.out2 || c.mode == GEMM_QKV || c.mode == GEMM_RESIDUAL || c.w_layer % 8 || c.w_layer >> 32 ||
-                    (!halves && c.op[1].K > 0)))
+    if (layered && ((c.mode != GEMM_SWIGLU && c.mode != GEMM_STORE_F32) || batched || c.grp || c.out2 || c.w_layer % 8 || c.w_layer >> 32 || (!halves && c.op[1].K > 0)))
         return (int)cudaErrorInvalidValue;
     const int maps = c.out2 ? 2 : 1;
     for (int pr = 0; pr < maps; ++pr)
@@ -632,7 +630,6 @@ int launch_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream)
     const int tile_n = halves ? BN / 2 : BN;
     p.batch = batched ? c.batch : 1;
     p.out_batch = batched ? c.out_batch : 0;
-    p.layers = layered ? c.layers : 1;
     p.nprob = batched ? c.batch : layered ? c.layers : maps;
     p.N = c.N;
     p.T = c.T;
@@ -664,10 +661,7 @@ int launch_pair(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream)
     }
     p.trace = 2 * pairs <= c.trace_ctas ? c.trace : nullptr;
     auto go = [&](auto kern) { return (int)launch_k_cluster(kern, dim3(2 * pairs), dim3(kPairThreads), dim3(2, 1, 1), PairCfg<BN>::SMEM, stream, c.pdl, p); };
-    if (layered) {
-        if (c.mode == GEMM_SWIGLU) return go(k_gemm_pair<BN, GEMM_SWIGLU, PAIR_LAYERS>);
-        return c.mode == GEMM_STORE_F32 ? go(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_LAYERS>) : (int)cudaErrorInvalidValue;
-    }
+    if (layered) return halves ? go(k_gemm_pair<BN, GEMM_SWIGLU, PAIR_LAYERS>) : go(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_LAYERS>);
     switch (c.mode) {
         case GEMM_STORE_F32: return split ? go(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_SPLIT>) : go(k_gemm_pair<BN, GEMM_STORE_F32, PAIR_TILES>);
         case GEMM_STORE_BF16: return split ? go(k_gemm_pair<BN, GEMM_STORE_BF16, PAIR_SPLIT>) : go(k_gemm_pair<BN, GEMM_STORE_BF16, PAIR_TILES>);

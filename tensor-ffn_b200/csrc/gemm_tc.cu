@@ -912,10 +912,12 @@ int launch_bn(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream, i
         // four layers, K 22016, N 2048: 32 tokens 381 with 16 splits, 364 with 8; 64 tokens in 32-wide tiles 462, in 64-wide ones 428
         // and 406; K 17920, N 1536: 64 tokens 390, 352, 352).
         const int most = (BN != 32 && BN != 64) || c.grp || c.bin_counts ? 2 * ws.num_sms : ws.num_sms + ws.num_sms / 3;
-        // Whole tiles on half to four fifths of the SMs stay whole: their halves would be two to an SM here and one there, and need
-        // clusters (K 2048, 96 and 113 tiles of first products in one launch: 10.7 -> 9.8 us, a step of
-        // one sequence, 8 layers, 450 -> 430, of 16 461 -> 450).
-        const bool whole = !c.grp && !c.bin_counts && splits == 1 && tiles * 2 > ws.num_sms && tiles * 10 < ws.num_sms * 8;
+        // Tiles that the loop above left whole, up to four fifths of the SMs (84 to 118 of 148), stay whole: their halves would be two
+        // to an SM here and one there, and need clusters. Back to back with early starts, us a launch whole and in halves, 84 and 118
+        // tiles: 16 tokens, K 512 4.5, 6.7 and 5.3, 7.0; K 2048 10.9, 12.3 and 12.5, 15.7; K 17920 62.4, 65.0 and 80.0, 101.8; 64
+        // tokens, K 2048 12.0, 15.5 and 14.0, 17.2; K 17920 67.5, 72.4 and 84.7, 87.9; 100 tokens, K 2048 13.5, 29.8 and 15.2, 31.2; K
+        // 17920 75.0, 98.8 and 90.3, 107.2. A step of one sequence, 8 layers 2 048 wide, first products of 96 and 113 tiles: 450 -> 430.
+        const bool whole = !c.grp && !c.bin_counts && splits == 1 && tiles * 10 < ws.num_sms * 8;
         while (!whole && splits < kMaxSplits && tiles * splits * 2 <= most && total_kb / (splits * 2) >= min_kb) splits *= 2;
     }
     if (splits != 1 && splits != 2 && splits != 4 && splits != 8 && splits != 16) return (int)cudaErrorInvalidValue;

@@ -156,7 +156,7 @@ struct PairSplit {
     double us, whole_us;
 };
 PairSplit pair_split(long long tiles, int kb, int bn, int num_sms);
-// one launch over independent layers: modes STORE_F32, STORE_BF16, SWIGLU, one operand pair
+// One launch over independent layers: modes STORE_F32 (one operand pair) and SWIGLU
 [[nodiscard]] int launch_gemm_layers(const GemmCall& c, const GemmWorkspace& ws, cudaStream_t stream);
 // The same products in true fp32 (fp32 X and out, fp32 FMA, weights still bf16): modes STORE_F32, STORE_BF16, RELU2 and
 // SWIGLU (which then store fp32), grouped and batched launches included; two operand pairs only in a plain launch. The operands' X pointers
