@@ -119,7 +119,8 @@ int tffn_expert_set_scale(tffn_expert* e, float scale); /* ExpertModel::output_s
  * input of every layer), d_out_delta = DEVICE fp32 [num_layers][batch_tokens][hidden] =
  * scale * (bf16(silu(bf16(x Wg^T)) * bf16(x Wu^T)) Wd^T), scale = the expert's output scale (the trainer
  * uses kExpertOutputScale = 0.01: set it with tffn_expert_set_scale). Runs on `stream` (0: the default
- * stream) and returns when the result is complete. */
+ * stream) and returns when the result is complete. Up to 128 MB of
+ * working memory stay with the expert between calls. */
 int tffn_expert_forward(const tffn_expert* e, const void* d_x_norm, float* d_out_delta, int batch_tokens, void* stream);
 float tffn_expert_get_scale(const tffn_expert* e);
 void tffn_expert_free(tffn_expert* e); /* expert_free (expert.cu:33-42) */
